@@ -449,7 +449,7 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
                 return (int64_t)launch_build_tall(g, h->v.as<double>(), h->xt.as<double>(), h->dvec.as<double>(), nf,
                                                   h->a.as<double>(), s);
             });
-            launches += launch_factor_chunk(g, nf, h->a.as<double>(), h->linv.as<double>(), h->qacc.as<double>(),
+            launches += launch_factor_chunk(g, nf, h->a.as<double>(), h->qacc.as<double>(),
                                             h->err.as<unsigned long long>(), s, prof.enabled ? &prof : nullptr,
                                             upd_variant, fp64_oz ? h->panel32.p : nullptr,
                                             h->tc_sched.as<unsigned long long>(), h->persistent_ctas);
@@ -664,8 +664,7 @@ int64_t batch_screen(gwb200_handle* w, BatchLane& lane, cudaStream_t s, int max_
                 }
             }
         } else
-            launches += launch_factor_chunk(c.g, c.nmat, lane.a.as<double>(), lane.linv.as<double>(),
-                                            lane.qacc.as<double>(), err, s, nullptr, variants[k],
+            launches += launch_factor_chunk(c.g, c.nmat, lane.a.as<double>(), lane.qacc.as<double>(), err, s, nullptr, variants[k],
                                             oz ? lane.panel.p : nullptr, sched, max_ctas);
         launches += launch_forms_scatter(gp, c.ngroups, lane.qacc.as<double>(), c.g.m_pad, s);
     }

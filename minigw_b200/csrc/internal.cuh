@@ -119,15 +119,21 @@ int launch_scale_vectors(const double* delta, int64_t n, int64_t n_pad, const do
                          double* dvec, cudaStream_t s);
 int launch_build_tall(const TallGeometry& g, const double* v, const double* xt, const double* dvec, int64_t nf,
                       double* a, cudaStream_t s);
-// Blocked Cholesky of the tall matrices of nf frequencies (outer blocks of two 64-wide inner
-// blocks); returns launches issued.
+// Blocked Cholesky of the tall matrices of nf frequencies (outer blocks of 128 columns); returns
+// launches issued.
 // `variant`: index into the FP64 update kernel table (tune_update_variant); -1: GWB200_UPDATE_VARIANT
 // if set, else the default; kUpdateOzaki: the outer trailing updates run as the int8 emulation of
 // kernels_oz.cu with `oz` as its slice workspace (oz_slice_bytes_per_freq(g) per frequency) and
-// `sched` as its work counter (look-left updates on the default DMMA kernel).
-int launch_factor_chunk(const TallGeometry& g, int64_t nf, double* a, double* linv, double* qacc,
+// `sched` as its work counter.
+int launch_factor_chunk(const TallGeometry& g, int64_t nf, double* a, double* qacc,
                         unsigned long long* err_pivot, cudaStream_t s, UpdateProfiler* prof, int variant,
                         void* oz = nullptr, unsigned long long* sched = nullptr, int max_ctas = 0);
+// kernels_panel.cu: the panel step of columns [k, k + width), width 64 or 128: the diagonal block
+// (replaced by its inverse factor) and every row below it; the squared norms of the right-hand-side
+// rows are added to qacc.  Returns launches issued.
+int launch_panel64(const TallGeometry& g, int64_t nf, double* a, int64_t k, int64_t width, double* qacc,
+                   unsigned long long* err_pivot, cudaStream_t s);
+int64_t panel_grid(int64_t tiles, int64_t nf);
 // kernels_oz.cu: FP64 trailing update C -= P P^T (K = 128 from kb0, columns [c_begin, n_pad), rows
 // [c_begin, rows)) from exact int8 products of 6-digit row slices (tcgen05 kind::i8).  Two launches.
 size_t oz_slice_bytes_per_freq(const TallGeometry& g);

@@ -139,152 +139,7 @@ __device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
                  : "d"(a), "d"(b));
 }
 
-template <int LD, int KD>
-__device__ __forceinline__ void tile_mma(const double* __restrict__ As, const double* __restrict__ Bs,
-                                         double (&acc)[2][4][2], double sgn) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    const int r0 = 16 * (w >> 1), c0 = 32 * (w & 1);
-#pragma unroll 4
-    for (int kk = 0; kk < KD; kk += 4) {
-        double af[2], bf[4];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) af[i] = sgn * As[(r0 + 8 * i + g) * LD + kk + t];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bf[j] = Bs[(c0 + 8 * j + g) * LD + kk + t];
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) dmma_8x8x4(acc[i][j], af[i], bf[j]);
-    }
-}
-
-__device__ __forceinline__ void tile_mma_64(const double* __restrict__ As, const double* __restrict__ Bs,
-                                            double (&acc)[2][4][2], double sgn) {
-    tile_mma<kLds, kNb>(As, Bs, acc, sgn);
-}
-
-// Copy a 64x64 tile (global row stride ld) into shared memory (stride kLds), 16-byte loads.
-__device__ __forceinline__ void load_tile_64(double* __restrict__ s, const double* __restrict__ gsrc, int64_t ld) {
-    for (int idx = threadIdx.x; idx < 64 * 32; idx += blockDim.x) {
-        const int r = idx >> 5, c2 = idx & 31;
-        const double2 v = *reinterpret_cast<const double2*>(gsrc + (size_t)r * ld + 2 * c2);
-        *reinterpret_cast<double2*>(s + r * kLds + 2 * c2) = v;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Step 1: factor the diagonal block A[k:k+64, k:k+64] of each frequency in shared memory,
-// write L back and its inverse to linv (64x64 row-major, zero above the diagonal).
-// A pivot that is not > 0 (or NaN) records the 1-based global pivot row in *err_pivot
-// (minimum over all frequencies) and is replaced by 1 so the factorisation stays finite.
-__global__ void __launch_bounds__(256) k_potrf_diag(double* __restrict__ a, int64_t ld, int64_t stride, int64_t k,
-                                                    double* __restrict__ linv, unsigned long long* err_pivot) {
-    extern __shared__ double smem[];
-    constexpr int L = kNb + 1;
-    double* T = smem;            // 64 x 65: the block, then L
-    double* Y = smem + kNb * L;  // 64 x 65: L^{-1}
-    double* A = a + (size_t)blockIdx.x * stride + k * ld + k;
-    const int tid = threadIdx.x;
-    for (int idx = tid; idx < kNb * kNb; idx += blockDim.x) {
-        const int i = idx / kNb, j = idx % kNb;
-        T[i * L + j] = (j <= i) ? A[(size_t)i * ld + j] : 0.0;
-    }
-    __syncthreads();
-    for (int j = 0; j < kNb; ++j) {
-        if (tid == 0) {
-            double piv = T[j * L + j];
-            if (!(piv > 0.0)) {
-                atomicMin(err_pivot, (unsigned long long)(k + j + 1));
-                piv = 1.0;
-            }
-            T[j * L + j] = sqrt(piv);
-        }
-        __syncthreads();
-        const double rjj = 1.0 / T[j * L + j];
-        for (int i = j + 1 + tid; i < kNb; i += blockDim.x) T[i * L + j] *= rjj;
-        __syncthreads();
-        // rank-1 update of the trailing lower triangle on a 16 x 16 thread grid (no index division)
-        for (int i = j + 1 + (tid >> 4); i < kNb; i += 16) {
-            const double lij = T[i * L + j];
-            for (int l = j + 1 + (tid & 15); l <= i; l += 16) T[i * L + l] -= lij * T[l * L + j];
-        }
-        __syncthreads();
-    }
-    for (int idx = tid; idx < kNb * kNb; idx += blockDim.x) {
-        const int i = idx / kNb, j = idx % kNb;
-        if (j <= i) A[(size_t)i * ld + j] = T[i * L + j];
-    }
-    // Inverse of the lower-triangular block by forward substitution: column `col` is owned by the
-    // four lanes 4*col..4*col+3 of one warp (all 256 threads busy), which split each dot product
-    // and combine it with two xor-shuffles.
-    {
-        const int col = tid >> 2, part = tid & 3;
-        for (int i = 0; i < kNb; ++i) {
-            double sum = 0.0;
-            if (i > col)
-                for (int l = col + part; l < i; l += 4) sum = fma(T[i * L + l], Y[l * L + col], sum);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-            if (part == 0) {
-                double y;
-                if (i < col) y = 0.0;
-                else if (i == col) y = 1.0 / T[i * L + i];
-                else y = -sum / T[i * L + i];
-                Y[i * L + col] = y;
-            }
-            __syncwarp();
-        }
-    }
-    __syncthreads();
-    double* out = linv + (size_t)blockIdx.x * kNb * kNb;
-    for (int idx = tid; idx < kNb * kNb; idx += blockDim.x) out[idx] = Y[(idx / kNb) * L + idx % kNb];
-}
-
-// Step 2: panel solve.  Rows [k+64, rows) of block column k: P = A[:, k:k+64] * Linv^T, in place.
-// Rows in the right-hand-side block also add their squared norms to qacc (one thread per row,
-// fixed order, so the accumulation is deterministic).
-__global__ void __launch_bounds__(256) k_trsm_panel(double* __restrict__ a, int64_t ld, int64_t stride, int64_t k,
-                                                    int64_t n_pad, int64_t rows, const double* __restrict__ linv,
-                                                    double* __restrict__ qacc, int64_t ldq) {
-    extern __shared__ double smem[];
-    double* Ps = smem;              // 64 x kLds
-    double* Ls = smem + 64 * kLds;  // 64 x kLds
-    const int f = blockIdx.y;
-    const int64_t r0 = k + kNb + (int64_t)blockIdx.x * kNb;
-    if (r0 >= rows) return;
-    double* A = a + (size_t)f * stride;
-    load_tile_64(Ps, A + r0 * ld + k, ld);
-    load_tile_64(Ls, linv + (size_t)f * kNb * kNb, kNb);
-    __syncthreads();
-    double acc[2][4][2] = {};
-    tile_mma_64(Ps, Ls, acc, 1.0);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    const int rr = 16 * (w >> 1), cc = 32 * (w & 1);
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            Ps[(rr + 8 * i + g) * kLds + cc + 8 * j + 2 * t] = acc[i][j][0];
-            Ps[(rr + 8 * i + g) * kLds + cc + 8 * j + 2 * t + 1] = acc[i][j][1];
-        }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < 64 * 32; idx += blockDim.x) {
-        const int r = idx >> 5, c2 = idx & 31;
-        *reinterpret_cast<double2*>(A + (size_t)(r0 + r) * ld + k + 2 * c2) =
-            *reinterpret_cast<const double2*>(Ps + r * kLds + 2 * c2);
-    }
-    if (r0 >= n_pad && threadIdx.x < kNb) {
-        const int r = threadIdx.x;
-        double s = 0.0;
-        for (int j = 0; j < kNb; ++j) s = fma(Ps[r * kLds + j], Ps[r * kLds + j], s);
-        qacc[(size_t)f * ldq + (r0 - n_pad + r)] += s;
-    }
-}
-
-// Step 3: update C -= sum_chunks P_i P_j^T of the output column tiles [tc0, tc0+T) (64-wide,
+// Trailing update C -= sum_chunks P_i P_j^T of the output column tiles [tc0, tc0+T) (64-wide,
 // absolute tile indices): every tile on or below the diagonal in the square block, then every
 // tile of the right-hand-side rows.  The contraction runs over nk 64-wide column chunks of the
 // factored panels starting at column kb0, one chunk in shared memory at a time (cp.async), so
@@ -611,63 +466,31 @@ const char* update_variant_name(int v) {
     return (v >= 0 && v < kNumVariants) ? kVariants[v].name : "?";
 }
 
-int launch_factor_chunk(const TallGeometry& g, int64_t nf, double* a, double* linv, double* qacc,
-                        unsigned long long* err_pivot, cudaStream_t s, UpdateProfiler* prof, int variant, void* oz,
-                        unsigned long long* sched, int max_ctas) {
-    const size_t smem = 2 * 64 * kLds * sizeof(double);
-    const size_t smem_potrf = 2 * kNb * (kNb + 1) * sizeof(double);
-    GWB_CUDA(cudaFuncSetAttribute(k_trsm_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const bool use_oz = oz && variant == kUpdateOzaki;  // outer updates emulated; look-left on DMMA
+int launch_factor_chunk(const TallGeometry& g, int64_t nf, double* a, double* qacc, unsigned long long* err_pivot,
+                        cudaStream_t s, UpdateProfiler* prof, int variant, void* oz, unsigned long long* sched,
+                        int max_ctas) {
+    const bool use_oz = oz && variant == kUpdateOzaki;
     if (variant < 0 || variant >= kNumVariants)  // untuned caller: GWB200_UPDATE_VARIANT, else the default
         variant = env_update_variant() >= 0 ? env_update_variant() : kDefaultUpdateVariant;
-    const UpdateVariant& uv = kVariants[variant];
-    GWB_CUDA(cudaFuncSetAttribute(uv.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)uv.smem));
-    GWB_CUDA(cudaFuncSetAttribute(k_potrf_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_potrf));
     const int64_t nsq = g.n_pad / kNb;   // square tile rows/cols
-    const int64_t nrt = g.rows / kNb;    // all tile rows
-    constexpr int64_t kInner = 2;        // 64-wide inner blocks per outer block
+    constexpr int64_t kOuter = 2;        // 64-wide tiles per outer block
+    if (!use_oz && nsq > kOuter)
+        GWB_CUDA(cudaFuncSetAttribute(kVariants[variant].fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)kVariants[variant].smem));
     int launches = 0;
-    // with the int8-emulated outer updates, the profiler times those alone (the look-left updates
-    // that stay on DMMA are a few percent of the flops)
-    UpdateProfiler* lprof = use_oz ? nullptr : prof;
-    auto update = [&](int64_t kb0, int nk, int64_t tc0, int64_t T) {
-        const int64_t L = nsq - tc0;
-        const int64_t tiles = T * L - T * (T - 1) / 2 + T * (nrt - nsq);
-        if (tiles <= 0) return;
-        dim3 grid((unsigned)tiles, (unsigned)nf);
-        if (lprof) lprof->begin();
-        uv.fn<<<grid, uv.threads, uv.smem, s>>>(a, g.ld, g.stride, kb0, nk, tc0, T, nsq);
-        GWB_LAUNCH("k_update");
-        if (lprof) lprof->end((double)nf * update_flops(g, kb0, nk, tc0 * kNb, (tc0 + T) * kNb));
-        ++launches;
-    };
-    for (int64_t ob = 0; ob < nsq; ob += kInner) {
-        const int64_t q = std::min(kInner, nsq - ob);
-        for (int64_t j = 0; j < q; ++j) {
-            const int64_t kt = ob + j;
-            const int64_t k = kt * kNb;
-            if (j > 0) update(ob * kNb, (int)j, kt, 1);  // look-left: earlier inner blocks onto this column
-            k_potrf_diag<<<(unsigned)nf, 256, smem_potrf, s>>>(a, g.ld, g.stride, k, linv, err_pivot);
-            GWB_LAUNCH("k_potrf_diag");
+    for (int64_t ob = 0; ob < nsq; ob += kOuter) {
+        const int64_t q = std::min(kOuter, nsq - ob), tc0 = ob + q;
+        launches += launch_panel64(g, nf, a, ob * kNb, q * kNb, qacc, err_pivot, s);
+        if (tc0 >= nsq) break;
+        // trailing update, K = 128 (columns remain only behind a full outer block)
+        if (prof) prof->begin();
+        if (use_oz) {
+            launches += launch_update64_oz(g, nf, a, ob * kNb, tc0 * kNb, oz, sched, err_pivot, s, max_ctas);
+        } else {
+            launch_variant(variant, g, nf, a, ob * kNb, (int)q, tc0, nsq - tc0, s);
             ++launches;
-            const int64_t below = g.rows - (k + kNb);
-            if (below > 0) {
-                dim3 grid((unsigned)(below / kNb), (unsigned)nf);
-                k_trsm_panel<<<grid, 256, smem, s>>>(a, g.ld, g.stride, k, g.n_pad, g.rows, linv, qacc, g.m_pad);
-                GWB_LAUNCH("k_trsm_panel");
-                ++launches;
-            }
         }
-        const int64_t tc0 = ob + q;
-        if (tc0 < nsq) {  // outer-block trailing update, K = 64*q (= 128 whenever columns remain)
-            if (use_oz && q == kInner) {
-                if (prof) prof->begin();
-                launches += launch_update64_oz(g, nf, a, ob * kNb, tc0 * kNb, oz, sched, err_pivot, s, max_ctas);
-                if (prof) prof->end((double)nf * update_flops(g, ob * kNb, (int)q, tc0 * kNb, nsq * kNb));
-            } else {
-                update(ob * kNb, (int)q, tc0, nsq - tc0);
-            }
-        }
+        if (prof) prof->end((double)nf * update_flops(g, ob * kNb, (int)q, tc0 * kNb, nsq * kNb));
     }
     return launches;
 }

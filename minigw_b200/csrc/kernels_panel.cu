@@ -1,0 +1,185 @@
+// kernels_panel.cu -- the panel step of the plain form's blocked Cholesky (FP64): per outer block
+// of 128 columns (64 where only 64 are left) one kernel for the diagonal block and one for the
+// rows below it.
+//
+//   k_diag64    one CTA per frequency: Cholesky of the diagonal block and its inverse
+//               (panel_common.cuh); the inverse replaces the block in the tall matrix (the factor
+//               itself is not read again: the screened forms need the solved rows alone).
+//   k_panel64   rows below: P = A L^{-T} with the whole block's inverse, so the second 64 columns
+//               need no separate update by the first.  The inverse is triangular, so column tile c
+//               (8 wide) takes k < 8 (c + 1) only: 0.53 of the square product, less work than two
+//               64-wide solves and the update between them (0.75).  Bound by the FP64 tensor pipe.
+//               A CTA keeps the inverse in shared memory and walks row tiles of 32, the next tile
+//               loaded while one is multiplied; each warp owns 16 rows and column tiles
+//               {g, 7-g, 8+g, 15-g}, the same work for every g.
+#include "panel_common.cuh"
+
+#include <algorithm>
+
+namespace gwb200 {
+namespace {
+
+using namespace panel;
+
+constexpr int kRowTile = 32;
+
+template <int NB>
+__global__ void __launch_bounds__(kPanelThreads) k_diag64(double* __restrict__ a, int64_t ld, int64_t stride, int64_t k,
+                                                          unsigned long long* err_pivot) {
+    extern __shared__ __align__(16) double psm[];
+    constexpr int LD = DiagShape<NB>::kLd;
+    double* S = psm;
+    double* A = a + (size_t)blockIdx.x * stride + k * ld + k;
+    for (int idx = threadIdx.x; idx < NB * (LD / 2); idx += kPanelThreads) {
+        const int i = idx / (LD / 2), j = 2 * (idx % (LD / 2));
+        double2 v = make_double2(0.0, 0.0);
+        if (j <= i) v = *reinterpret_cast<const double2*>(A + (size_t)i * ld + j);
+        if (j + 1 > i) v.y = 0.0;
+        *reinterpret_cast<double2*>(S + i * LD + j) = v;
+    }
+    __syncthreads();
+    factor_diag<NB, false>(S, S + DiagShape<NB>::kBlockDoubles, k, err_pivot);
+    // the inverse in place of the block; above the diagonal zeros (not the upper right 64 x 64, which
+    // nothing reads)
+    for (int idx = threadIdx.x; idx < NB * NB; idx += kPanelThreads) {
+        const int i = idx / NB, j = idx % NB;
+        if (j < (i < kNb ? kNb : NB)) A[(size_t)i * ld + j] = j <= i ? S[j * LD + i + 1] : 0.0;
+    }
+}
+
+template <int NB>
+struct PanelShape {
+    static constexpr int kLd = NB + 4;  // = 4 mod 16 (fragment loads on distinct banks)
+    static constexpr int kTiles = NB / 32;  // column tiles of 8 per warp
+    static constexpr size_t kSmem = sizeof(double) * ((size_t)NB * kLd + 2 * kRowTile * kLd + 4 * kRowTile);
+};
+
+__device__ __forceinline__ void cp_async16(double* dst, const double* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+
+template <int NB>
+__global__ void __launch_bounds__(kPanelThreads, 1)
+    k_panel64(double* __restrict__ a, int64_t ld, int64_t stride, int64_t k, int64_t n_pad, int ntile,
+              double* __restrict__ qacc, int64_t ldq) {
+    extern __shared__ __align__(16) double psm[];
+    using Sh = PanelShape<NB>;
+    constexpr int LD = Sh::kLd, NT = Sh::kTiles;
+    double* Y = psm;
+    double* Xs = Y + NB * LD;
+    double* red = Xs + 2 * kRowTile * LD;
+    double* A = a + (size_t)blockIdx.y * stride;
+    const int64_t row0 = k + NB;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    const int r0 = 16 * (w & 1), cg = w >> 1;
+    auto load_rows = [&](int tile, int buf) {
+        const double* src = A + (size_t)(row0 + (int64_t)tile * kRowTile) * ld + k;
+        double* dst = Xs + buf * kRowTile * LD;
+        for (int idx = threadIdx.x; idx < kRowTile * (NB / 2); idx += kPanelThreads) {
+            const int r = idx / (NB / 2), c = 2 * (idx % (NB / 2));
+            cp_async16(dst + r * LD + c, src + (size_t)r * ld + c);
+        }
+        asm volatile("cp.async.commit_group;\n" ::);
+    };
+    for (int idx = threadIdx.x; idx < NB * (NB / 2); idx += kPanelThreads) {
+        const int r = idx / (NB / 2), c = 2 * (idx % (NB / 2));
+        if (c < (r < kNb ? kNb : NB)) cp_async16(Y + r * LD + c, A + (size_t)(k + r) * ld + k + c);
+    }
+    load_rows(blockIdx.x, 0);
+    int buf = 0;
+    for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x, buf ^= 1) {
+        if (tile + (int)gridDim.x < ntile) {
+            load_rows(tile + gridDim.x, buf ^ 1);
+            asm volatile("cp.async.wait_group 1;\n" ::);
+        } else {
+            asm volatile("cp.async.wait_group 0;\n" ::);
+        }
+        __syncthreads();
+        const double* X = Xs + buf * kRowTile * LD + (r0 + g) * LD + t;
+        // column tiles of this warp, ascending: cg, 7 - cg(, 8 + cg, 15 - cg)
+        auto col = [&](int i) { return (i >> 1) * 8 + ((i & 1) ? 7 - cg : cg); };
+        double acc[2][NT][2] = {};
+        int ks = 0;
+#pragma unroll
+        for (int first = 0; first < NT; ++first) {  // tiles `first`.. still have columns k <= c
+            const int kend = 2 * (col(first) + 1);
+            for (; ks < kend; ++ks) {
+                const double a0 = X[4 * ks], a1 = X[8 * LD + 4 * ks];
+#pragma unroll
+                for (int i = first; i < NT; ++i) {
+                    const double b = Y[(8 * col(i) + g) * LD + 4 * ks + t];
+                    dmma(acc[0][i], a0, b);
+                    dmma(acc[1][i], a1, b);
+                }
+            }
+        }
+        const int64_t row = row0 + (int64_t)tile * kRowTile + r0 + g;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int i = 0; i < NT; ++i)
+                *reinterpret_cast<double2*>(A + (size_t)(row + 8 * h) * ld + k + 8 * col(i) + 2 * t) =
+                    make_double2(acc[h][i][0], acc[h][i][1]);
+        const bool rhs = row0 + (int64_t)tile * kRowTile >= n_pad;  // n_pad is a multiple of the tile
+        if (rhs) {  // squared row norms, summed in a fixed order
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                double s = 0.0;
+#pragma unroll
+                for (int i = 0; i < NT; ++i) s = fma(acc[h][i][1], acc[h][i][1], fma(acc[h][i][0], acc[h][i][0], s));
+                s += __shfl_xor_sync(0xffffffffu, s, 1);
+                s += __shfl_xor_sync(0xffffffffu, s, 2);
+                if (t == 0) red[cg * kRowTile + r0 + 8 * h + g] = s;
+            }
+        }
+        __syncthreads();
+        if (rhs && threadIdx.x < kRowTile) {
+            const int r = threadIdx.x;
+            qacc[(size_t)blockIdx.y * ldq + (row0 + (int64_t)tile * kRowTile - n_pad) + r] +=
+                (red[r] + red[kRowTile + r]) + (red[2 * kRowTile + r] + red[3 * kRowTile + r]);
+        }
+    }
+}
+
+template <int NB>
+int launch_block(const TallGeometry& g, int64_t nf, double* a, int64_t k, double* qacc, unsigned long long* err_pivot,
+                 cudaStream_t s) {
+    GWB_CUDA(cudaFuncSetAttribute(k_diag64<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DiagShape<NB>::kSmem));
+    k_diag64<NB><<<(unsigned)nf, kPanelThreads, DiagShape<NB>::kSmem, s>>>(a, g.ld, g.stride, k, err_pivot);
+    GWB_LAUNCH("k_diag64");
+    const int64_t tiles = (g.rows - (k + NB)) / kRowTile;
+    if (tiles <= 0) return 1;
+    GWB_CUDA(cudaFuncSetAttribute(k_panel64<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PanelShape<NB>::kSmem));
+    k_panel64<NB><<<dim3((unsigned)panel_grid(tiles, nf), (unsigned)nf), kPanelThreads, PanelShape<NB>::kSmem, s>>>(
+        a, g.ld, g.stride, k, g.n_pad, (int)tiles, qacc, g.m_pad);
+    GWB_LAUNCH("k_panel64");
+    return 2;
+}
+
+}  // namespace
+
+// CTAs per frequency for `tiles` row tiles of nf frequencies, one CTA per SM: the fewest tile times
+// over the waves, counting two for a CTA's load of the inverse.
+int64_t panel_grid(int64_t tiles, int64_t nf) {
+    const int64_t sms = 148;
+    int64_t best = 1;
+    double best_cost = 0.0;
+    for (int64_t gx = 1; gx <= std::min<int64_t>(tiles, 64); ++gx) {
+        const double waves = (double)((nf * gx + sms - 1) / sms);
+        const double cost = waves * ((double)((tiles + gx - 1) / gx) + 2.0);
+        if (gx == 1 || cost < best_cost) {
+            best = gx;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
+int launch_panel64(const TallGeometry& g, int64_t nf, double* a, int64_t k, int64_t width, double* qacc,
+                   unsigned long long* err_pivot, cudaStream_t s) {
+    return width == 2 * kNb ? launch_block<128>(g, nf, a, k, qacc, err_pivot, s)
+                            : launch_block<64>(g, nf, a, k, qacc, err_pivot, s);
+}
+
+}  // namespace gwb200

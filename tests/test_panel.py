@@ -1,0 +1,64 @@
+"""The panel step of the plain form (diagonal block with its inverse, rows below) at the sizes where
+its tiles begin and end: 64- and 128-wide blocks, 16-wide panels, 32-row tiles, and the pivot it reports."""
+import numpy as np
+import pytest
+
+from minigw_b200.gw_input import GwSlices
+
+pytestmark = pytest.mark.gpu
+
+
+def _system(n, rank, nstates, seed):
+    """nocc = 1, so n = nmo - 1: V_ph = F F^T of the given rank, random right-hand sides."""
+    rng = np.random.default_rng(seed)
+    nmo = n + 1
+    mo = np.concatenate([[-0.6], np.sort(rng.uniform(0.05, 3.0, n))])
+    f = rng.standard_normal((n, rank)) * 0.4
+    panel = rng.standard_normal((nstates * nmo, n)) * 0.2
+    return GwSlices(mo_energy=mo, nocc=1, fermi_energy=-0.2, states=np.arange(nstates), vph=f @ f.T, panel=panel,
+                    xdiag=np.zeros((nmo, 1)), vxc_diag=np.zeros(nmo))
+
+
+def _forms(sl, omegas):
+    """x^T W_c x = -||L^{-1} D^{1/2} x||^2 with numpy in FP64."""
+    delta = sl.mo_energy[1:] - sl.mo_energy[0]
+    out = []
+    for w in omegas:
+        d = np.sqrt(4.0 * delta / (w * w + delta * delta))
+        low = np.linalg.cholesky(np.eye(len(d)) + d[:, None] * sl.vph * d[None, :])
+        out.append(-(np.linalg.solve(low, (sl.panel * d).T) ** 2).sum(axis=0))
+    return np.array(out).reshape(len(omegas), len(sl.states), -1)
+
+
+@pytest.mark.parametrize("n,nstates", [(1, 1), (15, 1), (16, 2), (17, 1), (63, 1), (64, 1), (65, 1), (127, 1), (128, 1),
+                                       (129, 1), (191, 1), (192, 1), (193, 2), (257, 1), (320, 3)])
+def test_forms_at_block_edges(n, nstates):
+    from minigw_b200 import B200Backend
+
+    sl = _system(n, max(1, n // 2), nstates, 100 + n)
+    omegas = np.array([1e-3, 0.4, 7.0])
+    with B200Backend(0) as be:
+        be.load_slices(sl)
+        q, _ = be.screened_forms(omegas, sl.states)
+    ref = _forms(sl, omegas)
+    # the bound of the other form tests: condition <= ~1e3 here, FP64 sums of length n
+    assert np.abs(q - ref).max() <= 1e-11 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("n,pivot", [(40, 0), (40, 15), (40, 16), (100, 63), (100, 64), (200, 127), (200, 128), (200, 199)])
+def test_reported_pivot(n, pivot):
+    from minigw_b200 import B200Backend
+    from minigw_b200._lib import GwB200Error
+
+    sl = _system(n, 3, 1, 7)
+    sl.vph = np.zeros((n, n))
+    sl.vph[pivot, pivot] = -1e6  # eps is diagonal, negative at this one row
+    with B200Backend(0) as be:
+        be.load_slices(sl)
+        with pytest.raises(GwB200Error) as e:
+            be.screened_forms(np.array([0.3, 1.0]), sl.states)
+        assert e.value.status == "GWB200_NOT_SPD" and f"pivot {pivot + 1} " in str(e.value)
+        sl.vph[pivot, pivot] = 0.0
+        be.load_slices(sl)  # the handle is usable afterwards
+        q, _ = be.screened_forms(np.array([0.3]), sl.states)
+    assert np.abs(q - _forms(sl, [0.3])).max() <= 1e-11 * np.abs(q).max()
