@@ -85,8 +85,8 @@ struct PinnedBuf {
 struct BatchLane {
     cudaStream_t stream = nullptr;  // lanes >= 1 (created on first use)
     cudaEvent_t done = nullptr;
-    DevBuf a, linv, qacc, panel, sched, refine;  // refine: the refined mixed form's correction terms
-    size_t bytes() const { return a.bytes + linv.bytes + qacc.bytes + panel.bytes + refine.bytes; }
+    DevBuf a, qacc, panel, sched, refine;  // refine: the refined mixed form's correction terms
+    size_t bytes() const { return a.bytes + qacc.bytes + panel.bytes + refine.bytes; }
 };
 constexpr int kMaxBatchLanes = 4;
 
@@ -331,7 +331,7 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
     }
     GWB_CUDA(cudaMemsetAsync(h->err.p, 0xFF, sizeof(unsigned long long), s));
 
-    // Frequency chunk size from the HBM budget: tall matrices + scale vectors + 64x64 inverses.
+    // Frequency chunk size from the HBM budget: tall matrices + scale vectors (+ 64x64 inverses: complex form).
     const bool mixed_tc = mixed && mixed_update_on_tcgen05(h);
     // plain form: the int8 emulation of the outer updates is a candidate of the update autotuner
     // (its slice workspace is part of the budget) unless GWB200_FP64_UPDATE=dmma; memory-capped
@@ -344,10 +344,10 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
         fac = refine_factor(h, s);
         r_pad = fac.r_pad;
     }
-    const size_t per_freq = mixed ? sizeof(float) * ((size_t)g.stride + kNb * kNb) + sizeof(double) * (g.n_pad + g.m_pad) +
+    const size_t per_freq = mixed ? sizeof(float) * (size_t)g.stride + sizeof(double) * (g.n_pad + g.m_pad) +
                                         (mixed_tc ? tc_panel_bytes_per_freq(g) : 0) +
                                         (refine ? refine_bytes_per_freq(g, r_pad) : 0)
-                                  : sizeof(double) * planes * ((size_t)g.stride + g.n_pad + kNb * kNb + g.m_pad) +
+                                  : sizeof(double) * planes * ((size_t)g.stride + g.n_pad + (cplx ? kNb * kNb : 0) + g.m_pad) +
                                         (fp64_oz ? oz_slice_bytes_per_freq(g) : 0);
     // GWB200_MAX_FREQ_CHUNK caps the chunk (tests use it to exercise the multi-chunk path).
     int64_t cap = 0;
@@ -380,15 +380,15 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
     }
     size_buffer(h, h->a, (mixed ? sizeof(float) : sizeof(double) * planes) * (size_t)fc * g.stride);
     size_buffer(h, h->dvec, sizeof(double) * planes * (size_t)fc * g.n_pad);
-    size_buffer(h, h->linv, (mixed ? sizeof(float) : sizeof(double) * planes) * (size_t)fc * kNb * kNb);
+    if (cplx) size_buffer(h, h->linv, sizeof(double) * planes * (size_t)fc * kNb * kNb);
     size_buffer(h, h->qacc, sizeof(double) * planes * (size_t)fc * g.m_pad);
     if (mixed_tc) {
         size_buffer(h, h->panel32, tc_panel_bytes_per_freq(g) * (size_t)fc);
-        h->tc_sched.ensure(sizeof(unsigned long long));
+        h->tc_sched.ensure(sched_bytes(g));
     }
     if (fp64_oz) {
         size_buffer(h, h->panel32, oz_slice_bytes_per_freq(g) * (size_t)fc);
-        h->tc_sched.ensure(sizeof(unsigned long long));
+        h->tc_sched.ensure(sched_bytes(g));
     }
     if (refine) size_buffer(h, h->refine, refine_bytes_per_freq(g, r_pad) * (size_t)fc);
 
@@ -430,12 +430,13 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
                 return (int64_t)launch_build_tall32(g, h->v.as<double>(), h->xt.as<double>(), h->dvec.as<double>(), nf,
                                                     h->a.as<float>(), s);
             });
-            launches += launch_factor_chunk32(g, nf, h->a.as<float>(), h->linv.as<float>(), h->qacc.as<double>(),
+            launches += launch_factor_chunk32(g, nf, h->a.as<float>(), h->qacc.as<double>(),
                                               h->err.as<unsigned long long>(), s, prof.enabled ? &prof : nullptr,
                                               mixed_tc ? h->panel32.as<float>() : nullptr,
-                                              h->tc_sched.as<unsigned long long>(), h->persistent_ctas);
+                                              h->tc_sched.as<unsigned long long>(), h->persistent_ctas,
+                                              /*keep_rows=*/refine);
             if (refine)  // qacc <- 2 x^T y - z^T z - y^T V y (FP64 energy functional at the FP32 solve)
-                launches += launch_refine_chunk(g, nf, h->a.as<float>(), h->linv.as<float>(), h->xt.as<double>(),
+                launches += launch_refine_chunk(g, nf, h->a.as<float>(), h->xt.as<double>(),
                                                 h->dvec.as<double>(), fac, h->refine.p,
                                                 h->qacc.as<double>(), h->err.as<unsigned long long>(), s,
                                                 mixed_tc ? h->panel32.as<float>() : nullptr,
@@ -609,17 +610,17 @@ std::vector<BatchChunk> batch_chunks(const std::vector<gwb200_handle*>& hs, cons
     return chunks;
 }
 
-// Workspace bytes of a set of chunks: the largest tall matrices, inverses, accumulators, operands.
+// Workspace bytes of a set of chunks: the largest tall matrices, accumulators, operands, counters.
 struct BatchNeed {
-    size_t a = 0, linv = 0, qacc = 0, panel = 0, refine = 0;
-    size_t total() const { return a + linv + qacc + panel + refine; }
+    size_t a = 0, qacc = 0, panel = 0, sched = 0, refine = 0;
+    size_t total() const { return a + qacc + panel + refine; }
 };
 void batch_need(const std::vector<BatchChunk>& chunks, bool mixed, bool oz, bool refine, BatchNeed& need) {
     const size_t el = mixed ? sizeof(float) : sizeof(double);
     for (const BatchChunk& c : chunks) {
         const size_t nm = (size_t)c.nmat;
         need.a = std::max(need.a, el * nm * (size_t)c.g.stride);
-        need.linv = std::max(need.linv, el * nm * kNb * kNb);
+        need.sched = std::max(need.sched, sched_bytes(c.g));
         need.qacc = std::max(need.qacc, sizeof(double) * nm * (size_t)c.g.m_pad);
         const size_t op = mixed ? tc_panel_bytes_per_freq(c.g) : (oz ? oz_slice_bytes_per_freq(c.g) : 0);
         need.panel = std::max(need.panel, op * nm);
@@ -642,9 +643,9 @@ int64_t batch_screen(gwb200_handle* w, BatchLane& lane, cudaStream_t s, int max_
         GWB_CUDA(cudaMemsetAsync(lane.qacc.p, 0, sizeof(double) * (size_t)c.nmat * c.g.m_pad, s));
         launches += launch_build_tall_batch(c.g, gp, c.ngroups, mixed, lane.a.p, s);
         if (mixed) {
-            launches += launch_factor_chunk32(c.g, c.nmat, lane.a.as<float>(), lane.linv.as<float>(),
-                                              lane.qacc.as<double>(), err, s, nullptr,
-                                              mixed_tc ? lane.panel.as<float>() : nullptr, sched, max_ctas);
+            launches += launch_factor_chunk32(c.g, c.nmat, lane.a.as<float>(), lane.qacc.as<double>(), err, s,
+                                              nullptr, mixed_tc ? lane.panel.as<float>() : nullptr, sched, max_ctas,
+                                              /*keep_rows=*/refine);
             if (refine) {  // each molecule's factor reversed in its own n_pad, one backward solve of the
                            // chunk, then each molecule's correction in its own geometry
                 for (int64_t q = 0; q < c.ngroups; ++q) {
@@ -652,7 +653,7 @@ int64_t batch_screen(gwb200_handle* w, BatchLane& lane, cudaStream_t s, int max_
                     launches += launch_refine_flip(c.g, gr.nf, lane.a.as<float>() + (size_t)gr.mat0 * c.g.stride,
                                                    gr.n_pad, s);
                 }
-                launches += launch_refine_solve(c.g, c.nmat, lane.a.as<float>(), lane.linv.as<float>(), err, s,
+                launches += launch_refine_solve(c.g, c.nmat, lane.a.as<float>(), err, s,
                                                 mixed_tc ? lane.panel.as<float>() : nullptr, sched, max_ctas,
                                                 /*flip=*/false);
                 for (int64_t q = 0; q < c.ngroups; ++q) {
@@ -754,7 +755,7 @@ int gwb200_destroy(gwb200_handle* h) {
         b->release();
     for (BatchLane& l : h->lanes) {
         if (l.stream) cudaStreamSynchronize(l.stream);
-        for (DevBuf* b : {&l.a, &l.linv, &l.qacc, &l.panel, &l.sched, &l.refine}) b->release();
+        for (DevBuf* b : {&l.a, &l.qacc, &l.panel, &l.sched, &l.refine}) b->release();
         if (l.done) cudaEventDestroy(l.done);
         if (l.stream) cudaStreamDestroy(l.stream);
     }
@@ -1358,7 +1359,7 @@ std::vector<int64_t> batch_graph_key(const gwb200_handle* w, const std::vector<g
     put(w->batch_fork);
     for (int l = 0; l < lanes; ++l) {
         const BatchLane& ln = w->lanes[l];
-        for (const DevBuf* b : {&ln.a, &ln.linv, &ln.qacc, &ln.panel, &ln.sched, &ln.refine}) put(b->p);
+        for (const DevBuf* b : {&ln.a, &ln.qacc, &ln.panel, &ln.sched, &ln.refine}) put(b->p);
         put(ln.stream);
         put(ln.done);
     }
@@ -1514,17 +1515,16 @@ int gwb200_run_g0w0_batch(gwb200_handle* const* systems, int64_t nsys, const int
             // lane holds one this call does not use (the correction terms of an earlier refined
             // batch, the operand panel of another form), free them all before allocating, so the
             // new sizes fit the budget they were planned in
-            const bool grow = need.a > ln.a.bytes || need.linv > ln.linv.bytes || need.qacc > ln.qacc.bytes ||
+            const bool grow = need.a > ln.a.bytes || need.qacc > ln.qacc.bytes ||
                               need.panel > ln.panel.bytes || need.refine > ln.refine.bytes;
             const bool unused = (!need.panel && ln.panel.bytes) || (!need.refine && ln.refine.bytes);
             if (grow || unused)
-                for (DevBuf* b : {&ln.a, &ln.linv, &ln.qacc, &ln.panel, &ln.refine}) b->release();
+                for (DevBuf* b : {&ln.a, &ln.qacc, &ln.panel, &ln.refine}) b->release();
             size_buffer(w, ln.a, need.a);
-            size_buffer(w, ln.linv, need.linv);
             size_buffer(w, ln.qacc, need.qacc);
             if (need.panel) size_buffer(w, ln.panel, need.panel);
             if (need.refine) size_buffer(w, ln.refine, need.refine);
-            ln.sched.ensure(sizeof(unsigned long long));
+            ln.sched.ensure(need.sched);
             if (l > 0 && !ln.stream) {
                 GWB_CUDA(cudaStreamCreateWithFlags(&ln.stream, cudaStreamNonBlocking));
                 GWB_CUDA(cudaEventCreateWithFlags(&ln.done, cudaEventDisableTiming));

@@ -133,7 +133,8 @@ int launch_factor_chunk(const TallGeometry& g, int64_t nf, double* a, double* qa
 // rows are added to qacc.  Returns launches issued.
 int launch_panel64(const TallGeometry& g, int64_t nf, double* a, int64_t k, int64_t width, double* qacc,
                    unsigned long long* err_pivot, cudaStream_t s);
-int64_t panel_grid(int64_t tiles, int64_t nf);
+// CTAs per frequency of a panel kernel over `tiles` row tiles of nf frequencies, per_sm CTAs per SM
+int64_t panel_grid(int64_t tiles, int64_t nf, int64_t per_sm);
 // kernels_oz.cu: FP64 trailing update C -= P P^T (K = 128 from kb0, columns [c_begin, n_pad), rows
 // [c_begin, rows)) from exact int8 products of 6-digit row slices (tcgen05 kind::i8).  Two launches.
 size_t oz_slice_bytes_per_freq(const TallGeometry& g);
@@ -186,10 +187,17 @@ double measure_fp64_peak_tflops(cudaStream_t s);
 int launch_build_tall32(const TallGeometry& g, const double* v, const double* xt, const double* dvec, int64_t nf,
                         float* a, cudaStream_t s);
 // panel != NULL: the outer trailing updates run on tcgen05 (kernels_tc.cu) with `panel` as the
-// split-panel workspace (tc_panel_bytes_per_freq(g) bytes per frequency); NULL: mma.sync.
-int launch_factor_chunk32(const TallGeometry& g, int64_t nf, float* a, float* linv, double* qacc,
-                          unsigned long long* err_pivot, cudaStream_t s, UpdateProfiler* prof, float* panel,
-                          unsigned long long* sched, int max_ctas = 0, bool solve_only = false);
+// split-panel workspace (tc_panel_bytes_per_freq(g) bytes per frequency) and `sched` as their work
+// counters (sched_bytes(g)); NULL: mma.sync.  The 64 x 64 diagonal blocks end as their inverse
+// factors.  keep_rows: the solved rows are wanted in the tall matrices afterwards (the refinement's
+// backward solve); without it the tcgen05 path leaves them in `panel` alone.  solve_only: solve the
+// right-hand sides against a factor that is already there.
+int launch_factor_chunk32(const TallGeometry& g, int64_t nf, float* a, double* qacc, unsigned long long* err_pivot,
+                          cudaStream_t s, UpdateProfiler* prof, float* panel, unsigned long long* sched, int max_ctas,
+                          bool keep_rows, bool solve_only = false);
+// Work counters of the persistent updates of one factorisation, one per outer block.
+inline size_t sched_bytes(const TallGeometry& g) { return sizeof(unsigned long long) * (size_t)(g.n_pad / (2 * kNb) + 1); }
+int launch_clear_sched(const TallGeometry& g, unsigned long long* sched, cudaStream_t s);
 // kernels_refine.cu: FP64 energy-functional correction of the mixed form.  launch_pchol factors
 // V = C C^T (pivoted, FP64; `work` of pchol_bytes(n)), returns the rank r and C^T (r_pad x n_pad,
 // r_pad = max(64, r rounded up to 64)) in *ct_out (inside `work`).  launch_refine_chunk runs after
@@ -206,7 +214,7 @@ struct RefineFactor {
 size_t refine_bytes_per_freq(const TallGeometry& g, int64_t r_pad);
 size_t pchol_bytes(int64_t n);
 int64_t launch_pchol(const double* v, int64_t n, void* work, double** ct_out, cudaStream_t s);
-int launch_refine_chunk(const TallGeometry& g, int64_t nf, float* a, float* linv, const double* xt,
+int launch_refine_chunk(const TallGeometry& g, int64_t nf, float* a, const double* xt,
                         const double* dvec, const RefineFactor& fac, void* work, double* qacc,
                         unsigned long long* err_pivot, cudaStream_t s, float* panel, unsigned long long* sched,
                         int max_ctas);
@@ -231,19 +239,20 @@ int launch_refine_terms_oz(const TallGeometry& ga, int64_t nf, const float* a, c
 // the reversal over g.n_pad); the correction terms of one molecule (own geometry gm) for its nf
 // matrices from `a`, into qacc (row stride ldq).
 int launch_refine_flip(const TallGeometry& ga, int64_t nf, float* a, int64_t n_flip, cudaStream_t s);
-int launch_refine_solve(const TallGeometry& g, int64_t nf, float* a, float* linv, unsigned long long* err_pivot,
+int launch_refine_solve(const TallGeometry& g, int64_t nf, float* a, unsigned long long* err_pivot,
                         cudaStream_t s, float* panel, unsigned long long* sched, int max_ctas, bool flip);
 int launch_refine_terms(const TallGeometry& ga, int64_t nf, const float* a, const TallGeometry& gm, const double* xt,
                         const double* dvec, const RefineFactor& fac, void* work, double* qacc, int64_t ldq,
                         unsigned long long* err, cudaStream_t s);
-// kernels_tc.cu: tcgen05 3xTF32 trailing update C -= P P^T of the mixed form (K = kdim columns from
-// kb0, output columns [c_begin, n_pad), rows [c_begin, rows)).  Two launches; `sched` is one
-// device word the kernel's work counter lives in.  A device wait that expires records pivot 0 in
-// err_pivot.
+// kernels_tc.cu: tcgen05 3xTF32 trailing update C -= P P^T of the mixed form (K = 128, output
+// columns [c_begin, n_pad), rows [c_begin, rows)) from the split rows in `panel` (tc_panel_rows(g,
+// c_begin) rows per frequency, k_panel32's layout).  `sched` is one cleared device word, the
+// kernel's work counter.  A device wait that expires records pivot 0 in err_pivot.
 size_t tc_panel_bytes_per_freq(const TallGeometry& g);
-int launch_update32_tc(const TallGeometry& g, int64_t nf, float* a, int64_t kb0, int kdim, int64_t c_begin,
-                       float* panel, unsigned long long* sched, unsigned long long* err_pivot, cudaStream_t s,
-                       int max_ctas = 0, int64_t row_min = 0);
+int64_t tc_panel_rows(const TallGeometry& g, int64_t c_begin);
+int launch_update32_tc(const TallGeometry& g, int64_t nf, float* a, int64_t c_begin, const float* panel,
+                       unsigned long long* sched, unsigned long long* err_pivot, cudaStream_t s, int max_ctas = 0,
+                       int64_t row_min = 0);
 // kernels_c64.cu: eta != 0 (complex symmetric M = I - S V S, S = diag(Pi0)^1/2).  Planes a_re/a_im
 // of geometry g; svec 2*n_pad, linv 2*64*64, qacc 2*m_pad doubles per frequency.
 int launch_factor_chunk_c(const TallGeometry& g, int64_t nf, const double* delta, const double* omega, double eta,

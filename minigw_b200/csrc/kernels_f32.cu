@@ -11,7 +11,7 @@
 //   * the squared norms, the G0 frequency contraction, Pade and QP in FP64.
 // There is no FP64 refinement: the result carries FP32-level error (stated, not hidden, by
 // bench.py and the tests).
-#include "internal.cuh"
+#include "panel_common.cuh"
 
 #include <cmath>
 
@@ -67,6 +67,20 @@ __device__ __forceinline__ void tile_mma_3xtf32(const float* __restrict__ As, co
     }
 }
 
+// The C fragments of tile_mma_3xtf32 to a 64 x 64 tile in shared memory (row stride LD).
+template <int LD>
+__device__ __forceinline__ void store_fragments(float* __restrict__ s, const float (&acc)[4][4]) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    const int r0 = 16 * (w >> 1), c0 = 32 * (w & 1);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            *reinterpret_cast<float2*>(s + (r0 + g + 8 * h) * LD + c0 + 8 * j + 2 * t) =
+                make_float2(acc[j][2 * h], acc[j][2 * h + 1]);
+}
+
 __device__ __forceinline__ void cp_async_16f(float* smem_dst, const float* gsrc) {
     const unsigned saddr = (unsigned)__cvta_generic_to_shared(smem_dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(saddr), "l"(gsrc));
@@ -104,116 +118,180 @@ __global__ void k_build_tall32(int64_t n, int64_t m, int64_t n_pad, int64_t ld, 
     }
 }
 
-// Diagonal block in FP64 (from the FP32 tall matrix), written back as FP32 L and FP32 L^{-1}.
-// One 64 x 65 FP64 tile: L in the lower triangle, Y = L^{-1} (lower too) transposed into the
-// upper triangle (Y[l][c] at T[c][l], l > c) with its diagonal in Yd, so 6 CTAs fit an SM.
-// invert_only: the block already holds a Cholesky factor (the solve-only pass of the mixed form's
-// refinement); only its inverse is formed and the block is left as it is.
-__global__ void __launch_bounds__(256) k_potrf_diag32(float* __restrict__ a, int64_t ld, int64_t stride, int64_t k,
-                                                      float* __restrict__ linv, unsigned long long* err_pivot,
-                                                      int invert_only) {
-    extern __shared__ double smem[];
-    constexpr int L = kNb + 1;
-    double* T = smem;
-    double* Yd = smem + kNb * L;
-    float* A = a + (size_t)blockIdx.x * stride + k * ld + k;
+// Diagonal step of outer block [k, k + NB): the 64 x 64 diagonal blocks are factored and inverted
+// in FP64 (panel_common.cuh) and their inverses, rounded to FP32, replace them in the tall matrix;
+// for NB = 128 the block between them is solved (L21 = A21 L11^{-T}) and the second diagonal block
+// updated (A22 -= L21 L21^T) in 3xTF32 first, as for the rows below.  One CTA per matrix.
+constexpr size_t kDiag32Smem = panel::DiagShape<kNb>::kSmem + 2 * 64 * kLdf * sizeof(float);
+
+template <int NB>
+__global__ void __launch_bounds__(256) k_diag32(float* __restrict__ a, int64_t ld, int64_t stride, int64_t k,
+                                                unsigned long long* err_pivot) {
+    extern __shared__ __align__(16) double smem[];
+    using Sh = panel::DiagShape<kNb>;
+    constexpr int LD = Sh::kLd;
+    double* S = smem;
+    double* work = S + Sh::kBlockDoubles;
+    float* Yf = reinterpret_cast<float*>(work + Sh::kWorkDoubles);
+    float* Pf = Yf + 64 * kLdf;
     const int tid = threadIdx.x;
-    for (int idx = tid; idx < kNb * kNb; idx += blockDim.x) {
-        const int i = idx / kNb, j = idx % kNb;
-        T[i * L + j] = (j <= i) ? (double)A[(size_t)i * ld + j] : 0.0;
+    float* A = a + (size_t)blockIdx.x * stride + k * ld + k;
+    for (int idx = tid; idx < kNb * LD; idx += 256) {
+        const int i = idx / LD, j = idx % LD;
+        S[idx] = j <= i ? (double)A[(size_t)i * ld + j] : 0.0;
     }
-    __syncthreads();
-    for (int j = 0; j < kNb && !invert_only; ++j) {
-        if (tid == 0) {
-            double piv = T[j * L + j];
-            if (!(piv > 0.0)) {
-                atomicMin(err_pivot, (unsigned long long)(k + j + 1));
-                piv = 1.0;
-            }
-            T[j * L + j] = sqrt(piv);
-        }
-        __syncthreads();
-        const double rjj = 1.0 / T[j * L + j];
-        for (int i = j + 1 + tid; i < kNb; i += blockDim.x) T[i * L + j] *= rjj;
-        __syncthreads();
-        // rank-1 update of the trailing lower triangle on a 16 x 16 thread grid (no index division)
-        for (int i = j + 1 + (tid >> 4); i < kNb; i += 16) {
-            const double lij = T[i * L + j];
-            for (int l = j + 1 + (tid & 15); l <= i; l += 16) T[i * L + l] -= lij * T[l * L + j];
-        }
-        __syncthreads();
-    }
-    if (!invert_only)
-        for (int idx = tid; idx < kNb * kNb; idx += blockDim.x) {
+    if (NB == 128) load_f32_async<64, kLdf>(Pf, A + (size_t)kNb * ld, ld);
+    asm volatile("cp.async.commit_group;\n" ::);
+    auto inverse_out = [&](float* dst) {
+        for (int idx = tid; idx < kNb * kNb; idx += 256) {
             const int i = idx / kNb, j = idx % kNb;
-            if (j <= i) A[(size_t)i * ld + j] = (float)T[i * L + j];
+            const float y = j <= i ? (float)S[j * LD + i + 1] : 0.0f;
+            Yf[i * kLdf + j] = y;
+            dst[(size_t)i * ld + j] = y;
         }
-    {
-        const int col = tid >> 2, part = tid & 3;
-        for (int i = 0; i < kNb; ++i) {
-            double sum = 0.0;
-            if (i > col)
-                for (int l = col + part; l < i; l += 4) sum = fma(T[i * L + l], l == col ? Yd[col] : T[col * L + l], sum);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-            if (part == 0) {
-                if (i == col) Yd[col] = 1.0 / T[i * L + i];
-                else if (i > col) T[col * L + i] = -sum / T[i * L + i];
-            }
-            __syncwarp();
-        }
-    }
+    };
     __syncthreads();
-    float* out = linv + (size_t)blockIdx.x * kNb * kNb;
-    for (int idx = tid; idx < kNb * kNb; idx += blockDim.x) {
-        const int r = idx / kNb, c = idx % kNb;
-        out[idx] = r > c ? (float)T[c * L + r] : (r == c ? (float)Yd[r] : 0.0f);
+    panel::factor_diag<kNb, false>(S, work, k, err_pivot);
+    inverse_out(A);
+    if (NB == 128) {
+        const int lane = tid & 31, w = tid >> 5;
+        const int g = lane >> 2, t = lane & 3;
+        const int rr = 16 * (w >> 1), cc = 32 * (w & 1);
+        float* A21 = A + (size_t)kNb * ld;
+        float* A22 = A21 + kNb;
+        asm volatile("cp.async.wait_group 0;\n" ::);
+        __syncthreads();
+        float acc[4][4] = {};
+        tile_mma_3xtf32<kLdf, 64>(Pf, Yf, acc, 1.0f);
+        __syncthreads();
+        store_fragments<kLdf>(Pf, acc);
+        __syncthreads();
+        for (int idx = tid; idx < 64 * 16; idx += 256) {
+            const int r = idx >> 4, c4 = idx & 15;
+            *reinterpret_cast<float4*>(A21 + (size_t)r * ld + 4 * c4) = *reinterpret_cast<const float4*>(Pf + r * kLdf + 4 * c4);
+        }
+        float upd[4][4] = {};
+        tile_mma_3xtf32<kLdf, 64>(Pf, Pf, upd, -1.0f);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int i = rr + g + 8 * (e >> 1), c = cc + 8 * j + 2 * t + (e & 1);
+                S[i * LD + c] = c <= i ? (double)(A22[(size_t)i * ld + c] + upd[j][e]) : 0.0;
+            }
+        if (tid < kNb) S[tid * LD + kNb] = 0.0;  // the last identity column
+        __syncthreads();
+        panel::factor_diag<kNb, false>(S, work, k + kNb, err_pivot);
+        inverse_out(A22);
     }
 }
 
-// Panel solve P <- P Linv^T on the tensor cores (3xTF32) for the 64-row blocks from row0 on; RHS
-// rows add their squared norms (FP64) to qacc unless it is null.
-__global__ void __launch_bounds__(256) k_trsm_panel32(float* __restrict__ a, int64_t ld, int64_t stride, int64_t k,
-                                                      int64_t row0, int64_t n_pad, const float* __restrict__ linv,
-                                                      double* __restrict__ qacc, int64_t ldq) {
-    extern __shared__ float fsm[];
-    float* Ps = fsm;
-    float* Ls = fsm + 64 * kLdf;
-    const int f = blockIdx.y;
-    const int64_t r0 = row0 + (int64_t)blockIdx.x * kNb;
-    float* A = a + (size_t)f * stride;
-    load_f32_async<64, kLdf>(Ps, A + r0 * ld + k, ld);
-    load_f32_async<64, kLdf>(Ls, linv + (size_t)f * kNb * kNb, kNb);
-    asm volatile("cp.async.commit_group;\n" ::);
-    asm volatile("cp.async.wait_group 0;\n" ::);
-    __syncthreads();
-    float acc[4][4] = {};
-    tile_mma_3xtf32<kLdf, 64>(Ps, Ls, acc, 1.0f);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+// The rows below an outer block, 64-row tiles from row0 on: P1 = A1 L11^{-T}, A2 -= P1 L21^T,
+// P2 = A2 L22^{-T} (3xTF32; a 64-wide block is P1 alone), in one pass with the block's three tiles
+// kept in shared memory (as separate solves and an update between them the tile moved three times).
+// Bound by the tensor pipe's TF32 rate in three products per tile.
+//   solve_row0  rows before it are finished (the solve-only pass): passed through to `panel` alone
+//   rows_end    rows to write to `panel` (beyond `rows` zeros)
+//   panel       the solved rows' hi / lo parts for the tcgen05 update (tc::panel_position); null: none
+//   keep        write the solved rows back to the tall matrix
+//   qacc        squared norms (FP64) of the right-hand-side rows are added; null: none
+template <int NB>
+__global__ void __launch_bounds__(256, 2)
+    k_panel32(float* __restrict__ a, int64_t ld, int64_t stride, int64_t k, int64_t row0, int64_t rows, int64_t rows_end,
+              int64_t solve_row0, int64_t n_pad, float* __restrict__ panel, int keep, double* __restrict__ qacc,
+              int64_t ldq) {
+    extern __shared__ __align__(16) float fsm[];
+    constexpr int kTile = 64 * kLdf;
+    float* P1 = fsm;
+    float* P2 = P1 + kTile;  // NB == 128 only, as the last two
+    float* Y1 = NB == 128 ? P2 + kTile : P2;
+    float* L21 = Y1 + kTile;
+    float* Y2 = L21 + kTile;
+    const int tid = threadIdx.x;
+    const int lane = tid & 31, w = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const int rr = 16 * (w >> 1), cc = 32 * (w & 1);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        Ps[(rr + g) * kLdf + cc + 8 * j + 2 * t] = acc[j][0];
-        Ps[(rr + g) * kLdf + cc + 8 * j + 2 * t + 1] = acc[j][1];
-        Ps[(rr + g + 8) * kLdf + cc + 8 * j + 2 * t] = acc[j][2];
-        Ps[(rr + g + 8) * kLdf + cc + 8 * j + 2 * t + 1] = acc[j][3];
+    const int rr0 = 16 * (w >> 1), cc0 = 32 * (w & 1);
+    float* A = a + (size_t)blockIdx.y * stride;
+    const float* D = A + (size_t)k * ld + k;
+    load_f32_async<64, kLdf>(Y1, D, ld);
+    if (NB == 128) {
+        load_f32_async<64, kLdf>(L21, D + (size_t)kNb * ld, ld);
+        load_f32_async<64, kLdf>(Y2, D + (size_t)kNb * ld + kNb, ld);
     }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < 64 * 16; idx += blockDim.x) {
-        const int r = idx >> 4, c4 = idx & 15;
-        *reinterpret_cast<float4*>(A + (size_t)(r0 + r) * ld + k + 4 * c4) =
-            *reinterpret_cast<const float4*>(Ps + r * kLdf + 4 * c4);
-    }
-    if (qacc && r0 >= n_pad && threadIdx.x < kNb) {
-        const int r = threadIdx.x;
-        double s = 0.0;
-        for (int j = 0; j < kNb; ++j) {
-            const double y = (double)Ps[r * kLdf + j];
-            s = fma(y, y, s);
+    const int64_t rp = rows_end - row0;
+    float4* hi = reinterpret_cast<float4*>(panel + (size_t)blockIdx.y * 2 * (NB / 32) * rp * 32);
+    float4* lo = hi + (size_t)(NB / 32) * rp * 8;
+    for (int64_t r0 = row0 + (int64_t)blockIdx.x * kNb; r0 < rows_end; r0 += (int64_t)gridDim.x * kNb) {
+        const bool inside = r0 < rows;
+        const bool solve = inside && r0 >= solve_row0;
+        if (inside) {
+            load_f32_async<64, kLdf>(P1, A + r0 * ld + k, ld);
+            if (NB == 128) load_f32_async<64, kLdf>(P2, A + r0 * ld + k + kNb, ld);
         }
-        qacc[(size_t)f * ldq + (r0 - n_pad + r)] += s;
+        asm volatile("cp.async.commit_group;\n" ::);
+        asm volatile("cp.async.wait_group 0;\n" ::);
+        __syncthreads();
+        if (solve) {
+            float acc[4][4] = {};
+            tile_mma_3xtf32<kLdf, 64>(P1, Y1, acc, 1.0f);
+            __syncthreads();
+            store_fragments<kLdf>(P1, acc);
+            __syncthreads();
+            if (NB == 128) {
+                float upd[4][4] = {};
+                tile_mma_3xtf32<kLdf, 64>(P1, L21, upd, -1.0f);
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        P2[(rr0 + g + 8 * (e >> 1)) * kLdf + cc0 + 8 * j + 2 * t + (e & 1)] += upd[j][e];
+                __syncthreads();
+                float acc2[4][4] = {};
+                tile_mma_3xtf32<kLdf, 64>(P2, Y2, acc2, 1.0f);
+                __syncthreads();
+                store_fragments<kLdf>(P2, acc2);
+                __syncthreads();
+            }
+            if (keep)
+                for (int idx = tid; idx < 64 * (NB / 4); idx += 256) {
+                    const int r = idx / (NB / 4), c = 4 * (idx % (NB / 4));
+                    *reinterpret_cast<float4*>(A + (size_t)(r0 + r) * ld + k + c) =
+                        *reinterpret_cast<const float4*>((c < kNb ? P1 : P2 - kNb) + r * kLdf + c);
+                }
+            if (qacc && r0 >= n_pad) {  // four threads per row, fixed order
+                const int r = tid >> 2, part = tid & 3;
+                double s = 0.0;
+                for (int c = part; c < NB; c += 4) {
+                    const double y = (double)(c < kNb ? P1 : P2 - kNb)[r * kLdf + c];
+                    s = fma(y, y, s);
+                }
+                s += __shfl_xor_sync(0xffffffffu, s, 1);
+                s += __shfl_xor_sync(0xffffffffu, s, 2);
+                if (part == 0) qacc[(size_t)blockIdx.y * ldq + (r0 - n_pad + r)] += s;
+            }
+        }
+        if (panel) {
+            for (int idx = tid; idx < 64 * (NB / 4); idx += 256) {
+                const int kb = idx >> 9, r = (idx >> 3) & 63, c = idx & 7;  // K slice of 32, row, 16-byte chunk
+                const int col = 32 * kb + 4 * c;
+                float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (inside) x = *reinterpret_cast<const float4*>((col < kNb ? P1 : P2 - kNb) + r * kLdf + col);
+                float4 h, l;
+                h.x = __uint_as_float(to_tf32(x.x));
+                h.y = __uint_as_float(to_tf32(x.y));
+                h.z = __uint_as_float(to_tf32(x.z));
+                h.w = __uint_as_float(to_tf32(x.w));
+                l.x = __uint_as_float(to_tf32(x.x - h.x));
+                l.y = __uint_as_float(to_tf32(x.y - h.y));
+                l.z = __uint_as_float(to_tf32(x.z - h.z));
+                l.w = __uint_as_float(to_tf32(x.w - h.w));
+                const int64_t rr = r0 - row0 + r;
+                const size_t dst = ((size_t)kb * rp + rr) * 8 + (c ^ (int)(rr & 7));
+                hi[dst] = h;
+                lo[dst] = l;
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -296,63 +374,66 @@ int launch_build_tall32(const TallGeometry& g, const double* v, const double* xt
     return 1;
 }
 
-int launch_factor_chunk32(const TallGeometry& g, int64_t nf, float* a, float* linv, double* qacc,
-                          unsigned long long* err_pivot, cudaStream_t s, UpdateProfiler* prof, float* panel,
-                          unsigned long long* sched, int max_ctas, bool solve_only) {
-    const size_t smem_tile = 2 * 64 * kLdf * sizeof(float);
-    const size_t smem_update = 4 * 64 * kLdkf * sizeof(float);
-    const size_t smem_potrf = (kNb * (kNb + 1) + kNb) * sizeof(double);
-    GWB_CUDA(cudaFuncSetAttribute(k_trsm_panel32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_tile));
-    GWB_CUDA(cudaFuncSetAttribute(k_update32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_update));
-    GWB_CUDA(cudaFuncSetAttribute(k_potrf_diag32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_potrf));
-    const int64_t nsq = g.n_pad / kNb, nrt = g.rows / kNb;
-    constexpr int64_t kInner = 2;
+namespace {
+
+template <int NB>
+int launch_block32(const TallGeometry& g, int64_t nf, float* a, int64_t k, double* qacc, unsigned long long* err_pivot,
+                   cudaStream_t s, float* panel, bool solve_only, bool keep) {
     int launches = 0;
-    // with the tcgen05 outer updates, the profiler times those alone (the look-left updates that
-    // stay on mma.sync are a few percent of the flops)
-    UpdateProfiler* lprof = panel ? nullptr : prof;
-    auto update = [&](int64_t kb0, int nk, int64_t tc0, int64_t T) {
-        const int64_t L = nsq - tc0;
-        const int64_t tiles = (solve_only ? 0 : T * L - T * (T - 1) / 2) + T * (nrt - nsq);
-        if (tiles <= 0) return;
-        if (lprof) lprof->begin();
-        k_update32<<<dim3((unsigned)tiles, (unsigned)nf), 256, smem_update, s>>>(a, g.ld, g.stride, kb0, nk, tc0, T, nsq,
-                                                                                  solve_only ? 1 : 0);
-        GWB_LAUNCH("k_update32");
-        if (lprof) lprof->end((double)nf * update_flops32(g, kb0, nk, tc0 * kNb, (tc0 + T) * kNb));
+    if (!solve_only) {
+        GWB_CUDA(cudaFuncSetAttribute(k_diag32<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiag32Smem));
+        k_diag32<NB><<<(unsigned)nf, 256, kDiag32Smem, s>>>(a, g.ld, g.stride, k, err_pivot);
+        GWB_LAUNCH("k_diag32");
         ++launches;
-    };
-    for (int64_t ob = 0; ob < nsq; ob += kInner) {
-        const int64_t q = std::min(kInner, nsq - ob);
-        for (int64_t j = 0; j < q; ++j) {
-            const int64_t kt = ob + j, k = kt * kNb;
-            if (j > 0) update(ob * kNb, (int)j, kt, 1);
-            k_potrf_diag32<<<(unsigned)nf, 256, smem_potrf, s>>>(a, g.ld, g.stride, k, linv, err_pivot,
-                                                                 solve_only ? 1 : 0);
-            GWB_LAUNCH("k_potrf_diag32");
-            ++launches;
-            // the panel rows below the block: all of them while factoring, the RHS rows alone when
-            // solving against a finished factor
-            const int64_t row0 = solve_only ? g.n_pad : k + kNb;
-            const int64_t below = g.rows - row0;
-            if (below > 0) {
-                k_trsm_panel32<<<dim3((unsigned)(below / kNb), (unsigned)nf), 256, smem_tile, s>>>(
-                    a, g.ld, g.stride, k, row0, g.n_pad, linv, solve_only ? nullptr : qacc, g.m_pad);
-                GWB_LAUNCH("k_trsm_panel32");
+    }
+    // the rows below: all of them for the update's operands, else while factoring; the solve-only
+    // pass works on the right-hand sides alone
+    const int64_t row0 = solve_only && !panel ? g.n_pad : k + NB;
+    const int64_t rows_end = panel ? row0 + tc_panel_rows(g, row0) : g.rows;
+    const int64_t tiles = (rows_end - row0) / kNb;
+    if (tiles <= 0) return launches;
+    const size_t smem = (NB == 128 ? 5 : 2) * 64 * kLdf * sizeof(float);
+    GWB_CUDA(cudaFuncSetAttribute(k_panel32<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_panel32<NB><<<dim3((unsigned)panel_grid(tiles, nf, 2), (unsigned)nf), 256, smem, s>>>(
+        a, g.ld, g.stride, k, row0, g.rows, rows_end, solve_only ? g.n_pad : row0, g.n_pad, panel, keep ? 1 : 0, qacc,
+        g.m_pad);
+    GWB_LAUNCH("k_panel32");
+    return launches + 1;
+}
+
+}  // namespace
+
+int launch_factor_chunk32(const TallGeometry& g, int64_t nf, float* a, double* qacc, unsigned long long* err_pivot,
+                          cudaStream_t s, UpdateProfiler* prof, float* panel, unsigned long long* sched, int max_ctas,
+                          bool keep_rows, bool solve_only) {
+    const size_t smem_update = 4 * 64 * kLdkf * sizeof(float);
+    GWB_CUDA(cudaFuncSetAttribute(k_update32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_update));
+    const int64_t nsq = g.n_pad / kNb, nrt = g.rows / kNb;
+    constexpr int64_t kOuter = 2;
+    int launches = 0;
+    if (panel && nsq > kOuter) launches += launch_clear_sched(g, sched, s);
+    for (int64_t ob = 0; ob < nsq; ob += kOuter) {
+        const int64_t q = std::min(kOuter, nsq - ob), tc0 = ob + q;
+        float* pan = tc0 < nsq ? panel : nullptr;  // operands of the trailing update, when there is one
+        const bool keep = keep_rows || !panel;     // the mma.sync update reads the rows themselves
+        launches += q == kOuter ? launch_block32<128>(g, nf, a, ob * kNb, qacc, err_pivot, s, pan, solve_only, keep)
+                                : launch_block32<64>(g, nf, a, ob * kNb, qacc, err_pivot, s, pan, solve_only, keep);
+        if (tc0 >= nsq) break;
+        if (prof) prof->begin();
+        if (pan) {  // trailing update on tcgen05
+            launches += launch_update32_tc(g, nf, a, tc0 * kNb, pan, sched + ob / kOuter, err_pivot, s, max_ctas,
+                                           solve_only ? g.n_pad : 0);
+        } else {
+            const int64_t T = nsq - tc0;
+            const int64_t tiles = (solve_only ? 0 : T * (T + 1) / 2) + T * (nrt - nsq);
+            if (tiles > 0) {
+                k_update32<<<dim3((unsigned)tiles, (unsigned)nf), 256, smem_update, s>>>(
+                    a, g.ld, g.stride, ob * kNb, (int)q, tc0, T, nsq, solve_only ? 1 : 0);
+                GWB_LAUNCH("k_update32");
                 ++launches;
             }
         }
-        const int64_t tc0 = ob + q;
-        if (tc0 < nsq) {
-            if (panel) {  // outer trailing update on tcgen05
-                if (prof) prof->begin();
-                launches += launch_update32_tc(g, nf, a, ob * kNb, (int)(q * kNb), tc0 * kNb, panel, sched, err_pivot, s,
-                                                max_ctas, solve_only ? g.n_pad : 0);
-                if (prof) prof->end((double)nf * update_flops32(g, ob * kNb, (int)q, tc0 * kNb, nsq * kNb));
-            } else {
-                update(ob * kNb, (int)q, tc0, nsq - tc0);
-            }
-        }
+        if (prof) prof->end((double)nf * update_flops32(g, ob * kNb, (int)q, tc0 * kNb, nsq * kNb));
     }
     return launches;
 }

@@ -437,7 +437,10 @@ int tune_update_variant(const TallGeometry& g, int64_t nf, double* a, cudaStream
         }
     }
     if (oz) {  // the int8 emulation of the outer update (kernels_oz.cu), slicing included
-        const float ms = time_it([&] { launch_update64_oz(g, nf, a, 0, 2 * kNb, oz, sched, err_pivot, s); });
+        const float ms = time_it([&] {
+            launch_clear_sched(g, sched, s);
+            launch_update64_oz(g, nf, a, 0, 2 * kNb, oz, sched, err_pivot, s);
+        });
         times[kUpdateOzaki] = ms;
         if (ms < best_ms) {
             best_ms = ms;
@@ -478,6 +481,7 @@ int launch_factor_chunk(const TallGeometry& g, int64_t nf, double* a, double* qa
         GWB_CUDA(cudaFuncSetAttribute(kVariants[variant].fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)kVariants[variant].smem));
     int launches = 0;
+    if (use_oz && nsq > kOuter) launches += launch_clear_sched(g, sched, s);
     for (int64_t ob = 0; ob < nsq; ob += kOuter) {
         const int64_t q = std::min(kOuter, nsq - ob), tc0 = ob + q;
         launches += launch_panel64(g, nf, a, ob * kNb, q * kNb, qacc, err_pivot, s);
@@ -485,7 +489,7 @@ int launch_factor_chunk(const TallGeometry& g, int64_t nf, double* a, double* qa
         // trailing update, K = 128 (columns remain only behind a full outer block)
         if (prof) prof->begin();
         if (use_oz) {
-            launches += launch_update64_oz(g, nf, a, ob * kNb, tc0 * kNb, oz, sched, err_pivot, s, max_ctas);
+            launches += launch_update64_oz(g, nf, a, ob * kNb, tc0 * kNb, oz, sched + ob / kOuter, err_pivot, s, max_ctas);
         } else {
             launch_variant(variant, g, nf, a, ob * kNb, (int)q, tc0, nsq - tc0, s);
             ++launches;

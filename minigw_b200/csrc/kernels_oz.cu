@@ -590,7 +590,6 @@ int launch_update64_oz(const TallGeometry& g, int64_t nf, double* a, int64_t kb0
     us.NS = (T + kOzSeg - 1) / kOzSeg;
     us.per_f = NI * us.NS;
     us.total = nf * us.per_f;
-    GWB_CUDA(cudaMemsetAsync(sched, 0, sizeof(unsigned long long), s));
     const char* expire = std::getenv("GWB200_TEST_EXPIRE_WAIT");
     const int withhold = (expire && expire[0] == '1') ? 1 : 0;
     const unsigned grid = (unsigned)std::min<int64_t>(us.total, max_ctas > 0 ? std::min(max_ctas, sm_count()) : sm_count());

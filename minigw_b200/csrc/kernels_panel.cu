@@ -21,16 +21,17 @@ namespace {
 
 using namespace panel;
 
+constexpr int kPanelThreads = 256;
 constexpr int kRowTile = 32;
 
 template <int NB>
-__global__ void __launch_bounds__(kPanelThreads) k_diag64(double* __restrict__ a, int64_t ld, int64_t stride, int64_t k,
+__global__ void __launch_bounds__(DiagShape<NB>::kThreads) k_diag64(double* __restrict__ a, int64_t ld, int64_t stride, int64_t k,
                                                           unsigned long long* err_pivot) {
     extern __shared__ __align__(16) double psm[];
     constexpr int LD = DiagShape<NB>::kLd;
     double* S = psm;
     double* A = a + (size_t)blockIdx.x * stride + k * ld + k;
-    for (int idx = threadIdx.x; idx < NB * (LD / 2); idx += kPanelThreads) {
+    for (int idx = threadIdx.x; idx < NB * (LD / 2); idx += DiagShape<NB>::kThreads) {
         const int i = idx / (LD / 2), j = 2 * (idx % (LD / 2));
         double2 v = make_double2(0.0, 0.0);
         if (j <= i) v = *reinterpret_cast<const double2*>(A + (size_t)i * ld + j);
@@ -41,7 +42,7 @@ __global__ void __launch_bounds__(kPanelThreads) k_diag64(double* __restrict__ a
     factor_diag<NB, false>(S, S + DiagShape<NB>::kBlockDoubles, k, err_pivot);
     // the inverse in place of the block; above the diagonal zeros (not the upper right 64 x 64, which
     // nothing reads)
-    for (int idx = threadIdx.x; idx < NB * NB; idx += kPanelThreads) {
+    for (int idx = threadIdx.x; idx < NB * NB; idx += DiagShape<NB>::kThreads) {
         const int i = idx / NB, j = idx % NB;
         if (j < (i < kNb ? kNb : NB)) A[(size_t)i * ld + j] = j <= i ? S[j * LD + i + 1] : 0.0;
     }
@@ -146,12 +147,12 @@ template <int NB>
 int launch_block(const TallGeometry& g, int64_t nf, double* a, int64_t k, double* qacc, unsigned long long* err_pivot,
                  cudaStream_t s) {
     GWB_CUDA(cudaFuncSetAttribute(k_diag64<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DiagShape<NB>::kSmem));
-    k_diag64<NB><<<(unsigned)nf, kPanelThreads, DiagShape<NB>::kSmem, s>>>(a, g.ld, g.stride, k, err_pivot);
+    k_diag64<NB><<<(unsigned)nf, DiagShape<NB>::kThreads, DiagShape<NB>::kSmem, s>>>(a, g.ld, g.stride, k, err_pivot);
     GWB_LAUNCH("k_diag64");
     const int64_t tiles = (g.rows - (k + NB)) / kRowTile;
     if (tiles <= 0) return 1;
     GWB_CUDA(cudaFuncSetAttribute(k_panel64<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PanelShape<NB>::kSmem));
-    k_panel64<NB><<<dim3((unsigned)panel_grid(tiles, nf), (unsigned)nf), kPanelThreads, PanelShape<NB>::kSmem, s>>>(
+    k_panel64<NB><<<dim3((unsigned)panel_grid(tiles, nf, 1), (unsigned)nf), kPanelThreads, PanelShape<NB>::kSmem, s>>>(
         a, g.ld, g.stride, k, g.n_pad, (int)tiles, qacc, g.m_pad);
     GWB_LAUNCH("k_panel64");
     return 2;
@@ -159,14 +160,13 @@ int launch_block(const TallGeometry& g, int64_t nf, double* a, int64_t k, double
 
 }  // namespace
 
-// CTAs per frequency for `tiles` row tiles of nf frequencies, one CTA per SM: the fewest tile times
-// over the waves, counting two for a CTA's load of the inverse.
-int64_t panel_grid(int64_t tiles, int64_t nf) {
-    const int64_t sms = 148;
+// The fewest tile times over the waves, counting two for a CTA's load of the block's tiles.
+int64_t panel_grid(int64_t tiles, int64_t nf, int64_t per_sm) {
+    const int64_t slots = 148 * per_sm;
     int64_t best = 1;
     double best_cost = 0.0;
     for (int64_t gx = 1; gx <= std::min<int64_t>(tiles, 64); ++gx) {
-        const double waves = (double)((nf * gx + sms - 1) / sms);
+        const double waves = (double)((nf * gx + slots - 1) / slots);
         const double cost = waves * ((double)((tiles + gx - 1) / gx) + 2.0);
         if (gx == 1 || cost < best_cost) {
             best = gx;

@@ -14,7 +14,8 @@
 //
 // Steps per frequency chunk (after the mixed factorisation of the chunk):
 //   k_flip_tiles32 + k_reverse_rows32  turn L~ into P L~^T P (P the index reversal of [0, n_pad)),
-//                 which is lower triangular, and reverse every RHS row: the backward solve
+//                 which is lower triangular (the diagonal blocks hold their inverses, and the
+//                 reversal of an inverse is the inverse of the reversal), and reverse every RHS row: the backward solve
 //                 L~^T z = w becomes the forward solve (P L~^T P)(P z) = P w, which the mixed
 //                 factorisation's kernels run in their solve-only mode (the RHS rows alone against
 //                 the finished factor) -> the RHS rows end as (P z_j)^T;
@@ -423,11 +424,11 @@ int launch_refine_flip(const TallGeometry& ga, int64_t nf, float* a, int64_t n_f
     return 2;
 }
 
-int launch_refine_solve(const TallGeometry& g, int64_t nf, float* a, float* linv, unsigned long long* err_pivot,
+int launch_refine_solve(const TallGeometry& g, int64_t nf, float* a, unsigned long long* err_pivot,
                         cudaStream_t s, float* panel, unsigned long long* sched, int max_ctas, bool flip) {
     int launches = flip ? launch_refine_flip(g, nf, a, g.n_pad, s) : 0;
-    launches += launch_factor_chunk32(g, nf, a, linv, nullptr, err_pivot, s, nullptr, panel, sched, max_ctas,
-                                      /*solve_only=*/true);
+    launches += launch_factor_chunk32(g, nf, a, nullptr, err_pivot, s, nullptr, panel, sched, max_ctas,
+                                      /*keep_rows=*/true, /*solve_only=*/true);
     return launches;
 }
 
@@ -466,11 +467,11 @@ int launch_refine_terms(const TallGeometry& ga, int64_t nf, const float* a, cons
     return launches + 1;
 }
 
-int launch_refine_chunk(const TallGeometry& g, int64_t nf, float* a, float* linv, const double* xt,
+int launch_refine_chunk(const TallGeometry& g, int64_t nf, float* a, const double* xt,
                         const double* dvec, const RefineFactor& fac, void* work, double* qacc,
                         unsigned long long* err_pivot, cudaStream_t s, float* panel, unsigned long long* sched,
                         int max_ctas) {
-    return launch_refine_solve(g, nf, a, linv, err_pivot, s, panel, sched, max_ctas, /*flip=*/true) +
+    return launch_refine_solve(g, nf, a, err_pivot, s, panel, sched, max_ctas, /*flip=*/true) +
            launch_refine_terms(g, nf, a, g, xt, dvec, fac, work, qacc, g.m_pad, err_pivot, s);
 }
 

@@ -1,17 +1,18 @@
 // kernels_tc.cu -- the mixed form's trailing update on the 5th-generation tensor cores (tcgen05).
 //
-// After an outer block of K = 64 or 128 columns [kb0, kb0+K) has been factored, every element of
+// After an outer block of K = 128 columns [kb0, kb0+K) has been factored, every element of
 // the trailing lower part C = A[r][c] (c_begin <= c < n_pad, c <= r < rows) takes
 // C -= P_r . P_c with P the FP32 panel A[:, kb0:kb0+K).  The products use the 3xTF32 split
 // (x = hi + lo, hi = rna_tf32(x), lo = rna_tf32(x - hi); x.y ~ lo.hi + hi.lo + hi.hi, in that
 // order per 8-deep K step) accumulated in FP32: the same arithmetic, in the same order, as the
 // mma.sync update of kernels_f32.cu.
 //
-// Two launches per update:
-//   k_split_panel32  writes hi and lo of the panel rows [c_begin, rows) in the 128-byte-swizzled
-//                    K-major layout the tensor core reads ([K slice of 32 floats][row][128 bytes],
-//                    rows padded with zeros to a multiple of 128), so that every operand slice of a
-//                    tile is one contiguous 16 KB block (one cp.async.bulk);
+// The solved rows come from k_panel32 (kernels_f32.cu) already split: hi and lo of the panel rows
+// [c_begin, rows) in the 128-byte-swizzled K-major layout the tensor core reads ([K slice of 32
+// floats][row][128 bytes], the 16-byte chunk c of row r at chunk position c ^ (r % 8), rows padded
+// with zeros to a multiple of 128), so that every operand slice of a tile is one contiguous 16 KB
+// block (one cp.async.bulk).
+//
 //   k_update32_tc    a persistent, warp-specialised kernel, one CTA per SM (18 warps, 226 KB of
 //                    shared memory, all 512 TMEM columns):
 //                      warp 0     producer: takes work units from a global counter and hands them
@@ -124,45 +125,6 @@ __device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* map, uint32
                  "r"(src), "r"(x), "r"(y), "r"(z)
                  : "memory");
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-}
-__device__ __forceinline__ float rna_tf32(float x) {
-    uint32_t r;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-    return __uint_as_float(r);
-}
-
-// hi/lo of panel rows [c_begin, rows) x columns [kb0, kb0 + 32 nkc) in the 128-byte-swizzled
-// K-major layout: [K slice of 32 floats][row][128 bytes], the 16-byte chunk c of row rr stored at
-// chunk position c ^ (rr % 8); rows [rows - c_begin, rp) are zero.  Per frequency: hi at
-// panel + f*2*nkc*rp*32, lo nkc*rp*32 floats later.  One thread per 16-byte chunk.
-__global__ void k_split_panel32(const float* __restrict__ a, int64_t ld, int64_t stride, int64_t kb0, int nkc,
-                                int64_t c_begin, int64_t rows, int64_t rp, float* __restrict__ panel) {
-    const int f = blockIdx.y;
-    const float* A = a + (size_t)f * stride;
-    float4* hi = reinterpret_cast<float4*>(panel + (size_t)f * 2 * nkc * rp * 32);
-    float4* lo = hi + (size_t)nkc * rp * 8;
-    const int64_t total = (int64_t)nkc * rp * 8;
-    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t srow = idx >> 3;  // kb * rp + rr
-        const int c = (int)(idx & 7);
-        const int64_t kb = srow / rp, rr = srow - kb * rp;
-        const int64_t r = c_begin + rr;
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < rows) x = *reinterpret_cast<const float4*>(A + (size_t)r * ld + kb0 + 32 * kb + 4 * c);
-        float4 h, l;
-        h.x = rna_tf32(x.x);
-        h.y = rna_tf32(x.y);
-        h.z = rna_tf32(x.z);
-        h.w = rna_tf32(x.w);
-        l.x = rna_tf32(x.x - h.x);
-        l.y = rna_tf32(x.y - h.y);
-        l.z = rna_tf32(x.z - h.z);
-        l.w = rna_tf32(x.w - h.w);
-        const int64_t dst = srow * 8 + (c ^ (int)(rr & 7));
-        hi[dst] = h;
-        lo[dst] = l;
-    }
 }
 
 // Work units: (frequency, 128-row tile i, segment of kTcSeg column tiles of 128).  Column tile c
@@ -514,22 +476,29 @@ size_t tc_panel_bytes_per_freq(const TallGeometry& g) {
     return (size_t)2 * (128 / 4) * (size_t)rp * 16;
 }
 
-int launch_update32_tc(const TallGeometry& g, int64_t nf, float* a, int64_t kb0, int kdim, int64_t c_begin,
-                       float* panel, unsigned long long* sched, unsigned long long* err, cudaStream_t s, int max_ctas,
+namespace {
+// The work counters of a pass's updates, one per outer block, cleared in one launch.
+__global__ void k_clear_sched(unsigned long long* __restrict__ sched, int count) {
+    for (int i = threadIdx.x; i < count; i += blockDim.x) sched[i] = 0ull;
+}
+}  // namespace
+
+int launch_clear_sched(const TallGeometry& g, unsigned long long* sched, cudaStream_t s) {
+    k_clear_sched<<<1, 256, 0, s>>>(sched, (int)(sched_bytes(g) / sizeof(unsigned long long)));
+    GWB_LAUNCH("k_clear_sched");
+    return 1;
+}
+
+int64_t tc_panel_rows(const TallGeometry& g, int64_t c_begin) { return round_up(g.rows - c_begin, kTcM); }
+
+int launch_update32_tc(const TallGeometry& g, int64_t nf, float* a, int64_t c_begin, const float* panel,
+                       unsigned long long* sched, unsigned long long* err, cudaStream_t s, int max_ctas,
                        int64_t row_min) {
-    if (kdim <= 0 || kdim > 128 || kdim % kTcKc != 0)
-        fail(GWB200_BAD_SHAPE, "tcgen05 update: K must be 32, 64, 96 or 128");
     const int64_t T = (g.n_pad - c_begin + kTcN - 1) / kTcN;  // the last column tile may be 64 wide
     if (T <= 0 || nf <= 0) return 0;
     const int64_t H = g.rows - c_begin;
     const int64_t NI = (H + kTcM - 1) / kTcM, rp = NI * kTcM;
-    const int nkc = kdim / kTcKc;
-    {
-        const int64_t total = (int64_t)nkc * rp * 8;
-        const unsigned gx = (unsigned)std::min<int64_t>((total + 255) / 256, 4096);
-        k_split_panel32<<<dim3(gx, (unsigned)nf), 256, 0, s>>>(a, g.ld, g.stride, kb0, nkc, c_begin, g.rows, rp, panel);
-        GWB_LAUNCH("k_split_panel32");
-    }
+    const int nkc = 128 / kTcKc;
     GWB_CUDA(cudaFuncSetAttribute(k_update32_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
     // C of the chunk as a 3-D FP32 tensor (columns, rows, frequencies), 32 x 32 boxes, 128B swizzle
     CUtensorMap cmap;
@@ -560,7 +529,6 @@ int launch_update32_tc(const TallGeometry& g, int64_t nf, float* a, int64_t kb0,
     const int64_t i0 = std::max<int64_t>(0, (row_min - c_begin) / kTcM);
     us.per_f = (NI - i0) * us.NS;
     us.total = nf * us.per_f;
-    GWB_CUDA(cudaMemsetAsync(sched, 0, sizeof(unsigned long long), s));
     const unsigned grid = (unsigned)std::min<int64_t>(us.total, max_ctas > 0 ? std::min(max_ctas, sm_count()) : sm_count());
     // GWB200_TEST_EXPIRE_WAIT=1 (tests only): one CTA withholds its first operand stage, so a
     // device wait expires and the call reports GWB200_DEVICE_TIMEOUT with the context intact.
@@ -569,7 +537,7 @@ int launch_update32_tc(const TallGeometry& g, int64_t nf, float* a, int64_t kb0,
     k_update32_tc<<<grid, kTcThreads, kTcSmem, s>>>(a, g.ld, g.stride, c_begin, g.rows, g.n_pad, row_min, nkc, panel, rp,
                                                      us, sched, err, withhold, cmap);
     GWB_LAUNCH("k_update32_tc");
-    return 2;
+    return 1;
 }
 
 } // namespace gwb200
