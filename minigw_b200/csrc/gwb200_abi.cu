@@ -128,13 +128,14 @@ struct gwb200_handle {
     bool complex_forms = false;  // the last compute_forms ran the eta != 0 (complex) path
     DevBuf pqo, xdiag, mo, vxc_diag, delta, v, sigx, flag;  // pqo: the (pq|o.) block of the ERI
     // per-call workspaces (grow-only, reused across calls)
-    DevBuf xt, dvec, a, linv, qacc, qall, sigma, omega, weight, states, err, qp, qp_scratch, omega_out;
+    DevBuf xt, dvec, a, linv, qacc, qall, sigma, omega, weight, states, err, qp, omega_out;
     DevBuf panel32;   // operand workspace of the tcgen05 trailing updates (mixed: FP32 hi/lo split;
                       // plain with GWB200_FP64_UPDATE=ozaki: int8 digit slices + exponents)
     DevBuf tc_sched;  // work counter of the tcgen05 update kernel
     // GWB200_MIXED_REFINED: pivoted Cholesky factor of the resident V_ph (computed on first use after
     // a load; pchol_rank < 0: not yet) and the per-chunk refinement workspace
     DevBuf pchol, pchol_sl, refine;  // pchol_sl: the factor's int8 digit slices
+    DevBuf sweep;                    // gwb200_pade_sweep: grid, row, points
     DevBuf qx, sigmx;                // gwb200_sigma_c_matrix: cross forms, Sigma_c between the states
     int64_t pchol_rank = -1;
     double* pchol_ct = nullptr;
@@ -365,7 +366,7 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
         size_t budget = (size_t)((double)avail * 0.85);
         if (h->mem_limit > 0) {  // the handle's cap minus what the system and panels already hold
             const size_t resident = h->pqo.bytes + h->xdiag.bytes + h->v.bytes + h->xt.bytes + h->qall.bytes +
-                                    h->sigma.bytes + h->qp_scratch.bytes + h->pchol.bytes + h->pchol_sl.bytes +
+                                    h->sigma.bytes + h->pchol.bytes + h->pchol_sl.bytes +
                                     h->qx.bytes + h->sigmx.bytes + ((size_t)1 << 20);
             const size_t lim = (size_t)h->mem_limit;
             const size_t room = lim > resident ? lim - resident : 0;
@@ -528,11 +529,9 @@ void contract_on_device(gwb200_handle* h, int64_t nf_int, int64_t nstates, gwb20
 void qp_on_device(gwb200_handle* h, int64_t nfreq, int64_t npade, int64_t nstates) {
     cudaStream_t s = h->stream;
     h->qp.ensure(sizeof(double) * h->nmo);
-    h->qp_scratch.ensure(qp_scratch_bytes(nfreq, nstates));
     launch_fill(h->qp.as<double>(), std::numeric_limits<double>::quiet_NaN(), h->nmo, s);
-    launch_qp(h->sigma.as<double>(), h->omega.as<double>(), nfreq, h->nmo, h->states.as<int64_t>(), nstates, npade,
-              h->mo.as<double>(), h->fermi, h->sigx.as<double>(), h->vxc_diag.as<double>(), h->qp.as<double>(),
-              h->qp_scratch.p, s);
+    launch_qp(h->sigma.as<double>(), h->omega.as<double>(), nfreq, h->states.as<int64_t>(), nstates, npade,
+              h->mo.as<double>(), h->fermi, h->sigx.as<double>(), h->vxc_diag.as<double>(), h->qp.as<double>(), s);
 }
 
 // ---- many molecules in shared launches (gwb200_run_g0w0_batch; kernels in kernels_batch.cu) ----
@@ -751,7 +750,7 @@ int gwb200_destroy(gwb200_handle* h) {
     h->stage_out.release();
     for (DevBuf* b : {&h->pchol, &h->pchol_sl, &h->refine, &h->pqo, &h->xdiag, &h->mo, &h->vxc_diag, &h->delta, &h->v, &h->sigx, &h->flag, &h->xt, &h->dvec, &h->a,
                       &h->linv, &h->qacc, &h->qall, &h->sigma, &h->omega, &h->weight, &h->states, &h->err, &h->qp,
-                      &h->qp_scratch, &h->omega_out, &h->panel32, &h->tc_sched, &h->batch_desc, &h->qx, &h->sigmx})
+                      &h->sweep, &h->omega_out, &h->panel32, &h->tc_sched, &h->batch_desc, &h->qx, &h->sigmx})
         b->release();
     for (BatchLane& l : h->lanes) {
         if (l.stream) cudaStreamSynchronize(l.stream);
@@ -1159,30 +1158,16 @@ int gwb200_pade_sweep(gwb200_handle* h, const double* omega, int64_t nfreq, cons
         if (nfreq <= 0 || npts <= 0) fail(GWB200_BAD_SHAPE, "nfreq and npts must be positive");
         if (npade <= 0) fail(GWB200_BAD_SHAPE, "Pade: npar must be positive");
         cudaStream_t s = h->stream;
-        DevBuf dom, drow, dout, dscr;
-        try {
-            dom.ensure(sizeof(double) * nfreq);
-            drow.ensure(sizeof(double) * 2 * nfreq);
-            dout.ensure(sizeof(double) * 3 * (size_t)npts);
-            dscr.ensure(qp_scratch_bytes(nfreq, pade_sweep_blocks(npts)));
-            GWB_CUDA(cudaMemcpyAsync(dom.p, omega, sizeof(double) * nfreq, cudaMemcpyHostToDevice, s));
-            GWB_CUDA(cudaMemcpyAsync(drow.p, sigma_row, sizeof(double) * 2 * nfreq, cudaMemcpyHostToDevice, s));
-            launch_pade_sweep(drow.as<double>(), dom.as<double>(), nfreq, npade, npts, fermi, x_start, interval,
-                              dout.as<double>(), dscr.p, s);
-            GWB_CUDA(cudaMemcpyAsync(out, dout.p, sizeof(double) * 3 * (size_t)npts, cudaMemcpyDeviceToHost, s));
-            GWB_CUDA(cudaStreamSynchronize(s));
-        } catch (...) {
-            cudaStreamSynchronize(s);
-            dom.release();
-            drow.release();
-            dout.release();
-            dscr.release();
-            throw;
-        }
-        dom.release();
-        drow.release();
-        dout.release();
-        dscr.release();
+        // kept by the handle: allocating and freeing them per call synchronised the device each time
+        h->sweep.ensure(sizeof(double) * ((size_t)nfreq * 3 + 3 * (size_t)npts));
+        double* dom = h->sweep.as<double>();
+        double* drow = dom + nfreq;
+        double* dout = drow + 2 * nfreq;
+        GWB_CUDA(cudaMemcpyAsync(dom, omega, sizeof(double) * nfreq, cudaMemcpyHostToDevice, s));
+        GWB_CUDA(cudaMemcpyAsync(drow, sigma_row, sizeof(double) * 2 * nfreq, cudaMemcpyHostToDevice, s));
+        launch_pade_sweep(drow, dom, nfreq, npade, npts, fermi, x_start, interval, dout, s);
+        GWB_CUDA(cudaMemcpyAsync(out, dout, sizeof(double) * 3 * (size_t)npts, cudaMemcpyDeviceToHost, s));
+        GWB_CUDA(cudaStreamSynchronize(s));
     });
 }
 
@@ -1270,7 +1255,7 @@ size_t batch_avail(const gwb200_handle* w) {
     size_t avail = free_b + held;
     if (w->mem_limit > 0) {
         size_t resident = (size_t)1 << 20;
-        for (const DevBuf* b : {&w->pqo, &w->xdiag, &w->v, &w->xt, &w->dvec, &w->qall, &w->sigma, &w->qp_scratch, &w->a,
+        for (const DevBuf* b : {&w->pqo, &w->xdiag, &w->v, &w->xt, &w->dvec, &w->qall, &w->sigma, &w->a,
                                 &w->linv, &w->qacc, &w->panel32})
             resident += b->bytes;
         const size_t lim = (size_t)w->mem_limit;
@@ -1346,7 +1331,7 @@ std::vector<int64_t> batch_graph_key(const gwb200_handle* w, const std::vector<g
         gkey.push_back(nstates[i]);
         gkey.insert(gkey.end(), states[i], states[i] + nstates[i]);
         gkey.push_back(h->bound_states.empty() ? 0 : 1);
-        for (const DevBuf* b : {&h->pqo, &h->v, &h->xt, &h->dvec, &h->qall, &h->sigma, &h->qp, &h->qp_scratch, &h->omega,
+        for (const DevBuf* b : {&h->pqo, &h->v, &h->xt, &h->dvec, &h->qall, &h->sigma, &h->qp, &h->omega,
                                 &h->weight, &h->states, &h->delta, &h->mo, &h->sigx, &h->vxc_diag})
             put(b->p);
         put(h->pchol_ct);
@@ -1574,7 +1559,6 @@ int gwb200_run_g0w0_batch(gwb200_handle* const* systems, int64_t nsys, const int
             gwb200_handle* h = hs[(size_t)i];
             h->sigma.ensure(sizeof(double) * 2 * (size_t)h->nmo * fs[(size_t)i]);
             h->qp.ensure(sizeof(double) * h->nmo);
-            h->qp_scratch.ensure(qp_scratch_bytes(fs[(size_t)i], nstates[i]));
         }
         // the lanes fork off the lead stream and join back onto it around each phase
         auto lane_stream = [&](int l) { return l == 0 ? s : w->lanes[l].stream; };

@@ -41,124 +41,171 @@ __device__ __forceinline__ cplx c_div(cplx x, cplx y) {
     return {__ddiv_rn(__dadd_rn(__dmul_rn(b, ratio), a), denom),
             __ddiv_rn(__dsub_rn(b, __dmul_rn(a, ratio)), denom)};
 }
-__device__ __forceinline__ double c_abs(cplx a) { return hypot(a.re, a.im); }
+// c_abs(a) < 1e-20 (hypot), decided without the square root wherever the larger part alone decides it:
+// max(|re|, |im|) <= hypot <= sqrt(2) max up to rounding.
+__device__ __noinline__ bool hypot_below(cplx a) { return hypot(a.re, a.im) < 1e-20; }
+__device__ __forceinline__ bool c_small(cplx a) {
+    if (fabs(a.re) > 1.001e-20 || fabs(a.im) > 1.001e-20) return false;
+    return hypot_below(a);
+}
+
+// x / y by c_div's steps with shorter chains and no branch.  A quotient a / b comes from the
+// correctly rounded reciprocal y of b, a quotient q within one ulp and its exact residual r = a - b q
+// as fma(r, y, q), which is the correctly rounded quotient, the bits of __ddiv_rn (P. Markstein, IBM
+// J. Res. Dev. 34(1), 1990; y likewise from a reciprocal within one ulp, unless b's significand is
+// all ones).  Both parts share denom's reciprocal, whose first approximation comes from the
+// unrounded ratio, so that it does not wait for the rounded one.  `ok` is cleared, and the result
+// void, unless the divisor's larger part is within 2^-60 .. 2^400 (so it is not c_small), the ratio of
+// its parts and both numerators are at least 2^-300 and finite (no residual underflows; zeros,
+// infinities and NaN are out), its parts differ in their leading words (their order is decided on
+// those) and neither divisor ends in 32 ones.
+__device__ __noinline__ cplx c_div_general(cplx x, cplx y) { return c_div(x, y); }
+__device__ __forceinline__ double rcp_iter(double b) {  // 1 / b within one ulp: a third-order iteration
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    const double e = fma(-b, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ double rcp_step(double b, double y) { return fma(y, fma(-b, y, 1.0), y); }
+// y0 within a few ulp of 1 / b, y its correct rounding
+__device__ __forceinline__ double quotient(double a, double b, double y0, double y) {
+    double q = a * y0;
+    q = fma(fma(-b, q, a), y0, q);
+    return fma(fma(-b, q, a), y, q);
+}
+__device__ __forceinline__ unsigned hi_abs(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
+__device__ __forceinline__ bool exponent_in(double v, unsigned lo, unsigned hi) {  // 2^(lo - 1023) <= |v| < 2^(hi - 1023)
+    return hi_abs(v) - (lo << 20) < ((hi - lo) << 20);
+}
+__device__ __forceinline__ cplx c_div_chain(cplx x, cplx y, bool& ok) {
+    const double a = x.re, b = x.im;
+    const unsigned hre = hi_abs(y.re), him = hi_abs(y.im);
+    const bool swap = hre < him;
+    const double s = swap ? y.re : y.im, big = swap ? y.im : y.re;
+    const double y0 = rcp_iter(big);
+    const double d0 = rcp_iter(fma(s, s * y0, big));  // of denom, to a few ulp
+    const double ratio = quotient(s, big, y0, rcp_step(big, y0));
+    const double denom = __dadd_rn(__dmul_rn(s, ratio), big);
+    const double p = swap ? a : b, q = swap ? b : a;
+    const double nr = __dadd_rn(__dmul_rn(p, ratio), q);
+    const double t = __dmul_rn(q, ratio);
+    const double ni = swap ? __dsub_rn(t, a) : __dsub_rn(b, t);
+    const double d1 = rcp_step(denom, rcp_step(denom, d0));
+    const double re = quotient(nr, denom, d0, d1), im = quotient(ni, denom, d0, d1);
+    ok = ok && hre != him && exponent_in(big, 1023 - 60, 1023 + 400) && exponent_in(ratio, 1023 - 300, 1024) &&
+         exponent_in(nr, 1023 - 300, 1023 + 400) && exponent_in(ni, 1023 - 300, 1023 + 400) &&
+         __double2loint(big) != -1 && __double2loint(denom) != -1;
+    return {re, im};
+}
 
 constexpr int kMaxPade = 128;
 
-// Thiele continued-fraction coefficients (src/gw/pade.cpp:10-63).  Only the previous column
-// of the reference's table g is live, so it is kept as one vector `col` updated in place:
-// after column ip, col[ip] = g(ip, ip) = coeffs[ip].
-__device__ int pade_coeffs(const cplx* __restrict__ x, const cplx* __restrict__ y, int n, int npar, cplx* coeffs,
-                           cplx* xs) {
+// Thiele continued-fraction coefficients (src/gw/pade.cpp:10-63) by one warp: only the previous
+// column of the reference's table g is live, kept as `coeffs` updated in place (lane i holds rows i,
+// i + 32, ...), so after column ip coeffs[ip] = g(ip, ip).  The rows of a column are independent.
+// row: sigma(i omega) as interleaved complex numbers; xs_im: the sample points i * xs_im.
+__device__ int pade_coeffs(const double* __restrict__ row, const double* __restrict__ omega, int n, int npar,
+                           cplx* coeffs, double* xs_im) {
+    const int lane = threadIdx.x & 31;
     const int na = npar < n ? npar : n;
-    if (na == 1) {
-        coeffs[0] = y[0];
-        xs[0] = x[0];
-        return 1;
+    const int step = na > 1 ? n / (na - 1) : 1;
+    for (int i = lane; i < na; i += 32) {
+        const int f = (na > 1 && i == na - 1) ? n - 1 : i * step;
+        xs_im[i] = omega[f];
+        coeffs[i] = {row[2 * f], row[2 * f + 1]};
     }
-    cplx col[kMaxPade];
-    const int step = n / (na - 1);
-    if (step == 0) {
-        for (int i = 0; i < na; ++i) {
-            xs[i] = x[i];
-            col[i] = y[i];
-        }
-    } else {
-        int idat = 0;
-        for (int ip = 0; ip < na - 1; ++ip) {
-            xs[ip] = x[idat];
-            col[ip] = y[idat];
-            idat += step;
-        }
-        xs[na - 1] = x[n - 1];
-        col[na - 1] = y[n - 1];
-    }
-    coeffs[0] = col[0];
+    __syncwarp();
     for (int ip = 1; ip < na; ++ip) {
-        const cplx pivot = col[ip - 1];
-        for (int id = ip; id < na; ++id) {
-            const cplx num = c_sub(pivot, col[id]);
-            const cplx den = c_mul(c_sub(xs[id], xs[ip - 1]), col[id]);
-            col[id] = (c_abs(den) < 1e-20) ? c_div(num, cplx{1e-20, 0.0}) : c_div(num, den);
+        const cplx pivot = coeffs[ip - 1];
+        const cplx x0{0.0, xs_im[ip - 1]};
+        for (int id = ip + lane; id < na; id += 32) {
+            const cplx c = coeffs[id];
+            const cplx num = c_sub(pivot, c);
+            const cplx den = c_mul(c_sub(cplx{0.0, xs_im[id]}, x0), c);
+            bool ok = true;
+            cplx v = c_div_chain(num, den, ok);
+            if (!ok) v = c_div_general(num, c_small(den) ? cplx{1e-20, 0.0} : den);
+            coeffs[id] = v;
         }
-        coeffs[ip] = col[ip];
+        __syncwarp();
     }
     return na;
 }
 
-// Backward evaluation at real z (src/gw/pade.cpp:65-101).
-__device__ cplx pade_eval(const cplx* coeffs, int npar, double z, const cplx* xs) {
-    if (npar == 0) return {0.0, 0.0};
-    if (npar == 1) return coeffs[0];
-    const cplx zt{z, 0.0};
+// Backward evaluation at real z (src/gw/pade.cpp:65-101); num(k) = coeffs[k + 1] (z - xs[k]).  The
+// chain runs through without a branch and is done again step by step if one of its steps was not
+// covered.
+template <class Num>
+__device__ __noinline__ cplx pade_eval_general(cplx first, int npar, Num num) {
     cplx val{1.0, 0.0};
-    for (int kr = npar - 1; kr > 0; --kr) {
-        const int k = kr - 1;
-        const cplx num = c_mul(coeffs[k + 1], c_sub(zt, xs[k]));
-        if (c_abs(val) < 1e-20) val = cplx{1e-20, 0.0};
-        val = c_add(cplx{1.0, 0.0}, c_div(num, val));
+    for (int k = npar - 2; k >= 0; --k) {
+        if (c_small(val)) val = cplx{1e-20, 0.0};
+        val = c_add(cplx{1.0, 0.0}, c_div(num(k), val));
     }
-    if (c_abs(val) < 1e-20) return c_div(coeffs[0], cplx{1e-20, 0.0});
-    return c_div(coeffs[0], val);
+    return c_div(first, c_small(val) ? cplx{1e-20, 0.0} : val);
+}
+template <class Num>
+__device__ __forceinline__ cplx pade_eval(cplx first, int npar, Num num) {
+    if (npar == 1) return first;
+    // the innermost step divides by exactly 1: c_div(x, 1) is x + 0 componentwise
+    const cplx inner = num(npar - 2);
+    cplx val = c_add(cplx{1.0, 0.0}, cplx{__dadd_rn(__dmul_rn(inner.im, 0.0), inner.re),
+                                          __dsub_rn(inner.im, __dmul_rn(inner.re, 0.0))});
+    bool ok = true;
+#pragma unroll 2
+    for (int k = npar - 3; k >= 0; --k) val = c_add(cplx{1.0, 0.0}, c_div_chain(num(k), val, ok));
+    val = c_div_chain(first, val, ok);
+    return ok ? val : pade_eval_general(first, npar, num);
+}
+__device__ __forceinline__ cplx pade_num(const cplx* coeffs, const double* xs_im, double z, int k) {
+    return c_mul(coeffs[k + 1], c_sub(cplx{z, 0.0}, cplx{0.0, xs_im[k]}));
 }
 
-// One thread per requested state: Pade fit of Sigma_c(p, iw) and the fixed-point QP update
-// (src/gw/qp_solver.cpp:18-43), <= 200 iterations, tolerance 1e-6.
-__global__ void k_qp(const double* __restrict__ sigma, const double* __restrict__ omega, int nfreq, int nmo,
-                     const int64_t* __restrict__ states, int nstates, int npade, const double* __restrict__ mo,
-                     double fermi, const double* __restrict__ sigx, const double* __restrict__ vxc_diag,
-                     double* __restrict__ qp, cplx* __restrict__ scratch) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nstates) return;
-    const int p = (int)states[s];
-    cplx* x = scratch + (size_t)s * 2 * nfreq;
-    cplx* y = x + nfreq;
-    for (int f = 0; f < nfreq; ++f) {
-        x[f] = {0.0, omega[f]};
-        y[f] = {sigma[2 * ((size_t)p * nfreq + f)], sigma[2 * ((size_t)p * nfreq + f) + 1]};
-    }
-    cplx coeffs[kMaxPade], xs[kMaxPade];
-    const int na = pade_coeffs(x, y, nfreq, npade, coeffs, xs);
-    const double e = mo[p];
+// One warp per requested state: Pade fit of Sigma_c(p, iw) and the fixed-point QP update
+// (src/gw/qp_solver.cpp:18-43), <= 200 iterations, tolerance 1e-6.  Bound by the chain of the
+// evaluations (a state that does not settle takes all 200); the numerators of an evaluation do not
+// depend on each other and are formed by the lanes before it.  60 states, 16 parameters, 100
+// frequencies: 441 us (1347 us with one thread per state, __ddiv_rn and hypot at every step).
+__global__ void __launch_bounds__(32) k_qp(const double* __restrict__ sigma, const double* __restrict__ omega,
+                                           int nfreq, const int64_t* __restrict__ states, int npade,
+                                           const double* __restrict__ mo, double fermi, const double* __restrict__ sigx,
+                                           const double* __restrict__ vxc_diag, double* __restrict__ qp) {
+    __shared__ cplx coeffs[kMaxPade], num[kMaxPade];
+    __shared__ double xs_im[kMaxPade];
+    const int lane = threadIdx.x;
+    const int p = (int)states[blockIdx.x];
+    const int na = pade_coeffs(sigma + 2 * (size_t)p * nfreq, omega, nfreq, npade, coeffs, xs_im);
+    const double e = mo[p], sx = sigx[p], vx = vxc_diag[p];
+    const cplx first = coeffs[0];
     double cur = e;
     for (int it = 0; it < 200; ++it) {
         const double target = __dsub_rn(cur, fermi);
-        const cplx sc = pade_eval(coeffs, na, target, xs);
-        const double nq = __dsub_rn(__dadd_rn(__dadd_rn(e, sc.re), sigx[p]), vxc_diag[p]);
-        if (fabs(__dsub_rn(nq, cur)) < 1e-6) {
-            cur = nq;
-            break;
-        }
+        for (int k = lane; k < na - 1; k += 32) num[k] = pade_num(coeffs, xs_im, target, k);
+        __syncwarp();
+        const cplx sc = pade_eval(first, na, [&](int k) { return num[k]; });
+        __syncwarp();
+        const double nq = __dsub_rn(__dadd_rn(__dadd_rn(e, sc.re), sx), vx);
+        const bool done = fabs(__dsub_rn(nq, cur)) < 1e-6;
         cur = nq;
+        if (done) break;
     }
-    qp[p] = cur;
+    if (lane == 0) qp[p] = cur;
 }
 
 // E_c.out sweep (src/io.cpp:94-108): coefficients once per block, one point per thread.
-__global__ void k_pade_sweep(const double* __restrict__ sigma_row, const double* __restrict__ omega, int nfreq,
-                             int npade, int npts, double fermi, double x_start, double interval,
-                             double* __restrict__ out, cplx* __restrict__ scratch) {
-    __shared__ cplx coeffs_s[kMaxPade], xs_s[kMaxPade];
-    __shared__ int na_s;
-    if (threadIdx.x == 0) {
-        cplx* x = scratch + (size_t)blockIdx.x * 2 * nfreq;
-        cplx* y = x + nfreq;
-        for (int f = 0; f < nfreq; ++f) {
-            x[f] = {0.0, omega[f]};
-            y[f] = {sigma_row[2 * f], sigma_row[2 * f + 1]};
-        }
-        cplx coeffs[kMaxPade], xs[kMaxPade];
-        const int na = pade_coeffs(x, y, nfreq, npade, coeffs, xs);
-        for (int i = 0; i < na; ++i) {
-            coeffs_s[i] = coeffs[i];
-            xs_s[i] = xs[i];
-        }
-        na_s = na;
-    }
+__global__ void __launch_bounds__(128) k_pade_sweep(const double* __restrict__ sigma_row,
+                                                    const double* __restrict__ omega, int nfreq, int npade, int npts,
+                                                    double fermi, double x_start, double interval,
+                                                    double* __restrict__ out) {
+    __shared__ cplx coeffs[kMaxPade];
+    __shared__ double xs_im[kMaxPade];
+    const int na = npade < nfreq ? npade : nfreq;
+    if (threadIdx.x < 32) pade_coeffs(sigma_row, omega, nfreq, npade, coeffs, xs_im);
     __syncthreads();
+    const cplx first = coeffs[0];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npts; i += gridDim.x * blockDim.x) {
         const double e = __dsub_rn(__dadd_rn(x_start, __dmul_rn((double)i, interval)), fermi);
-        const cplx v = pade_eval(coeffs_s, na_s, e, xs_s);
+        const cplx v = pade_eval(first, na, [&](int k) { return pade_num(coeffs, xs_im, e, k); });
         out[3 * (size_t)i + 0] = __dmul_rn(__dadd_rn(e, fermi), 27.211386245988);
         out[3 * (size_t)i + 1] = v.re;
         out[3 * (size_t)i + 2] = v.im;
@@ -252,27 +299,20 @@ int launch_fill(double* p, double v, int64_t n, cudaStream_t s) {
     return 1;
 }
 
-size_t qp_scratch_bytes(int64_t nfreq, int64_t nstates) { return 2 * sizeof(cplx) * (size_t)nfreq * (size_t)nstates; }
-
-int launch_qp(const double* sigma, const double* omega, int64_t nfreq, int64_t nmo, const int64_t* states,
-              int64_t nstates, int64_t npade, const double* mo, double fermi, const double* sigx,
-              const double* vxc_diag, double* qp, void* scratch, cudaStream_t s) {
+int launch_qp(const double* sigma, const double* omega, int64_t nfreq, const int64_t* states, int64_t nstates,
+              int64_t npade, const double* mo, double fermi, const double* sigx, const double* vxc_diag, double* qp,
+              cudaStream_t s) {
     if (npade > kMaxPade) fail(GWB200_BAD_SHAPE, "npade exceeds the device Pade limit of 128");
-    k_qp<<<(unsigned)((nstates + 63) / 64), 64, 0, s>>>(sigma, omega, (int)nfreq, (int)nmo, states, (int)nstates,
-                                                         (int)npade, mo, fermi, sigx, vxc_diag, qp,
-                                                         static_cast<cplx*>(scratch));
+    k_qp<<<(unsigned)nstates, 32, 0, s>>>(sigma, omega, (int)nfreq, states, (int)npade, mo, fermi, sigx, vxc_diag, qp);
     GWB_LAUNCH("k_qp");
     return 1;
 }
 
-int pade_sweep_blocks(int64_t npts) { return (int)std::min<int64_t>((npts + 255) / 256, 148); }
-
 int launch_pade_sweep(const double* sigma_row, const double* omega, int64_t nfreq, int64_t npade, int64_t npts,
-                      double fermi, double x_start, double interval, double* out, void* scratch, cudaStream_t s) {
+                      double fermi, double x_start, double interval, double* out, cudaStream_t s) {
     if (npade > kMaxPade) fail(GWB200_BAD_SHAPE, "npade exceeds the device Pade limit of 128");
-    k_pade_sweep<<<(unsigned)pade_sweep_blocks(npts), 256, 0, s>>>(sigma_row, omega, (int)nfreq, (int)npade,
-                                                                   (int)npts, fermi, x_start, interval, out,
-                                                                   static_cast<cplx*>(scratch));
+    k_pade_sweep<<<(unsigned)std::min<int64_t>((npts + 127) / 128, 8 * 148), 128, 0, s>>>(
+        sigma_row, omega, (int)nfreq, (int)npade, (int)npts, fermi, x_start, interval, out);
     GWB_LAUNCH("k_pade_sweep");
     return 1;
 }
