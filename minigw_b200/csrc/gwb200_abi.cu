@@ -128,7 +128,7 @@ struct gwb200_handle {
     bool complex_forms = false;  // the last compute_forms ran the eta != 0 (complex) path
     DevBuf pqo, xdiag, mo, vxc_diag, delta, v, sigx, flag;  // pqo: the (pq|o.) block of the ERI
     // per-call workspaces (grow-only, reused across calls)
-    DevBuf xt, dvec, a, linv, qacc, qall, sigma, omega, weight, states, err, qp, omega_out;
+    DevBuf xt, dvec, a, qacc, qall, sigma, omega, weight, states, err, qp, omega_out;
     DevBuf panel32;   // operand workspace of the tcgen05 trailing updates (mixed: FP32 hi/lo split;
                       // plain with GWB200_FP64_UPDATE=ozaki: int8 digit slices + exponents)
     DevBuf tc_sched;  // work counter of the tcgen05 update kernel
@@ -332,7 +332,7 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
     }
     GWB_CUDA(cudaMemsetAsync(h->err.p, 0xFF, sizeof(unsigned long long), s));
 
-    // Frequency chunk size from the HBM budget: tall matrices + scale vectors (+ 64x64 inverses: complex form).
+    // Frequency chunk size from the HBM budget: tall matrices, scale vectors, accumulators, operands.
     const bool mixed_tc = mixed && mixed_update_on_tcgen05(h);
     // plain form: the int8 emulation of the outer updates is a candidate of the update autotuner
     // (its slice workspace is part of the budget) unless GWB200_FP64_UPDATE=dmma; memory-capped
@@ -348,7 +348,7 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
     const size_t per_freq = mixed ? sizeof(float) * (size_t)g.stride + sizeof(double) * (g.n_pad + g.m_pad) +
                                         (mixed_tc ? tc_panel_bytes_per_freq(g) : 0) +
                                         (refine ? refine_bytes_per_freq(g, r_pad) : 0)
-                                  : sizeof(double) * planes * ((size_t)g.stride + g.n_pad + (cplx ? kNb * kNb : 0) + g.m_pad) +
+                                  : sizeof(double) * planes * ((size_t)g.stride + g.n_pad + g.m_pad) +
                                         (fp64_oz ? oz_slice_bytes_per_freq(g) : 0);
     // GWB200_MAX_FREQ_CHUNK caps the chunk (tests use it to exercise the multi-chunk path).
     int64_t cap = 0;
@@ -361,7 +361,7 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
         size_t free_b = 0, total_b = 0;
         GWB_CUDA(cudaMemGetInfo(&free_b, &total_b));
         const size_t have =
-            h->a.bytes + h->dvec.bytes + h->linv.bytes + h->qacc.bytes + h->panel32.bytes + h->refine.bytes;
+            h->a.bytes + h->dvec.bytes + h->qacc.bytes + h->panel32.bytes + h->refine.bytes;
         size_t avail = free_b + have;  // what the chunk buffers may occupy
         size_t budget = (size_t)((double)avail * 0.85);
         if (h->mem_limit > 0) {  // the handle's cap minus what the system and panels already hold
@@ -381,7 +381,6 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
     }
     size_buffer(h, h->a, (mixed ? sizeof(float) : sizeof(double) * planes) * (size_t)fc * g.stride);
     size_buffer(h, h->dvec, sizeof(double) * planes * (size_t)fc * g.n_pad);
-    if (cplx) size_buffer(h, h->linv, sizeof(double) * planes * (size_t)fc * kNb * kNb);
     size_buffer(h, h->qacc, sizeof(double) * planes * (size_t)fc * g.m_pad);
     if (mixed_tc) {
         size_buffer(h, h->panel32, tc_panel_bytes_per_freq(g) * (size_t)fc);
@@ -416,7 +415,7 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
             double* a_re = h->a.as<double>();
             launches += launch_factor_chunk_c(g, nf, h->delta.as<double>(), h->omega.as<double>() + f0, eta,
                                               h->v.as<double>(), h->xt.as<double>(), a_re, a_re + (size_t)nf * g.stride,
-                                              h->dvec.as<double>(), h->linv.as<double>(), h->qacc.as<double>(),
+                                              h->dvec.as<double>(), h->qacc.as<double>(),
                                               h->err.as<unsigned long long>(), s);
             launches += launch_forms_out_c(h->qacc.as<double>(), nf, m, g.m_pad,
                                            h->qall.as<double>() + f0 * 2 * g.m_pad, g.m_pad, s);
@@ -749,7 +748,7 @@ int gwb200_destroy(gwb200_handle* h) {
     h->stage_in.release();
     h->stage_out.release();
     for (DevBuf* b : {&h->pchol, &h->pchol_sl, &h->refine, &h->pqo, &h->xdiag, &h->mo, &h->vxc_diag, &h->delta, &h->v, &h->sigx, &h->flag, &h->xt, &h->dvec, &h->a,
-                      &h->linv, &h->qacc, &h->qall, &h->sigma, &h->omega, &h->weight, &h->states, &h->err, &h->qp,
+                      &h->qacc, &h->qall, &h->sigma, &h->omega, &h->weight, &h->states, &h->err, &h->qp,
                       &h->sweep, &h->omega_out, &h->panel32, &h->tc_sched, &h->batch_desc, &h->qx, &h->sigmx})
         b->release();
     for (BatchLane& l : h->lanes) {
@@ -828,7 +827,7 @@ void load_system_impl(gwb200_handle* h, int64_t nmo, int64_t nocc, const double*
     const size_t nmo2 = (size_t)nmo * nmo;
     const int64_t nvir = nmo - nocc, n = nocc * nvir;
     if (h->mem_limit > 0)  // drop the previous request's workspaces before sizing this system
-        for (DevBuf* b : {&h->xt, &h->dvec, &h->a, &h->linv, &h->qacc, &h->qall, &h->panel32, &h->pchol, &h->pchol_sl,
+        for (DevBuf* b : {&h->xt, &h->dvec, &h->a, &h->qacc, &h->qall, &h->panel32, &h->pchol, &h->pchol_sl,
                           &h->refine, &h->qx, &h->sigmx})
             b->release();
     if (bound) {
@@ -1256,7 +1255,7 @@ size_t batch_avail(const gwb200_handle* w) {
     if (w->mem_limit > 0) {
         size_t resident = (size_t)1 << 20;
         for (const DevBuf* b : {&w->pqo, &w->xdiag, &w->v, &w->xt, &w->dvec, &w->qall, &w->sigma, &w->a,
-                                &w->linv, &w->qacc, &w->panel32})
+                                &w->qacc, &w->panel32})
             resident += b->bytes;
         const size_t lim = (size_t)w->mem_limit;
         avail = std::min(avail, lim > resident ? lim - resident : (size_t)0);

@@ -250,10 +250,10 @@ int launch_update32_tc(const TallGeometry& g, int64_t nf, float* a, int64_t c_be
                        unsigned long long* sched, unsigned long long* err_pivot, cudaStream_t s, int max_ctas = 0,
                        int64_t row_min = 0);
 // kernels_c64.cu: eta != 0 (complex symmetric M = I - S V S, S = diag(Pi0)^1/2).  Planes a_re/a_im
-// of geometry g; svec 2*n_pad, linv 2*64*64, qacc 2*m_pad doubles per frequency.
+// of geometry g; svec 2*n_pad, qacc 2*m_pad doubles per frequency.
 int launch_factor_chunk_c(const TallGeometry& g, int64_t nf, const double* delta, const double* omega, double eta,
-                          const double* v, const double* xt, double* a_re, double* a_im, double* svec, double* linv,
-                          double* qacc, unsigned long long* err_pivot, cudaStream_t s);
+                          const double* v, const double* xt, double* a_re, double* a_im, double* svec, double* qacc,
+                          unsigned long long* err_pivot, cudaStream_t s);
 int launch_forms_out_c(const double* qacc, int64_t nf, int64_t m, int64_t ldq, double* q_out, int64_t ldq_out,
                        cudaStream_t s);
 int launch_sigma_contract_c(const double* qall, int64_t nf_int, int64_t nstates, int64_t nmo, int64_t ldq,
@@ -273,7 +273,7 @@ struct BatchGroup {
 int launch_build_tall_batch(const TallGeometry& g, const BatchGroup* groups, int64_t ngroups, bool fp32, void* a,
                             cudaStream_t s);
 int launch_forms_scatter(const BatchGroup* groups, int64_t ngroups, const double* qacc, int64_t ldq, cudaStream_t s);
-// device bytes of one batched matrix (tall matrix, 64x64 inverse, scale vector, norm accumulators,
+// device bytes of one batched matrix (tall matrix, scale vector, norm accumulators,
 // tcgen05 / int8 operand workspace)
 size_t batch_bytes_per_matrix(const TallGeometry& g, bool mixed, bool fp64_oz, bool refine = false);
 // bucket sizes over the molecules sorted by (n, m): minimises block-step latency + padded work

@@ -10,46 +10,12 @@
 // non-finite one is reported like the real path's non-positive pivot.  Every complex tile product
 // is four FP64 DMMA tile products on separate real and imaginary planes.  At eta = 0 this path
 // gives the real path's numbers (S = i D^1/2); the real path is used there.
-#include "internal.cuh"
+#include "panel_common.cuh"
 
 #include <cmath>
 
 namespace gwb200 {
 namespace {
-
-__device__ __forceinline__ void dmma_8x8x4c(double (&c)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                 : "+d"(c[0]), "+d"(c[1])
-                 : "d"(a), "d"(b));
-}
-
-// acc += sgn * As(64x64) * Bs(64x64)^T from shared memory (stride kLds); same warp layout as the
-// real path: warp w owns rows 16*(w/2)..+15, cols 32*(w%2)..+31.
-__device__ __forceinline__ void tile_mma_c(const double* __restrict__ As, const double* __restrict__ Bs,
-                                           double (&acc)[2][4][2], double sgn) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    const int r0 = 16 * (w >> 1), c0 = 32 * (w & 1);
-#pragma unroll 4
-    for (int kk = 0; kk < kNb; kk += 4) {
-        double af[2], bf[4];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) af[i] = sgn * As[(r0 + 8 * i + g) * kLds + kk + t];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bf[j] = Bs[(c0 + 8 * j + g) * kLds + kk + t];
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) dmma_8x8x4c(acc[i][j], af[i], bf[j]);
-    }
-}
-
-__device__ __forceinline__ void load_tile_c(double* __restrict__ s, const double* __restrict__ gsrc, int64_t ld) {
-    for (int idx = threadIdx.x; idx < 64 * 32; idx += blockDim.x) {
-        const int r = idx >> 5, c2 = idx & 31;
-        *reinterpret_cast<double2*>(s + r * kLds + 2 * c2) = *reinterpret_cast<const double2*>(gsrc + (size_t)r * ld + 2 * c2);
-    }
-}
 
 // principal square root of x + i y
 __device__ __forceinline__ void csqrt_dev(double x, double y, double& sr, double& si) {
@@ -124,205 +90,482 @@ __global__ void k_build_tall_c(int64_t n, int64_t m, int64_t n_pad, int64_t ld, 
     }
 }
 
-// Complex 64x64 diagonal block: L L^T (no conjugation) in shared memory, then L^{-1}.
-__global__ void __launch_bounds__(256) k_potrf_diag_c(double* __restrict__ a_re, double* __restrict__ a_im, int64_t ld,
-                                                      int64_t stride, int64_t k, double* __restrict__ linv,
-                                                      unsigned long long* err_pivot) {
-    extern __shared__ double smem[];
-    constexpr int L = kNb + 1;
-    double* Tr = smem;
-    double* Ti = Tr + kNb * L;
-    double* Yr = Ti + kNb * L;
-    double* Yi = Yr + kNb * L;
-    double* Ar = a_re + (size_t)blockIdx.x * stride + k * ld + k;
-    double* Ai = a_im + (size_t)blockIdx.x * stride + k * ld + k;
-    const int tid = threadIdx.x;
-    for (int idx = tid; idx < kNb * kNb; idx += blockDim.x) {
-        const int i = idx / kNb, j = idx % kNb;
-        Tr[i * L + j] = (j <= i) ? Ar[(size_t)i * ld + j] : 0.0;
-        Ti[i * L + j] = (j <= i) ? Ai[(size_t)i * ld + j] : 0.0;
+// ---------------------------------------------------------------------------------------------
+// Diagonal block, as in panel_common.cuh with complex entries: [A ; I] in 16-wide panels, the
+// panel's 16 rows and 16 identity rows in one warp's registers, four columns per exchange; both
+// planes of the 64-wide block share L (below) and the identity rows (column c at [r][c + 1]).
+// Within a panel the columns stay unscaled (L D L^T): the chain takes 1 / d per pivot, and the
+// square roots of the 16 pivots are taken at its end, one per lane.  (A complex pivot step with
+// barriers and divisions per column and the inverse by substitution: 165 us per 64 columns.)
+
+constexpr int kLdc = kNb + 4;
+constexpr int kPlane = kNb * kLdc;
+constexpr int kCWork = 2 * 2 * 16 * panel::kWtLd + 2 * 2 * 64 + 2 * 16 + 2 * 16;  // doubles
+
+struct cd {
+    double r, i;
+};
+__device__ __forceinline__ cd operator*(cd a, cd b) { return {fma(a.r, b.r, -(a.i * b.i)), fma(a.r, b.i, a.i * b.r)}; }
+__device__ __forceinline__ void sub_prod(cd& c, cd a, cd b) {  // c -= a b
+    c.r = fma(a.i, b.i, fma(-a.r, b.r, c.r));
+    c.i = fma(-a.i, b.r, fma(-a.r, b.i, c.i));
+}
+__device__ __forceinline__ cd ld2(const double* p) {
+    const double2 v = *reinterpret_cast<const double2*>(p);
+    return {v.x, v.y};
+}
+__device__ __forceinline__ void st2(double* p, cd v) { *reinterpret_cast<double2*>(p) = make_double2(v.r, v.i); }
+
+// 1 / d.  kPlain: conj(d) / |d|^2 with |d|^2's reciprocal from a third-order iteration; a pivot whose
+// larger part is outside 2^-400 .. 2^400 clears the result's validity through `bad` and the caller
+// starts over without kPlain: there a pivot of modulus <= 1e-300 or a non-finite one is recorded in
+// `bad` and counts as 1, and the division is scaled.
+template <bool kPlain>
+__device__ __forceinline__ cd pivot_inverse(cd& d, int j, unsigned& bad) {
+    if (kPlain) {
+        const unsigned h = max((unsigned)__double2hiint(d.r) & 0x7fffffffu, (unsigned)__double2hiint(d.i) & 0x7fffffffu);
+        bad |= (unsigned)!(h - ((1023u - 400u) << 20) < (800u << 20));
+        const double m = fma(d.r, d.r, d.i * d.i);
+        double y;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(m));
+        const double e = fma(-m, y, 1.0);
+        y = fma(y, fma(e, e, e), y);
+        return {d.r * y, -d.i * y};
     }
-    __syncthreads();
-    for (int j = 0; j < kNb; ++j) {
-        if (tid == 0) {
-            double xr = Tr[j * L + j], xi = Ti[j * L + j];
-            const double mod = hypot(xr, xi);
-            if (!(mod > 1e-300) || !isfinite(mod)) {
-                atomicMin(err_pivot, (unsigned long long)(k + j + 1));
-                xr = 1.0;
-                xi = 0.0;
+    const double mod = hypot(d.r, d.i);
+    if (!(mod > 1e-300) || !isfinite(mod)) {
+        bad |= 1u << j;
+        d = {1.0, 0.0};
+        return d;
+    }
+    return {d.r / mod / mod, -(d.i / mod / mod)};
+}
+
+template <bool kPlain>
+__device__ __forceinline__ unsigned factor_rows16c(const double* __restrict__ Sr, const double* __restrict__ Si,
+                                                   cd (&x)[16], double* __restrict__ rows2, double* __restrict__ piv,
+                                                   double* __restrict__ scale, int c0) {
+    const int lane = threadIdx.x & 31, r = lane & 15;
+    const bool ident = lane >= 16;
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+        x[c] = {ident && c == r ? 1.0 : 0.0, 0.0};
+        if (!ident && c <= r) x[c] = {Sr[(c0 + r) * kLdc + c0 + c], Si[(c0 + r) * kLdc + c0 + c]};
+    }
+    unsigned bad = 0;
+    cd xt[4] = {};      // this lane's row of the last four columns times 1 / d
+    cd mine = {1.0, 0.0};  // pivot r
+#pragma unroll
+    for (int q = 0; q < 16; q += 4) {
+        if (!ident && (r >> 2) == (q >> 2))
+#pragma unroll
+            for (int c = 0; c < 4; ++c) st2(piv + 8 * (r & 3) + 2 * c, x[q + c]);
+        __syncwarp();
+        if (q > 0) {  // the previous four columns' update of the columns behind this block
+            const double* rows = rows2 + ((q >> 2) & 1 ? 0 : 128);
+#pragma unroll
+            for (int c = q + 4; c < 16; ++c)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) sub_prod(x[c], xt[j], ld2(rows + 8 * c + 2 * j));
+        }
+        cd l[4][4], inv[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int c = 0; c <= i; ++c) l[i][c] = ld2(piv + 8 * i + 2 * c);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            inv[j] = pivot_inverse<kPlain>(l[j][j], q + j, bad);
+            if (r == q + j) mine = l[j][j];
+#pragma unroll
+            for (int i = j + 1; i < 4; ++i) {
+                const cd t = l[i][j] * inv[j];
+#pragma unroll
+                for (int c = j + 1; c <= i; ++c) sub_prod(l[i][c], t, l[c][j]);
             }
-            double sr, si;
-            csqrt_dev(xr, xi, sr, si);
-            Tr[j * L + j] = sr;
-            Ti[j * L + j] = si;
         }
-        __syncthreads();
-        const double dr = Tr[j * L + j], di = Ti[j * L + j];
-        const double dn = dr * dr + di * di;
-        for (int i = j + 1 + tid; i < kNb; i += blockDim.x) {  // a_ij / d
-            const double xr = Tr[i * L + j], xi = Ti[i * L + j];
-            Tr[i * L + j] = (xr * dr + xi * di) / dn;
-            Ti[i * L + j] = (xi * dr - xr * di) / dn;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {  // this lane's row against the block
+#pragma unroll
+            for (int c = 0; c < j; ++c) sub_prod(x[q + j], xt[c], l[j][c]);
+            if (!ident && r == q + j) x[q + j] = l[j][j];
+            xt[j] = x[q + j] * inv[j];
         }
-        __syncthreads();
-        const int rem = kNb - 1 - j;
-        for (int idx = tid; idx < rem * rem; idx += blockDim.x) {
-            const int i = j + 1 + idx / rem, l = j + 1 + idx % rem;
-            if (l <= i) {
-                const double ar = Tr[i * L + j], ai = Ti[i * L + j], br = Tr[l * L + j], bi = Ti[l * L + j];
-                Tr[i * L + l] -= ar * br - ai * bi;
-                Ti[i * L + l] -= ar * bi + ai * br;
+        if (q < 12) {  // these columns of the block's rows, and their update of the next four columns
+            double* rows = rows2 + ((q >> 2) & 1 ? 128 : 0);
+            if (!ident)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) st2(rows + 8 * r + 2 * j, x[q + j]);
+            __syncwarp();
+#pragma unroll
+            for (int c = q + 4; c < q + 8; ++c)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) sub_prod(x[c], xt[j], ld2(rows + 8 * c + 2 * j));
+        }
+    }
+    // columns scaled by 1 / sqrt(d) (either root: only L L^T matters)
+    cd s;
+    csqrt_dev(mine.r, mine.i, s.r, s.i);
+    unsigned none = 0;
+    s = pivot_inverse<false>(s, 0, none);
+    if (!ident) st2(scale + 2 * r, s);
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < 16; ++c) x[c] = x[c] * ld2(scale + 2 * c);
+    return bad;
+}
+
+// The block in Sr / Si (lower triangle, zeros above) -> transposed inverse, L^{-1}[c][r] at
+// [r][c + 1]; as panel::factor_diag.  256 threads, after a barrier; ends with a barrier.
+__device__ void factor_diag_c(double* __restrict__ Sr, double* __restrict__ Si, double* __restrict__ work, int64_t k0,
+                              unsigned long long* err) {
+    constexpr int kWarps = 8;
+    constexpr int WL = panel::kWtLd, kW = 16 * WL;
+    double* rows2 = work;
+    double* piv = rows2 + 2 * 128;
+    double* scale = piv + 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    for (int c0 = 0; c0 < kNb; c0 += 16) {
+        double* Wr = scale + 32 + (c0 & 16 ? 2 * kW : 0);  // [c][r] of the panel's inverse, two buffers
+        double* Wi = Wr + kW;
+        if (warp == 0) {
+            cd x[16];
+            unsigned bad = factor_rows16c<true>(Sr, Si, x, rows2, piv, scale, c0);
+            if (bad) {
+                __syncwarp();
+                bad = factor_rows16c<false>(Sr, Si, x, rows2, piv, scale, c0);
             }
-        }
-        __syncthreads();
-    }
-    for (int idx = tid; idx < kNb * kNb; idx += blockDim.x) {
-        const int i = idx / kNb, j = idx % kNb;
-        if (j <= i) {
-            Ar[(size_t)i * ld + j] = Tr[i * L + j];
-            Ai[(size_t)i * ld + j] = Ti[i * L + j];
-        }
-    }
-    if (tid < kNb) {  // forward substitution, one column of L^{-1} per thread
-        const int col = tid;
-        for (int i = 0; i < kNb; ++i) {
-            double yr, yi;
-            if (i < col) {
-                yr = yi = 0.0;
-            } else {
-                double sr = (i == col) ? 1.0 : 0.0, si = 0.0;
-                for (int l = col; l < i; ++l) {
-                    sr -= Tr[i * L + l] * Yr[l * L + col] - Ti[i * L + l] * Yi[l * L + col];
-                    si -= Tr[i * L + l] * Yi[l * L + col] + Ti[i * L + l] * Yr[l * L + col];
+            if (bad && lane == 0) atomicMin(err, (unsigned long long)(k0 + c0 + __ffs(bad)));
+            if (lane >= 16)
+#pragma unroll
+                for (int c = 0; c < 16; ++c) {
+                    Wr[c * WL + lane - 16] = x[c].r;
+                    Wi[c * WL + lane - 16] = x[c].i;
                 }
-                const double dr = Tr[i * L + i], di = Ti[i * L + i], dn = dr * dr + di * di;
-                yr = (sr * dr + si * di) / dn;
-                yi = (si * dr - sr * di) / dn;
+        }
+        __syncthreads();
+        // the panel's other rows (A below, identity above): X <- X L_p^{-T}
+        constexpr int kRowTiles = (kNb - 16) / 8;
+        if (warp < kRowTiles) {
+            const bool below = 8 * warp >= c0;
+            const int off = ((below ? 8 * warp + 16 : 8 * warp) + g) * kLdc + c0 + (below ? 0 : 1);
+            double ar[2][2] = {}, ai[2][2] = {};
+            double xr[4], xi[4];
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+                xr[kk] = Sr[off + 4 * kk + t];
+                xi[kk] = Si[off + 4 * kk + t];
             }
-            Yr[i * L + col] = yr;
-            Yi[i * L + col] = yi;
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const double br = Wr[(8 * h + g) * WL + 4 * kk + t], bi = Wi[(8 * h + g) * WL + 4 * kk + t];
+                    panel::dmma(ar[h], xr[kk], br);
+                    panel::dmma(ai[h], xr[kk], bi);
+                    panel::dmma(ar[h], -xi[kk], bi);
+                    panel::dmma(ai[h], xi[kk], br);
+                }
+            __syncwarp();
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    Sr[off + 8 * h + 2 * t + e] = ar[h][e];
+                    Si[off + 8 * h + 2 * t + e] = ai[h][e];
+                }
+        } else if (warp == kWarps - 1 && lane < 16) {  // the panel's own identity rows
+#pragma unroll
+            for (int c = 0; c < 16; ++c)
+                if (c >= lane) {
+                    Sr[(c0 + lane) * kLdc + c0 + c + 1] = Wr[c * WL + lane];
+                    Si[(c0 + lane) * kLdc + c0 + c + 1] = Wi[c * WL + lane];
+                }
+        }
+        __syncthreads();
+        // trailing columns, 16 x 16 tile groups: X -= X_p (row c of L_p)^T
+        const int c1 = c0 + 16;
+        const int ng = (kNb - c1) / 16, n_low = ng * (ng + 1) / 2, n_all = n_low + (c1 / 16) * ng;
+        auto group = [&](int row, int col, int shift, const double* Xr, const double* Xi, int rs, int ks) {
+            double br[2][4], bi[2][4];
+#pragma unroll
+            for (int v = 0; v < 2; ++v)
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) {
+                    br[v][kk] = Sr[(col + 8 * v + g) * kLdc + c0 + 4 * kk + t];
+                    bi[v][kk] = Si[(col + 8 * v + g) * kLdc + c0 + 4 * kk + t];
+                }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                double ar[2][2], ai[2][2];
+                const int off = (row + 8 * h + g) * kLdc + col + 2 * t + shift;
+#pragma unroll
+                for (int v = 0; v < 2; ++v)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        ar[v][e] = Sr[off + 8 * v + e];
+                        ai[v][e] = Si[off + 8 * v + e];
+                    }
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) {
+                    const int at = (8 * h + g) * rs + (4 * kk + t) * ks;
+                    const double xr = Xr[at], xi = Xi[at];
+#pragma unroll
+                    for (int v = 0; v < 2; ++v) {
+                        panel::dmma(ar[v], -xr, br[v][kk]);
+                        panel::dmma(ai[v], -xr, bi[v][kk]);
+                        panel::dmma(ar[v], xi, bi[v][kk]);
+                        panel::dmma(ai[v], -xi, br[v][kk]);
+                    }
+                }
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    if (row == col && v > h) continue;  // above the diagonal: identity columns live there
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        Sr[off + 8 * v + e] = ar[v][e];
+                        Si[off + 8 * v + e] = ai[v][e];
+                    }
+                }
+            }
+        };
+        auto group_low = [&](int row, int col) {
+            group(row, col, 0, Sr + row * kLdc + c0, Si + row * kLdc + c0, kLdc, 1);
+        };
+        if (ng > 0) {
+            if (warp == 0) {  // the next panel's diagonal block, then on to factoring it
+                group_low(c1, c1);
+                __syncwarp();
+            } else if (warp & 3) {  // the warps that share warp 0's FP64 pipe stay out of its way
+                for (int x = warp - (warp >> 2); x < n_all; x += kWarps - kWarps / 4) {
+                    if (x < n_low) {
+                        int gi = 0, base = 0;
+                        while (base + gi + 1 <= x) base += ++gi;
+                        group_low(c1 + 16 * gi, c1 + 16 * (x - base));
+                    } else {
+                        const int y = x - n_low, row = 16 * (y / ng), col = c1 + 16 * (y % ng);
+                        const int at = row * kLdc + c0 + 1;
+                        if (row < c0)
+                            group(row, col, 1, Sr + at, Si + at, kLdc, 1);
+                        else  // this panel's own identity rows, from the zero-filled copy
+                            group(row, col, 1, Wr, Wi, 1, WL);
+                    }
+                }
+            }
         }
     }
     __syncthreads();
-    double* out = linv + (size_t)blockIdx.x * 2 * kNb * kNb;
-    for (int idx = tid; idx < kNb * kNb; idx += blockDim.x) {
-        out[idx] = Yr[(idx / kNb) * L + idx % kNb];
-        out[kNb * kNb + idx] = Yi[(idx / kNb) * L + idx % kNb];
+}
+
+__global__ void __launch_bounds__(256) k_diag_c(double* __restrict__ a_re, double* __restrict__ a_im, int64_t ld,
+                                                int64_t stride, int64_t k, unsigned long long* err_pivot) {
+    extern __shared__ __align__(16) double smem[];
+    double* Sr = smem;
+    double* Si = Sr + kPlane;
+    const size_t base = (size_t)blockIdx.x * stride + k * ld + k;
+    for (int idx = threadIdx.x; idx < kPlane; idx += 256) {
+        const int i = idx / kLdc, j = idx % kLdc;
+        Sr[idx] = j <= i ? a_re[base + (size_t)i * ld + j] : 0.0;
+        Si[idx] = j <= i ? a_im[base + (size_t)i * ld + j] : 0.0;
+    }
+    __syncthreads();
+    factor_diag_c(Sr, Si, Si + kPlane, k, err_pivot);
+    for (int idx = threadIdx.x; idx < kNb * kNb; idx += 256) {  // the inverse in place of the block
+        const int i = idx / kNb, j = idx % kNb;
+        a_re[base + (size_t)i * ld + j] = j <= i ? Sr[j * kLdc + i + 1] : 0.0;
+        a_im[base + (size_t)i * ld + j] = j <= i ? Si[j * kLdc + i + 1] : 0.0;
     }
 }
 
-// Panel solve: P <- P * Linv^T (complex) for rows below the block; RHS rows add sum_j y_j^2 to q.
-__global__ void __launch_bounds__(256) k_trsm_panel_c(double* __restrict__ a_re, double* __restrict__ a_im, int64_t ld,
-                                                      int64_t stride, int64_t k, int64_t n_pad,
-                                                      const double* __restrict__ linv, double* __restrict__ qacc,
-                                                      int64_t ldq) {
-    extern __shared__ double smem[];
-    double* Pr = smem;
-    double* Pi = Pr + 64 * kLds;
-    double* Lr = Pi + 64 * kLds;
-    double* Li = Lr + 64 * kLds;
-    const int f = blockIdx.y;
-    const int64_t r0 = k + kNb + (int64_t)blockIdx.x * kNb;
-    double* Ar = a_re + (size_t)f * stride;
-    double* Ai = a_im + (size_t)f * stride;
-    load_tile_c(Pr, Ar + r0 * ld + k, ld);
-    load_tile_c(Pi, Ai + r0 * ld + k, ld);
-    const double* lv = linv + (size_t)f * 2 * kNb * kNb;
-    load_tile_c(Lr, lv, kNb);
-    load_tile_c(Li, lv + kNb * kNb, kNb);
-    __syncthreads();
-    double accr[2][4][2] = {}, acci[2][4][2] = {};
-    tile_mma_c(Pr, Lr, accr, 1.0);
-    tile_mma_c(Pi, Li, accr, -1.0);
-    tile_mma_c(Pr, Li, acci, 1.0);
-    tile_mma_c(Pi, Lr, acci, 1.0);
-    __syncthreads();
+__device__ __forceinline__ void cp_async16c(double* dst, const double* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+// 32 or 64 rows of `w` doubles of both planes into shared memory (row stride ldm), one plane `plane` apart
+__device__ __forceinline__ void load_rows_c(double* dst, int plane, int ldm, const double* re, const double* im, int64_t ld,
+                                            int rows, int w) {
+    for (int idx = threadIdx.x; idx < rows * (w / 2); idx += blockDim.x) {
+        const int r = idx / (w / 2), c = 2 * (idx % (w / 2));
+        cp_async16c(dst + r * ldm + c, re + (size_t)r * ld + c);
+        cp_async16c(dst + plane + r * ldm + c, im + (size_t)r * ld + c);
+    }
+}
+
+// Rows below the block, 32-row tiles: P <- P L^{-T} with the triangular inverse (column tile c takes
+// k < 8 (c + 1)); right-hand-side rows add sum_j p_j^2 to q.  A CTA keeps the inverse and walks its
+// tiles; two CTAs per SM cover each other's loads.  Warp: 16 rows, column tiles {g, 7-g}.
+constexpr int kTileC = 32 * kLdc;
+constexpr size_t kPanelSmemC = sizeof(double) * (2 * kPlane + 2 * kTileC + 2 * 4 * 32);
+
+__global__ void __launch_bounds__(256, 2) k_panel_c(double* __restrict__ a_re, double* __restrict__ a_im, int64_t ld,
+                                                    int64_t stride, int64_t k, int64_t n_pad, int ntile,
+                                                    double* __restrict__ qacc, int64_t ldq) {
+    extern __shared__ __align__(16) double smem[];
+    double* Y = smem;
+    double* X = Y + 2 * kPlane;
+    double* red = X + 2 * kTileC;
+    const size_t f0 = (size_t)blockIdx.y * stride;
+    const int64_t row0 = k + kNb;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const int rr = 16 * (w >> 1), cc = 32 * (w & 1);
+    const int r0 = 16 * (w & 1), cg = w >> 1;
+    load_rows_c(Y, kPlane, kLdc, a_re + f0 + k * ld + k, a_im + f0 + k * ld + k, ld, kNb, kNb);
+    for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+        const int64_t row = row0 + (int64_t)tile * 32;
+        const size_t at = f0 + row * ld + k;
+        load_rows_c(X, kTileC, kLdc, a_re + at, a_im + at, ld, 32, kNb);
+        asm volatile("cp.async.commit_group;\n" ::);
+        asm volatile("cp.async.wait_group 0;\n" ::);
+        __syncthreads();
+        double ar[2][2][2] = {}, ai[2][2][2] = {};
+        auto steps = [&](int from, int to, int first) {
+            for (int ks = from; ks < to; ++ks) {
+                const double* xp = X + (r0 + g) * kLdc + 4 * ks + t;
+                const double xr0 = xp[0], xr1 = xp[8 * kLdc], xi0 = xp[kTileC], xi1 = xp[kTileC + 8 * kLdc];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                Pr[(rr + 8 * i + g) * kLds + cc + 8 * j + 2 * t + e] = accr[i][j][e];
-                Pi[(rr + 8 * i + g) * kLds + cc + 8 * j + 2 * t + e] = acci[i][j][e];
+                for (int i = 0; i < 2; ++i) {
+                    if (i < first) continue;
+                    const double* yp = Y + (8 * (i ? 7 - cg : cg) + g) * kLdc + 4 * ks + t;
+                    const double br = yp[0], bi = yp[kPlane];
+                    panel::dmma(ar[0][i], xr0, br);
+                    panel::dmma(ar[1][i], xr1, br);
+                    panel::dmma(ai[0][i], xr0, bi);
+                    panel::dmma(ai[1][i], xr1, bi);
+                    panel::dmma(ar[0][i], -xi0, bi);
+                    panel::dmma(ar[1][i], -xi1, bi);
+                    panel::dmma(ai[0][i], xi0, br);
+                    panel::dmma(ai[1][i], xi1, br);
+                }
             }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < 64 * 32; idx += blockDim.x) {
-        const int r = idx >> 5, c2 = idx & 31;
-        *reinterpret_cast<double2*>(Ar + (size_t)(r0 + r) * ld + k + 2 * c2) =
-            *reinterpret_cast<const double2*>(Pr + r * kLds + 2 * c2);
-        *reinterpret_cast<double2*>(Ai + (size_t)(r0 + r) * ld + k + 2 * c2) =
-            *reinterpret_cast<const double2*>(Pi + r * kLds + 2 * c2);
-    }
-    if (r0 >= n_pad && threadIdx.x < kNb) {
-        const int r = threadIdx.x;
-        double sr = 0.0, si = 0.0;
-        for (int j = 0; j < kNb; ++j) {
-            const double yr = Pr[r * kLds + j], yi = Pi[r * kLds + j];
-            sr += yr * yr - yi * yi;
-            si += 2.0 * yr * yi;
+        };
+        steps(0, 2 * (cg + 1), 0);
+        steps(2 * (cg + 1), 2 * (8 - cg), 1);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const size_t p = at + (size_t)(r0 + 8 * h + g) * ld + 8 * (i ? 7 - cg : cg) + 2 * t;
+                *reinterpret_cast<double2*>(a_re + p) = make_double2(ar[h][i][0], ar[h][i][1]);
+                *reinterpret_cast<double2*>(a_im + p) = make_double2(ai[h][i][0], ai[h][i][1]);
+            }
+        const bool rhs = row >= n_pad;
+        if (rhs) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                double sr = 0.0, si = 0.0;
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const double yr = ar[h][i][e], yi = ai[h][i][e];
+                        sr += yr * yr - yi * yi;
+                        si += 2.0 * yr * yi;
+                    }
+                for (int o = 1; o < 4; o <<= 1) {
+                    sr += __shfl_xor_sync(0xffffffffu, sr, o);
+                    si += __shfl_xor_sync(0xffffffffu, si, o);
+                }
+                if (t == 0) {
+                    red[cg * 32 + r0 + 8 * h + g] = sr;
+                    red[128 + cg * 32 + r0 + 8 * h + g] = si;
+                }
+            }
         }
-        qacc[(size_t)f * 2 * ldq + (r0 - n_pad + r)] += sr;
-        qacc[(size_t)f * 2 * ldq + ldq + (r0 - n_pad + r)] += si;
+        __syncthreads();
+        if (rhs && threadIdx.x < 64) {
+            const int r = threadIdx.x & 31, pl = threadIdx.x >> 5;
+            const double* p = red + 128 * pl + r;
+            qacc[((size_t)blockIdx.y * 2 + pl) * ldq + (row - n_pad) + r] += (p[0] + p[32]) + (p[64] + p[96]);
+        }
     }
 }
 
-// Trailing update C -= P_i P_j^T (complex, K = 64) over lower square tiles and all RHS tiles.
-__global__ void __launch_bounds__(256) k_update_c(double* __restrict__ a_re, double* __restrict__ a_im, int64_t ld,
-                                                  int64_t stride, int64_t k, int64_t t_sq, int64_t t_rhs) {
-    extern __shared__ double smem[];
-    double* Pir = smem;
-    double* Pii = Pir + 64 * kLds;
-    double* Pjr = Pii + 64 * kLds;
-    double* Pji = Pjr + 64 * kLds;
-    const int f = blockIdx.y;
-    const int64_t x = blockIdx.x;
-    const int64_t n_sq = t_sq * (t_sq + 1) / 2;
-    int64_t ti, tj;
-    if (x < n_sq) {
-        ti = (int64_t)((sqrt(8.0 * (double)x + 1.0) - 1.0) * 0.5);
-        while (ti * (ti + 1) / 2 > x) --ti;
-        while ((ti + 1) * (ti + 2) / 2 <= x) ++ti;
-        tj = x - ti * (ti + 1) / 2;
+// C -= P_i P_j^T (complex) over K = 64 nk columns from kb0, output column tiles [tc0, tc0 + T): square
+// tiles on or below the diagonal, then all right-hand-side rows; the real form's k_update with two
+// planes.  64 x 64 tiles, K in 16-wide slices through a two-stage cp.async pipeline, two CTAs per SM
+// (one 64-deep load per tile with one CTA per SM left the loads exposed: 18 TFLOP/s).
+constexpr int kKcc = 16, kLdkc = kKcc + 4, kSliceC = 64 * kLdkc;
+constexpr size_t kUpdateSmemC = sizeof(double) * 2 * 4 * kSliceC;
+
+__global__ void __launch_bounds__(256, 2) k_update_c(double* __restrict__ a_re, double* __restrict__ a_im, int64_t ld,
+                                                     int64_t stride, int64_t kb0, int nk, int64_t tc0, int64_t T,
+                                                     int64_t nsq) {
+    extern __shared__ __align__(16) double smem[];
+    const int64_t x = blockIdx.x, L = nsq - tc0;
+    const int64_t n_square = T * L - T * (T - 1) / 2;
+    int64_t c, tr;
+    if (x < n_square) {
+        const double b = 2.0 * (double)L + 1.0;
+        c = (int64_t)((b - sqrt(fmax(b * b - 8.0 * (double)x, 0.0))) * 0.5);
+        auto cum = [L](int64_t cc) { return cc * L - cc * (cc - 1) / 2; };
+        while (c > 0 && cum(c) > x) --c;
+        while (c + 1 < T && cum(c + 1) <= x) ++c;
+        tr = tc0 + c + (x - cum(c));
     } else {
-        const int64_t y = x - n_sq;
-        ti = t_sq + y / t_sq;
-        tj = y % t_sq;
-        if (ti >= t_sq + t_rhs) return;
+        const int64_t y = x - n_square;
+        c = y % T;
+        tr = nsq + y / T;
     }
-    const int64_t base = k + kNb;
-    const int64_t ri = base + ti * kNb, cj = base + tj * kNb;
-    double* Ar = a_re + (size_t)f * stride;
-    double* Ai = a_im + (size_t)f * stride;
-    load_tile_c(Pir, Ar + ri * ld + k, ld);
-    load_tile_c(Pii, Ai + ri * ld + k, ld);
-    load_tile_c(Pjr, Ar + cj * ld + k, ld);
-    load_tile_c(Pji, Ai + cj * ld + k, ld);
-    __syncthreads();
-    double accr[2][4][2] = {}, acci[2][4][2] = {};
-    tile_mma_c(Pir, Pjr, accr, -1.0);
-    tile_mma_c(Pii, Pji, accr, 1.0);
-    tile_mma_c(Pir, Pji, acci, -1.0);
-    tile_mma_c(Pii, Pjr, acci, -1.0);
+    const size_t f0 = (size_t)blockIdx.y * stride;
+    const int64_t ri = tr * kNb, cj = (tc0 + c) * kNb;
+    const int nsub = nk * (kNb / kKcc);
+    auto stage = [&](int st) { return smem + (st & 1) * 4 * kSliceC; };
+    auto load = [&](int sc) {
+        const int64_t kc = kb0 + (int64_t)sc * kKcc;
+        load_rows_c(stage(sc), kSliceC, kLdkc, a_re + f0 + ri * ld + kc, a_im + f0 + ri * ld + kc, ld, 64, kKcc);
+        load_rows_c(stage(sc) + 2 * kSliceC, kSliceC, kLdkc, a_re + f0 + cj * ld + kc, a_im + f0 + cj * ld + kc, ld, 64,
+                    kKcc);
+        asm volatile("cp.async.commit_group;\n" ::);
+    };
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const int rr = 16 * (w >> 1), cc = 32 * (w & 1);
+    const int r0 = 16 * (w >> 1), c0 = 32 * (w & 1);
+    double ar[2][4][2] = {}, ai[2][4][2] = {};
+    load(0);
+    for (int sc = 0; sc < nsub; ++sc) {
+        if (sc + 1 < nsub) {
+            load(sc + 1);
+            asm volatile("cp.async.wait_group 1;\n" ::);
+        } else {
+            asm volatile("cp.async.wait_group 0;\n" ::);
+        }
+        __syncthreads();
+        const double* A = stage(sc) + (r0 + g) * kLdkc + t;
+        const double* B = stage(sc) + 2 * kSliceC + (c0 + g) * kLdkc + t;
+#pragma unroll
+        for (int kk = 0; kk < kKcc; kk += 4) {
+            double xr[2], xi[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                xr[i] = -A[8 * i * kLdkc + kk];
+                xi[i] = A[kSliceC + 8 * i * kLdkc + kk];
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const double br = B[8 * j * kLdkc + kk], bi = B[kSliceC + 8 * j * kLdkc + kk];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    panel::dmma(ar[i][j], xr[i], br);
+                    panel::dmma(ai[i][j], xr[i], bi);
+                    panel::dmma(ar[i][j], xi[i], bi);
+                    panel::dmma(ai[i][j], -xi[i], br);
+                }
+            }
+        }
+        __syncthreads();
+    }
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const size_t off = (size_t)(ri + rr + 8 * i + g) * ld + cj + cc + 8 * j + 2 * t;
-            double2 vr = *reinterpret_cast<double2*>(Ar + off), vi = *reinterpret_cast<double2*>(Ai + off);
-            vr.x += accr[i][j][0];
-            vr.y += accr[i][j][1];
-            vi.x += acci[i][j][0];
-            vi.y += acci[i][j][1];
-            *reinterpret_cast<double2*>(Ar + off) = vr;
-            *reinterpret_cast<double2*>(Ai + off) = vi;
+            const size_t off = f0 + (size_t)(ri + r0 + 8 * i + g) * ld + cj + c0 + 8 * j + 2 * t;
+            double2 vr = *reinterpret_cast<double2*>(a_re + off), vi = *reinterpret_cast<double2*>(a_im + off);
+            vr.x += ar[i][j][0];
+            vr.y += ar[i][j][1];
+            vi.x += ai[i][j][0];
+            vi.y += ai[i][j][1];
+            *reinterpret_cast<double2*>(a_re + off) = vr;
+            *reinterpret_cast<double2*>(a_im + off) = vi;
         }
 }
 
@@ -384,14 +627,12 @@ __global__ void __launch_bounds__(256) k_sigma_contract_c(const double* __restri
 } // namespace
 
 int launch_factor_chunk_c(const TallGeometry& g, int64_t nf, const double* delta, const double* omega, double eta,
-                          const double* v, const double* xt, double* a_re, double* a_im, double* svec, double* linv,
-                          double* qacc, unsigned long long* err_pivot, cudaStream_t s) {
-    const size_t smem4 = 4 * 64 * kLds * sizeof(double);
-    const size_t smem_potrf = 4 * kNb * (kNb + 1) * sizeof(double);
-    GWB_CUDA(cudaFuncSetAttribute(k_potrf_diag_c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_potrf));
-    GWB_CUDA(cudaFuncSetAttribute(k_trsm_panel_c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem4));
-    GWB_CUDA(cudaFuncSetAttribute(k_update_c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem4));
-    int launches = 0;
+                          const double* v, const double* xt, double* a_re, double* a_im, double* svec, double* qacc,
+                          unsigned long long* err_pivot, cudaStream_t s) {
+    const size_t smem_diag = sizeof(double) * (2 * kPlane + kCWork);
+    GWB_CUDA(cudaFuncSetAttribute(k_diag_c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_diag));
+    GWB_CUDA(cudaFuncSetAttribute(k_panel_c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmemC));
+    GWB_CUDA(cudaFuncSetAttribute(k_update_c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUpdateSmemC));
     k_scale_vectors_c<<<dim3((unsigned)((g.n_pad + 255) / 256), (unsigned)nf), 256, 0, s>>>(delta, (int)g.n, (int)g.n_pad,
                                                                                           omega, eta, svec);
     GWB_LAUNCH("k_scale_vectors_c");
@@ -399,26 +640,26 @@ int launch_factor_chunk_c(const TallGeometry& g, int64_t nf, const double* delta
         g.n, g.m, g.n_pad, g.ld, g.stride, g.rows, v, xt, svec, (int)nf, a_re, a_im);
     GWB_LAUNCH("k_build_tall_c");
     GWB_CUDA(cudaMemsetAsync(qacc, 0, sizeof(double) * 2 * (size_t)nf * g.m_pad, s));
-    launches += 2;
-    for (int64_t k = 0; k < g.n_pad; k += kNb) {
-        k_potrf_diag_c<<<(unsigned)nf, 256, smem_potrf, s>>>(a_re, a_im, g.ld, g.stride, k, linv, err_pivot);
-        GWB_LAUNCH("k_potrf_diag_c");
+    int launches = 2;
+    const int64_t nsq = g.n_pad / kNb, nrt = g.rows / kNb;
+    auto update = [&](int64_t kb0, int nk, int64_t tc0, int64_t T) {
+        const int64_t L = nsq - tc0, tiles = T * L - T * (T - 1) / 2 + T * (nrt - nsq);
+        if (tiles <= 0) return;
+        k_update_c<<<dim3((unsigned)tiles, (unsigned)nf), 256, kUpdateSmemC, s>>>(a_re, a_im, g.ld, g.stride, kb0, nk, tc0,
+                                                                                T, nsq);
+        GWB_LAUNCH("k_update_c");
         ++launches;
-        const int64_t below = g.rows - (k + kNb);
-        if (below > 0) {
-            k_trsm_panel_c<<<dim3((unsigned)(below / kNb), (unsigned)nf), 256, smem4, s>>>(a_re, a_im, g.ld, g.stride, k,
-                                                                                      g.n_pad, linv, qacc, g.m_pad);
-            GWB_LAUNCH("k_trsm_panel_c");
-            ++launches;
-        }
-        const int64_t t_sq = (g.n_pad - (k + kNb)) / kNb;
-        if (t_sq > 0) {
-            const int64_t t_rhs = g.m_pad / kNb;
-            const int64_t tiles = t_sq * (t_sq + 1) / 2 + t_rhs * t_sq;
-            k_update_c<<<dim3((unsigned)tiles, (unsigned)nf), 256, smem4, s>>>(a_re, a_im, g.ld, g.stride, k, t_sq, t_rhs);
-            GWB_LAUNCH("k_update_c");
-            ++launches;
-        }
+    };
+    for (int64_t b = 0; b < nsq; ++b) {  // outer blocks of two 64-wide blocks
+        if (b & 1) update((b - 1) * kNb, 1, b, 1);  // the first block onto the second's columns
+        k_diag_c<<<(unsigned)nf, 256, smem_diag, s>>>(a_re, a_im, g.ld, g.stride, b * kNb, err_pivot);
+        GWB_LAUNCH("k_diag_c");
+        const int64_t tiles = (g.rows - (b + 1) * kNb) / 32;
+        k_panel_c<<<dim3((unsigned)panel_grid(tiles, nf, 2), (unsigned)nf), 256, kPanelSmemC, s>>>(
+            a_re, a_im, g.ld, g.stride, b * kNb, g.n_pad, (int)tiles, qacc, g.m_pad);
+        GWB_LAUNCH("k_panel_c");
+        launches += 2;
+        if ((b & 1) && b + 1 < nsq) update((b - 1) * kNb, 2, b + 1, nsq - b - 1);
     }
     return launches;
 }

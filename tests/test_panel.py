@@ -62,3 +62,43 @@ def test_reported_pivot(n, pivot):
         be.load_slices(sl)  # the handle is usable afterwards
         q, _ = be.screened_forms(np.array([0.3]), sl.states)
     assert np.abs(q - _forms(sl, [0.3])).max() <= 1e-11 * np.abs(q).max()
+
+
+def _forms_complex(sl, omegas, eta):
+    """x^T W_c x with W_c = (I - diag(Pi0) V)^{-1} diag(Pi0), numpy in complex FP64."""
+    delta = sl.mo_energy[1:] - sl.mo_energy[0]
+    out = []
+    for w in omegas:
+        p = 2.0 * (1.0 / (1j * w - delta + 1j * eta) - 1.0 / (1j * w + delta - 1j * eta))
+        y = np.linalg.solve(np.eye(len(p)) - p[:, None] * sl.vph, p[:, None] * sl.panel.T)
+        out.append((sl.panel.T * y).sum(axis=0))
+    return np.array(out).reshape(len(omegas), len(sl.states), -1)
+
+
+@pytest.mark.parametrize("n,nstates", [(1, 1), (15, 1), (16, 1), (17, 2), (63, 1), (64, 1), (65, 1), (128, 1), (129, 1),
+                                       (193, 1), (257, 2)])
+def test_complex_forms_at_block_edges(n, nstates):
+    from minigw_b200 import B200Backend
+
+    sl = _system(n, max(1, n // 2), nstates, 300 + n)
+    omegas = np.array([1e-3, 0.4, 7.0])
+    with B200Backend(0) as be:
+        be.load_slices(sl)
+        q, _ = be.screened_forms_complex(omegas, sl.states, eta=0.02)
+    ref = _forms_complex(sl, omegas, 0.02)
+    assert np.abs(q - ref).max() <= 1e-11 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("pivot", [0, 15, 16, 63, 64, 99])
+def test_complex_reported_pivot(pivot):
+    from minigw_b200 import B200Backend
+    from minigw_b200._lib import GwB200Error
+
+    sl = _system(100, 3, 1, 7)
+    sl.vph = np.zeros((100, 100))
+    sl.vph[pivot, pivot] = np.nan
+    with B200Backend(0) as be:
+        be.load_slices(sl)
+        with pytest.raises(GwB200Error) as e:
+            be.screened_forms_complex(np.array([0.3]), sl.states, eta=0.02)
+        assert e.value.status == "GWB200_NOT_SPD" and f"pivot {pivot + 1} " in str(e.value)
