@@ -332,12 +332,15 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
     }
     GWB_CUDA(cudaMemsetAsync(h->err.p, 0xFF, sizeof(unsigned long long), s));
 
+    // small systems need no tall matrices (unless the solved rows are wanted): one launch, one chunk
+    const bool small = !mixed && !cplx && !after_factor && small_system(g);
+
     // Frequency chunk size from the HBM budget: tall matrices, scale vectors, accumulators, operands.
     const bool mixed_tc = mixed && mixed_update_on_tcgen05(h);
     // plain form: the int8 emulation of the outer updates is a candidate of the update autotuner
     // (its slice workspace is part of the budget) unless GWB200_FP64_UPDATE=dmma; memory-capped
     // handles use it only when it is forced (GWB200_FP64_UPDATE=ozaki)
-    const bool fp64_oz = !mixed && !cplx && fp64_update_mode() != 1 && (h->mem_limit <= 0 || fp64_update_mode() == 2);
+    const bool fp64_oz = !mixed && !cplx && !small && fp64_update_mode() != 1 && (h->mem_limit <= 0 || fp64_update_mode() == 2);
     // refined mixed form: V_ph = C C^T once per loaded system (its rank sizes the correction's work)
     int64_t r_pad = 0;
     RefineFactor fac{};
@@ -355,7 +358,9 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
     if (const char* env = std::getenv("GWB200_MAX_FREQ_CHUNK")) cap = std::max<long long>(0, std::atoll(env));
     const int64_t key[5] = {(int64_t)per_freq, nfreq, cap, (int64_t)g.stride, h->mem_limit};
     int64_t fc;
-    if (std::equal(key, key + 5, h->chunk_key)) {
+    if (small) {
+        fc = cap > 0 ? std::min<int64_t>(nfreq, cap) : nfreq;
+    } else if (std::equal(key, key + 5, h->chunk_key)) {
         fc = h->chunk_fc;  // same geometry as the last call: its buffers are already sized
     } else {
         size_t free_b = 0, total_b = 0;
@@ -379,9 +384,11 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
         std::copy(key, key + 5, h->chunk_key);
         h->chunk_fc = fc;
     }
-    size_buffer(h, h->a, (mixed ? sizeof(float) : sizeof(double) * planes) * (size_t)fc * g.stride);
-    size_buffer(h, h->dvec, sizeof(double) * planes * (size_t)fc * g.n_pad);
-    size_buffer(h, h->qacc, sizeof(double) * planes * (size_t)fc * g.m_pad);
+    if (!small) {
+        size_buffer(h, h->a, (mixed ? sizeof(float) : sizeof(double) * planes) * (size_t)fc * g.stride);
+        size_buffer(h, h->dvec, sizeof(double) * planes * (size_t)fc * g.n_pad);
+        size_buffer(h, h->qacc, sizeof(double) * planes * (size_t)fc * g.m_pad);
+    }
     if (mixed_tc) {
         size_buffer(h, h->panel32, tc_panel_bytes_per_freq(g) * (size_t)fc);
         h->tc_sched.ensure(sched_bytes(g));
@@ -411,6 +418,13 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
     int upd_variant = -1;  // FP64 update kernel, tuned on the first chunk (full size) of this geometry
     for (int64_t f0 = 0; f0 < nfreq; f0 += fc) {
         const int64_t nf = std::min(fc, nfreq - f0);
+        if (small) {
+            launches += launch_small64(g, nf, h->delta.as<double>(), h->omega.as<double>() + f0, h->v.as<double>(),
+                                       h->xt.as<double>(), h->qall.as<double>() + f0 * g.m_pad, g.m_pad,
+                                       h->err.as<unsigned long long>(), s);
+            ++chunks;
+            continue;
+        }
         if (cplx) {
             double* a_re = h->a.as<double>();
             launches += launch_factor_chunk_c(g, nf, h->delta.as<double>(), h->omega.as<double>() + f0, eta,

@@ -133,6 +133,11 @@ int launch_factor_chunk(const TallGeometry& g, int64_t nf, double* a, double* qa
 // rows are added to qacc.  Returns launches issued.
 int launch_panel64(const TallGeometry& g, int64_t nf, double* a, int64_t k, int64_t width, double* qacc,
                    unsigned long long* err_pivot, cudaStream_t s);
+// Small systems (n <= 128): the forms q[f][j] = x_j^T W_c x_j (rows ldq apart) of nf frequencies straight
+// from V, the panel rows and the frequencies in one launch, without tall matrices.
+bool small_system(const TallGeometry& g);
+int launch_small64(const TallGeometry& g, int64_t nf, const double* delta, const double* omega, const double* v,
+                   const double* xt, double* q, int64_t ldq, unsigned long long* err_pivot, cudaStream_t s);
 // CTAs per frequency of a panel kernel over `tiles` row tiles of nf frequencies, per_sm CTAs per SM
 int64_t panel_grid(int64_t tiles, int64_t nf, int64_t per_sm);
 // kernels_oz.cu: FP64 trailing update C -= P P^T (K = 128 from kb0, columns [c_begin, n_pad), rows

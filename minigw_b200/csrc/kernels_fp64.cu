@@ -10,7 +10,7 @@
 // blocked Cholesky: its lower rows become (L^{-1} D^1/2 X)^T, whose row norms are the
 // quadratic forms.  All arithmetic is FP64; the O(n^3) and O(n^2 m) work runs on FP64
 // tensor cores (mma.sync m8n8k4 f64, DMMA).
-#include "internal.cuh"
+#include "panel_common.cuh"
 
 #include <array>
 #include <cstdio>
@@ -91,10 +91,7 @@ __global__ void k_scale_vectors(const double* __restrict__ delta, int n, int n_p
     const double w = omega[f];
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n_pad; c += gridDim.x * blockDim.x) {
         double val = 0.0;
-        if (c < n) {
-            const double d = delta[c];
-            val = sqrt(4.0 * d / (w * w + d * d));
-        }
+        if (c < n) val = panel::scale_value(delta[c], w);
         dvec[(size_t)f * n_pad + c] = val;
     }
 }

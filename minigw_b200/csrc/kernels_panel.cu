@@ -12,6 +12,9 @@
 //               A CTA keeps the inverse in shared memory and walks row tiles of 32, the next tile
 //               loaded while one is multiplied; each warp owns 16 rows and column tiles
 //               {g, 7-g, 8+g, 15-g}, the same work for every g.
+//
+//   k_small64   systems of at most 128 particle-hole pairs: everything between the frequencies and
+//               the forms in one kernel, see there.
 #include "panel_common.cuh"
 
 #include <algorithm>
@@ -143,6 +146,104 @@ __global__ void __launch_bounds__(kPanelThreads, 1)
     }
 }
 
+// Whole frequencies of a small system (n <= NB <= 128), one CTA each: the scale vector, eps, its factor
+// and inverse in shared memory, then the right-hand sides in 32-row tiles, of which only the forms
+// leave the SM.  The arithmetic and its order are those of k_scale_vectors, k_build_tall, k_diag64,
+// k_panel64 and k_negate_copy, whose five launches and tall matrices it replaces: at this size they
+// spent their time in launches and the matrices' way through memory (24 orbitals, 200 frequencies:
+// 113 us of kernels; this one 39).  NB is the next of 64, 96 and 128, so that up to n = 96 two CTAs
+// share an SM.
+template <int NB>
+struct SmallShape {
+    static constexpr int kXLd = NB + 4;
+    static constexpr size_t kSmem = DiagShape<NB>::kSmem + sizeof(double) * ((size_t)kRowTile * kXLd + NB + 4 * kRowTile);
+};
+
+template <int NB>
+__global__ void __launch_bounds__(DiagShape<NB>::kThreads) k_small64(int n, int m, const double* __restrict__ delta,
+                                                                     const double* __restrict__ omega,
+                                                                     const double* __restrict__ v,
+                                                                     const double* __restrict__ xt, double* __restrict__ q,
+                                                                     int64_t ldq, unsigned long long* err_pivot) {
+    extern __shared__ __align__(16) double psm[];
+    using Sh = DiagShape<NB>;
+    constexpr int LD = Sh::kLd, XL = SmallShape<NB>::kXLd, NT = NB / 32;
+    double* S = psm;
+    double* work = S + Sh::kBlockDoubles;
+    double* X = work + Sh::kWorkDoubles;
+    double* d = X + kRowTile * XL;
+    double* red = d + NB;
+    const int f = blockIdx.x;
+    const double w = omega[f];
+    for (int c = threadIdx.x; c < NB; c += Sh::kThreads) d[c] = c < n ? scale_value(delta[c], w) : 0.0;
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < NB * LD; idx += Sh::kThreads) {
+        const int i = idx / LD, j = idx % LD;
+        double x = 0.0;
+        if (j <= i) x = fma(d[i] * (i < n ? v[(size_t)i * n + j] : 0.0), d[j], i == j ? 1.0 : 0.0);
+        S[idx] = x;
+    }
+    __syncthreads();
+    factor_diag<NB, false>(S, work, 0, err_pivot);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    const int r0 = 16 * (warp & 1), cg = warp >> 1;
+    auto col = [&](int i) { return (i >> 1) * 8 + ((i & 1) ? 7 - cg : cg); };  // as in k_panel64
+    for (int row = 0; row < m; row += kRowTile) {
+        for (int idx = threadIdx.x; idx < kRowTile * NB; idx += Sh::kThreads) {
+            const int r = idx / NB, c = idx % NB;
+            X[r * XL + c] = (row + r < m && c < n) ? d[c] * xt[(size_t)(row + r) * n + c] : 0.0;
+        }
+        __syncthreads();
+        if (warp < 8) {
+            const double* Xp = X + (r0 + g) * XL + t;
+            double acc[2][NT][2] = {};
+            int ks = 0;
+#pragma unroll
+            for (int first = 0; first < NT; ++first) {
+                const int kend = 2 * (col(first) + 1);
+                for (; ks < kend; ++ks) {
+                    const double a0 = Xp[4 * ks], a1 = Xp[8 * XL + 4 * ks];
+                    const int k = 4 * ks + t;
+#pragma unroll
+                    for (int i = first; i < NT; ++i) {
+                        const int c = 8 * col(i) + g;
+                        const double b = k <= c ? S[k * LD + c + 1] : 0.0;
+                        dmma(acc[0][i], a0, b);
+                        dmma(acc[1][i], a1, b);
+                    }
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                double s = 0.0;
+#pragma unroll
+                for (int i = 0; i < NT; ++i) s = fma(acc[h][i][1], acc[h][i][1], fma(acc[h][i][0], acc[h][i][0], s));
+                s += __shfl_xor_sync(0xffffffffu, s, 1);
+                s += __shfl_xor_sync(0xffffffffu, s, 2);
+                if (t == 0) red[cg * kRowTile + r0 + 8 * h + g] = s;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < kRowTile && row + (int)threadIdx.x < m) {
+            const int r = threadIdx.x;
+            q[(size_t)f * ldq + row + r] =
+                -((red[r] + red[kRowTile + r]) + (red[2 * kRowTile + r] + red[3 * kRowTile + r]));
+        }
+    }
+}
+
+template <int NB>
+int launch_small(const TallGeometry& g, int64_t nf, const double* delta, const double* omega, const double* v,
+                 const double* xt, double* q, int64_t ldq, unsigned long long* err_pivot, cudaStream_t s) {
+    const size_t smem = SmallShape<NB>::kSmem;
+    GWB_CUDA(cudaFuncSetAttribute(k_small64<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_small64<NB><<<(unsigned)nf, DiagShape<NB>::kThreads, smem, s>>>((int)g.n, (int)g.m, delta, omega, v, xt, q, ldq,
+                                                                     err_pivot);
+    GWB_LAUNCH("k_small64");
+    return 1;
+}
+
 template <int NB>
 int launch_block(const TallGeometry& g, int64_t nf, double* a, int64_t k, double* qacc, unsigned long long* err_pivot,
                  cudaStream_t s) {
@@ -174,6 +275,15 @@ int64_t panel_grid(int64_t tiles, int64_t nf, int64_t per_sm) {
         }
     }
     return best;
+}
+
+bool small_system(const TallGeometry& g) { return g.n <= 128; }
+
+int launch_small64(const TallGeometry& g, int64_t nf, const double* delta, const double* omega, const double* v,
+                   const double* xt, double* q, int64_t ldq, unsigned long long* err_pivot, cudaStream_t s) {
+    if (g.n <= 64) return launch_small<64>(g, nf, delta, omega, v, xt, q, ldq, err_pivot, s);
+    if (g.n <= 96) return launch_small<96>(g, nf, delta, omega, v, xt, q, ldq, err_pivot, s);
+    return launch_small<128>(g, nf, delta, omega, v, xt, q, ldq, err_pivot, s);
 }
 
 int launch_panel64(const TallGeometry& g, int64_t nf, double* a, int64_t k, int64_t width, double* qacc,

@@ -33,6 +33,11 @@ struct DiagShape {
     static constexpr int kThreads = 4 * NB;  // enough warps to update the trailing tiles beside warp 0
 };
 
+// sqrt(D) with D = -Pi0(i w) = 4 delta / (w^2 + delta^2), rounded the same wherever it is formed.
+__device__ __forceinline__ double scale_value(double delta, double w) {
+    return sqrt(__dmul_rn(4.0, delta) / __fma_rn(w, w, __dmul_rn(delta, delta)));
+}
+
 __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
                  : "+d"(c[0]), "+d"(c[1])
