@@ -7,6 +7,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <functional>
+#include <initializer_list>
 #include <limits>
 #include <map>
 #include <mutex>
@@ -126,9 +127,19 @@ struct gwb200_handle {
     double fermi = 0.0;
     bool bad_gap = false;
     bool complex_forms = false;  // the last compute_forms ran the eta != 0 (complex) path
-    DevBuf pqo, xdiag, mo, vxc_diag, delta, v, sigx, flag;  // pqo: the (pq|o.) block of the ERI
+    DevBuf pqo, xdiag, mo, vxc_diag, delta, v, sigx;  // pqo: the (pq|o.) block of the ERI
     // per-call workspaces (grow-only, reused across calls)
-    DevBuf xt, dvec, a, qacc, qall, sigma, omega, weight, states, err, qp, omega_out;
+    DevBuf xt, dvec, a, qacc, qall, omega_out;
+    // A call's small inputs and results, one copy each way: `in` holds the pivot word (set by the
+    // upload), the grid, the state list (and a batch's group tables), `out` Sigma_c of the requested
+    // states [nstates][nfreq] and their QP energies; `call` points into them (a batch member's into
+    // its lead handle's).
+    DevBuf in, out;
+    struct {
+        double *omega = nullptr, *weight = nullptr, *sigma = nullptr, *qp = nullptr;
+        int64_t* states = nullptr;
+    } call;
+    unsigned long long* err() const { return in.as<unsigned long long>(); }
     DevBuf panel32;   // operand workspace of the tcgen05 trailing updates (mixed: FP32 hi/lo split;
                       // plain with GWB200_FP64_UPDATE=ozaki: int8 digit slices + exponents)
     DevBuf tc_sched;  // work counter of the tcgen05 update kernel
@@ -139,7 +150,6 @@ struct gwb200_handle {
     DevBuf qx, sigmx;                // gwb200_sigma_c_matrix: cross forms, Sigma_c between the states
     int64_t pchol_rank = -1;
     double* pchol_ct = nullptr;
-    DevBuf batch_desc;  // BatchGroup tables of gwb200_run_g0w0_batch (when this handle leads a batch)
     BatchLane lanes[kMaxBatchLanes];  // streams + workspaces of the batches this handle leads
     cudaEvent_t batch_fork = nullptr;
     cudaGraphExec_t batch_exec = nullptr;   // the last batch sequence captured as a CUDA graph
@@ -308,29 +318,28 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
     const TallGeometry g = make_geometry(h->n, m);
     int64_t launches = 0;
 
-    h->omega.ensure(sizeof(double) * nfreq);
-    h->states.ensure(sizeof(int64_t) * nstates);
     const bool bound = !h->bound_states.empty();
     if (bound && !std::equal(states, states + nstates, h->bound_states.begin(), h->bound_states.end()))
         fail(GWB200_BAD_ARGUMENT, "the state list must be the one given to gwb200_load_system_states");
     if (!bound) size_buffer(h, h->xt, sizeof(double) * (size_t)m * h->n);
     size_buffer(h, h->qall, sizeof(double) * planes * (size_t)nfreq * g.m_pad);
-    h->err.ensure(sizeof(unsigned long long));
-    {  // grid, states and (optionally) weights through the pinned staging buffer, all up front
+    {  // pivot word, grid, weights (optional) and states: one pinned upload
         const size_t nb_om = sizeof(double) * nfreq, nb_st = sizeof(int64_t) * nstates;
-        h->stage_in.ensure(2 * nb_om + nb_st);
+        const size_t nb_in = sizeof(unsigned long long) + 2 * nb_om + nb_st;
+        h->in.ensure(nb_in);
+        h->stage_in.ensure(nb_in);
         char* st_p = h->stage_in.as<char>();
+        std::memset(st_p, 0xFF, sizeof(unsigned long long));
+        st_p += sizeof(unsigned long long);
         std::memcpy(st_p, omega, nb_om);
-        std::memcpy(st_p + nb_om, states, nb_st);
-        GWB_CUDA(cudaMemcpyAsync(h->omega.p, st_p, nb_om, cudaMemcpyHostToDevice, s));
-        GWB_CUDA(cudaMemcpyAsync(h->states.p, st_p + nb_om, nb_st, cudaMemcpyHostToDevice, s));
-        if (weight) {
-            h->weight.ensure(nb_om);
-            std::memcpy(st_p + nb_om + nb_st, weight, nb_om);
-            GWB_CUDA(cudaMemcpyAsync(h->weight.p, st_p + nb_om + nb_st, nb_om, cudaMemcpyHostToDevice, s));
-        }
+        if (weight) std::memcpy(st_p + nb_om, weight, nb_om);
+        else std::memset(st_p + nb_om, 0, nb_om);
+        std::memcpy(st_p + 2 * nb_om, states, nb_st);
+        GWB_CUDA(cudaMemcpyAsync(h->in.p, h->stage_in.p, nb_in, cudaMemcpyHostToDevice, s));
+        h->call.omega = h->in.as<double>() + 1;
+        h->call.weight = h->call.omega + nfreq;
+        h->call.states = reinterpret_cast<int64_t*>(h->call.weight + nfreq);
     }
-    GWB_CUDA(cudaMemsetAsync(h->err.p, 0xFF, sizeof(unsigned long long), s));
 
     // small systems need no tall matrices (unless the solved rows are wanted): one launch, one chunk
     const bool small = !mixed && !cplx && !after_factor && small_system(g);
@@ -371,7 +380,7 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
         size_t budget = (size_t)((double)avail * 0.85);
         if (h->mem_limit > 0) {  // the handle's cap minus what the system and panels already hold
             const size_t resident = h->pqo.bytes + h->xdiag.bytes + h->v.bytes + h->xt.bytes + h->qall.bytes +
-                                    h->sigma.bytes + h->pchol.bytes + h->pchol_sl.bytes +
+                                    h->out.bytes + h->pchol.bytes + h->pchol_sl.bytes +
                                     h->qx.bytes + h->sigmx.bytes + ((size_t)1 << 20);
             const size_t lim = (size_t)h->mem_limit;
             const size_t room = lim > resident ? lim - resident : 0;
@@ -402,7 +411,7 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
     GWB_CUDA(cudaEventRecord(h->ev[0], s));
     if (!bound)
         launches += kprof(h, kKprofGatherPanel, 16.0 * (double)m * (double)h->n, [&] {
-            return (int64_t)launch_gather_panel(h->pqo.as<double>(), h->nmo, h->nocc, h->states.as<int64_t>(), nstates,
+            return (int64_t)launch_gather_panel(h->pqo.as<double>(), h->nmo, h->nocc, h->call.states, nstates,
                                                 h->xt.as<double>(), s);
         });
     GWB_CUDA(cudaEventRecord(h->ev[1], s));
@@ -419,24 +428,24 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
     for (int64_t f0 = 0; f0 < nfreq; f0 += fc) {
         const int64_t nf = std::min(fc, nfreq - f0);
         if (small) {
-            launches += launch_small64(g, nf, h->delta.as<double>(), h->omega.as<double>() + f0, h->v.as<double>(),
+            launches += launch_small64(g, nf, h->delta.as<double>(), h->call.omega + f0, h->v.as<double>(),
                                        h->xt.as<double>(), h->qall.as<double>() + f0 * g.m_pad, g.m_pad,
-                                       h->err.as<unsigned long long>(), s);
+                                       h->err(), s);
             ++chunks;
             continue;
         }
         if (cplx) {
             double* a_re = h->a.as<double>();
-            launches += launch_factor_chunk_c(g, nf, h->delta.as<double>(), h->omega.as<double>() + f0, eta,
+            launches += launch_factor_chunk_c(g, nf, h->delta.as<double>(), h->call.omega + f0, eta,
                                               h->v.as<double>(), h->xt.as<double>(), a_re, a_re + (size_t)nf * g.stride,
                                               h->dvec.as<double>(), h->qacc.as<double>(),
-                                              h->err.as<unsigned long long>(), s);
+                                              h->err(), s);
             launches += launch_forms_out_c(h->qacc.as<double>(), nf, m, g.m_pad,
                                            h->qall.as<double>() + f0 * 2 * g.m_pad, g.m_pad, s);
             ++chunks;
             continue;
         }
-        launches += launch_scale_vectors(h->delta.as<double>(), g.n, g.n_pad, h->omega.as<double>() + f0, nf,
+        launches += launch_scale_vectors(h->delta.as<double>(), g.n, g.n_pad, h->call.omega + f0, nf,
                                          h->dvec.as<double>(), s);
         GWB_CUDA(cudaMemsetAsync(h->qacc.p, 0, sizeof(double) * (size_t)nf * g.m_pad, s));
         if (mixed) {
@@ -445,27 +454,27 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
                                                     h->a.as<float>(), s);
             });
             launches += launch_factor_chunk32(g, nf, h->a.as<float>(), h->qacc.as<double>(),
-                                              h->err.as<unsigned long long>(), s, prof.enabled ? &prof : nullptr,
+                                              h->err(), s, prof.enabled ? &prof : nullptr,
                                               mixed_tc ? h->panel32.as<float>() : nullptr,
                                               h->tc_sched.as<unsigned long long>(), h->persistent_ctas,
                                               /*keep_rows=*/refine);
             if (refine)  // qacc <- 2 x^T y - z^T z - y^T V y (FP64 energy functional at the FP32 solve)
                 launches += launch_refine_chunk(g, nf, h->a.as<float>(), h->xt.as<double>(),
                                                 h->dvec.as<double>(), fac, h->refine.p,
-                                                h->qacc.as<double>(), h->err.as<unsigned long long>(), s,
+                                                h->qacc.as<double>(), h->err(), s,
                                                 mixed_tc ? h->panel32.as<float>() : nullptr,
                                                 h->tc_sched.as<unsigned long long>(), h->persistent_ctas);
         } else {
             if (upd_variant < 0)
                 upd_variant = tune_update_variant(g, nf, h->a.as<double>(), s, fp64_oz ? h->panel32.p : nullptr,
-                                                  h->tc_sched.as<unsigned long long>(), h->err.as<unsigned long long>(),
+                                                  h->tc_sched.as<unsigned long long>(), h->err(),
                                                   /*timed=*/h->mem_limit <= 0);
             launches += kprof(h, kKprofBuildTall, build_bytes(nf, 8.0), [&] {
                 return (int64_t)launch_build_tall(g, h->v.as<double>(), h->xt.as<double>(), h->dvec.as<double>(), nf,
                                                   h->a.as<double>(), s);
             });
             launches += launch_factor_chunk(g, nf, h->a.as<double>(), h->qacc.as<double>(),
-                                            h->err.as<unsigned long long>(), s, prof.enabled ? &prof : nullptr,
+                                            h->err(), s, prof.enabled ? &prof : nullptr,
                                             upd_variant, fp64_oz ? h->panel32.p : nullptr,
                                             h->tc_sched.as<unsigned long long>(), h->persistent_ctas);
             if (after_factor) {
@@ -491,9 +500,25 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
     if (prof.enabled && st) prof.collect(st);
 }
 
-void finish_forms(gwb200_handle* h, gwb200_stats* st) {
-    h->stage_out.ensure(sizeof(unsigned long long));
-    GWB_CUDA(cudaMemcpyAsync(h->stage_out.p, h->err.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, h->stream));
+// Reads the pivot word and `nb` bytes of results at `src` back (one synchronisation; the results at
+// result_stage(h) afterwards) and reports a failed factorisation.
+char* result_stage(gwb200_handle* h) { return h->stage_out.as<char>() + sizeof(unsigned long long); }
+
+struct Readback {
+    const void* src;
+    size_t bytes;
+};
+
+void finish_forms(gwb200_handle* h, gwb200_stats* st, std::initializer_list<Readback> results = {}) {
+    size_t nb = sizeof(unsigned long long);
+    for (const Readback& r : results) nb += r.bytes;
+    h->stage_out.ensure(nb);
+    GWB_CUDA(cudaMemcpyAsync(h->stage_out.p, h->in.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, h->stream));
+    char* o = result_stage(h);
+    for (const Readback& r : results) {
+        GWB_CUDA(cudaMemcpyAsync(o, r.src, r.bytes, cudaMemcpyDeviceToHost, h->stream));
+        o += r.bytes;
+    }
     GWB_CUDA(cudaStreamSynchronize(h->stream));
     const unsigned long long piv = *h->stage_out.as<unsigned long long>();
     if (piv == 0)  // a bounded device wait expired (pivots are 1-based)
@@ -508,8 +533,27 @@ void finish_forms(gwb200_handle* h, gwb200_stats* st) {
     }
 }
 
+// Sigma_c of the requested states ([nstates][nf] complex at `rows`) into the caller's nmo x nf array,
+// zero elsewhere.
+void scatter_sigma(const gwb200_handle* h, const char* rows, const int64_t* states, int64_t nstates, int64_t nf,
+                   double* sigma_out) {
+    const size_t nb_row = sizeof(double) * 2 * (size_t)nf;
+    std::memset(sigma_out, 0, nb_row * (size_t)h->nmo);
+    for (int64_t i = 0; i < nstates; ++i) std::memcpy(sigma_out + 2 * (size_t)(states[i] * nf), rows + (size_t)i * nb_row, nb_row);
+}
+void scatter_qp(const gwb200_handle* h, const char* rows, const int64_t* states, int64_t nstates, double* qp_out) {
+    std::fill(qp_out, qp_out + h->nmo, std::numeric_limits<double>::quiet_NaN());
+    for (int64_t i = 0; i < nstates; ++i) std::memcpy(qp_out + states[i], rows + sizeof(double) * (size_t)i, sizeof(double));
+}
+// Sizes `out` for nstates x nf results and points `call` at them.
+void size_results(gwb200_handle* h, int64_t nstates, int64_t nf) {
+    h->out.ensure(sizeof(double) * (size_t)nstates * (2 * (size_t)nf + 1));
+    h->call.sigma = h->out.as<double>();
+    h->call.qp = h->call.sigma + 2 * (size_t)nstates * nf;
+}
+
 // G0-weighted frequency contraction of h->qall (the nf_int frequencies compute_forms solved, with
-// the weights it uploaded) into h->sigma (nmo x nf_out complex, zero rows for unrequested states).
+// the weights it uploaded) into h->call.sigma ([nstates][nf_out] complex).
 // omega_out_dev = NULL: the output grid is the integration grid.  Records ev[3].
 void contract_on_device(gwb200_handle* h, int64_t nf_int, int64_t nstates, gwb200_stats* st,
                         const double* omega_out_dev = nullptr, int64_t nf_out = -1) {
@@ -517,34 +561,28 @@ void contract_on_device(gwb200_handle* h, int64_t nf_int, int64_t nstates, gwb20
     const int64_t m = nstates * h->nmo;
     const int64_t ldq = make_geometry(h->n, m).m_pad;
     if (!omega_out_dev) {
-        omega_out_dev = h->omega.as<double>();
+        omega_out_dev = h->call.omega;
         nf_out = nf_int;
     }
-    const size_t sig_bytes = sizeof(double) * 2 * (size_t)h->nmo * nf_out;
-    h->sigma.ensure(sig_bytes);
-    GWB_CUDA(cudaMemsetAsync(h->sigma.p, 0, sig_bytes, s));
+    const size_t sig_bytes = sizeof(double) * 2 * (size_t)h->nmo * nf_out;  // as the caller gets it
     if (h->complex_forms)
         st->kernel_launches += launch_sigma_contract_c(h->qall.as<double>(), nf_int, nstates, h->nmo, ldq,
-                                                       h->states.as<int64_t>(), h->mo.as<double>(), h->fermi,
-                                                       h->omega.as<double>(), h->weight.as<double>(), omega_out_dev,
-                                                       nf_out, h->sigma.as<double>(), s);
+                                                       h->mo.as<double>(), h->fermi, h->call.omega, h->call.weight, omega_out_dev,
+                                                       nf_out, h->call.sigma, s);
     else  // algorithmic bytes: the forms read once, Sigma_c written once
         st->kernel_launches += kprof(h, kKprofContract, 8.0 * (double)nf_int * (double)m + (double)sig_bytes, [&] {
             return (int64_t)launch_sigma_contract(h->qall.as<double>(), nf_int, nstates, h->nmo, ldq,
-                                                  h->states.as<int64_t>(), h->mo.as<double>(), h->fermi,
-                                                  h->omega.as<double>(), h->weight.as<double>(), omega_out_dev, nf_out,
-                                                  h->sigma.as<double>(), s);
+                                                  h->mo.as<double>(), h->fermi, h->call.omega, h->call.weight, omega_out_dev, nf_out,
+                                                  h->call.sigma, s);
         });
     GWB_CUDA(cudaEventRecord(h->ev[3], s));
 }
 
-// Pade + QP fixed point on h->sigma / h->omega / h->states (already on the device) into h->qp.
+// Pade + QP fixed point of the requested states on h->call's Sigma_c rows into h->call.qp.
 void qp_on_device(gwb200_handle* h, int64_t nfreq, int64_t npade, int64_t nstates) {
     cudaStream_t s = h->stream;
-    h->qp.ensure(sizeof(double) * h->nmo);
-    launch_fill(h->qp.as<double>(), std::numeric_limits<double>::quiet_NaN(), h->nmo, s);
-    launch_qp(h->sigma.as<double>(), h->omega.as<double>(), nfreq, h->states.as<int64_t>(), nstates, npade,
-              h->mo.as<double>(), h->fermi, h->sigx.as<double>(), h->vxc_diag.as<double>(), h->qp.as<double>(), s);
+    launch_qp(h->call.sigma, h->call.omega, nfreq, h->call.states, nstates, npade, h->mo.as<double>(), h->fermi,
+              h->sigx.as<double>(), h->vxc_diag.as<double>(), h->call.qp, s);
 }
 
 // ---- many molecules in shared launches (gwb200_run_g0w0_batch; kernels in kernels_batch.cu) ----
@@ -647,7 +685,7 @@ int64_t batch_screen(gwb200_handle* w, BatchLane& lane, cudaStream_t s, int max_
                      const std::vector<BatchGroup>& hgroups, const std::vector<int>& variants, bool mixed,
                      bool mixed_tc, bool oz, bool refine) {
     int64_t launches = 0;
-    unsigned long long* err = w->err.as<unsigned long long>();
+    unsigned long long* err = w->err();
     unsigned long long* sched = lane.sched.as<unsigned long long>();
     for (size_t k : idx) {
         const BatchChunk& c = chunks[k];
@@ -761,9 +799,9 @@ int gwb200_destroy(gwb200_handle* h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     h->stage_in.release();
     h->stage_out.release();
-    for (DevBuf* b : {&h->pchol, &h->pchol_sl, &h->refine, &h->pqo, &h->xdiag, &h->mo, &h->vxc_diag, &h->delta, &h->v, &h->sigx, &h->flag, &h->xt, &h->dvec, &h->a,
-                      &h->qacc, &h->qall, &h->sigma, &h->omega, &h->weight, &h->states, &h->err, &h->qp,
-                      &h->sweep, &h->omega_out, &h->panel32, &h->tc_sched, &h->batch_desc, &h->qx, &h->sigmx})
+    for (DevBuf* b : {&h->pchol, &h->pchol_sl, &h->refine, &h->pqo, &h->xdiag, &h->mo, &h->vxc_diag, &h->delta, &h->v, &h->sigx, &h->xt, &h->dvec, &h->a,
+                      &h->qacc, &h->qall, &h->in, &h->out, &h->sweep, &h->omega_out, &h->panel32, &h->tc_sched, &h->qx,
+                      &h->sigmx})
         b->release();
     for (BatchLane& l : h->lanes) {
         if (l.stream) cudaStreamSynchronize(l.stream);
@@ -856,9 +894,33 @@ void load_system_impl(gwb200_handle* h, int64_t nmo, int64_t nocc, const double*
     h->sigx.ensure(sizeof(double) * nmo);
     h->delta.ensure(sizeof(double) * n);
     size_buffer(h, h->v, sizeof(double) * (size_t)n * n);
-    h->flag.ensure(sizeof(int));
-    std::vector<double> vd((size_t)nmo);
-    for (int64_t p = 0; p < nmo; ++p) vd[(size_t)p] = sl ? sl->vxc_diag[p] : vxc[p * nmo + p];
+    // the small arrays through the pinned buffer: orbital energies, the vxc diagonal and the exchange
+    // diagonal eri[p,i,p,i], whose nocc elements per p lie nmo^2 + 1 apart (as copies of single
+    // elements, one call per p, they took longer than the rest of the upload)
+    h->stage_in.ensure(sizeof(double) * (size_t)(2 * nmo + nmo * nocc));
+    double* hmo = h->stage_in.as<double>();
+    double* hvxc = hmo + nmo;
+    double* hxd = hvxc + nmo;
+    std::memcpy(hmo, mo_energy, sizeof(double) * nmo);
+    for (int64_t p = 0; p < nmo; ++p) hvxc[p] = sl ? sl->vxc_diag[p] : vxc[p * nmo + p];
+    if (sl) {
+        std::memcpy(hxd, sl->xdiag, sizeof(double) * nmo * nocc);
+    } else {
+        for (int64_t p = 0; p < nmo; ++p)
+            for (int64_t i = 0; i < nocc; ++i) hxd[p * nocc + i] = eri[((size_t)(p * nmo + i) * nmo + p) * nmo + i];
+    }
+    GWB_CUDA(cudaMemcpyAsync(h->mo.p, hmo, sizeof(double) * nmo, cudaMemcpyHostToDevice, s));
+    GWB_CUDA(cudaMemcpyAsync(h->vxc_diag.p, hvxc, sizeof(double) * nmo, cudaMemcpyHostToDevice, s));
+    GWB_CUDA(cudaMemcpyAsync(h->xdiag.p, hxd, sizeof(double) * nmo * nocc, cudaMemcpyHostToDevice, s));
+    // some e_a - e_i not > 0 (NaN included): the smallest virtual against the largest occupied energy
+    bool bad = false;
+    double top = -std::numeric_limits<double>::infinity(), bottom = std::numeric_limits<double>::infinity();
+    for (int64_t p = 0; p < nmo; ++p) {
+        if (std::isnan(mo_energy[p])) bad = true;
+        if (p < nocc) top = std::max(top, mo_energy[p]);
+        else bottom = std::min(bottom, mo_energy[p]);
+    }
+    bad = bad || !(bottom - top > 0.0);
     if (sl) {  // already in the device layouts: contiguous copies
         GWB_CUDA(cudaMemcpyAsync(h->v.p, sl->vph, sizeof(double) * (size_t)n * n, cudaMemcpyHostToDevice, s));
         GWB_CUDA(cudaMemcpyAsync(h->xt.p, sl->panel, sizeof(double) * (size_t)nstates * nmo * n, cudaMemcpyHostToDevice,
@@ -889,28 +951,17 @@ void load_system_impl(gwb200_handle* h, int64_t nmo, int64_t nocc, const double*
         GWB_CUDA(cudaMemcpy2DAsync(h->pqo.p, sizeof(double) * nocc * nmo, eri, sizeof(double) * nmo2,
                                    sizeof(double) * nocc * nmo, nmo2, cudaMemcpyHostToDevice, s));
     }
-    // exchange diagonal eri[p,i,p,i]: for each p, nocc elements with stride nmo^2 + 1
-    if (sl) GWB_CUDA(cudaMemcpyAsync(h->xdiag.p, sl->xdiag, sizeof(double) * nmo * nocc, cudaMemcpyHostToDevice, s));
-    for (int64_t p = 0; p < nmo && !sl; ++p)
-        GWB_CUDA(cudaMemcpy2DAsync(h->xdiag.as<double>() + p * nocc, sizeof(double),
-                                   eri + ((size_t)p * nmo * nmo + p) * nmo, sizeof(double) * (nmo2 + 1),
-                                   sizeof(double), nocc, cudaMemcpyHostToDevice, s));
-    GWB_CUDA(cudaMemcpyAsync(h->mo.p, mo_energy, sizeof(double) * nmo, cudaMemcpyHostToDevice, s));
-    GWB_CUDA(cudaMemcpyAsync(h->vxc_diag.p, vd.data(), sizeof(double) * nmo, cudaMemcpyHostToDevice, s));
-    GWB_CUDA(cudaMemsetAsync(h->flag.p, 0, sizeof(int), s));
-    launch_delta(h->mo.as<double>(), nmo, nocc, h->delta.as<double>(), h->flag.as<int>(), s);
+    launch_delta(h->mo.as<double>(), nmo, nocc, h->delta.as<double>(), s);
     if (!bound)
         kprof(h, kKprofGatherVph, 16.0 * (double)n * (double)n,
               [&] { return (int64_t)launch_gather_vph(h->pqo.as<double>(), nmo, nocc, h->v.as<double>(), s); });
     launch_sigma_x_diag(h->xdiag.as<double>(), nmo, nocc, h->sigx.as<double>(), s);
-    int bad = 0;
-    GWB_CUDA(cudaMemcpyAsync(&bad, h->flag.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     GWB_CUDA(cudaStreamSynchronize(s));
     h->nmo = nmo;
     h->nocc = nocc;
     h->n = n;
     h->fermi = fermi_energy;
-    h->bad_gap = bad != 0;
+    h->bad_gap = bad;
     if (bound) h->bound_states.assign(states, states + nstates);
     h->loaded = true;
 }
@@ -943,10 +994,10 @@ int gwb200_read_resident(gwb200_handle* h, const int64_t* states, int64_t nstate
                 if (!std::equal(states, states + nstates, h->bound_states.begin(), h->bound_states.end()))
                     fail(GWB200_BAD_ARGUMENT, "the state list must be the one given to gwb200_load_system_states");
             } else {  // the panel rows a screening call would gather from the resident (pq|o.) block
-                h->states.ensure(sizeof(int64_t) * nstates);
+                h->in.ensure(sizeof(int64_t) * nstates);
                 size_buffer(h, h->xt, nb);
-                GWB_CUDA(cudaMemcpyAsync(h->states.p, states, sizeof(int64_t) * nstates, cudaMemcpyHostToDevice, s));
-                launch_gather_panel(h->pqo.as<double>(), h->nmo, h->nocc, h->states.as<int64_t>(), nstates,
+                GWB_CUDA(cudaMemcpyAsync(h->in.p, states, sizeof(int64_t) * nstates, cudaMemcpyHostToDevice, s));
+                launch_gather_panel(h->pqo.as<double>(), h->nmo, h->nocc, h->in.as<int64_t>(), nstates,
                                     h->xt.as<double>(), s);
             }
             GWB_CUDA(cudaMemcpyAsync(panel_out, h->xt.p, nb, cudaMemcpyDeviceToHost, s));
@@ -1022,15 +1073,12 @@ int gwb200_sigma_c(gwb200_handle* h, const double* omega, const double* weight, 
         gwb200_stats* st = stats ? stats : &local;
         *st = gwb200_stats{};
         compute_forms(h, omega, nfreq, states, nstates, eta, precision, st, weight);
+        size_results(h, nstates, nfreq);
         contract_on_device(h, nfreq, nstates, st);
-        finish_forms(h, st);
+        finish_forms(h, st, {{h->call.sigma, sizeof(double) * 2 * (size_t)nstates * nfreq}});
         st->device_ms_contract = elapsed(h->ev[2], h->ev[3]);
         st->device_ms_total = elapsed(h->ev[0], h->ev[3]);
-        const size_t nb_sig = sizeof(double) * 2 * (size_t)h->nmo * nfreq;
-        h->stage_out.ensure(nb_sig);
-        GWB_CUDA(cudaMemcpyAsync(h->stage_out.p, h->sigma.p, nb_sig, cudaMemcpyDeviceToHost, h->stream));
-        GWB_CUDA(cudaStreamSynchronize(h->stream));
-        std::memcpy(sigma_out, h->stage_out.p, nb_sig);
+        scatter_sigma(h, result_stage(h), states, nstates, nfreq, sigma_out);
     });
 }
 
@@ -1055,16 +1103,13 @@ int gwb200_sigma_c_matrix(gwb200_handle* h, const double* omega, const double* w
         const size_t sig_bytes = sizeof(double) * 2 * (size_t)ns * ns * nfreq;
         size_buffer(h, h->sigmx, sig_bytes);
         st->kernel_launches += launch_sigma_contract_pairs(
-            h->qx.as<double>(), nfreq, h->nmo, ns, h->mo.as<double>(), h->fermi, h->omega.as<double>(),
-            h->weight.as<double>(), h->omega.as<double>(), nfreq, h->sigmx.as<double>(), s);
+            h->qx.as<double>(), nfreq, h->nmo, ns, h->mo.as<double>(), h->fermi, h->call.omega, h->call.weight,
+            h->call.omega, nfreq, h->sigmx.as<double>(), s);
         GWB_CUDA(cudaEventRecord(h->ev[3], s));
-        finish_forms(h, st);
+        finish_forms(h, st, {{h->sigmx.p, sig_bytes}});
         st->device_ms_contract = elapsed(h->ev[2], h->ev[3]);
         st->device_ms_total = elapsed(h->ev[0], h->ev[3]);
-        h->stage_out.ensure(sig_bytes);
-        GWB_CUDA(cudaMemcpyAsync(h->stage_out.p, h->sigmx.p, sig_bytes, cudaMemcpyDeviceToHost, s));
-        GWB_CUDA(cudaStreamSynchronize(s));
-        std::memcpy(sigma_out, h->stage_out.p, sig_bytes);
+        std::memcpy(sigma_out, result_stage(h), sig_bytes);
     });
 }
 
@@ -1079,7 +1124,6 @@ int gwb200_sigma_c_shard(gwb200_handle* h, const double* omega, const double* we
         gwb200_stats local{};
         gwb200_stats* st = stats ? stats : &local;
         *st = gwb200_stats{};
-        const size_t sig_bytes = sizeof(double) * 2 * (size_t)h->nmo * nfreq;
         if (f_begin == f_end) {  // empty shard: contributes nothing
             std::fill(sigma_partial_out, sigma_partial_out + 2 * (size_t)h->nmo * nfreq, 0.0);
             return;
@@ -1088,12 +1132,12 @@ int gwb200_sigma_c_shard(gwb200_handle* h, const double* omega, const double* we
         h->omega_out.ensure(sizeof(double) * nfreq);
         GWB_CUDA(cudaMemcpyAsync(h->omega_out.p, omega, sizeof(double) * nfreq, cudaMemcpyHostToDevice, s));
         compute_forms(h, omega + f_begin, f_end - f_begin, states, nstates, eta, precision, st, weight + f_begin);
+        size_results(h, nstates, nfreq);
         contract_on_device(h, f_end - f_begin, nstates, st, h->omega_out.as<double>(), nfreq);
-        finish_forms(h, st);
+        finish_forms(h, st, {{h->call.sigma, sizeof(double) * 2 * (size_t)nstates * nfreq}});
         st->device_ms_contract = elapsed(h->ev[2], h->ev[3]);
         st->device_ms_total = elapsed(h->ev[0], h->ev[3]);
-        GWB_CUDA(cudaMemcpyAsync(sigma_partial_out, h->sigma.p, sig_bytes, cudaMemcpyDeviceToHost, s));
-        GWB_CUDA(cudaStreamSynchronize(s));
+        scatter_sigma(h, result_stage(h), states, nstates, nfreq, sigma_partial_out);
     });
 }
 
@@ -1110,23 +1154,19 @@ int gwb200_run_g0w0(gwb200_handle* h, int64_t nfreq, int64_t npade, const int64_
         std::vector<double> omega((size_t)nfreq), weight((size_t)nfreq);
         transformed_legendre_grid(nfreq, omega.data(), weight.data());
         compute_forms(h, omega.data(), nfreq, states, nstates, eta, precision, st, weight.data());
+        size_results(h, nstates, nfreq);
         contract_on_device(h, nfreq, nstates, st);
         qp_on_device(h, nfreq, npade, nstates);
-        st->kernel_launches += 2;
-        finish_forms(h, st);
+        st->kernel_launches += 1;
+        const size_t nb_sig = sizeof(double) * 2 * (size_t)nstates * nfreq, nb_qp = sizeof(double) * nstates,
+                     nb_v = sizeof(double) * h->nmo;
+        finish_forms(h, st, {{h->call.sigma, nb_sig + nb_qp}, {h->sigx.p, nb_v}});
         st->device_ms_contract = elapsed(h->ev[2], h->ev[3]);
         st->device_ms_total = elapsed(h->ev[0], h->ev[3]);
-        cudaStream_t s = h->stream;
-        const size_t nb_sig = sizeof(double) * 2 * (size_t)h->nmo * nfreq, nb_v = sizeof(double) * h->nmo;
-        h->stage_out.ensure(nb_sig + 2 * nb_v);
-        char* o = h->stage_out.as<char>();
-        GWB_CUDA(cudaMemcpyAsync(o, h->sigma.p, nb_sig, cudaMemcpyDeviceToHost, s));
-        GWB_CUDA(cudaMemcpyAsync(o + nb_sig, h->sigx.p, nb_v, cudaMemcpyDeviceToHost, s));
-        GWB_CUDA(cudaMemcpyAsync(o + nb_sig + nb_v, h->qp.p, nb_v, cudaMemcpyDeviceToHost, s));
-        GWB_CUDA(cudaStreamSynchronize(s));
-        if (sigma_out) std::memcpy(sigma_out, o, nb_sig);
-        if (sigma_x_out) std::memcpy(sigma_x_out, o + nb_sig, nb_v);
-        if (qp_out) std::memcpy(qp_out, o + nb_sig + nb_v, nb_v);
+        const char* o = result_stage(h);
+        if (sigma_out) scatter_sigma(h, o, states, nstates, nfreq, sigma_out);
+        if (qp_out) scatter_qp(h, o + nb_sig, states, nstates, qp_out);
+        if (sigma_x_out) std::memcpy(sigma_x_out, o + nb_sig + nb_qp, nb_v);
         if (omega_out) std::copy(omega.begin(), omega.end(), omega_out);
         if (weight_out) std::copy(weight.begin(), weight.end(), weight_out);
     });
@@ -1150,16 +1190,27 @@ int gwb200_qp(gwb200_handle* h, const double* omega, int64_t nfreq, const double
         if (npade <= 0) fail(GWB200_BAD_SHAPE, "Pade: npar must be positive");
         check_states(h, states, nstates);
         cudaStream_t s = h->stream;
-        const size_t sig_bytes = sizeof(double) * 2 * (size_t)h->nmo * nfreq;
-        h->omega.ensure(sizeof(double) * nfreq);
-        h->sigma.ensure(sig_bytes);
-        h->states.ensure(sizeof(int64_t) * nstates);
-        GWB_CUDA(cudaMemcpyAsync(h->omega.p, omega, sizeof(double) * nfreq, cudaMemcpyHostToDevice, s));
-        GWB_CUDA(cudaMemcpyAsync(h->sigma.p, sigma, sig_bytes, cudaMemcpyHostToDevice, s));
-        GWB_CUDA(cudaMemcpyAsync(h->states.p, states, sizeof(int64_t) * nstates, cudaMemcpyHostToDevice, s));
+        // grid, the states' rows and the state list: one pinned upload; one read back
+        const size_t nb_om = sizeof(double) * nfreq, nb_st = sizeof(int64_t) * nstates;
+        const size_t nb_sig = 2 * nb_om * (size_t)nstates, nb_qp = sizeof(double) * nstates;
+        h->in.ensure(nb_om + nb_sig + nb_st);
+        h->stage_in.ensure(nb_om + nb_sig + nb_st);
+        char* p = h->stage_in.as<char>();
+        std::memcpy(p, omega, nb_om);
+        for (int64_t i = 0; i < nstates; ++i)
+            std::memcpy(p + nb_om + 2 * nb_om * (size_t)i, sigma + 2 * (size_t)(states[i] * nfreq), 2 * nb_om);
+        std::memcpy(p + nb_om + nb_sig, states, nb_st);
+        GWB_CUDA(cudaMemcpyAsync(h->in.p, p, nb_om + nb_sig + nb_st, cudaMemcpyHostToDevice, s));
+        h->call.omega = h->in.as<double>();
+        h->call.sigma = h->call.omega + nfreq;
+        h->call.states = reinterpret_cast<int64_t*>(h->call.sigma + 2 * (size_t)nstates * nfreq);
+        h->out.ensure(nb_qp);
+        h->call.qp = h->out.as<double>();
         qp_on_device(h, nfreq, npade, nstates);
-        GWB_CUDA(cudaMemcpyAsync(qp_out, h->qp.p, sizeof(double) * h->nmo, cudaMemcpyDeviceToHost, s));
+        h->stage_out.ensure(nb_qp);
+        GWB_CUDA(cudaMemcpyAsync(h->stage_out.p, h->call.qp, nb_qp, cudaMemcpyDeviceToHost, s));
         GWB_CUDA(cudaStreamSynchronize(s));
+        scatter_qp(h, h->stage_out.as<char>(), states, nstates, qp_out);
     });
 }
 
@@ -1268,7 +1319,7 @@ size_t batch_avail(const gwb200_handle* w) {
     size_t avail = free_b + held;
     if (w->mem_limit > 0) {
         size_t resident = (size_t)1 << 20;
-        for (const DevBuf* b : {&w->pqo, &w->xdiag, &w->v, &w->xt, &w->dvec, &w->qall, &w->sigma, &w->a,
+        for (const DevBuf* b : {&w->pqo, &w->xdiag, &w->v, &w->xt, &w->dvec, &w->qall, &w->out, &w->a,
                                 &w->qacc, &w->panel32})
             resident += b->bytes;
         const size_t lim = (size_t)w->mem_limit;
@@ -1344,15 +1395,16 @@ std::vector<int64_t> batch_graph_key(const gwb200_handle* w, const std::vector<g
         gkey.push_back(nstates[i]);
         gkey.insert(gkey.end(), states[i], states[i] + nstates[i]);
         gkey.push_back(h->bound_states.empty() ? 0 : 1);
-        for (const DevBuf* b : {&h->pqo, &h->v, &h->xt, &h->dvec, &h->qall, &h->sigma, &h->qp, &h->omega,
-                                &h->weight, &h->states, &h->delta, &h->mo, &h->sigx, &h->vxc_diag})
+        for (const DevBuf* b : {&h->pqo, &h->v, &h->xt, &h->dvec, &h->qall, &h->delta, &h->mo, &h->sigx, &h->vxc_diag})
             put(b->p);
+        for (const void* p : {(const void*)h->call.omega, (const void*)h->call.weight, (const void*)h->call.states,
+                              (const void*)h->call.sigma, (const void*)h->call.qp})
+            put(p);
         put(h->pchol_ct);
         put(h->pchol_sl.p);
         gkey.push_back(h->pchol_rank);
     }
-    put(w->batch_desc.p);
-    put(w->err.p);
+    put(w->in.p);
     put(w->stage_in.p);
     put(w->batch_fork);
     for (int l = 0; l < lanes; ++l) {
@@ -1456,16 +1508,12 @@ int gwb200_run_g0w0_batch(gwb200_handle* const* systems, int64_t nsys, const int
             gwb200_handle* h = hs[(size_t)i];
             const TallGeometry gi = make_geometry(h->n, ms[(size_t)i]);
             const int64_t nfreq = fs[(size_t)i];
-            h->omega.ensure(sizeof(double) * nfreq);
-            h->weight.ensure(sizeof(double) * nfreq);
-            h->states.ensure(sizeof(int64_t) * nstates[i]);
             if (h->bound_states.empty()) size_buffer(h, h->xt, sizeof(double) * (size_t)ms[(size_t)i] * h->n);
             size_buffer(h, h->dvec, sizeof(double) * (size_t)nfreq * gi.n_pad);
             size_buffer(h, h->qall, sizeof(double) * (size_t)nfreq * gi.m_pad);
             h->complex_forms = false;
             nb_states += sizeof(int64_t) * nstates[i];
         }
-        w->err.ensure(sizeof(unsigned long long));
         int lane_ctas = 0;
         const int lanes = batch_lanes(w, nsys, &lane_ctas);
 
@@ -1529,7 +1577,16 @@ int gwb200_run_g0w0_batch(gwb200_handle* const* systems, int64_t nsys, const int
             }
         }
         if (!w->batch_fork) GWB_CUDA(cudaEventCreateWithFlags(&w->batch_fork, cudaEventDisableTiming));
-        w->batch_desc.ensure(sizeof(BatchGroup) * groups.size());
+        // the call's inputs in one upload: the pivot word, one grid (omega, weights) per distinct frequency
+        // count, the state lists, the group tables
+        std::map<int64_t, size_t> grid_off;
+        size_t groups_off = sizeof(unsigned long long);
+        for (int64_t f : fs)
+            if (grid_off.emplace(f, groups_off).second) groups_off += 2 * sizeof(double) * (size_t)f;
+        const size_t states_off = groups_off;
+        groups_off += nb_states;
+        const size_t nb_in = groups_off + sizeof(BatchGroup) * groups.size();
+        w->in.ensure(nb_in);
         std::vector<std::vector<std::vector<size_t>>> assign;
         for (const auto& ch : chunks) assign.push_back(batch_assign(ch, lanes, batch_step_us(mixed), batch_tflops(mixed)));
         // FP64: the update kernel of each chunk geometry (timed before anything is built: the
@@ -1541,37 +1598,37 @@ int gwb200_run_g0w0_batch(gwb200_handle* const* systems, int64_t nsys, const int
                                             : tune_update_variant(ch.g, ch.nmat, w->lanes[0].a.as<double>(), s,
                                                                   oz ? w->lanes[0].panel.p : nullptr,
                                                                   w->lanes[0].sched.as<unsigned long long>(),
-                                                                  w->err.as<unsigned long long>(), w->mem_limit <= 0));
+                                                                  w->err(), w->mem_limit <= 0));
 
-        // the lead handle's pinned staging buffer, filled on the host before anything is issued:
-        // grid, every member's state list, group tables
-        // one grid (omega, weights) per distinct frequency count, then the state lists, then the
-        // group tables
-        std::map<int64_t, size_t> grid_off;
-        size_t nb_grids = 0;
-        for (int64_t f : fs)
-            if (grid_off.emplace(f, nb_grids).second) nb_grids += 2 * sizeof(double) * (size_t)f;
-        const size_t nb_groups = sizeof(BatchGroup) * groups.size();
-        w->stage_in.ensure(nb_grids + nb_states + nb_groups);
+        // the lead handle's pinned staging buffer, filled on the host before anything is issued
+        w->stage_in.ensure(nb_in);
         char* sp = w->stage_in.as<char>();
+        std::memset(sp, 0xFF, sizeof(unsigned long long));
         for (const auto& [f, off] : grid_off)
             transformed_legendre_grid(f, reinterpret_cast<double*>(sp + off),
                                       reinterpret_cast<double*>(sp + off) + f);
-        std::vector<size_t> st_off((size_t)nsys);
+        std::memcpy(sp + groups_off, groups.data(), sizeof(BatchGroup) * groups.size());
+        // results of all members, each [nstates][nfreq] complex and nstates QP energies, read back at once
+        size_t nb_out = 0;
+        std::vector<size_t> out_off;
+        for (int64_t i = 0; i < nsys; ++i) {
+            out_off.push_back(nb_out);
+            nb_out += sizeof(double) * (size_t)nstates[i] * (2 * (size_t)fs[(size_t)i] + 1);
+        }
+        w->out.ensure(nb_out);
         {
-            size_t off = nb_grids;
+            size_t off = states_off;
             for (int64_t i = 0; i < nsys; ++i) {
-                st_off[(size_t)i] = off;
+                gwb200_handle* h = hs[(size_t)i];
+                const int64_t nfreq = fs[(size_t)i];
                 std::memcpy(sp + off, states[i], sizeof(int64_t) * nstates[i]);
+                h->call.omega = reinterpret_cast<double*>(w->in.as<char>() + grid_off.at(nfreq));
+                h->call.weight = h->call.omega + nfreq;
+                h->call.states = reinterpret_cast<int64_t*>(w->in.as<char>() + off);
+                h->call.sigma = reinterpret_cast<double*>(w->out.as<char>() + out_off[(size_t)i]);
+                h->call.qp = h->call.sigma + 2 * (size_t)nstates[i] * nfreq;
                 off += sizeof(int64_t) * nstates[i];
             }
-        }
-        const size_t groups_off = nb_grids + nb_states;
-        std::memcpy(sp + groups_off, groups.data(), nb_groups);
-        for (int64_t i = 0; i < nsys; ++i) {  // every buffer the device sequence touches, sized now
-            gwb200_handle* h = hs[(size_t)i];
-            h->sigma.ensure(sizeof(double) * 2 * (size_t)h->nmo * fs[(size_t)i]);
-            h->qp.ensure(sizeof(double) * h->nmo);
         }
         // the lanes fork off the lead stream and join back onto it around each phase
         auto lane_stream = [&](int l) { return l == 0 ? s : w->lanes[l].stream; };
@@ -1585,28 +1642,22 @@ int gwb200_run_g0w0_batch(gwb200_handle* const* systems, int64_t nsys, const int
                 GWB_CUDA(cudaStreamWaitEvent(s, w->lanes[l].done, 0));
             }
         };
-        const BatchGroup* dgroups = w->batch_desc.as<BatchGroup>();
+        const BatchGroup* dgroups = reinterpret_cast<const BatchGroup*>(w->in.as<char>() + groups_off);
         // the device sequence in three phases: uploads and member preparation; the screening of a
         // plan (each lane runs its chunks); members' contractions and QP updates
         auto prefix = [&]() {
             int64_t n_launch = 0;
-            GWB_CUDA(cudaMemcpyAsync(w->batch_desc.p, sp + groups_off, nb_groups, cudaMemcpyHostToDevice, s));
-            GWB_CUDA(cudaMemsetAsync(w->err.p, 0xFF, sizeof(unsigned long long), s));
+            GWB_CUDA(cudaMemcpyAsync(w->in.p, sp, nb_in, cudaMemcpyHostToDevice, s));
             fork();
             for (int64_t i = 0; i < nsys; ++i) {
                 gwb200_handle* h = hs[(size_t)i];
                 cudaStream_t ls = lane_stream((int)(i % lanes));
                 const int64_t nfreq = fs[(size_t)i];
-                const size_t nb_om = sizeof(double) * nfreq, goff = grid_off.at(nfreq);
-                GWB_CUDA(cudaMemcpyAsync(h->omega.p, sp + goff, nb_om, cudaMemcpyHostToDevice, ls));
-                GWB_CUDA(cudaMemcpyAsync(h->weight.p, sp + goff + nb_om, nb_om, cudaMemcpyHostToDevice, ls));
-                GWB_CUDA(cudaMemcpyAsync(h->states.p, sp + st_off[(size_t)i], sizeof(int64_t) * nstates[i],
-                                         cudaMemcpyHostToDevice, ls));
                 if (h->bound_states.empty())
-                    n_launch += launch_gather_panel(h->pqo.as<double>(), h->nmo, h->nocc, h->states.as<int64_t>(),
-                                                    nstates[i], h->xt.as<double>(), ls);
+                    n_launch += launch_gather_panel(h->pqo.as<double>(), h->nmo, h->nocc, h->call.states, nstates[i],
+                                                    h->xt.as<double>(), ls);
                 n_launch += launch_scale_vectors(h->delta.as<double>(), h->n, make_geometry(h->n, ms[(size_t)i]).n_pad,
-                                                 h->omega.as<double>(), nfreq, h->dvec.as<double>(), ls);
+                                                 h->call.omega, nfreq, h->dvec.as<double>(), ls);
             }
             join();
             return n_launch;
@@ -1629,7 +1680,7 @@ int gwb200_run_g0w0_batch(gwb200_handle* const* systems, int64_t nsys, const int
                 qp_on_device(hs[(size_t)i], fs[(size_t)i], ps[(size_t)i], nstates[i]);
             }
             join();
-            return scratch.kernel_launches + 2 * nsys;
+            return scratch.kernel_launches + nsys;
         };
 
         // CUDA graph of the whole sequence for a repeated batch (one plan, nothing to time):
@@ -1714,20 +1765,10 @@ int gwb200_run_g0w0_batch(gwb200_handle* const* systems, int64_t nsys, const int
         }
         st->kernel_launches = launches;
         // results and the pivot word back in one synchronisation
-        size_t nb_out = sizeof(unsigned long long);
-        for (int64_t i = 0; i < nsys; ++i)
-            nb_out += sizeof(double) * (2 * (size_t)hs[(size_t)i]->nmo * fs[(size_t)i] + hs[(size_t)i]->nmo);
-        w->stage_out.ensure(nb_out);
+        w->stage_out.ensure(sizeof(unsigned long long) + nb_out);
         char* op = w->stage_out.as<char>();
-        GWB_CUDA(cudaMemcpyAsync(op, w->err.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-        size_t o = sizeof(unsigned long long);
-        for (int64_t i = 0; i < nsys; ++i) {
-            const gwb200_handle* h = hs[(size_t)i];
-            const size_t nb_sig = sizeof(double) * 2 * (size_t)h->nmo * fs[(size_t)i], nb_qp = sizeof(double) * h->nmo;
-            GWB_CUDA(cudaMemcpyAsync(op + o, h->sigma.p, nb_sig, cudaMemcpyDeviceToHost, s));
-            GWB_CUDA(cudaMemcpyAsync(op + o + nb_sig, h->qp.p, nb_qp, cudaMemcpyDeviceToHost, s));
-            o += nb_sig + nb_qp;
-        }
+        GWB_CUDA(cudaMemcpyAsync(op, w->in.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+        GWB_CUDA(cudaMemcpyAsync(op + sizeof(unsigned long long), w->out.p, nb_out, cudaMemcpyDeviceToHost, s));
         GWB_CUDA(cudaStreamSynchronize(s));
         unsigned long long piv = 0;
         std::memcpy(&piv, op, sizeof(piv));
@@ -1737,13 +1778,12 @@ int gwb200_run_g0w0_batch(gwb200_handle* const* systems, int64_t nsys, const int
             fail(GWB200_NOT_SPD, "eps(iw) of a batch member is not positive definite: Cholesky pivot " +
                                      std::to_string(piv) + " <= 0");
         }
-        o = sizeof(unsigned long long);
         for (int64_t i = 0; i < nsys; ++i) {
             const gwb200_handle* h = hs[(size_t)i];
-            const size_t nb_sig = sizeof(double) * 2 * (size_t)h->nmo * fs[(size_t)i], nb_qp = sizeof(double) * h->nmo;
-            if (sigma_out && sigma_out[i]) std::memcpy(sigma_out[i], op + o, nb_sig);
-            if (qp_out && qp_out[i]) std::memcpy(qp_out[i], op + o + nb_sig, nb_qp);
-            o += nb_sig + nb_qp;
+            const char* rows = op + sizeof(unsigned long long) + out_off[(size_t)i];
+            if (sigma_out && sigma_out[i]) scatter_sigma(h, rows, states[i], nstates[i], fs[(size_t)i], sigma_out[i]);
+            if (qp_out && qp_out[i])
+                scatter_qp(h, rows + sizeof(double) * 2 * (size_t)nstates[i] * fs[(size_t)i], states[i], nstates[i], qp_out[i]);
         }
         double flops = 0.0;
         int64_t nmax = 0, mmax = 0;

@@ -114,7 +114,7 @@ int launch_gather_panel(const double* pqo, int64_t nmo, int64_t nocc, const int6
                         double* xt, cudaStream_t s);
 // xdiag[p*nocc + i] = eri[p,i,p,i]
 int launch_sigma_x_diag(const double* xdiag, int64_t nmo, int64_t nocc, double* out, cudaStream_t s);
-int launch_delta(const double* mo, int64_t nmo, int64_t nocc, double* delta, int* bad_gap, cudaStream_t s);
+int launch_delta(const double* mo, int64_t nmo, int64_t nocc, double* delta, cudaStream_t s);
 int launch_scale_vectors(const double* delta, int64_t n, int64_t n_pad, const double* omega, int64_t nf,
                          double* dvec, cudaStream_t s);
 int launch_build_tall(const TallGeometry& g, const double* v, const double* xt, const double* dvec, int64_t nf,
@@ -169,13 +169,11 @@ int launch_cross_forms(const TallGeometry& g, int64_t nf, const double* a, int64
 int launch_sigma_contract_pairs(const double* qx, int64_t nf_int, int64_t nmo, int64_t nstates, const double* mo,
                                 double fermi, const double* omega_int, const double* weight_int,
                                 const double* omega_out, int64_t nf_out, double* sigma, cudaStream_t s);
-// Contraction of the screened forms of nf_int integration frequencies onto nf_out output
+// Contraction ([nstates][nf_out] complex) of the screened forms of nf_int integration frequencies onto nf_out output
 // frequencies (the full grid; a shard of integration frequencies gives a partial sum).
 int launch_sigma_contract(const double* qall, int64_t nf_int, int64_t nstates, int64_t nmo, int64_t ldq,
-                          const int64_t* states, const double* mo, double fermi, const double* omega_int,
-                          const double* weight_int, const double* omega_out, int64_t nf_out, double* sigma,
-                          cudaStream_t s);
-int launch_fill(double* p, double v, int64_t n, cudaStream_t s);
+                          const double* mo, double fermi, const double* omega_int, const double* weight_int,
+                          const double* omega_out, int64_t nf_out, double* sigma, cudaStream_t s);
 int launch_qp(const double* sigma, const double* omega, int64_t nfreq, const int64_t* states, int64_t nstates,
               int64_t npade, const double* mo, double fermi, const double* sigx, const double* vxc_diag, double* qp,
               cudaStream_t s);
@@ -262,9 +260,8 @@ int launch_factor_chunk_c(const TallGeometry& g, int64_t nf, const double* delta
 int launch_forms_out_c(const double* qacc, int64_t nf, int64_t m, int64_t ldq, double* q_out, int64_t ldq_out,
                        cudaStream_t s);
 int launch_sigma_contract_c(const double* qall, int64_t nf_int, int64_t nstates, int64_t nmo, int64_t ldq,
-                            const int64_t* states, const double* mo, double fermi, const double* omega_int,
-                            const double* weight_int, const double* omega_out, int64_t nf_out, double* sigma,
-                            cudaStream_t s);
+                            const double* mo, double fermi, const double* omega_int, const double* weight_int,
+                            const double* omega_out, int64_t nf_out, double* sigma, cudaStream_t s);
 // kernels_batch.cu: one molecule's run of consecutive matrices in a batched chunk (device table).
 struct BatchGroup {
     const double* v;     // V_ph, n x n

@@ -582,7 +582,7 @@ __global__ void k_forms_out_c(const double* __restrict__ qacc, int m, int64_t ld
 // Sigma contraction with complex forms (interleaved [f][2*ldq]):
 // Sigma_c(p_s, i w_n) = -(1/pi) sum_{f', k} w_{f'} g(k, n, f') q[f', s, k].
 __global__ void __launch_bounds__(256) k_sigma_contract_c(const double* __restrict__ qall, int nf_int, int nmo,
-                                                          int64_t ldq, const int64_t* __restrict__ states,
+                                                          int64_t ldq,
                                                           const double* __restrict__ mo, double fermi,
                                                           const double* __restrict__ omega_int,
                                                           const double* __restrict__ weight_int,
@@ -617,10 +617,9 @@ __global__ void __launch_bounds__(256) k_sigma_contract_c(const double* __restri
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        const size_t p = (size_t)states[s];
         const double inv_pi = 1.0 / 3.141592653589793238462643383279502884;
-        sigma[2 * (p * nf_out + fn)] = red[0][0] * inv_pi;
-        sigma[2 * (p * nf_out + fn) + 1] = red[1][0] * inv_pi;
+        sigma[2 * ((size_t)s * nf_out + fn)] = red[0][0] * inv_pi;
+        sigma[2 * ((size_t)s * nf_out + fn) + 1] = red[1][0] * inv_pi;
     }
 }
 
@@ -673,11 +672,10 @@ int launch_forms_out_c(const double* qacc, int64_t nf, int64_t m, int64_t ldq, d
 }
 
 int launch_sigma_contract_c(const double* qall, int64_t nf_int, int64_t nstates, int64_t nmo, int64_t ldq,
-                            const int64_t* states, const double* mo, double fermi, const double* omega_int,
-                            const double* weight_int, const double* omega_out, int64_t nf_out, double* sigma,
-                            cudaStream_t s) {
+                            const double* mo, double fermi, const double* omega_int, const double* weight_int,
+                            const double* omega_out, int64_t nf_out, double* sigma, cudaStream_t s) {
     k_sigma_contract_c<<<dim3((unsigned)nf_out, (unsigned)nstates), 256, 0, s>>>(
-        qall, (int)nf_int, (int)nmo, ldq, states, mo, fermi, omega_int, weight_int, omega_out, (int)nf_out, sigma);
+        qall, (int)nf_int, (int)nmo, ldq, mo, fermi, omega_int, weight_int, omega_out, (int)nf_out, sigma);
     GWB_LAUNCH("k_sigma_contract_c");
     return 1;
 }

@@ -73,15 +73,12 @@ __global__ void k_sigma_x_diag(const double* __restrict__ xdiag, int nmo, int no
 }
 
 // delta[ph] = e_a - e_i with ph = i*nvir + a_vir (include/gw/particle_hole.hpp:22-35).
-__global__ void k_delta(const double* __restrict__ mo, int nmo, int nocc, double* __restrict__ delta,
-                        int* __restrict__ bad_gap) {
+__global__ void k_delta(const double* __restrict__ mo, int nmo, int nocc, double* __restrict__ delta) {
     const int nvir = nmo - nocc, n = nocc * nvir;
     const int ph = blockIdx.x * blockDim.x + threadIdx.x;
     if (ph >= n) return;
     const int i = ph / nvir, a = nocc + ph % nvir;
-    const double d = __dsub_rn(mo[a], mo[i]);
-    delta[ph] = d;
-    if (!(d > 0.0)) atomicExch(bad_gap, 1);
+    delta[ph] = __dsub_rn(mo[a], mo[i]);
 }
 
 // dvec[f, c] = sqrt(D_f[c]) with D = -Pi0(i w_f) = 4 delta / (w^2 + delta^2); zero padding.
@@ -350,9 +347,9 @@ int launch_sigma_x_diag(const double* xdiag, int64_t nmo, int64_t nocc, double* 
     return 1;
 }
 
-int launch_delta(const double* mo, int64_t nmo, int64_t nocc, double* delta, int* bad_gap, cudaStream_t s) {
+int launch_delta(const double* mo, int64_t nmo, int64_t nocc, double* delta, cudaStream_t s) {
     const int64_t n = nocc * (nmo - nocc);
-    k_delta<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(mo, (int)nmo, (int)nocc, delta, bad_gap);
+    k_delta<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(mo, (int)nmo, (int)nocc, delta);
     GWB_LAUNCH("k_delta");
     return 1;
 }

@@ -161,7 +161,7 @@ __device__ __forceinline__ cplx pade_num(const cplx* coeffs, const double* xs_im
     return c_mul(coeffs[k + 1], c_sub(cplx{z, 0.0}, cplx{0.0, xs_im[k]}));
 }
 
-// One warp per requested state: Pade fit of Sigma_c(p, iw) and the fixed-point QP update
+// One warp per requested state (row of sigma, entry of qp): Pade fit of Sigma_c(p, iw) and the fixed-point QP update
 // (src/gw/qp_solver.cpp:18-43), <= 200 iterations, tolerance 1e-6.  Bound by the chain of the
 // evaluations (a state that does not settle takes all 200); the numerators of an evaluation do not
 // depend on each other and are formed by the lanes before it.  60 states, 16 parameters, 100
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(32) k_qp(const double* __restrict__ sigma, con
     __shared__ double xs_im[kMaxPade];
     const int lane = threadIdx.x;
     const int p = (int)states[blockIdx.x];
-    const int na = pade_coeffs(sigma + 2 * (size_t)p * nfreq, omega, nfreq, npade, coeffs, xs_im);
+    const int na = pade_coeffs(sigma + 2 * (size_t)blockIdx.x * nfreq, omega, nfreq, npade, coeffs, xs_im);
     const double e = mo[p], sx = sigx[p], vx = vxc_diag[p];
     const cplx first = coeffs[0];
     double cur = e;
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(32) k_qp(const double* __restrict__ sigma, con
         cur = nq;
         if (done) break;
     }
-    if (lane == 0) qp[p] = cur;
+    if (lane == 0) qp[blockIdx.x] = cur;
 }
 
 // E_c.out sweep (src/io.cpp:94-108): coefficients once per block, one point per thread.
@@ -217,9 +217,9 @@ __global__ void __launch_bounds__(128) k_pade_sweep(const double* __restrict__ s
 // (the reference's accumulation, src/gw/sigma_c_driver.cpp:154-168, with W_c hoisted out of
 // the loop over w_n).  The integration frequencies f' (omega_int, weight_int, rows of qall) may be
 // a shard of the output grid (omega_out): the shards' results then add up to the full sum.
-// One block per (n, s); fixed-shape tree reduction (deterministic).
+// sigma: [state][output frequency].  One block per (n, s); fixed-shape tree reduction (deterministic).
 __global__ void __launch_bounds__(256) k_sigma_contract(const double* __restrict__ qall, int nf_int, int nmo,
-                                                        int64_t ldq, const int64_t* __restrict__ states,
+                                                        int64_t ldq,
                                                         const double* __restrict__ mo, double fermi,
                                                         const double* __restrict__ omega_int,
                                                         const double* __restrict__ weight_int,
@@ -253,15 +253,10 @@ __global__ void __launch_bounds__(256) k_sigma_contract(const double* __restrict
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        const size_t p = (size_t)states[s];
         const double inv_pi = 1.0 / 3.141592653589793238462643383279502884;
-        sigma[2 * (p * nf_out + fn)] = red[0][0] * inv_pi;
-        sigma[2 * (p * nf_out + fn) + 1] = red[1][0] * inv_pi;
+        sigma[2 * ((size_t)s * nf_out + fn)] = red[0][0] * inv_pi;
+        sigma[2 * ((size_t)s * nf_out + fn) + 1] = red[1][0] * inv_pi;
     }
-}
-
-__global__ void k_fill(double* __restrict__ p, double v, int64_t n) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) p[i] = v;
 }
 
 // Short FP64 DMMA throughput probe (8 warps/block, 4 independent accumulators per warp).
@@ -283,19 +278,12 @@ __global__ void k_dmma_probe(double* out, int iters) {
 } // namespace
 
 int launch_sigma_contract(const double* qall, int64_t nf_int, int64_t nstates, int64_t nmo, int64_t ldq,
-                          const int64_t* states, const double* mo, double fermi, const double* omega_int,
-                          const double* weight_int, const double* omega_out, int64_t nf_out, double* sigma,
-                          cudaStream_t s) {
+                          const double* mo, double fermi, const double* omega_int, const double* weight_int,
+                          const double* omega_out, int64_t nf_out, double* sigma, cudaStream_t s) {
     dim3 grid((unsigned)nf_out, (unsigned)nstates);
-    k_sigma_contract<<<grid, 256, 0, s>>>(qall, (int)nf_int, (int)nmo, ldq, states, mo, fermi, omega_int, weight_int,
+    k_sigma_contract<<<grid, 256, 0, s>>>(qall, (int)nf_int, (int)nmo, ldq, mo, fermi, omega_int, weight_int,
                                           omega_out, (int)nf_out, sigma);
     GWB_LAUNCH("k_sigma_contract");
-    return 1;
-}
-
-int launch_fill(double* p, double v, int64_t n, cudaStream_t s) {
-    k_fill<<<(unsigned)std::min<int64_t>((n + 255) / 256, 1024), 256, 0, s>>>(p, v, n);
-    GWB_LAUNCH("k_fill");
     return 1;
 }
 
