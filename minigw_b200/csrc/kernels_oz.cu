@@ -27,7 +27,7 @@
 //                      warp 0     producer: units from a global counter handed on through a
 //                                 4-slot mbarrier ring; loads the unit's A slices 3-6 (128 rows,
 //                                 64 KB, resident for the unit) and streams the B slices (64
-//                                 rows, 8 KB each) through a 15-stage ring;
+//                                 rows, 8 KB each) through a ring of five pairs;
 //                      warp 1     TMEM allocation; lane 0 issues tcgen05.mma kind::i8 (M = 128,
 //                                 N = 64, K = 32 per instruction; A slices 1-2, which take part
 //                                 in 12 of the 26 products, from TMEM (columns 448-511), the
@@ -36,9 +36,9 @@
 //                      warps 2-9  epilogue: at each unit start, write A slices 1-2 into TMEM;
 //                                 per tile, warp w reads lane quadrant w % 4, 32 columns (16
 //                                 columns per tcgen05.wait::ld), combines the levels, scales by
-//                                 2^{e_r + e_c}, stages -value per row (128 bytes per half) and
-//                                 adds it to C with a bulk reduction (cp.reduce.async.bulk
-//                                 .add.f64) per row and half.
+//                                 2^{e_r + e_c}, stages -value per row (256 bytes) and adds it
+//                                 to C with one bulk reduction (cp.reduce.async.bulk .add.f64)
+//                                 per row.
 // The accumulators are drained in two level groups so that the tensor core does not wait for the
 // whole drain: per tile the MMAs of group X (levels 4-8, 23 of the 26 products) run first and are
 // committed, then those of group Y (levels 2-3, 3 products).  The epilogue reads group X (keeping
@@ -67,21 +67,21 @@ constexpr int kOzSlices = 6;                 // digit slices per value
 constexpr int kOzLevels = 7;                 // levels s + t = 2..8, one accumulator each
 constexpr int kOzMaxSum = kOzLevels - 1;     // 0-based slice indices: products with sa + t <= 6
 constexpr int kOzSeg = 32;                   // column tiles per work unit
-constexpr int kOzStages = 15;                // B ring depth (one slice per stage): a tile's 6, the 2 held
-                                             // for group Y, and 7 ahead
+constexpr int kOzStages = 5;                 // B ring depth, in pairs of slices (three per tile)
 constexpr int kOzTmemSlices = 2;             // A slices 1-2 (12 of the 26 products) read from TMEM
 constexpr int kSchedSlots = 4;
 constexpr int kSliceA = kOzM * 128;          // one slice of 128 rows: 16 KB
 constexpr int kSliceB = kOzN * 128;          // of 64 rows: 8 KB
+constexpr int kStageB = 2 * kSliceB;
 constexpr int kEpiWarps = 8;                 // 4 lane quadrants x 2 column halves of 32
 constexpr int kOzThreads = 32 * (2 + kEpiWarps);
 constexpr int kTmemCols = 512;               // 7 levels x 64 columns, then A slices 1-2 (32 each)
 constexpr int kTmemA = kOzLevels * kOzN;     // first column of the A slices held in TMEM
 static_assert(kTmemA + 32 * kOzTmemSlices <= kTmemCols, "TMEM columns");
-constexpr int kStgRow = 128 + 16;            // staging row stride: 16 doubles + 16 bytes (banks)
+constexpr int kStgRow = 256 + 16;            // staging row stride: 32 doubles + 16 bytes (banks)
 constexpr int kStgBytes = 32 * kStgRow;      // per epilogue warp
 constexpr int kHeader = 1024;
-constexpr int kOzSmem = kHeader + 1024 + (kOzSlices - kOzTmemSlices) * kSliceA + kOzStages * kSliceB + kEpiWarps * kStgBytes;
+constexpr int kOzSmem = kHeader + 1024 + (kOzSlices - kOzTmemSlices) * kSliceA + kOzStages * kStageB + kEpiWarps * kStgBytes;
 
 constexpr int kOffFull = 0;
 constexpr int kOffEmpty = kOffFull + 8 * kOzStages;
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
     const uint32_t base = smem_u32(osm);
     const uint32_t abuf = (base + kHeader + 1023u) & ~1023u;  // A slices 3-6, 1024-aligned
     const uint32_t ring = abuf + (kOzSlices - kOzTmemSlices) * kSliceA;  // B stages (A slices 3-6 before)
-    const uint32_t stg0 = ring + kOzStages * kSliceB;          // epilogue staging rows
+    const uint32_t stg0 = ring + kOzStages * kStageB;          // epilogue staging rows
     volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(osm + kOffAbort);
     volatile int64_t* uslot = reinterpret_cast<volatile int64_t*>(osm + kOffUnit);
     auto full = [&](int s) { return base + kOffFull + 8 * s; };
@@ -255,83 +255,61 @@ __global__ void __launch_bounds__(kOzThreads, 1)
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(osm + kOffTmem);
     const size_t fbytes = oz_freq_bytes(rp);
 
-    if (warp == 0) {
-        // ---- producer ----
+    if (warp == 0 && lane == 0) {
+        // ---- producer (one thread: handing a stage over costs ~400 cycles, ~1,300 with the warp in step) ----
         int s = 0, js = 0;
         uint32_t ph = 0, aph = 0, jph = 0;
         uint32_t filled = 0, fill_par = 0;
-        bool a_filled = false;
-        for (;;) {
+        bool a_filled = false, ok = true;
+        const size_t slice_bytes = (size_t)rp * 128;
+        while (ok) {
             int f = 0;
             int64_t i = 0, c0 = 0, c1 = 0, u = 0;
-            if (lane == 0) {
-                do {
-                    u = (int64_t)atomicAdd(sched, 1ull);
-                } while (u < us.total && !decode_unit(us, u, f, i, c0, c1));
-                if (u > us.total) u = us.total;
-            }
-            u = __shfl_sync(0xffffffffu, u, 0);
-            uint32_t got = 1;
-            if (lane == 0) {
-                got = mbar_wait(uempty(js), jph ^ 1u, abort_flag, err) ? 1u : 0u;
-                if (got) {
-                    uslot[js] = u;
-                    mbar_arrive(ufull(js));
-                }
-            }
-            got = __shfl_sync(0xffffffffu, got, 0);
-            if (!got) break;
+            do {
+                u = (int64_t)atomicAdd(sched, 1ull);
+            } while (u < us.total && !decode_unit(us, u, f, i, c0, c1));
+            if (u > us.total) u = us.total;
+            if (!mbar_wait(uempty(js), jph ^ 1u, abort_flag, err)) break;
+            uslot[js] = u;
+            mbar_arrive(ufull(js));
             if (++js == kSchedSlots) {
                 js = 0;
                 jph ^= 1u;
             }
             if (u >= us.total) break;
-            decode_unit(us, u, f, i, c0, c1);
             const uint8_t* slices = buf + (size_t)f * fbytes;
-            if (lane == 0) got = mbar_wait(aempty, aph ^ 1u, abort_flag, err) ? 1u : 0u;
-            got = __shfl_sync(0xffffffffu, got, 0);
-            if (!got) break;
-            if (lane == 0) mbar_expect_tx(afull, (uint32_t)((kOzSlices - kOzTmemSlices) * kSliceA));
-            __syncwarp();
-            if (lane < kOzSlices - kOzTmemSlices)  // one 16 KB copy per smem slice (slices 3-6)
-                bulk_g2s(abuf + lane * kSliceA, slices + ((size_t)(lane + kOzTmemSlices) * rp + i * kOzM) * 128, kSliceA,
-                         afull);
+            if (!mbar_wait(aempty, aph ^ 1u, abort_flag, err)) break;
+            mbar_expect_tx(afull, (uint32_t)((kOzSlices - kOzTmemSlices) * kSliceA));
+            for (int j = kOzTmemSlices; j < kOzSlices; ++j)  // one 16 KB copy per smem slice (slices 3-6)
+                bulk_g2s(abuf + (j - kOzTmemSlices) * kSliceA, slices + (size_t)j * slice_bytes + i * kSliceA, kSliceA, afull);
             a_filled = true;
             aph ^= 1u;
-            bool ok = true;
             for (int64_t c = c0; ok && c < c1; ++c) {
-                for (int t = 0; t < kOzSlices; ++t) {
-                    if (lane == 0) got = mbar_wait(empty(s), ph ^ 1u, abort_flag, err) ? 1u : 0u;
-                    got = __shfl_sync(0xffffffffu, got, 0);
-                    if (!got) {
+                const uint8_t* src = slices + c * kSliceB;
+                for (int t = 0; t < kOzSlices; t += 2, src += 2 * slice_bytes) {
+                    if (!mbar_wait_fast(empty(s), ph ^ 1u, abort_flag, err)) {
                         ok = false;
                         break;
                     }
                     if (withhold_first_stage && blockIdx.x == 0 && filled == 0) {
                         withhold_first_stage = 0;  // test of the bounded waits (see kernels_tc.cu)
                     } else {
-                        if (lane == 0) {
-                            mbar_expect_tx(full(s), (uint32_t)kSliceB);
-                            bulk_g2s(ring + s * kSliceB, slices + ((size_t)t * rp + c * kOzN) * 128, kSliceB, full(s));
-                        }
+                        mbar_expect_tx(full(s), (uint32_t)kStageB);
+                        bulk_g2s(ring + s * kStageB, src, kSliceB, full(s));
+                        bulk_g2s(ring + s * kStageB + kSliceB, src + slice_bytes, kSliceB, full(s));
                         filled |= 1u << s;
                         fill_par = (fill_par & ~(1u << s)) | (ph << s);
                     }
-                    __syncwarp();
                     if (++s == kOzStages) {
                         s = 0;
                         ph ^= 1u;
                     }
                 }
             }
-            if (!ok) break;
         }
-        if (lane == 0) {
-            for (int q = 0; q < kOzStages; ++q)
-                if (filled & (1u << q)) mbar_drain(full(q), (fill_par >> q) & 1u);
-            if (a_filled) mbar_drain(afull, aph ^ 1u);
-        }
-        __syncwarp();
+        for (int q = 0; q < kOzStages; ++q)
+            if (filled & (1u << q)) mbar_drain(full(q), (fill_par >> q) & 1u);
+        if (a_filled) mbar_drain(afull, aph ^ 1u);
     } else if (warp == 1 && lane == 0) {
         // ---- MMA issuer ----
         const uint64_t desc_a0 = smem_desc_sw128(abuf), desc_b0 = smem_desc_sw128(ring);
@@ -352,14 +330,14 @@ __global__ void __launch_bounds__(kOzThreads, 1)
             if (!mbar_wait(atmem, aph, abort_flag, err)) break;
             tc_fence_after();
             aph ^= 1u;
-            // A slice sa+1 against B slice t+1 (in stage st) into level sa + t + 2.  Products are
+            // A slice sa+1 against B slice t+1 (of stage st) into level sa + t + 2.  Products are
             // issued with t ascending, so the first product of level sa + t has the smallest t
             // the level allows, t0 = max(0, sa + t - (kOzSlices - 1)); it starts the accumulator
             // at kk = 0 (level 8 has no t = 0 product: it starts at sa = 6, t = 2, 1-based)
             auto pair = [&](int sa, int t, int st) {
                 // descriptors differ from the stage / A bases only in the address field (bytes >>
                 // 4, below 2^14 for shared memory): constant offsets, no carries
-                const uint64_t db0 = desc_b0 + (uint64_t)((uint32_t)(st * kSliceB) >> 4);
+                const uint64_t db0 = desc_b0 + (uint64_t)((uint32_t)(st * kStageB + (t & 1) * kSliceB) >> 4);
                 const uint32_t d = tmem + (uint32_t)((sa + t) * kOzN);
                 const bool starts = t == (sa + t > kOzSlices - 1 ? sa + t - (kOzSlices - 1) : 0);
 #pragma unroll
@@ -379,22 +357,21 @@ __global__ void __launch_bounds__(kOzThreads, 1)
                     break;
                 }
                 tc_fence_after();
-                int st01[2] = {0, 0};  // stages of B slices 1-2, held for group Y
+                const int s0 = s;  // B slices 1-2, held for group Y
 #pragma unroll
-                for (int t = 0; t < kOzSlices; ++t) {
+                for (int t2 = 0; t2 < kOzSlices; t2 += 2) {
                     if (!mbar_wait_fast(full(s), ph, abort_flag, err)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-#pragma unroll
-                    for (int sa = 0; sa < kOzSlices; ++sa)
-                        if (sa + t >= 2 && sa + t <= kOzMaxSum) pair(sa, t, s);
-                    if (t < 2)
-                        st01[t] = s;
-                    else
-                        mma_commit(empty(s));
                     issued = true;
+#pragma unroll
+                    for (int t = t2; t < t2 + 2; ++t)
+#pragma unroll
+                        for (int sa = 0; sa < kOzSlices; ++sa)
+                            if (sa + t >= 2 && sa + t <= kOzMaxSum) pair(sa, t, s);
+                    if (t2 > 0) mma_commit(empty(s));
                     if (++s == kOzStages) {
                         s = 0;
                         ph ^= 1u;
@@ -408,11 +385,10 @@ __global__ void __launch_bounds__(kOzThreads, 1)
                     break;
                 }
                 tc_fence_after();
-                pair(0, 0, st01[0]);
-                pair(1, 0, st01[0]);
-                pair(0, 1, st01[1]);
-                mma_commit(empty(st01[0]));
-                mma_commit(empty(st01[1]));
+                pair(0, 0, s0);
+                pair(1, 0, s0);
+                pair(0, 1, s0);
+                mma_commit(empty(s0));
                 mma_commit(tfull(1));
                 acc_ph ^= 1u;
             }
@@ -470,11 +446,12 @@ __global__ void __launch_bounds__(kOzThreads, 1)
                 if (lane == 0) mbar_arrive(atmem);
             }
             const int64_t r = c_begin + rr;
-            const int er = exps[rr];
+            // upper word of -2^{e_r - 56}; a column's exponent is added to its exponent field
+            const int scale_hi = (int)(0x80000000u | (uint32_t)((exps[rr] - 56 + 1023) << 20));
             for (int64_t c = c0; c < c1; ++c) {
                 const int64_t cj = c_begin + c * kOzN + half * 32;  // this warp's first column
                 const bool valid = r < rows && r >= c_begin + c * kOzN;
-                const int ec_lane = exps[c * kOzN + half * 32 + lane];  // exponent of column cj + lane
+                const int4* ec = reinterpret_cast<const int4*>(exps + c * kOzN + half * 32);  // the columns' exponents
                 // Levels combined exactly: adjacent pairs in int32 (|S_l| <= 6 64^2 128 < 2^22, so
                 // S2 2^7 + S3, S4 2^7 + S5, S6 2^7 + S7 < 2^30), then hi = (S2 2^7 + S3) 2^14 +
                 // S4 2^7 + S5 < 2^44 and lo = (S6 2^7 + S7) 2^7 + S8 < 2^37 in int64 (held as an
@@ -527,34 +504,39 @@ __global__ void __launch_bounds__(kOzThreads, 1)
                     tmem_ld16_nowait(lanes + (uint32_t)(kOzN + 16 * h16), v[1]);
                     tmem_wait_ld();
                     if (h16 == 1) release_group(1);
-                    double val[16];
+                    // the staged row's last reduction has read it
+                    if (h16 == 0 && reduced) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const int32_t p23 = (int32_t)v[0][j] * 128 + (int32_t)v[1][j];
-                        const int ej = __shfl_sync(0xffffffffu, ec_lane, 16 * h16 + j);
-                        // (p23 2^35 + m) rounded once is 2^56 times the value rounded once: the
-                        // 2^-56 joins the exact power-of-two scale (one FP64 multiply less; the
-                        // epilogue's FP64 work is on this kernel's critical path)
-                        val[j] = -fma((double)p23, 0x1p35, m_d[16 * h16 + j]) * pow2(er + ej - 56);
-                    }
-                    if (valid) {  // stage the half row (128 bytes), then one bulk reduction
-                        if (reduced) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    for (int j4 = 0; j4 < 4; ++j4) {
+                        const int4 e4 = __ldg(ec + 4 * h16 + j4);  // the same for every lane
+                        const int ej[4] = {e4.x, e4.y, e4.z, e4.w};
+                        double val[4];
 #pragma unroll
-                        for (int j = 0; j < 16; j += 2)
-                            asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(stg + 8u * j), "d"(val[j]),
-                                         "d"(val[j + 1])
+                        for (int k = 0; k < 4; ++k) {
+                            const int j = 4 * j4 + k;
+                            const int32_t p23 = (int32_t)v[0][j] * 128 + (int32_t)v[1][j];
+                            // (p23 2^35 + m) rounded once is 2^56 times the value rounded once: the
+                            // 2^-56 joins the exact power-of-two scale
+                            val[k] = fma((double)p23, 0x1p35, m_d[16 * h16 + j]) *
+                                     __hiloint2double(scale_hi + (ej[k] << 20), 0);
+                        }
+                        if (valid) {
+                            const uint32_t dst = stg + (uint32_t)(128 * h16 + 32 * j4);
+                            asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(dst), "d"(val[0]), "d"(val[1]) : "memory");
+                            asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(dst + 16u), "d"(val[2]), "d"(val[3])
                                          : "memory");
+                        }
                     }
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    if (valid) {
-                        double* dst = a + (size_t)f * stride + (size_t)r * ld + cj + 16 * h16;
-                        asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], 128;" ::"l"(
-                                         dst),
-                                     "r"(stg)
-                                     : "memory");
-                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                        reduced = true;
-                    }
+                }
+                // one bulk reduction per row: issuing one takes ~55 cycles per lane, whatever its size
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                if (valid) {
+                    double* dst = a + (size_t)f * stride + (size_t)r * ld + cj;
+                    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], 256;" ::"l"(dst),
+                                 "r"(stg)
+                                 : "memory");
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    reduced = true;
                 }
             }
         }
