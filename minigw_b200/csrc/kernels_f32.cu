@@ -69,8 +69,8 @@ __device__ __forceinline__ void tile_mma_3xtf32(const float* __restrict__ As, co
 
 // The C fragments of tile_mma_3xtf32 to a 64 x 64 tile in shared memory (row stride LD).
 template <int LD>
-__device__ __forceinline__ void store_fragments(float* __restrict__ s, const float (&acc)[4][4]) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+__device__ __forceinline__ void store_fragments(float* __restrict__ s, const float (&acc)[4][4], int w) {
+    const int lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int r0 = 16 * (w >> 1), c0 = 32 * (w & 1);
 #pragma unroll
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(256) k_diag32(float* __restrict__ a, int64_t l
         float acc[4][4] = {};
         tile_mma_3xtf32<kLdf, 64>(Pf, Yf, acc, 1.0f);
         __syncthreads();
-        store_fragments<kLdf>(Pf, acc);
+        store_fragments<kLdf>(Pf, acc, w);
         __syncthreads();
         for (int idx = tid; idx < 64 * 16; idx += 256) {
             const int r = idx >> 4, c4 = idx & 15;
@@ -186,112 +186,171 @@ __global__ void __launch_bounds__(256) k_diag32(float* __restrict__ a, int64_t l
     }
 }
 
-// The rows below an outer block, 64-row tiles from row0 on: P1 = A1 L11^{-T}, A2 -= P1 L21^T,
-// P2 = A2 L22^{-T} (3xTF32; a 64-wide block is P1 alone), in one pass with the block's three tiles
-// kept in shared memory (as separate solves and an update between them the tile moved three times).
-// Bound by the tensor pipe's TF32 rate in three products per tile.
+// The rows below an outer block, from row0 on: P1 = A1 L11^{-T}, A2 -= P1 L21^T, P2 = A2 L22^{-T}
+// (3xTF32; a 64-wide block is P1 alone), in one pass with the block's three tiles kept in shared
+// memory.  Every warp walks 16-row tiles of its own, all 64 output columns of a product at once, so
+// nothing but the warp is ever waited for.  Bound by the mma.sync TF32 rate (470 multiply-adds per
+// clock and SM, 5,000 cycles per 64 rows); with 16 x 32 warp tiles that split both operands at every
+// use and a barrier between the products it took 14,500.  The block's tiles are split once per CTA,
+// the two parts of a lane's two k values together (one 16-byte load per column tile and k step).  2000 pairs, 64 frequencies: 101 -> 74 us a launch.
 //   solve_row0  rows before it are finished (the solve-only pass): passed through to `panel` alone
 //   rows_end    rows to write to `panel` (beyond `rows` zeros)
-//   panel       the solved rows' hi / lo parts for the tcgen05 update (tc::panel_position); null: none
+//   panel       the solved rows' hi / lo parts for the tcgen05 update (the layout of kernels_tc.cu);
+//               null: none
 //   keep        write the solved rows back to the tall matrix
 //   qacc        squared norms (FP64) of the right-hand-side rows are added; null: none
+constexpr int kPanelWarps = 12;
+constexpr int kLdy = 144;        // split block row: 64 k as (hi, hi, lo, lo) of k, k + 4; = 16 mod 32 words
+constexpr int kBlk = 64 * kLdy;  // one split block
 template <int NB>
-__global__ void __launch_bounds__(256, 2)
+constexpr int kLdr = NB + 4;  // a warp's row stride
+template <int NB>
+constexpr size_t kPanel32Smem = sizeof(float) * ((NB == 128 ? 3 : 1) * kBlk + kPanelWarps * 16 * kLdr<NB>);
+
+// acc += sgn * (16 x 64 rows at X, stride LD) * (split block B)^T, the products of a k step in the order
+// lo.hi, hi.lo, hi.hi.
+template <int LD>
+__device__ __forceinline__ void rows_mma(const float* __restrict__ X, const float* __restrict__ B, float (&acc)[8][4],
+                                         float sgn) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const float* x0 = X + g * LD + t;
+    const float* b0 = B + g * kLdy + 4 * t;
+#pragma unroll 2
+    for (int k8 = 0; k8 < 8; ++k8) {
+        unsigned ah[4], al[4];
+        split_tf32(sgn * x0[8 * k8], ah[0], al[0]);
+        split_tf32(sgn * x0[8 * LD + 8 * k8], ah[1], al[1]);
+        split_tf32(sgn * x0[8 * k8 + 4], ah[2], al[2]);
+        split_tf32(sgn * x0[8 * LD + 8 * k8 + 4], ah[3], al[3]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint4 b = *reinterpret_cast<const uint4*>(b0 + 8 * j * kLdy + 16 * k8);
+            mma_tf32(acc[j], al, b.x, b.y);
+            mma_tf32(acc[j], ah, b.z, b.w);
+            mma_tf32(acc[j], ah, b.x, b.y);
+        }
+    }
+}
+
+template <int NB>
+__global__ void __launch_bounds__(32 * kPanelWarps, 1)
     k_panel32(float* __restrict__ a, int64_t ld, int64_t stride, int64_t k, int64_t row0, int64_t rows, int64_t rows_end,
               int64_t solve_row0, int64_t n_pad, float* __restrict__ panel, int keep, double* __restrict__ qacc,
               int64_t ldq) {
     extern __shared__ __align__(16) float fsm[];
-    constexpr int kTile = 64 * kLdf;
-    float* P1 = fsm;
-    float* P2 = P1 + kTile;  // NB == 128 only, as the last two
-    float* Y1 = NB == 128 ? P2 + kTile : P2;
-    float* L21 = Y1 + kTile;
-    float* Y2 = L21 + kTile;
-    const int tid = threadIdx.x;
-    const int lane = tid & 31, w = tid >> 5;
+    constexpr int kBlocks = NB == 128 ? 3 : 1;  // L11^{-1}, L21, L22^{-1}
+    constexpr int LD = kLdr<NB>;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const int rr0 = 16 * (w >> 1), cc0 = 32 * (w & 1);
+    float* B = fsm;
+    float* X = B + kBlocks * kBlk + warp * 16 * LD;
     float* A = a + (size_t)blockIdx.y * stride;
-    const float* D = A + (size_t)k * ld + k;
-    load_f32_async<64, kLdf>(Y1, D, ld);
-    if (NB == 128) {
-        load_f32_async<64, kLdf>(L21, D + (size_t)kNb * ld, ld);
-        load_f32_async<64, kLdf>(Y2, D + (size_t)kNb * ld + kNb, ld);
+    {
+        const float* D = A + (size_t)k * ld + k;
+        for (int idx = threadIdx.x; idx < kBlocks * 64 * 32; idx += 32 * kPanelWarps) {
+            const int blk = idx >> 11, r = (idx >> 5) & 63, k8 = (idx >> 2) & 7, tt = idx & 3;
+            const float* src = D + (size_t)(r + (blk > 0 ? kNb : 0)) * ld + 8 * k8 + tt + (blk > 1 ? kNb : 0);
+            uint4 v;
+            split_tf32(src[0], v.x, v.z);
+            split_tf32(src[4], v.y, v.w);
+            *reinterpret_cast<uint4*>(B + blk * kBlk + r * kLdy + 16 * k8 + 4 * tt) = v;
+        }
     }
+    __syncthreads();
     const int64_t rp = rows_end - row0;
     float4* hi = reinterpret_cast<float4*>(panel + (size_t)blockIdx.y * 2 * (NB / 32) * rp * 32);
     float4* lo = hi + (size_t)(NB / 32) * rp * 8;
-    for (int64_t r0 = row0 + (int64_t)blockIdx.x * kNb; r0 < rows_end; r0 += (int64_t)gridDim.x * kNb) {
+    auto store = [&](int col, const float (&acc)[8][4]) {  // fragments to this warp's rows
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                *reinterpret_cast<float2*>(X + (g + 8 * h) * LD + col + 8 * j + 2 * t) =
+                    make_float2(acc[j][2 * h], acc[j][2 * h + 1]);
+    };
+    for (int64_t r0 = row0 + (int64_t)(kPanelWarps * blockIdx.x + warp) * 16; r0 < rows_end;
+         r0 += (int64_t)kPanelWarps * gridDim.x * 16) {
         const bool inside = r0 < rows;
         const bool solve = inside && r0 >= solve_row0;
         if (inside) {
-            load_f32_async<64, kLdf>(P1, A + r0 * ld + k, ld);
-            if (NB == 128) load_f32_async<64, kLdf>(P2, A + r0 * ld + k + kNb, ld);
+            const float* src = A + (size_t)r0 * ld + k;
+            for (int idx = lane; idx < 16 * (NB / 4); idx += 32)
+                cp_async_16f(X + idx / (NB / 4) * LD + 4 * (idx % (NB / 4)),
+                             src + (size_t)(idx / (NB / 4)) * ld + 4 * (idx % (NB / 4)));
         }
         asm volatile("cp.async.commit_group;\n" ::);
         asm volatile("cp.async.wait_group 0;\n" ::);
-        __syncthreads();
+        __syncwarp();
         if (solve) {
-            float acc[4][4] = {};
-            tile_mma_3xtf32<kLdf, 64>(P1, Y1, acc, 1.0f);
-            __syncthreads();
-            store_fragments<kLdf>(P1, acc);
-            __syncthreads();
+            double s[2] = {0.0, 0.0};  // squared norms of rows g and g + 8, this lane's columns
+            auto add_norms = [&](const float (&acc)[8][4]) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const double y = (double)acc[j][e];
+                        s[e >> 1] = fma(y, y, s[e >> 1]);
+                    }
+            };
+            const bool norms = qacc && r0 >= n_pad;
+            {
+                float acc[8][4] = {};
+                rows_mma<LD>(X, B, acc, 1.0f);
+                __syncwarp();
+                store(0, acc);
+                if (norms) add_norms(acc);
+                __syncwarp();
+            }
             if (NB == 128) {
-                float upd[4][4] = {};
-                tile_mma_3xtf32<kLdf, 64>(P1, L21, upd, -1.0f);
+                {
+                    float upd[8][4] = {};
+                    rows_mma<LD>(X, B + kBlk, upd, -1.0f);
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
+                    for (int j = 0; j < 8; ++j)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        P2[(rr0 + g + 8 * (e >> 1)) * kLdf + cc0 + 8 * j + 2 * t + (e & 1)] += upd[j][e];
-                __syncthreads();
-                float acc2[4][4] = {};
-                tile_mma_3xtf32<kLdf, 64>(P2, Y2, acc2, 1.0f);
-                __syncthreads();
-                store_fragments<kLdf>(P2, acc2);
-                __syncthreads();
+                        for (int h = 0; h < 2; ++h) {
+                            float2* p = reinterpret_cast<float2*>(X + (g + 8 * h) * LD + kNb + 8 * j + 2 * t);
+                            float2 v = *p;
+                            v.x += upd[j][2 * h];
+                            v.y += upd[j][2 * h + 1];
+                            *p = v;
+                        }
+                    __syncwarp();
+                }
+                float acc[8][4] = {};
+                rows_mma<LD>(X + kNb, B + 2 * kBlk, acc, 1.0f);
+                __syncwarp();
+                store(kNb, acc);
+                if (norms) add_norms(acc);
+                __syncwarp();
             }
-            if (keep)
-                for (int idx = tid; idx < 64 * (NB / 4); idx += 256) {
-                    const int r = idx / (NB / 4), c = 4 * (idx % (NB / 4));
-                    *reinterpret_cast<float4*>(A + (size_t)(r0 + r) * ld + k + c) =
-                        *reinterpret_cast<const float4*>((c < kNb ? P1 : P2 - kNb) + r * kLdf + c);
+            if (norms) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    s[h] += __shfl_xor_sync(0xffffffffu, s[h], 1);
+                    s[h] += __shfl_xor_sync(0xffffffffu, s[h], 2);
+                    if (t == 0) qacc[(size_t)blockIdx.y * ldq + (r0 - n_pad + g + 8 * h)] += s[h];
                 }
-            if (qacc && r0 >= n_pad) {  // four threads per row, fixed order
-                const int r = tid >> 2, part = tid & 3;
-                double s = 0.0;
-                for (int c = part; c < NB; c += 4) {
-                    const double y = (double)(c < kNb ? P1 : P2 - kNb)[r * kLdf + c];
-                    s = fma(y, y, s);
-                }
-                s += __shfl_xor_sync(0xffffffffu, s, 1);
-                s += __shfl_xor_sync(0xffffffffu, s, 2);
-                if (part == 0) qacc[(size_t)blockIdx.y * ldq + (r0 - n_pad + r)] += s;
             }
         }
-        if (panel) {
-            for (int idx = tid; idx < 64 * (NB / 4); idx += 256) {
-                const int kb = idx >> 9, r = (idx >> 3) & 63, c = idx & 7;  // K slice of 32, row, 16-byte chunk
-                const int col = 32 * kb + 4 * c;
-                float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (inside) x = *reinterpret_cast<const float4*>((col < kNb ? P1 : P2 - kNb) + r * kLdf + col);
-                float4 h, l;
-                h.x = __uint_as_float(to_tf32(x.x));
-                h.y = __uint_as_float(to_tf32(x.y));
-                h.z = __uint_as_float(to_tf32(x.z));
-                h.w = __uint_as_float(to_tf32(x.w));
-                l.x = __uint_as_float(to_tf32(x.x - h.x));
-                l.y = __uint_as_float(to_tf32(x.y - h.y));
-                l.z = __uint_as_float(to_tf32(x.z - h.z));
-                l.w = __uint_as_float(to_tf32(x.w - h.w));
+        for (int idx = lane; idx < 16 * (NB / 4); idx += 32) {
+            const int r = idx / (NB / 4), c4 = idx % (NB / 4);
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (inside) x = *reinterpret_cast<const float4*>(X + r * LD + 4 * c4);
+            if (solve && keep) *reinterpret_cast<float4*>(A + (size_t)(r0 + r) * ld + k + 4 * c4) = x;
+            if (panel) {
+                unsigned h[4], l[4];
+                split_tf32(x.x, h[0], l[0]);
+                split_tf32(x.y, h[1], l[1]);
+                split_tf32(x.z, h[2], l[2]);
+                split_tf32(x.w, h[3], l[3]);
                 const int64_t rr = r0 - row0 + r;
-                const size_t dst = ((size_t)kb * rp + rr) * 8 + (c ^ (int)(rr & 7));
-                hi[dst] = h;
-                lo[dst] = l;
+                const size_t dst = ((size_t)(c4 >> 3) * rp + rr) * 8 + ((c4 & 7) ^ (int)(rr & 7));  // K slice of 32, chunk
+                hi[dst] = make_float4(__uint_as_float(h[0]), __uint_as_float(h[1]), __uint_as_float(h[2]), __uint_as_float(h[3]));
+                lo[dst] = make_float4(__uint_as_float(l[0]), __uint_as_float(l[1]), __uint_as_float(l[2]), __uint_as_float(l[3]));
             }
         }
-        __syncthreads();
+        __syncwarp();
     }
 }
 
@@ -390,11 +449,11 @@ int launch_block32(const TallGeometry& g, int64_t nf, float* a, int64_t k, doubl
     // pass works on the right-hand sides alone
     const int64_t row0 = solve_only && !panel ? g.n_pad : k + NB;
     const int64_t rows_end = panel ? row0 + tc_panel_rows(g, row0) : g.rows;
-    const int64_t tiles = (rows_end - row0) / kNb;
+    const int64_t tiles = (rows_end - row0) / 16;
     if (tiles <= 0) return launches;
-    const size_t smem = (NB == 128 ? 5 : 2) * 64 * kLdf * sizeof(float);
-    GWB_CUDA(cudaFuncSetAttribute(k_panel32<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_panel32<NB><<<dim3((unsigned)panel_grid(tiles, nf, 2), (unsigned)nf), 256, smem, s>>>(
+    GWB_CUDA(cudaFuncSetAttribute(k_panel32<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanel32Smem<NB>));
+    const int64_t gx = panel_grid((tiles + kPanelWarps - 1) / kPanelWarps, nf, 1);
+    k_panel32<NB><<<dim3((unsigned)gx, (unsigned)nf), 32 * kPanelWarps, kPanel32Smem<NB>, s>>>(
         a, g.ld, g.stride, k, row0, g.rows, rows_end, solve_only ? g.n_pad : row0, g.n_pad, panel, keep ? 1 : 0, qacc,
         g.m_pad);
     GWB_LAUNCH("k_panel32");

@@ -199,52 +199,41 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 
     const size_t half_floats = (size_t)nkc * rp * 32;  // hi (or lo) of one frequency
 
-    if (warp == 0) {
-        // ---- producer: takes units from the global counter, hands them on, streams B ----
+    if (warp == 0 && lane == 0) {
+        // ---- producer: takes units from the global counter, hands them on, streams B (one thread:
+        // with the warp in step a stage took three times as long to hand over) ----
         int s = 0, js = 0;
         uint32_t ph = 0, jph = 0;
         uint32_t filled = 0, fill_par = 0;  // per B stage: ever filled, parity of its last fill
-        for (;;) {
+        bool ok = true;
+        while (ok) {
             int f = 0;
             int64_t i = 0, c0 = 0, c1 = 0, u = 0;
-            if (lane == 0) {
-                do {
-                    u = (int64_t)atomicAdd(sched, 1ull);
-                } while (u < us.total && !decode_unit(us, u, f, i, c0, c1));
-                if (u > us.total) u = us.total;
-            }
-            u = __shfl_sync(0xffffffffu, u, 0);
-            uint32_t got = 1;
-            if (lane == 0) {
-                got = mbar_wait(uempty(js), jph ^ 1u, abort_flag, err) ? 1u : 0u;
-                if (got) {
-                    uslot[js] = u;
-                    mbar_arrive(ufull(js));
-                }
-            }
-            got = __shfl_sync(0xffffffffu, got, 0);
-            if (!got) break;
+            do {
+                u = (int64_t)atomicAdd(sched, 1ull);
+            } while (u < us.total && !decode_unit(us, u, f, i, c0, c1));
+            if (u > us.total) u = us.total;
+            if (!mbar_wait(uempty(js), jph ^ 1u, abort_flag, err)) break;
+            uslot[js] = u;
+            mbar_arrive(ufull(js));
             if (++js == kSchedSlots) {
                 js = 0;
                 jph ^= 1u;
             }
             if (u >= us.total) break;
-            decode_unit(us, u, f, i, c0, c1);
             const float* hi = panel + (size_t)f * 2 * half_floats;
             const float* lo = hi + half_floats;
             // the unit's A rows (read once, by the epilogue warps into TMEM when the unit starts):
             // bring them into L2 now, about a tile ahead of their use
-            if (lane < 2 * nkc) {
-                const int which = lane / nkc, kb = lane - which * nkc;
-                const float* src = (which == 0 ? hi : lo) + (size_t)((int64_t)kb * rp + i * kTcM) * 32;
-                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(kTcM * kRowBytes) : "memory");
-            }
-            bool ok = true;
-            for (int64_t c = c0; ok && c < c1; ++c) {
+            for (int which = 0; which < 2; ++which)
                 for (int kb = 0; kb < nkc; ++kb) {
-                    if (lane == 0) got = mbar_wait(empty(s), ph ^ 1u, abort_flag, err) ? 1u : 0u;
-                    got = __shfl_sync(0xffffffffu, got, 0);
-                    if (!got) {
+                    const float* src = (which == 0 ? hi : lo) + (size_t)((int64_t)kb * rp + i * kTcM) * 32;
+                    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(kTcM * kRowBytes) : "memory");
+                }
+            for (int64_t c = c0; ok && c < c1; ++c) {
+                const float* src = hi + (size_t)(c * kTcN) * 32;
+                for (int kb = 0; kb < nkc; ++kb, src += (size_t)rp * 32) {
+                    if (!mbar_wait_fast(empty(s), ph ^ 1u, abort_flag, err)) {
                         ok = false;
                         break;
                     }
@@ -253,12 +242,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         // thread's wait for it can only end by expiry (GWB200_DEVICE_TIMEOUT)
                         withhold_first_stage = 0;
                     } else {
-                        if (lane == 0) mbar_expect_tx(full(s), kStageBytes);
-                        __syncwarp();
-                        if (lane < 2) {  // one 16 KB copy each of hi and lo
-                            const float* src = (lane == 0 ? hi : lo) + (size_t)((int64_t)kb * rp + c * kTcN) * 32;
-                            bulk_g2s(ring + s * kStageBytes + lane * kSliceB, src, kSliceB, full(s));
-                        }
+                        mbar_expect_tx(full(s), kStageBytes);
+                        bulk_g2s(ring + s * kStageBytes, src, kSliceB, full(s));  // 16 KB each of hi and lo
+                        bulk_g2s(ring + s * kStageBytes + kSliceB, src + half_floats, kSliceB, full(s));
                         filled |= 1u << s;
                     }
                     fill_par = (fill_par & ~(1u << s)) | (ph << s);
@@ -268,14 +254,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     }
                 }
             }
-            if (!ok) break;
         }
         // every issued copy has landed before the CTA may exit (normally already consumed)
-        if (lane == 0) {
-            for (int q = 0; q < kTcStages; ++q)
-                if (filled & (1u << q)) mbar_drain(full(q), (fill_par >> q) & 1u);
-        }
-        __syncwarp();
+        for (int q = 0; q < kTcStages; ++q)
+            if (filled & (1u << q)) mbar_drain(full(q), (fill_par >> q) & 1u);
     } else if (warp == 1 && lane == 0) {
         // ---- MMA issuer: one thread waits, issues and commits ----
         int s = 0, ab = 0, js = 0;
