@@ -9,18 +9,19 @@
 // 119-169) applies unchanged, the Green's function depending on k only:
 //     Sigma_c(p_s, p_t; i w_n) = -(1/pi) sum_{f,k} w_f g_{n f k} q[f, k, s, t],
 //     g_{n f k} = a / (a^2 + w_f^2),  a = i w_n + E_F - e_k.
-//   k_cross_forms          one CTA per (k, frequency): the nstates rows staged in shared memory in
-//                          chunks of the row length, each thread the running dot products of its
-//                          (s <= t) pairs in a fixed order;
+//   k_cross_forms          one CTA per (k, frequency): the Gram matrix of the nstates rows on the FP64
+//                          tensor cores straight from global memory, an eighth of the row length per
+//                          warp, the warps' parts added in a fixed order;
 //   k_sigma_contract_pairs one CTA per (output frequency, pair s <= t): the contraction, a fixed
 //                          reduction tree; both triangles written.
 #include "internal.cuh"
 
+#include <type_traits>
+
 namespace gwb200 {
 namespace {
 
-constexpr int kXThreads = 256;
-constexpr int kXSmem = 48 * 1024;  // default dynamic shared memory, no opt-in needed
+constexpr int kXWarps = 8;
 
 // (s, t) with s <= t of upper-triangle index p (row-major: row s holds t = s .. ns-1).
 __device__ __forceinline__ void pair_of(int p, int ns, int& s, int& t) {
@@ -32,43 +33,61 @@ __device__ __forceinline__ void pair_of(int p, int ns, int& s, int& t) {
     t = s + p;
 }
 
-__global__ void __launch_bounds__(kXThreads) k_cross_forms(const double* __restrict__ a, int64_t ld, int64_t stride,
-                                                           int64_t n, int64_t n_pad, int nmo, int ns, int ch,
-                                                           double* __restrict__ qx) {
-    extern __shared__ double xsm[];
+// The ns rows (tall rows n_pad + s nmo + k) in tiles of 8: in an m8n8k4 product of a tile with another
+// the A fragment of the one and the B fragment of the other are both "row lane / 4, column lane % 4",
+// so one register per tile and four columns serves every pair.  Bound by reading the rows once (8
+// states, 1125 pairs, 90 orbitals, 48 frequencies: 311 MB in 64 us; one dot product per thread from
+// staged rows left 220 of 256 threads idle and took 258).  NT: tiles of 8 states.
+template <int NT>
+__global__ void __launch_bounds__(32 * kXWarps) k_cross_forms(const double* __restrict__ a, int64_t ld, int64_t stride,
+                                                              int64_t n_pad, int nmo, int ns, double* __restrict__ qx) {
+    constexpr int kPairs = NT * (NT + 1) / 2;
+    __shared__ double part[kXWarps][64];
     const int k = blockIdx.x, f = blockIdx.y;
-    const int npair = ns * (ns + 1) / 2;
-    const int ldr = ch + 1;  // odd row stride: the pair loop's reads spread over the banks
-    double* rows = xsm;
-    double* acc = xsm + (size_t)ns * ldr;
-    for (int p = threadIdx.x; p < npair; p += kXThreads) acc[p] = 0.0;
-    const double* A = a + (size_t)f * stride;
-    for (int64_t i0 = 0; i0 < n; i0 += ch) {
-        const int len = (int)min((int64_t)ch, n - i0);
-        __syncthreads();  // the previous chunk's reads are done
-        for (int idx = threadIdx.x; idx < ns * ch; idx += kXThreads) {
-            const int s = idx / ch, c = idx - s * ch;
-            rows[s * ldr + c] = c < len ? A[(size_t)(n_pad + (int64_t)s * nmo + k) * ld + i0 + c] : 0.0;
-        }
-        __syncthreads();
-        for (int p = threadIdx.x; p < npair; p += kXThreads) {
-            int s, t;
-            pair_of(p, ns, s, t);
-            const double* rs = rows + s * ldr;
-            const double* rt = rows + t * ldr;
-            double sum = acc[p];
-            for (int c = 0; c < len; ++c) sum = fma(rs[c], rt[c], sum);
-            acc[p] = sum;
-        }
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const double* rows[NT];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {  // a tile's missing states read the last one (their products are not stored)
+        const int s = min(8 * i + g, ns - 1);
+        rows[i] = a + (size_t)f * stride + (size_t)(n_pad + (int64_t)s * nmo + k) * ld + t;
     }
-    __syncthreads();
+    double acc[kPairs][2] = {};
+    // the rows are zero beyond n (identity padding), so whole 64-column blocks are read
+#pragma unroll 4
+    for (int64_t c = 4 * w; c < n_pad; c += 4 * kXWarps) {
+        double x[NT];
+#pragma unroll
+        for (int i = 0; i < NT; ++i) x[i] = rows[i][c];
+        int p = 0;
+#pragma unroll
+        for (int i = 0; i < NT; ++i)
+#pragma unroll
+            for (int j = i; j < NT; ++j, ++p)
+                asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                             : "+d"(acc[p][0]), "+d"(acc[p][1])
+                             : "d"(x[i]), "d"(x[j]));
+    }
     double* out = qx + ((size_t)f * nmo + k) * ns * ns;
-    for (int p = threadIdx.x; p < npair; p += kXThreads) {
-        int s, t;
-        pair_of(p, ns, s, t);
-        out[s * ns + t] = -acc[p];
-        out[t * ns + s] = -acc[p];
-    }
+    int p = 0;
+#pragma unroll
+    for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int j = i; j < NT; ++j, ++p) {
+            part[w][8 * g + 2 * t] = acc[p][0];
+            part[w][8 * g + 2 * t + 1] = acc[p][1];
+            __syncthreads();
+            if (threadIdx.x < 64) {
+                const int s = 8 * i + (threadIdx.x >> 3), u = 8 * j + (threadIdx.x & 7);
+                double sum = 0.0;
+#pragma unroll
+                for (int v = 0; v < kXWarps; ++v) sum += part[v][threadIdx.x];
+                if (s <= u && u < ns) {  // both triangles from one value
+                    out[s * ns + u] = -sum;
+                    out[u * ns + s] = -sum;
+                }
+            }
+            __syncthreads();
+        }
 }
 
 __global__ void __launch_bounds__(256) k_sigma_contract_pairs(const double* __restrict__ qx, int nf_int, int nmo,
@@ -121,14 +140,21 @@ __global__ void __launch_bounds__(256) k_sigma_contract_pairs(const double* __re
 int launch_cross_forms(const TallGeometry& g, int64_t nf, const double* a, int64_t nmo, int64_t nstates, double* qx,
                        cudaStream_t s) {
     const int ns = (int)nstates;
-    const int npair = ns * (ns + 1) / 2;
-    // rows chunk: ns rows of (ch + 1) doubles and the pair accumulators in 48 KB, ch a multiple of 32
-    int ch = (int)(((size_t)kXSmem / sizeof(double) - (size_t)npair) / (size_t)ns) - 1;
-    ch = std::max(32, ch / 32 * 32);
-    const size_t smem = sizeof(double) * ((size_t)ns * (ch + 1) + npair);
-    if (smem > (size_t)kXSmem) fail(GWB200_BAD_SHAPE, "too many states for the cross forms");
-    k_cross_forms<<<dim3((unsigned)nmo, (unsigned)nf), kXThreads, smem, s>>>(a, g.ld, g.stride, g.n, g.n_pad, (int)nmo,
-                                                                              ns, ch, qx);
+    if (ns < 1 || ns > 64) fail(GWB200_BAD_SHAPE, "too many states for the cross forms");
+    const dim3 grid((unsigned)nmo, (unsigned)nf);
+    auto run = [&](auto nt) {
+        k_cross_forms<decltype(nt)::value><<<grid, 32 * kXWarps, 0, s>>>(a, g.ld, g.stride, g.n_pad, (int)nmo, ns, qx);
+    };
+    switch ((ns + 7) / 8) {
+        case 1: run(std::integral_constant<int, 1>{}); break;
+        case 2: run(std::integral_constant<int, 2>{}); break;
+        case 3: run(std::integral_constant<int, 3>{}); break;
+        case 4: run(std::integral_constant<int, 4>{}); break;
+        case 5: run(std::integral_constant<int, 5>{}); break;
+        case 6: run(std::integral_constant<int, 6>{}); break;
+        case 7: run(std::integral_constant<int, 7>{}); break;
+        default: run(std::integral_constant<int, 8>{}); break;
+    }
     GWB_LAUNCH("k_cross_forms");
     return 1;
 }
