@@ -290,10 +290,15 @@ __device__ __forceinline__ void factor_diag(double* __restrict__ S, double* __re
                 }
         };
         if (ng > 0) {
-            if (warp == 0) {  // the next panel's diagonal block, then on to factoring it
+            // warp 0 updates the next panel's diagonal block and goes on to factor it; the others hold
+            // back until it has (they have time to spare, and shared memory is what they contend for: a block
+            // of 128 in 42,500 cycles without the barrier, 39,700 with it)
+            if (warp == 0) {
                 group(c1, c1, 0, S + c1 * LD + c0, LD, 1);
                 __syncwarp();
+                asm volatile("bar.arrive 1, %0;" ::"n"(32 * (1 + kWarps - kWarps / 4)) : "memory");
             } else if (warp & 3) {  // the warps that share warp 0's FP64 pipe stay out of its way
+                asm volatile("bar.sync 1, %0;" ::"n"(32 * (1 + kWarps - kWarps / 4)) : "memory");
                 for (int x = warp - (warp >> 2); x < n_all; x += kWarps - kWarps / 4) {  // group 0 is warp 0's
                     if (x < n_low) {
                         int gi = 0, base = 0;
