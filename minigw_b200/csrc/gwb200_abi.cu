@@ -120,6 +120,7 @@ struct gwb200_handle {
     int device = 0;
     cudaStream_t stream = nullptr;      // stream all work is issued on
     cudaStream_t own_stream = nullptr;  // the handle's own stream
+    SideStream side;                    // work beside `stream`, joined to it before a call's results are read
     cudaEvent_t ev[6] = {};
     // resident system
     bool loaded = false;
@@ -424,6 +425,7 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
     const char* prof_env = std::getenv("GWB200_PROFILE");
     UpdateProfiler prof(prof_env && prof_env[0] == '1', s);
     int64_t chunks = 0;
+    if (!small && !cplx && !mixed && g.n_pad > 2 * kNb && h->persistent_ctas == 0) h->side.ensure();
     int upd_variant = -1;  // FP64 update kernel, tuned on the first chunk (full size) of this geometry
     for (int64_t f0 = 0; f0 < nfreq; f0 += fc) {
         const int64_t nf = std::min(fc, nfreq - f0);
@@ -476,7 +478,8 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
             launches += launch_factor_chunk(g, nf, h->a.as<double>(), h->qacc.as<double>(),
                                             h->err(), s, prof.enabled ? &prof : nullptr,
                                             upd_variant, fp64_oz ? h->panel32.p : nullptr,
-                                            h->tc_sched.as<unsigned long long>(), h->persistent_ctas);
+                                            h->tc_sched.as<unsigned long long>(), h->persistent_ctas,
+                                            h->side.stream ? &h->side : nullptr);
             if (after_factor) {
                 (*after_factor)(g, f0, nf);
                 ++launches;
@@ -814,6 +817,7 @@ int gwb200_destroy(gwb200_handle* h) {
     if (h->batch_exec) cudaGraphExecDestroy(h->batch_exec);
     for (auto& e : h->ev)
         if (e) cudaEventDestroy(e);
+    h->side.destroy();
     if (h->own_stream) cudaStreamDestroy(h->own_stream);
     delete h;
     return GWB200_OK;

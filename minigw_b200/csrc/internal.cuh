@@ -73,6 +73,46 @@ inline TallGeometry make_geometry(int64_t n, int64_t m) {
     return g;
 }
 
+// A second stream of one handle for work beside its own, with the events that order the two.
+struct SideStream {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    void ensure() {
+        if (!stream) cuda_check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "side stream", __FILE__, __LINE__);
+        for (cudaEvent_t* e : {&fork, &join})
+            if (!*e) cuda_check(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "side event", __FILE__, __LINE__);
+    }
+    void destroy() {
+        if (stream) cudaStreamDestroy(stream);
+        if (fork) cudaEventDestroy(fork);
+        if (join) cudaEventDestroy(join);
+    }
+};
+
+// Work on the side stream, behind what `s` holds at the scope's start and before what `s` is given after the
+// scope (also where the scope is left by an exception).
+class SideScope {
+    const SideStream* side_;
+    cudaStream_t s_;
+    bool begun_ = false;
+
+  public:
+    SideScope(const SideStream* side, cudaStream_t s) : side_(side), s_(s) {
+        if (side_) cuda_check(cudaEventRecord(side_->fork, s_), "cudaEventRecord", __FILE__, __LINE__);
+    }
+    SideScope(const SideScope&) = delete;
+    SideScope& operator=(const SideScope&) = delete;
+    cudaStream_t stream() {
+        if (!side_) return s_;
+        if (!begun_) cuda_check(cudaStreamWaitEvent(side_->stream, side_->fork, 0), "cudaStreamWaitEvent", __FILE__, __LINE__);
+        begun_ = true;
+        return side_->stream;
+    }
+    ~SideScope() {
+        if (begun_ && cudaEventRecord(side_->join, side_->stream) == cudaSuccess) cudaStreamWaitEvent(s_, side_->join, 0);
+    }
+};
+
 // Optional event timing of every trailing-update launch (the dominant kernel).
 struct UpdateProfiler {
     bool enabled;
@@ -124,15 +164,20 @@ int launch_build_tall(const TallGeometry& g, const double* v, const double* xt, 
 // `variant`: index into the FP64 update kernel table (tune_update_variant); -1: GWB200_UPDATE_VARIANT
 // if set, else the default; kUpdateOzaki: the outer trailing updates run as the int8 emulation of
 // kernels_oz.cu with `oz` as its slice workspace (oz_slice_bytes_per_freq(g) per frequency) and
-// `sched` as its work counter.
+// `sched` as its work counter.  With `side` the next diagonal block is factored beside the trailing
+// update, the work on both streams ordered by the handle's events and joined to `s` on return.
 int launch_factor_chunk(const TallGeometry& g, int64_t nf, double* a, double* qacc,
                         unsigned long long* err_pivot, cudaStream_t s, UpdateProfiler* prof, int variant,
-                        void* oz = nullptr, unsigned long long* sched = nullptr, int max_ctas = 0);
-// kernels_panel.cu: the panel step of columns [k, k + width), width 64 or 128: the diagonal block
-// (replaced by its inverse factor) and every row below it; the squared norms of the right-hand-side
-// rows are added to qacc.  Returns launches issued.
+                        void* oz = nullptr, unsigned long long* sched = nullptr, int max_ctas = 0,
+                        const SideStream* side = nullptr);
+// kernels_panel.cu, the panel step of columns [k, k + width), width 64 or 128.  launch_diag64: the
+// diagonal block, replaced by its inverse factor; for k > 0 after its update by the 128 columns before
+// it.  launch_panel64: every row below; the squared norms of the right-hand-side rows are added to
+// qacc.  Both return the launches issued.
+int launch_diag64(const TallGeometry& g, int64_t nf, double* a, int64_t k, int64_t width, unsigned long long* err_pivot,
+                  cudaStream_t s);
 int launch_panel64(const TallGeometry& g, int64_t nf, double* a, int64_t k, int64_t width, double* qacc,
-                   unsigned long long* err_pivot, cudaStream_t s);
+                   cudaStream_t s);
 // Small systems (n <= 128): the forms q[f][j] = x_j^T W_c x_j (rows ldq apart) of nf frequencies straight
 // from V, the panel rows and the frequencies in one launch, without tall matrices.
 bool small_system(const TallGeometry& g);
@@ -143,9 +188,11 @@ int64_t panel_grid(int64_t tiles, int64_t nf, int64_t per_sm);
 // kernels_oz.cu: FP64 trailing update C -= P P^T (K = 128 from kb0, columns [c_begin, n_pad), rows
 // [c_begin, rows)) from exact int8 products of 6-digit row slices (tcgen05 kind::i8).  Two launches.
 size_t oz_slice_bytes_per_freq(const TallGeometry& g);
-// max_ctas > 0 caps the persistent grid (a handle that shares the GPU with other streams).
+// max_ctas > 0 caps the persistent grid (a handle that shares the GPU with other streams).  Rows below
+// c_begin + row_min (0, 64 or 128) are left alone.
 int launch_update64_oz(const TallGeometry& g, int64_t nf, double* a, int64_t kb0, int64_t c_begin, void* slices,
-                       unsigned long long* sched, unsigned long long* err_pivot, cudaStream_t s, int max_ctas = 0);
+                       unsigned long long* sched, unsigned long long* err_pivot, cudaStream_t s, int max_ctas = 0,
+                       int64_t row_min = 0);
 // Autotuner of the FP64 trailing-update kernel: GWB200_UPDATE_VARIANT if set, else the fastest
 // candidate on this geometry's largest trailing update, timed once per (device, n_pad, rows, nf)
 // per process in the workspace `a` (nf tall matrices) BEFORE the matrices are built there (the

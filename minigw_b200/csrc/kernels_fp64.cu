@@ -11,6 +11,7 @@
 // quadratic forms.  All arithmetic is FP64; the O(n^3) and O(n^2 m) work runs on FP64
 // tensor cores (mma.sync m8n8k4 f64, DMMA).
 #include "panel_common.cuh"
+#include "tc_common.cuh"
 
 #include <array>
 #include <cstdio>
@@ -134,13 +135,10 @@ __device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
 }
 
 // Trailing update C -= sum_chunks P_i P_j^T of the output column tiles [tc0, tc0+T) (64-wide,
-// absolute tile indices): every tile on or below the diagonal in the square block, then every
-// tile of the right-hand-side rows.  The contraction runs over nk 64-wide column chunks of the
-// factored panels starting at column kb0, one chunk in shared memory at a time (cp.async), so
-// K = 64*nk costs one read and one write of C: the outer-block trailing update uses nk = 2
-// (16 flop per byte of C traffic), the narrow look-left update of an inner block nk = 1..q-1.
-// C is loaded into registers before the chunk loop and added in the epilogue, so its latency
-// overlaps the MMAs.
+// absolute tile indices): every tile on or below the diagonal in the square block but the first
+// `skip` row tiles, then every tile of the right-hand-side rows.  The contraction runs over nk
+// 64-wide column chunks of the factored panels starting at column kb0 in K slices, so K = 64*nk
+// costs one read and one write of C: nk = 2 (16 flop per byte of C traffic).
 __device__ __forceinline__ void cp_async_16(double* smem_dst, const double* gsrc) {
     const unsigned saddr = (unsigned)__cvta_generic_to_shared(smem_dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(saddr), "l"(gsrc));
@@ -192,7 +190,7 @@ struct UpdateCfg {
 template <int WM, int WN, int KC, int STAGES>
 __global__ void __launch_bounds__(UpdateCfg<WM, WN, KC, STAGES>::kThreads, UpdateCfg<WM, WN, KC, STAGES>::kMinBlocks)
     k_update(double* __restrict__ a, int64_t ld, int64_t stride, int64_t kb0, int nk, int64_t tc0, int64_t T,
-             int64_t nsq) {
+             int64_t nsq, int64_t skip) {
     using Cfg = UpdateCfg<WM, WN, KC, STAGES>;
     constexpr int LD = Cfg::kLd;
     extern __shared__ double smem[];
@@ -210,6 +208,7 @@ __global__ void __launch_bounds__(UpdateCfg<WM, WN, KC, STAGES>::kThreads, Updat
         while (c > 0 && cum(c) > x) --c;
         while (c + 1 < T && cum(c + 1) <= x) ++c;
         tr = tc0 + c + (x - cum(c));
+        if (tr < tc0 + skip) return;
     } else {
         const int64_t y = x - n_square;
         c = y % T;
@@ -260,7 +259,7 @@ __global__ void __launch_bounds__(UpdateCfg<WM, WN, KC, STAGES>::kThreads, Updat
 
 // Variant table of the update kernel (selected by GWB200_UPDATE_VARIANT, default kDefaultUpdateVariant).
 struct UpdateVariant {
-    void (*fn)(double*, int64_t, int64_t, int64_t, int, int64_t, int64_t, int64_t);
+    void (*fn)(double*, int64_t, int64_t, int64_t, int, int64_t, int64_t, int64_t, int64_t);
     int threads;
     size_t smem;
     const char* name;
@@ -300,13 +299,13 @@ int env_update_variant() {  // GWB200_UPDATE_VARIANT forces a variant; -1 if uns
 }
 
 void launch_variant(int v, const TallGeometry& g, int64_t nf, double* a, int64_t kb0, int nk, int64_t tc0, int64_t T,
-                    cudaStream_t s) {
+                    cudaStream_t s, int64_t skip = 0) {
     const UpdateVariant& uv = kVariants[v];
     const int64_t nsq = g.n_pad / kNb, nrt = g.rows / kNb;
     const int64_t L = nsq - tc0;
     const int64_t tiles = T * L - T * (T - 1) / 2 + T * (nrt - nsq);
     if (tiles <= 0) return;
-    uv.fn<<<dim3((unsigned)tiles, (unsigned)nf), uv.threads, uv.smem, s>>>(a, g.ld, g.stride, kb0, nk, tc0, T, nsq);
+    uv.fn<<<dim3((unsigned)tiles, (unsigned)nf), uv.threads, uv.smem, s>>>(a, g.ld, g.stride, kb0, nk, tc0, T, nsq, skip);
     GWB_LAUNCH("k_update");
 }
 
@@ -378,6 +377,13 @@ static double update_flops(const TallGeometry& g, int64_t kb0, int nk, int64_t c
     const double cols = (double)(a1 - a0);
     const double lower = cols * (double)g.n - 0.5 * (double)(a0 + a1 - 1) * cols;  // sum_{c} (n - c)
     return 2.0 * (double)kt * (lower + (double)g.m * cols);
+}
+
+// ... and of its diagonal block of columns [c0, c1)
+static double diag_flops(const TallGeometry& g, int64_t kb0, int nk, int64_t c0, int64_t c1) {
+    const int64_t kt = std::max<int64_t>(0, std::min<int64_t>(kb0 + (int64_t)nk * kNb, g.n) - kb0);
+    const double cols = (double)(std::min(c1, g.n) - std::min(c0, g.n));
+    return (double)kt * cols * (cols + 1.0);
 }
 
 int tune_update_variant(const TallGeometry& g, int64_t nf, double* a, cudaStream_t s, void* oz,
@@ -465,7 +471,7 @@ const char* update_variant_name(int v) {
 
 int launch_factor_chunk(const TallGeometry& g, int64_t nf, double* a, double* qacc, unsigned long long* err_pivot,
                         cudaStream_t s, UpdateProfiler* prof, int variant, void* oz, unsigned long long* sched,
-                        int max_ctas) {
+                        int max_ctas, const SideStream* side) {
     const bool use_oz = oz && variant == kUpdateOzaki;
     if (variant < 0 || variant >= kNumVariants)  // untuned caller: GWB200_UPDATE_VARIANT, else the default
         variant = env_update_variant() >= 0 ? env_update_variant() : kDefaultUpdateVariant;
@@ -476,19 +482,31 @@ int launch_factor_chunk(const TallGeometry& g, int64_t nf, double* a, double* qa
                                       (int)kVariants[variant].smem));
     int launches = 0;
     if (use_oz && nsq > kOuter) launches += launch_clear_sched(g, sched, s);
+    launches += launch_diag64(g, nf, a, 0, std::min(kOuter, nsq) * kNb, err_pivot, s);
+    // The next diagonal block (one CTA per frequency, ~40 us) runs beside the trailing update: it is
+    // launched first and takes nf SMs, the update's CTAs the others and those that become free: 1098 ->
+    // 981 us for the forms of 737 pairs x 64 frequencies, 2845 -> 2634 for 1125 x 48.  With as many
+    // frequencies as SMs there is nothing beside it.
+    if (prof || max_ctas > 0 || nf >= tc::sm_count()) side = nullptr;
     for (int64_t ob = 0; ob < nsq; ob += kOuter) {
         const int64_t q = std::min(kOuter, nsq - ob), tc0 = ob + q;
-        launches += launch_panel64(g, nf, a, ob * kNb, q * kNb, qacc, err_pivot, s);
+        launches += launch_panel64(g, nf, a, ob * kNb, q * kNb, qacc, s);
         if (tc0 >= nsq) break;
-        // trailing update, K = 128 (columns remain only behind a full outer block)
+        const int64_t next = std::min(kOuter, nsq - tc0);
+        SideScope beside(side, s);
+        launches += launch_diag64(g, nf, a, tc0 * kNb, next * kNb, err_pivot, s);
+        // the rest of the trailing update, K = 128 (columns remain only behind a full outer block)
         if (prof) prof->begin();
         if (use_oz) {
-            launches += launch_update64_oz(g, nf, a, ob * kNb, tc0 * kNb, oz, sched + ob / kOuter, err_pivot, s, max_ctas);
+            launches += launch_update64_oz(g, nf, a, ob * kNb, tc0 * kNb, oz, sched + ob / kOuter, err_pivot,
+                                           beside.stream(), max_ctas, next * kNb);
         } else {
-            launch_variant(variant, g, nf, a, ob * kNb, (int)q, tc0, nsq - tc0, s);
+            launch_variant(variant, g, nf, a, ob * kNb, (int)q, tc0, nsq - tc0, beside.stream(), next);
             ++launches;
         }
-        if (prof) prof->end((double)nf * update_flops(g, ob * kNb, (int)q, tc0 * kNb, nsq * kNb));
+        if (prof)
+            prof->end((double)nf * (update_flops(g, ob * kNb, (int)q, tc0 * kNb, nsq * kNb) -
+                                    diag_flops(g, ob * kNb, (int)q, tc0 * kNb, (tc0 + next) * kNb)));
     }
     return launches;
 }

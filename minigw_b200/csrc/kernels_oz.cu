@@ -187,6 +187,7 @@ __global__ void __launch_bounds__(256) k_slice_panel64(const double* __restrict_
 
 struct UnitSpace {
     int64_t T, NI, NS, per_f, total;
+    int64_t row_min;  // panel rows above it are left alone (the next diagonal block's); row tiles from row_min / 128
 };
 
 // unit -> (frequency, row tile i, column tiles [c0, c1)); the longest row tiles first
@@ -450,7 +451,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
             const int scale_hi = (int)(0x80000000u | (uint32_t)((exps[rr] - 56 + 1023) << 20));
             for (int64_t c = c0; c < c1; ++c) {
                 const int64_t cj = c_begin + c * kOzN + half * 32;  // this warp's first column
-                const bool valid = r < rows && r >= c_begin + c * kOzN;
+                const bool valid = r < rows && rr >= max(us.row_min, c * kOzN);
                 const int4* ec = reinterpret_cast<const int4*>(exps + c * kOzN + half * 32);  // the columns' exponents
                 // Levels combined exactly: adjacent pairs in int32 (|S_l| <= 6 64^2 128 < 2^22, so
                 // S2 2^7 + S3, S4 2^7 + S5, S6 2^7 + S7 < 2^30), then hi = (S2 2^7 + S3) 2^14 +
@@ -556,7 +557,8 @@ __global__ void __launch_bounds__(kOzThreads, 1)
 size_t oz_slice_bytes_per_freq(const TallGeometry& g) { return oz_freq_bytes((g.rows + kOzM - 1) / kOzM * kOzM); }
 
 int launch_update64_oz(const TallGeometry& g, int64_t nf, double* a, int64_t kb0, int64_t c_begin, void* slices,
-                       unsigned long long* sched, unsigned long long* err, cudaStream_t s, int max_ctas) {
+                       unsigned long long* sched, unsigned long long* err, cudaStream_t s, int max_ctas,
+                       int64_t row_min) {
     const int64_t T = (g.n_pad - c_begin) / kOzN;
     if (T <= 0 || nf <= 0) return 0;
     const int64_t H = g.rows - c_begin;
@@ -570,8 +572,9 @@ int launch_update64_oz(const TallGeometry& g, int64_t nf, double* a, int64_t kb0
     us.T = T;
     us.NI = NI;
     us.NS = (T + kOzSeg - 1) / kOzSeg;
-    us.per_f = NI * us.NS;
+    us.per_f = (NI - row_min / kOzM) * us.NS;
     us.total = nf * us.per_f;
+    us.row_min = row_min;
     const char* expire = std::getenv("GWB200_TEST_EXPIRE_WAIT");
     const int withhold = (expire && expire[0] == '1') ? 1 : 0;
     const unsigned grid = (unsigned)std::min<int64_t>(us.total, max_ctas > 0 ? std::min(max_ctas, sm_count()) : sm_count());

@@ -4,7 +4,10 @@
 //
 //   k_diag64    one CTA per frequency: Cholesky of the diagonal block and its inverse
 //               (panel_common.cuh); the inverse replaces the block in the tall matrix (the factor
-//               itself is not read again: the screened forms need the solved rows alone).
+//               itself is not read again: the screened forms need the solved rows alone).  A chain of
+//               pivots on one SM, so the next block's runs beside the trailing update on the other
+//               SMs: it takes its own update by the panel first (31 us without, 40 with it, at any
+//               number of frequencies up to the SMs), which the trailing update leaves out.
 //   k_panel64   rows below: P = A L^{-T} with the whole block's inverse, so the second 64 columns
 //               need no separate update by the first.  The inverse is triangular, so column tile c
 //               (8 wide) takes k < 8 (c + 1) only: 0.53 of the square product, less work than two
@@ -27,28 +30,111 @@ using namespace panel;
 constexpr int kPanelThreads = 256;
 constexpr int kRowTile = 32;
 
-template <int NB>
+__device__ __forceinline__ void cp_async16(double* dst, const double* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+
+// With kUpdate the block first takes the update by the 128 columns before it, which the trailing
+// update then leaves out: the block depends on the previous panel alone and is factored while the
+// rest of the trailing update runs.
+template <int NB, bool kUpdate>
 __global__ void __launch_bounds__(DiagShape<NB>::kThreads) k_diag64(double* __restrict__ a, int64_t ld, int64_t stride, int64_t k,
                                                           unsigned long long* err_pivot) {
     extern __shared__ __align__(16) double psm[];
-    constexpr int LD = DiagShape<NB>::kLd;
+    constexpr int LD = DiagShape<NB>::kLd, kThreads = DiagShape<NB>::kThreads;
     double* S = psm;
     double* A = a + (size_t)blockIdx.x * stride + k * ld + k;
-    for (int idx = threadIdx.x; idx < NB * (LD / 2); idx += DiagShape<NB>::kThreads) {
-        const int i = idx / (LD / 2), j = 2 * (idx % (LD / 2));
-        double2 v = make_double2(0.0, 0.0);
-        if (j <= i) v = *reinterpret_cast<const double2*>(A + (size_t)i * ld + j);
-        if (j + 1 > i) v.y = 0.0;
-        *reinterpret_cast<double2*>(S + i * LD + j) = v;
+    if (kUpdate) {
+        // the panel's rows through the space of S and beyond, the block's lower 16 x 16 tiles in
+        // registers, tile x of the warps x mod kWarps
+        constexpr int kK = 2 * kNb, kLdP = kK + 4, kWarps = kThreads / 32;
+        constexpr int kTiles = (NB / 16) * (NB / 16 + 1) / 2, kPer = (kTiles + kWarps - 1) / kWarps;
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+        for (int idx = threadIdx.x; idx < NB * (kK / 2); idx += kThreads) {
+            const int r = idx / (kK / 2), c = 2 * (idx % (kK / 2));
+            cp_async16(psm + r * kLdP + c, A + (int64_t)r * ld + c - kK);
+        }
+        asm volatile("cp.async.commit_group;\n" ::);
+        double acc[kPer][2][2][2];
+        int row[kPer], col[kPer];
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+            const int x = w + u * kWarps;
+            int gi = 0, base = 0;
+            while (base + gi + 1 <= x) base += ++gi;
+            row[u] = 16 * gi;
+            col[u] = 16 * (x - base);
+            if (x < kTiles) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int v = 0; v < 2; ++v) {
+                        const double2 e = *reinterpret_cast<const double2*>(A + (size_t)(row[u] + 8 * h + g) * ld +
+                                                                             col[u] + 8 * v + 2 * t);
+                        acc[u][h][v][0] = e.x;
+                        acc[u][h][v][1] = e.y;
+                    }
+            }
+        }
+        asm volatile("cp.async.wait_group 0;\n" ::);
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+            if (w + u * kWarps >= kTiles) break;
+            const double* X = psm + (row[u] + g) * kLdP + t;
+            const double* Y = psm + (col[u] + g) * kLdP + t;
+#pragma unroll 4
+            for (int kk = 0; kk < kK; kk += 4) {
+                const double a0 = -X[kk], a1 = -X[8 * kLdP + kk], b0 = Y[kk], b1 = Y[8 * kLdP + kk];
+                dmma(acc[u][0][0], a0, b0);
+                dmma(acc[u][0][1], a0, b1);
+                dmma(acc[u][1][0], a1, b0);
+                dmma(acc[u][1][1], a1, b1);
+            }
+        }
+        __syncthreads();
+        // the block into S, zeros above its diagonal
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+            if (w + u * kWarps >= kTiles) break;
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    const int i = row[u] + 8 * h + g, j = col[u] + 8 * v + 2 * t;
+                    *reinterpret_cast<double2*>(S + i * LD + j) =
+                        make_double2(j <= i ? acc[u][h][v][0] : 0.0, j + 1 <= i ? acc[u][h][v][1] : 0.0);
+                }
+        }
+        for (int idx = threadIdx.x; idx < NB * (LD / 2); idx += kThreads) {
+            const int i = idx / (LD / 2), j = 2 * (idx % (LD / 2));
+            if ((j & ~15) > i) *reinterpret_cast<double2*>(S + i * LD + j) = make_double2(0.0, 0.0);
+        }
+    } else {
+        for (int idx = threadIdx.x; idx < NB * (LD / 2); idx += kThreads) {
+            const int i = idx / (LD / 2), j = 2 * (idx % (LD / 2));
+            double2 v = make_double2(0.0, 0.0);
+            if (j <= i) v = *reinterpret_cast<const double2*>(A + (size_t)i * ld + j);
+            if (j + 1 > i) v.y = 0.0;
+            *reinterpret_cast<double2*>(S + i * LD + j) = v;
+        }
     }
     __syncthreads();
     factor_diag<NB, false>(S, S + DiagShape<NB>::kBlockDoubles, k, err_pivot);
     // the inverse in place of the block; above the diagonal zeros (not the upper right 64 x 64, which
-    // nothing reads)
-    for (int idx = threadIdx.x; idx < NB * NB; idx += DiagShape<NB>::kThreads) {
-        const int i = idx / NB, j = idx % NB;
+    // nothing reads).  A warp takes 4 rows x 8 columns: the transposed reads are 2-way bank conflicts.
+    const int rr = (threadIdx.x >> 3) & 3, cc = threadIdx.x & 7;
+    for (int x = threadIdx.x >> 5; x < (NB / 4) * (NB / 8); x += kThreads / 32) {
+        const int i = 4 * (x / (NB / 8)) + rr, j = 8 * (x % (NB / 8)) + cc;
         if (j < (i < kNb ? kNb : NB)) A[(size_t)i * ld + j] = j <= i ? S[j * LD + i + 1] : 0.0;
     }
+}
+
+// shared memory of k_diag64: the block and the workspace, or the panel's rows
+template <int NB, bool kUpdate>
+constexpr size_t diag_smem() {
+    const size_t rows = sizeof(double) * (size_t)NB * (2 * kNb + 4);
+    return kUpdate && rows > DiagShape<NB>::kSmem ? rows : DiagShape<NB>::kSmem;
 }
 
 template <int NB>
@@ -57,10 +143,6 @@ struct PanelShape {
     static constexpr int kTiles = NB / 32;  // column tiles of 8 per warp
     static constexpr size_t kSmem = sizeof(double) * ((size_t)NB * kLd + 2 * kRowTile * kLd + 4 * kRowTile);
 };
-
-__device__ __forceinline__ void cp_async16(double* dst, const double* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
-}
 
 template <int NB>
 __global__ void __launch_bounds__(kPanelThreads, 1)
@@ -244,19 +326,23 @@ int launch_small(const TallGeometry& g, int64_t nf, const double* delta, const d
     return 1;
 }
 
-template <int NB>
-int launch_block(const TallGeometry& g, int64_t nf, double* a, int64_t k, double* qacc, unsigned long long* err_pivot,
-                 cudaStream_t s) {
-    GWB_CUDA(cudaFuncSetAttribute(k_diag64<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DiagShape<NB>::kSmem));
-    k_diag64<NB><<<(unsigned)nf, DiagShape<NB>::kThreads, DiagShape<NB>::kSmem, s>>>(a, g.ld, g.stride, k, err_pivot);
+template <int NB, bool kUpdate>
+void launch_diag(const TallGeometry& g, int64_t nf, double* a, int64_t k, unsigned long long* err_pivot, cudaStream_t s) {
+    constexpr size_t smem = diag_smem<NB, kUpdate>();
+    GWB_CUDA(cudaFuncSetAttribute(k_diag64<NB, kUpdate>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_diag64<NB, kUpdate><<<(unsigned)nf, DiagShape<NB>::kThreads, smem, s>>>(a, g.ld, g.stride, k, err_pivot);
     GWB_LAUNCH("k_diag64");
+}
+
+template <int NB>
+int launch_rows(const TallGeometry& g, int64_t nf, double* a, int64_t k, double* qacc, cudaStream_t s) {
     const int64_t tiles = (g.rows - (k + NB)) / kRowTile;
-    if (tiles <= 0) return 1;
+    if (tiles <= 0) return 0;
     GWB_CUDA(cudaFuncSetAttribute(k_panel64<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PanelShape<NB>::kSmem));
     k_panel64<NB><<<dim3((unsigned)panel_grid(tiles, nf, 1), (unsigned)nf), kPanelThreads, PanelShape<NB>::kSmem, s>>>(
         a, g.ld, g.stride, k, g.n_pad, (int)tiles, qacc, g.m_pad);
     GWB_LAUNCH("k_panel64");
-    return 2;
+    return 1;
 }
 
 }  // namespace
@@ -286,10 +372,18 @@ int launch_small64(const TallGeometry& g, int64_t nf, const double* delta, const
     return launch_small<128>(g, nf, delta, omega, v, xt, q, ldq, err_pivot, s);
 }
 
+int launch_diag64(const TallGeometry& g, int64_t nf, double* a, int64_t k, int64_t width, unsigned long long* err_pivot,
+                  cudaStream_t s) {
+    if (width == 2 * kNb)
+        k > 0 ? launch_diag<128, true>(g, nf, a, k, err_pivot, s) : launch_diag<128, false>(g, nf, a, k, err_pivot, s);
+    else
+        k > 0 ? launch_diag<64, true>(g, nf, a, k, err_pivot, s) : launch_diag<64, false>(g, nf, a, k, err_pivot, s);
+    return 1;
+}
+
 int launch_panel64(const TallGeometry& g, int64_t nf, double* a, int64_t k, int64_t width, double* qacc,
-                   unsigned long long* err_pivot, cudaStream_t s) {
-    return width == 2 * kNb ? launch_block<128>(g, nf, a, k, qacc, err_pivot, s)
-                            : launch_block<64>(g, nf, a, k, qacc, err_pivot, s);
+                   cudaStream_t s) {
+    return width == 2 * kNb ? launch_rows<128>(g, nf, a, k, qacc, s) : launch_rows<64>(g, nf, a, k, qacc, s);
 }
 
 }  // namespace gwb200

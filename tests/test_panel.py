@@ -45,6 +45,25 @@ def test_forms_at_block_edges(n, nstates):
     assert np.abs(q - ref).max() <= 1e-11 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("update", ["dmma", "ozaki"])
+@pytest.mark.parametrize("n", [129, 193, 256, 257, 321, 385])
+def test_next_block_beside_the_update(n, update, monkeypatch):
+    """The next diagonal block, 64 or 128 wide, left out of the trailing update and factored beside it (few
+    frequencies) or before it (more than there are SMs): the same forms bit for bit."""
+    from minigw_b200 import B200Backend
+
+    monkeypatch.setenv("GWB200_FP64_UPDATE", update)
+    sl = _system(n, n // 2, 1, 900 + n)
+    few = np.array([1e-3, 0.4, 7.0])
+    with B200Backend(0) as be:
+        be.load_slices(sl)
+        q, _ = be.screened_forms(few, sl.states)
+        many, _ = be.screened_forms(np.tile(few, 67), sl.states)
+    ref = _forms(sl, few)
+    assert np.abs(q - ref).max() <= 1e-11 * np.abs(ref).max()  # as above
+    np.testing.assert_array_equal(many.reshape(67, 3, -1), np.broadcast_to(q.reshape(3, -1), (67, 3, q[0].size)))
+
+
 @pytest.mark.parametrize("n,pivot", [(40, 0), (40, 15), (40, 16), (100, 63), (100, 64), (200, 127), (200, 128), (200, 199)])
 def test_reported_pivot(n, pivot):
     from minigw_b200 import B200Backend
