@@ -155,6 +155,7 @@ struct gwb200_handle {
     cudaEvent_t batch_fork = nullptr;
     cudaGraphExec_t batch_exec = nullptr;   // the last batch sequence captured as a CUDA graph
     std::vector<int64_t> batch_graph_key;   // what it was captured for (sizes, plan, every pointer)
+    std::vector<int64_t> batch_graph_seen;  // the last call's: captured when it comes twice in a row
     std::vector<int64_t> batch_graph_failed;  // a signature whose capture failed (issued eagerly)
     int64_t batch_graph_launches = 0;
     PinnedBuf stage_in, stage_out;
@@ -1688,8 +1689,10 @@ int gwb200_run_g0w0_batch(gwb200_handle* const* systems, int64_t nsys, const int
         };
 
         // CUDA graph of the whole sequence for a repeated batch (one plan, nothing to time):
-        // captured on the first such call, replayed while every pointer it holds and every scalar
-        // it passes by value is unchanged.
+        // captured on the second such call in a row, replayed while every pointer it holds and every
+        // scalar it passes by value is unchanged.  (A batch that never comes back, as most of a
+        // server's, is issued directly: capturing, instantiating and destroying its graph cost more
+        // than its launches, and other threads' calls waited for the destruction, 2.7 ms each.)
         // GWB200_BATCH_GRAPH=0 issues the launches one by one.
         const char* graph_env = std::getenv("GWB200_BATCH_GRAPH");
         const bool want_graph = cands.size() == 1 && !(graph_env && std::strcmp(graph_env, "0") == 0);
@@ -1701,7 +1704,7 @@ int gwb200_run_g0w0_batch(gwb200_handle* const* systems, int64_t nsys, const int
         size_t pick = 0;
         bool graphed = false;
         if (want_graph && gkey != w->batch_graph_failed) {
-            if (!w->batch_exec || gkey != w->batch_graph_key) {
+            if (gkey == w->batch_graph_seen && !(w->batch_exec && gkey == w->batch_graph_key)) {
                 if (w->batch_exec) cudaGraphExecDestroy(w->batch_exec);
                 w->batch_exec = nullptr;
                 w->batch_graph_key.clear();
@@ -1733,7 +1736,7 @@ int gwb200_run_g0w0_batch(gwb200_handle* const* systems, int64_t nsys, const int
                     w->batch_graph_failed = gkey;
                 }
             }
-            if (w->batch_exec) {
+            if (w->batch_exec && gkey == w->batch_graph_key) {
                 GWB_CUDA(cudaEventRecord(w->ev[0], s));
                 GWB_CUDA(cudaGraphLaunch(w->batch_exec, s));
                 GWB_CUDA(cudaEventRecord(w->ev[3], s));
@@ -1741,6 +1744,7 @@ int gwb200_run_g0w0_batch(gwb200_handle* const* systems, int64_t nsys, const int
                 graphed = true;
             }
         }
+        if (want_graph) w->batch_graph_seen = gkey;
         if (!graphed) {
             GWB_CUDA(cudaEventRecord(w->ev[0], s));
             launches += prefix();
