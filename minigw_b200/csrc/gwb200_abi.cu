@@ -747,11 +747,14 @@ std::vector<std::vector<size_t>> batch_assign(const std::vector<BatchChunk>& chu
     return out;
 }
 
-// Latency of one 64-wide block step and the sustained rate of the padded work, the cost model's
-// defaults (measured on config-4-like batches; GWB200_BATCH_STEP_US / GWB200_BATCH_TFLOPS override).
-double batch_step_us(bool mixed) {
+// Latency of one 64-wide block step, as far as the other lanes leave it bare, and the sustained rate of
+// the padded work, the cost model's defaults (GWB200_BATCH_STEP_US / GWB200_BATCH_TFLOPS override).
+// Measured on 16 molecules of 20 to 120 orbitals x 64 frequencies on 4 lanes, refined mixed form: 22.6
+// ms at 8-15 us, 23.9 at 30, 25.4 at 60, 30.7 at 240 (one bucket per molecule 22.2); plain form, 16 to
+// 96 orbitals: 9.7 ms at 8-15 us, 11.1 at 30, 12.2 at 80.
+double batch_step_us() {
     if (const char* e = std::getenv("GWB200_BATCH_STEP_US")) return std::max(0.0, std::atof(e));
-    return mixed ? 60.0 : 80.0;
+    return 12.0;
 }
 double batch_tflops(bool mixed) {
     if (const char* e = std::getenv("GWB200_BATCH_TFLOPS")) return std::max(1e-3, std::atof(e));
@@ -1351,7 +1354,7 @@ std::vector<std::vector<int64_t>> batch_candidates(const std::vector<int64_t>& k
         if (it != g_batch_plans.end()) return {it->second};
     }
     std::vector<std::vector<int64_t>> cands;
-    const double tau = batch_step_us(mixed), rate = batch_tflops(mixed);
+    const double tau = batch_step_us(), rate = batch_tflops(mixed);
     for (double mult : (mode == "tuned" ? std::vector<double>{1.0, 0.25, 4.0} : std::vector<double>{1.0})) {
         std::vector<int64_t> p = plan_buckets(n_sorted, m_sorted, f_sorted, mixed, lane_budget, tau * mult, rate);
         if (std::find(cands.begin(), cands.end(), p) == cands.end()) cands.push_back(p);
@@ -1441,7 +1444,7 @@ int gwb200_plan_buckets(int64_t nsys, const int64_t* nph, const int64_t* ncols, 
         }
         const std::vector<int64_t> sizes =
             plan_buckets(n_sorted, m_sorted, std::vector<int64_t>(n_sorted.size(), nfreq), mixed, (size_t)budget_bytes,
-                         step_us > 0 ? step_us : batch_step_us(mixed),
+                         step_us > 0 ? step_us : batch_step_us(),
                          tflops > 0 ? tflops : batch_tflops(mixed));
         size_t pos = 0;
         for (size_t b = 0; b < sizes.size(); ++b)
@@ -1593,7 +1596,7 @@ int gwb200_run_g0w0_batch(gwb200_handle* const* systems, int64_t nsys, const int
         const size_t nb_in = groups_off + sizeof(BatchGroup) * groups.size();
         w->in.ensure(nb_in);
         std::vector<std::vector<std::vector<size_t>>> assign;
-        for (const auto& ch : chunks) assign.push_back(batch_assign(ch, lanes, batch_step_us(mixed), batch_tflops(mixed)));
+        for (const auto& ch : chunks) assign.push_back(batch_assign(ch, lanes, batch_step_us(), batch_tflops(mixed)));
         // FP64: the update kernel of each chunk geometry (timed before anything is built: the
         // autotuner overwrites the workspace)
         std::vector<std::vector<int>> variants(cands.size());
