@@ -171,11 +171,11 @@ int launch_factor_chunk(const TallGeometry& g, int64_t nf, double* a, double* qa
                         void* oz = nullptr, unsigned long long* sched = nullptr, int max_ctas = 0,
                         const SideStream* side = nullptr);
 // kernels_panel.cu, the panel step of columns [k, k + width), width 64 or 128.  launch_diag64: the
-// diagonal block, replaced by its inverse factor; for k > 0 after its update by the 128 columns before
-// it.  launch_panel64: every row below; the squared norms of the right-hand-side rows are added to
+// diagonal block, replaced by its inverse factor, after its update by the `depth` columns before it (0,
+// 128 or 256).  launch_panel64: every row below; the squared norms of the right-hand-side rows are added to
 // qacc.  Both return the launches issued.
-int launch_diag64(const TallGeometry& g, int64_t nf, double* a, int64_t k, int64_t width, unsigned long long* err_pivot,
-                  cudaStream_t s);
+int launch_diag64(const TallGeometry& g, int64_t nf, double* a, int64_t k, int64_t width, int64_t depth,
+                  unsigned long long* err_pivot, cudaStream_t s);
 int launch_panel64(const TallGeometry& g, int64_t nf, double* a, int64_t k, int64_t width, double* qacc,
                    cudaStream_t s);
 // Small systems (n <= 128): the forms q[f][j] = x_j^T W_c x_j (rows ldq apart) of nf frequencies straight
@@ -185,14 +185,15 @@ int launch_small64(const TallGeometry& g, int64_t nf, const double* delta, const
                    const double* xt, double* q, int64_t ldq, unsigned long long* err_pivot, cudaStream_t s);
 // CTAs per frequency of a panel kernel over `tiles` row tiles of nf frequencies, per_sm CTAs per SM
 int64_t panel_grid(int64_t tiles, int64_t nf, int64_t per_sm);
-// kernels_oz.cu: FP64 trailing update C -= P P^T (K = 128 from kb0, columns [c_begin, n_pad), rows
-// [c_begin, rows)) from exact int8 products of 6-digit row slices (tcgen05 kind::i8).  Two launches.
+// kernels_oz.cu: FP64 trailing update C -= P P^T (columns [kb0, c_begin) of the panel, 128 or 256, into
+// columns [c_begin, c_end), rows [c_begin, rows)) from exact int8 products of 6-digit row slices
+// (tcgen05 kind::i8).  Two launches.
 size_t oz_slice_bytes_per_freq(const TallGeometry& g);
 // max_ctas > 0 caps the persistent grid (a handle that shares the GPU with other streams).  Rows below
 // c_begin + row_min (0, 64 or 128) are left alone.
-int launch_update64_oz(const TallGeometry& g, int64_t nf, double* a, int64_t kb0, int64_t c_begin, void* slices,
-                       unsigned long long* sched, unsigned long long* err_pivot, cudaStream_t s, int max_ctas = 0,
-                       int64_t row_min = 0);
+int launch_update64_oz(const TallGeometry& g, int64_t nf, double* a, int64_t kb0, int64_t c_begin, int64_t c_end,
+                       void* slices, unsigned long long* sched, unsigned long long* err_pivot, cudaStream_t s,
+                       int max_ctas = 0, int64_t row_min = 0);
 // Autotuner of the FP64 trailing-update kernel: GWB200_UPDATE_VARIANT if set, else the fastest
 // candidate on this geometry's largest trailing update, timed once per (device, n_pad, rows, nf)
 // per process in the workspace `a` (nf tall matrices) BEFORE the matrices are built there (the

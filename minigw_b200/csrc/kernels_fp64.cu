@@ -439,7 +439,7 @@ int tune_update_variant(const TallGeometry& g, int64_t nf, double* a, cudaStream
     if (oz) {  // the int8 emulation of the outer update (kernels_oz.cu), slicing included
         const float ms = time_it([&] {
             launch_clear_sched(g, sched, s);
-            launch_update64_oz(g, nf, a, 0, 2 * kNb, oz, sched, err_pivot, s);
+            launch_update64_oz(g, nf, a, 0, 2 * kNb, g.n_pad, oz, sched, err_pivot, s);
         });
         times[kUpdateOzaki] = ms;
         if (ms < best_ms) {
@@ -482,7 +482,7 @@ int launch_factor_chunk(const TallGeometry& g, int64_t nf, double* a, double* qa
                                       (int)kVariants[variant].smem));
     int launches = 0;
     if (use_oz && nsq > kOuter) launches += launch_clear_sched(g, sched, s);
-    launches += launch_diag64(g, nf, a, 0, std::min(kOuter, nsq) * kNb, err_pivot, s);
+    launches += launch_diag64(g, nf, a, 0, std::min(kOuter, nsq) * kNb, 0, err_pivot, s);
     // The next diagonal block (one CTA per frequency, ~40 us) runs beside the trailing update: it is
     // launched first and takes nf SMs, the update's CTAs the others and those that become free: 1098 ->
     // 981 us for the forms of 737 pairs x 64 frequencies, 2845 -> 2634 for 1125 x 48.  With as many
@@ -493,20 +493,26 @@ int launch_factor_chunk(const TallGeometry& g, int64_t nf, double* a, double* qa
         launches += launch_panel64(g, nf, a, ob * kNb, q * kNb, qacc, s);
         if (tc0 >= nsq) break;
         const int64_t next = std::min(kOuter, nsq - tc0);
+        // int8: outer blocks in pairs while columns remain behind the pair.  The first updates the
+        // second's columns alone, then both update the rest at K = 256.  (Pairs begin at multiples of
+        // 256 columns whatever n_pad, so a molecule's columns take the same steps in a batch's geometry.)
+        const bool wide = use_oz && nsq - ob / 4 * 4 > 4, second = wide && ob % 4 == 2;
+        const int64_t kb = (second ? ob - kOuter : ob) * kNb, c_end = wide && !second ? tc0 + next : nsq;
         SideScope beside(side, s);
-        launches += launch_diag64(g, nf, a, tc0 * kNb, next * kNb, err_pivot, s);
-        // the rest of the trailing update, K = 128 (columns remain only behind a full outer block)
+        launches += launch_diag64(g, nf, a, tc0 * kNb, next * kNb, tc0 * kNb - kb, err_pivot, s);
+        // the rest of the trailing update (columns remain only behind a full outer block)
         if (prof) prof->begin();
         if (use_oz) {
-            launches += launch_update64_oz(g, nf, a, ob * kNb, tc0 * kNb, oz, sched + ob / kOuter, err_pivot,
+            launches += launch_update64_oz(g, nf, a, kb, tc0 * kNb, c_end * kNb, oz, sched + ob / kOuter, err_pivot,
                                            beside.stream(), max_ctas, next * kNb);
         } else {
-            launch_variant(variant, g, nf, a, ob * kNb, (int)q, tc0, nsq - tc0, beside.stream(), next);
+            launch_variant(variant, g, nf, a, kb, (int)q, tc0, nsq - tc0, beside.stream(), next);
             ++launches;
         }
+        const int nk = (int)(tc0 - kb / kNb);
         if (prof)
-            prof->end((double)nf * (update_flops(g, ob * kNb, (int)q, tc0 * kNb, nsq * kNb) -
-                                    diag_flops(g, ob * kNb, (int)q, tc0 * kNb, (tc0 + next) * kNb)));
+            prof->end((double)nf * (update_flops(g, kb, nk, tc0 * kNb, c_end * kNb) -
+                                    diag_flops(g, kb, nk, tc0 * kNb, (tc0 + next) * kNb)));
     }
     return launches;
 }

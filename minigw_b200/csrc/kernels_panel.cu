@@ -34,12 +34,12 @@ __device__ __forceinline__ void cp_async16(double* dst, const double* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
 }
 
-// With kUpdate the block first takes the update by the 128 columns before it, which the trailing
+// With kUpdate the block first takes the update by the `depth` (128 or 256) columns before it, which the trailing
 // update then leaves out: the block depends on the previous panel alone and is factored while the
 // rest of the trailing update runs.
 template <int NB, bool kUpdate>
 __global__ void __launch_bounds__(DiagShape<NB>::kThreads) k_diag64(double* __restrict__ a, int64_t ld, int64_t stride, int64_t k,
-                                                          unsigned long long* err_pivot) {
+                                                          int depth, unsigned long long* err_pivot) {
     extern __shared__ __align__(16) double psm[];
     constexpr int LD = DiagShape<NB>::kLd, kThreads = DiagShape<NB>::kThreads;
     double* S = psm;
@@ -50,11 +50,14 @@ __global__ void __launch_bounds__(DiagShape<NB>::kThreads) k_diag64(double* __re
         constexpr int kK = 2 * kNb, kLdP = kK + 4, kWarps = kThreads / 32;
         constexpr int kTiles = (NB / 16) * (NB / 16 + 1) / 2, kPer = (kTiles + kWarps - 1) / kWarps;
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-        for (int idx = threadIdx.x; idx < NB * (kK / 2); idx += kThreads) {
-            const int r = idx / (kK / 2), c = 2 * (idx % (kK / 2));
-            cp_async16(psm + r * kLdP + c, A + (int64_t)r * ld + c - kK);
-        }
-        asm volatile("cp.async.commit_group;\n" ::);
+        auto load_rows = [&](int from) {
+            for (int idx = threadIdx.x; idx < NB * (kK / 2); idx += kThreads) {
+                const int r = idx / (kK / 2), c = 2 * (idx % (kK / 2));
+                cp_async16(psm + r * kLdP + c, A + (int64_t)r * ld + c - from);
+            }
+            asm volatile("cp.async.commit_group;\n" ::);
+        };
+        load_rows(depth);
         double acc[kPer][2][2][2];
         int row[kPer], col[kPer];
 #pragma unroll
@@ -76,23 +79,26 @@ __global__ void __launch_bounds__(DiagShape<NB>::kThreads) k_diag64(double* __re
                     }
             }
         }
-        asm volatile("cp.async.wait_group 0;\n" ::);
-        __syncthreads();
+        for (int from = depth; from > 0; from -= kK) {
+            if (from < depth) load_rows(from);
+            asm volatile("cp.async.wait_group 0;\n" ::);
+            __syncthreads();
 #pragma unroll
-        for (int u = 0; u < kPer; ++u) {
-            if (w + u * kWarps >= kTiles) break;
-            const double* X = psm + (row[u] + g) * kLdP + t;
-            const double* Y = psm + (col[u] + g) * kLdP + t;
+            for (int u = 0; u < kPer; ++u) {
+                if (w + u * kWarps >= kTiles) break;
+                const double* X = psm + (row[u] + g) * kLdP + t;
+                const double* Y = psm + (col[u] + g) * kLdP + t;
 #pragma unroll 4
-            for (int kk = 0; kk < kK; kk += 4) {
-                const double a0 = -X[kk], a1 = -X[8 * kLdP + kk], b0 = Y[kk], b1 = Y[8 * kLdP + kk];
-                dmma(acc[u][0][0], a0, b0);
-                dmma(acc[u][0][1], a0, b1);
-                dmma(acc[u][1][0], a1, b0);
-                dmma(acc[u][1][1], a1, b1);
+                for (int kk = 0; kk < kK; kk += 4) {
+                    const double a0 = -X[kk], a1 = -X[8 * kLdP + kk], b0 = Y[kk], b1 = Y[8 * kLdP + kk];
+                    dmma(acc[u][0][0], a0, b0);
+                    dmma(acc[u][0][1], a0, b1);
+                    dmma(acc[u][1][0], a1, b0);
+                    dmma(acc[u][1][1], a1, b1);
+                }
             }
+            __syncthreads();
         }
-        __syncthreads();
         // the block into S, zeros above its diagonal
 #pragma unroll
         for (int u = 0; u < kPer; ++u) {
@@ -327,10 +333,12 @@ int launch_small(const TallGeometry& g, int64_t nf, const double* delta, const d
 }
 
 template <int NB, bool kUpdate>
-void launch_diag(const TallGeometry& g, int64_t nf, double* a, int64_t k, unsigned long long* err_pivot, cudaStream_t s) {
+void launch_diag(const TallGeometry& g, int64_t nf, double* a, int64_t k, int64_t depth, unsigned long long* err_pivot,
+                 cudaStream_t s) {
     constexpr size_t smem = diag_smem<NB, kUpdate>();
     GWB_CUDA(cudaFuncSetAttribute(k_diag64<NB, kUpdate>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_diag64<NB, kUpdate><<<(unsigned)nf, DiagShape<NB>::kThreads, smem, s>>>(a, g.ld, g.stride, k, err_pivot);
+    k_diag64<NB, kUpdate><<<(unsigned)nf, DiagShape<NB>::kThreads, smem, s>>>(a, g.ld, g.stride, k, (int)depth,
+                                                                                 err_pivot);
     GWB_LAUNCH("k_diag64");
 }
 
@@ -372,12 +380,11 @@ int launch_small64(const TallGeometry& g, int64_t nf, const double* delta, const
     return launch_small<128>(g, nf, delta, omega, v, xt, q, ldq, err_pivot, s);
 }
 
-int launch_diag64(const TallGeometry& g, int64_t nf, double* a, int64_t k, int64_t width, unsigned long long* err_pivot,
-                  cudaStream_t s) {
-    if (width == 2 * kNb)
-        k > 0 ? launch_diag<128, true>(g, nf, a, k, err_pivot, s) : launch_diag<128, false>(g, nf, a, k, err_pivot, s);
-    else
-        k > 0 ? launch_diag<64, true>(g, nf, a, k, err_pivot, s) : launch_diag<64, false>(g, nf, a, k, err_pivot, s);
+int launch_diag64(const TallGeometry& g, int64_t nf, double* a, int64_t k, int64_t width, int64_t depth,
+                  unsigned long long* err_pivot, cudaStream_t s) {
+    auto run = width == 2 * kNb ? (depth > 0 ? launch_diag<128, true> : launch_diag<128, false>)
+                                : (depth > 0 ? launch_diag<64, true> : launch_diag<64, false>);
+    run(g, nf, a, k, depth, err_pivot, s);
     return 1;
 }
 

@@ -64,6 +64,27 @@ def test_next_block_beside_the_update(n, update, monkeypatch):
     np.testing.assert_array_equal(many.reshape(67, 3, -1), np.broadcast_to(q.reshape(3, -1), (67, 3, q[0].size)))
 
 
+@pytest.mark.parametrize("n", [257, 449, 512, 513, 577, 641])
+def test_int8_update_in_pairs_of_blocks(n, monkeypatch):
+    """One, two and three pairs of 128-column blocks with 64 or 128 columns or another block behind them: the
+    forms of numpy, and scaled exactly with right-hand sides that are scaled by a power of two."""
+    from minigw_b200 import B200Backend
+
+    monkeypatch.setenv("GWB200_FP64_UPDATE", "ozaki")
+    sl = _system(n, n // 2, 1, 1300 + n)
+    omegas = np.array([1e-2, 0.9])
+    with B200Backend(0) as be:
+        be.load_slices(sl)
+        q, _ = be.screened_forms(omegas, sl.states)
+        sl.panel = sl.panel * 2.0**-300
+        be.load_slices(sl)
+        small, _ = be.screened_forms(omegas, sl.states)
+        sl.panel = sl.panel * 2.0**300
+    ref = _forms(sl, omegas)
+    assert np.abs(q - ref).max() <= 1e-11 * np.abs(ref).max()  # as above
+    np.testing.assert_array_equal(small * 2.0**600, q)
+
+
 @pytest.mark.parametrize("n,pivot", [(40, 0), (40, 15), (40, 16), (100, 63), (100, 64), (200, 127), (200, 128), (200, 199)])
 def test_reported_pivot(n, pivot):
     from minigw_b200 import B200Backend
