@@ -426,7 +426,11 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
     const char* prof_env = std::getenv("GWB200_PROFILE");
     UpdateProfiler prof(prof_env && prof_env[0] == '1', s);
     int64_t chunks = 0;
-    if (!small && !cplx && !mixed && g.n_pad > 2 * kNb && h->persistent_ctas == 0) h->side.ensure();
+    const SideStream* side = nullptr;  // a capped handle's share of the GPU is taken by its own kernels
+    if (!small && !mixed && g.n_pad > kNb && h->persistent_ctas == 0) {
+        h->side.ensure();
+        side = &h->side;
+    }
     int upd_variant = -1;  // FP64 update kernel, tuned on the first chunk (full size) of this geometry
     for (int64_t f0 = 0; f0 < nfreq; f0 += fc) {
         const int64_t nf = std::min(fc, nfreq - f0);
@@ -442,7 +446,7 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
             launches += launch_factor_chunk_c(g, nf, h->delta.as<double>(), h->call.omega + f0, eta,
                                               h->v.as<double>(), h->xt.as<double>(), a_re, a_re + (size_t)nf * g.stride,
                                               h->dvec.as<double>(), h->qacc.as<double>(),
-                                              h->err(), s);
+                                              h->err(), s, side);
             launches += launch_forms_out_c(h->qacc.as<double>(), nf, m, g.m_pad,
                                            h->qall.as<double>() + f0 * 2 * g.m_pad, g.m_pad, s);
             ++chunks;
@@ -480,7 +484,7 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
                                             h->err(), s, prof.enabled ? &prof : nullptr,
                                             upd_variant, fp64_oz ? h->panel32.p : nullptr,
                                             h->tc_sched.as<unsigned long long>(), h->persistent_ctas,
-                                            h->side.stream ? &h->side : nullptr);
+                                            side);
             if (after_factor) {
                 (*after_factor)(g, f0, nf);
                 ++launches;

@@ -304,7 +304,7 @@ int launch_update32_tc(const TallGeometry& g, int64_t nf, float* a, int64_t c_be
 // of geometry g; svec 2*n_pad, qacc 2*m_pad doubles per frequency.
 int launch_factor_chunk_c(const TallGeometry& g, int64_t nf, const double* delta, const double* omega, double eta,
                           const double* v, const double* xt, double* a_re, double* a_im, double* svec, double* qacc,
-                          unsigned long long* err_pivot, cudaStream_t s);
+                          unsigned long long* err_pivot, cudaStream_t s, const SideStream* side = nullptr);
 int launch_forms_out_c(const double* qacc, int64_t nf, int64_t m, int64_t ldq, double* q_out, int64_t ldq_out,
                        cudaStream_t s);
 int launch_sigma_contract_c(const double* qall, int64_t nf_int, int64_t nstates, int64_t nmo, int64_t ldq,

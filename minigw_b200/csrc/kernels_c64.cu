@@ -11,6 +11,7 @@
 // is four FP64 DMMA tile products on separate real and imaginary planes.  At eta = 0 this path
 // gives the real path's numbers (S = i D^1/2); the real path is used there.
 #include "panel_common.cuh"
+#include "tc_common.cuh"
 
 #include <cmath>
 
@@ -358,26 +359,6 @@ __device__ void factor_diag_c(double* __restrict__ Sr, double* __restrict__ Si, 
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(256) k_diag_c(double* __restrict__ a_re, double* __restrict__ a_im, int64_t ld,
-                                                int64_t stride, int64_t k, unsigned long long* err_pivot) {
-    extern __shared__ __align__(16) double smem[];
-    double* Sr = smem;
-    double* Si = Sr + kPlane;
-    const size_t base = (size_t)blockIdx.x * stride + k * ld + k;
-    for (int idx = threadIdx.x; idx < kPlane; idx += 256) {
-        const int i = idx / kLdc, j = idx % kLdc;
-        Sr[idx] = j <= i ? a_re[base + (size_t)i * ld + j] : 0.0;
-        Si[idx] = j <= i ? a_im[base + (size_t)i * ld + j] : 0.0;
-    }
-    __syncthreads();
-    factor_diag_c(Sr, Si, Si + kPlane, k, err_pivot);
-    for (int idx = threadIdx.x; idx < kNb * kNb; idx += 256) {  // the inverse in place of the block
-        const int i = idx / kNb, j = idx % kNb;
-        a_re[base + (size_t)i * ld + j] = j <= i ? Sr[j * kLdc + i + 1] : 0.0;
-        a_im[base + (size_t)i * ld + j] = j <= i ? Si[j * kLdc + i + 1] : 0.0;
-    }
-}
-
 __device__ __forceinline__ void cp_async16c(double* dst, const double* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
 }
@@ -388,6 +369,115 @@ __device__ __forceinline__ void load_rows_c(double* dst, int plane, int ldm, con
         const int r = idx / (w / 2), c = 2 * (idx % (w / 2));
         cp_async16c(dst + r * ldm + c, re + (size_t)r * ld + c);
         cp_async16c(dst + plane + r * ldm + c, im + (size_t)r * ld + c);
+    }
+}
+
+// One CTA per frequency: the diagonal block, first updated by the `depth` (0, 64 or 128) columns before it
+// (the trailing update leaves it out, so that it is factored beside that update), replaced by its inverse
+// factor.
+__global__ void __launch_bounds__(256) k_diag_c(double* __restrict__ a_re, double* __restrict__ a_im, int64_t ld,
+                                                int64_t stride, int64_t k, int depth, unsigned long long* err_pivot) {
+    extern __shared__ __align__(16) double smem[];
+    double* Sr = smem;
+    double* Si = Sr + kPlane;
+    const size_t base = (size_t)blockIdx.x * stride + k * ld + k;
+    if (depth > 0) {
+        // 64 columns of the panel's rows at a time through S, the block's lower 16 x 16 tiles in registers
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+        constexpr int kLower = 10;  // lower 16 x 16 tiles of the block
+        double ar[2][2][2][2] = {}, ai[2][2][2][2] = {};
+        int row[2], col[2];
+        load_rows_c(Sr, kPlane, kLdc, a_re + base - depth, a_im + base - depth, ld, kNb, kNb);
+        asm volatile("cp.async.commit_group;\n" ::);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int x = w + 8 * u;
+            int gi = 0, first = 0;
+            while (first + gi + 1 <= x) first += ++gi;
+            row[u] = 16 * gi;
+            col[u] = 16 * (x - first);
+            if (x < kLower)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    const size_t at = base + (size_t)(row[u] + 8 * h + g) * ld + col[u] + 8 * v + 2 * t;
+                    const double2 re = *reinterpret_cast<const double2*>(a_re + at);
+                    const double2 im = *reinterpret_cast<const double2*>(a_im + at);
+                    ar[u][h][v][0] = re.x;
+                    ar[u][h][v][1] = re.y;
+                    ai[u][h][v][0] = im.x;
+                    ai[u][h][v][1] = im.y;
+                }
+        }
+        for (int from = depth; from > 0; from -= kNb) {
+            if (from < depth) {
+                load_rows_c(Sr, kPlane, kLdc, a_re + base - from, a_im + base - from, ld, kNb, kNb);
+                asm volatile("cp.async.commit_group;\n" ::);
+            }
+            asm volatile("cp.async.wait_group 0;\n" ::);
+            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                if (w + 8 * u >= kLower) continue;
+                const double* X = Sr + (row[u] + g) * kLdc + t;
+                const double* Y = Sr + (col[u] + g) * kLdc + t;
+#pragma unroll 2
+                for (int kk = 0; kk < kNb; kk += 4) {
+                    double xr[2], xi[2];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        xr[h] = -X[8 * h * kLdc + kk];
+                        xi[h] = X[kPlane + 8 * h * kLdc + kk];
+                    }
+#pragma unroll
+                    for (int v = 0; v < 2; ++v) {
+                        const double br = Y[8 * v * kLdc + kk], bi = Y[kPlane + 8 * v * kLdc + kk];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            panel::dmma(ar[u][h][v], xr[h], br);
+                            panel::dmma(ai[u][h][v], xr[h], bi);
+                            panel::dmma(ar[u][h][v], xi[h], bi);
+                            panel::dmma(ai[u][h][v], -xi[h], br);
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        // the block into S, zeros above its diagonal
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            if (w + 8 * u < kLower)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    const int i = row[u] + 8 * h + g, j = col[u] + 8 * v + 2 * t;
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        Sr[i * kLdc + j + q] = j + q <= i ? ar[u][h][v][q] : 0.0;
+                        Si[i * kLdc + j + q] = j + q <= i ? ai[u][h][v][q] : 0.0;
+                    }
+                }
+        }
+        for (int idx = threadIdx.x; idx < kPlane; idx += 256) {
+            const int i = idx / kLdc, j = idx % kLdc;
+            if ((j & ~15) > i) Sr[idx] = Si[idx] = 0.0;
+        }
+    } else {
+        for (int idx = threadIdx.x; idx < kPlane; idx += 256) {
+            const int i = idx / kLdc, j = idx % kLdc;
+            Sr[idx] = j <= i ? a_re[base + (size_t)i * ld + j] : 0.0;
+            Si[idx] = j <= i ? a_im[base + (size_t)i * ld + j] : 0.0;
+        }
+    }
+    __syncthreads();
+    factor_diag_c(Sr, Si, Si + kPlane, k, err_pivot);
+    for (int idx = threadIdx.x; idx < kNb * kNb; idx += 256) {  // the inverse in place of the block
+        const int i = idx / kNb, j = idx % kNb;
+        a_re[base + (size_t)i * ld + j] = j <= i ? Sr[j * kLdc + i + 1] : 0.0;
+        a_im[base + (size_t)i * ld + j] = j <= i ? Si[j * kLdc + i + 1] : 0.0;
     }
 }
 
@@ -491,7 +581,7 @@ __global__ void __launch_bounds__(256, 2) k_update_c(double* __restrict__ a_re, 
                                                      int64_t stride, int64_t kb0, int nk, int64_t tc0, int64_t T,
                                                      int64_t nsq) {
     extern __shared__ __align__(16) double smem[];
-    const int64_t x = blockIdx.x, L = nsq - tc0;
+    const int64_t x = blockIdx.x + 1, L = nsq - tc0;  // tile 0, the next diagonal block, is k_diag_c's
     const int64_t n_square = T * L - T * (T - 1) / 2;
     int64_t c, tr;
     if (x < n_square) {
@@ -627,7 +717,7 @@ __global__ void __launch_bounds__(256) k_sigma_contract_c(const double* __restri
 
 int launch_factor_chunk_c(const TallGeometry& g, int64_t nf, const double* delta, const double* omega, double eta,
                           const double* v, const double* xt, double* a_re, double* a_im, double* svec, double* qacc,
-                          unsigned long long* err_pivot, cudaStream_t s) {
+                          unsigned long long* err_pivot, cudaStream_t s, const SideStream* side) {
     const size_t smem_diag = sizeof(double) * (2 * kPlane + kCWork);
     GWB_CUDA(cudaFuncSetAttribute(k_diag_c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_diag));
     GWB_CUDA(cudaFuncSetAttribute(k_panel_c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmemC));
@@ -641,24 +731,29 @@ int launch_factor_chunk_c(const TallGeometry& g, int64_t nf, const double* delta
     GWB_CUDA(cudaMemsetAsync(qacc, 0, sizeof(double) * 2 * (size_t)nf * g.m_pad, s));
     int launches = 2;
     const int64_t nsq = g.n_pad / kNb, nrt = g.rows / kNb;
-    auto update = [&](int64_t kb0, int nk, int64_t tc0, int64_t T) {
-        const int64_t L = nsq - tc0, tiles = T * L - T * (T - 1) / 2 + T * (nrt - nsq);
-        if (tiles <= 0) return;
-        k_update_c<<<dim3((unsigned)tiles, (unsigned)nf), 256, kUpdateSmemC, s>>>(a_re, a_im, g.ld, g.stride, kb0, nk, tc0,
-                                                                                T, nsq);
-        GWB_LAUNCH("k_update_c");
-        ++launches;
-    };
-    for (int64_t b = 0; b < nsq; ++b) {  // outer blocks of two 64-wide blocks
-        if (b & 1) update((b - 1) * kNb, 1, b, 1);  // the first block onto the second's columns
-        k_diag_c<<<(unsigned)nf, 256, smem_diag, s>>>(a_re, a_im, g.ld, g.stride, b * kNb, err_pivot);
+    // the next diagonal block beside the trailing update, as in the plain form
+    if (nf >= tc::sm_count()) side = nullptr;
+    auto diag = [&](int64_t b, int64_t depth) {
+        k_diag_c<<<(unsigned)nf, 256, smem_diag, s>>>(a_re, a_im, g.ld, g.stride, b * kNb, (int)depth, err_pivot);
         GWB_LAUNCH("k_diag_c");
+    };
+    diag(0, 0);
+    for (int64_t b = 0; b < nsq; ++b) {  // outer blocks of two 64-wide blocks
         const int64_t tiles = (g.rows - (b + 1) * kNb) / 32;
         k_panel_c<<<dim3((unsigned)panel_grid(tiles, nf, 2), (unsigned)nf), 256, kPanelSmemC, s>>>(
             a_re, a_im, g.ld, g.stride, b * kNb, g.n_pad, (int)tiles, qacc, g.m_pad);
         GWB_LAUNCH("k_panel_c");
         launches += 2;
-        if ((b & 1) && b + 1 < nsq) update((b - 1) * kNb, 2, b + 1, nsq - b - 1);
+        if (b + 1 == nsq) break;
+        // behind the first block of two the second's columns (K = 64), behind the second all (K = 128)
+        const int nk = 1 + (int)(b & 1);
+        const int64_t tc0 = b + 1, T = nk == 1 ? 1 : nsq - tc0, L = nsq - tc0;
+        SideScope beside(side, s);
+        diag(b + 1, nk * kNb);
+        k_update_c<<<dim3((unsigned)(T * L - T * (T - 1) / 2 + T * (nrt - nsq) - 1), (unsigned)nf), 256, kUpdateSmemC,
+                     beside.stream()>>>(a_re, a_im, g.ld, g.stride, (tc0 - nk) * kNb, nk, tc0, T, nsq);
+        GWB_LAUNCH("k_update_c");
+        ++launches;
     }
     return launches;
 }
