@@ -126,96 +126,97 @@ __global__ void __launch_bounds__(256) k_slice_ct(const double* __restrict__ ct,
     if (lane == 0) exps[row] = e;
 }
 
-// One CTA per right-hand side j of one frequency (k_refine_prep's inputs): y_j = dvec * z_j in FP64,
+// One warp per right-hand side j of one frequency (k_refine_prep's inputs): y_j = dvec * z_j in FP64,
 // rounded to kBSl balanced digits below its row scale; the digits into B slices [kc][t][j][128 B] of
 // the frequency, the exponent into yexp; t1 = x_j . y^ and t2 = z^ . z^ (z^ = y^ / dvec) from the
-// rounded values (fixed-order sums).  The grid's x index is the frequency, so that the CTAs in flight
-// together share j and its row of xt (read from DRAM once, not once per frequency).
-constexpr int64_t kPrepMaxNpad = 25600;  // y staged in shared memory: 8 n_pad bytes <= 200 KB
-constexpr int kPrepThreads = 256;        // 8 warps: the block reductions keep one value per warp
+// rounded values (fixed-order sums).  A block's warps are eight frequencies of one j, so that they share
+// its row of xt.  Bound by the bytes of z and the digits and by their FP64 arithmetic; a warp reads its
+// row twice (the second time from L1) instead of staging y in shared memory: 389 us at 750 rows of 1980
+// x 64 frequencies, where a block per row with its barriers and one conversion per digit took 611.
+constexpr int64_t kPrepMaxNpad = 25600;
+constexpr int kPrepWarps = 8;
 
-__global__ void __launch_bounds__(kPrepThreads) k_refine_prep_oz(const float* __restrict__ a, int64_t ld, int64_t stride,
-                                                        int64_t row0, int64_t na, int64_t n, int64_t n_pad, int64_t nk,
-                                                        int64_t m, int64_t m_pad, const double* __restrict__ xt,
-                                                        const double* __restrict__ dvec, uint8_t* __restrict__ yslices,
-                                                        size_t fbytes, int32_t* __restrict__ yexp,
-                                                        double* __restrict__ t12) {
-    extern __shared__ double yrow[];  // n_pad
-    __shared__ double r1[kPrepThreads / 32], r2[kPrepThreads / 32], rm[kPrepThreads / 32];  // one value per warp
-    const int f = blockIdx.x;
+__global__ void __launch_bounds__(32 * kPrepWarps)
+    k_refine_prep_oz(const float* __restrict__ a, int64_t ld, int64_t stride, int64_t row0, int64_t na, int64_t n,
+                     int64_t n_pad, int64_t nk, int64_t m, int64_t m_pad, int nf, const double* __restrict__ xt,
+                     const double* __restrict__ dvec, uint8_t* __restrict__ yslices, size_t fbytes,
+                     int32_t* __restrict__ yexp, double* __restrict__ t12) {
+    const int f = blockIdx.x * kPrepWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (f >= nf) return;
     const int64_t j = blockIdx.y;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float* row = a + (size_t)f * stride + (size_t)(row0 + j) * ld;
     const double* d = dvec + (size_t)f * n_pad;
+    const double* x = xt + j * n;
     const bool live = j < m;
-    double mx = 0.0;
-    for (int64_t i = threadIdx.x; i < n_pad; i += blockDim.x) {
-        const double yi = (live && i < n) ? d[i] * (double)row[na - 1 - i] : 0.0;
-        yrow[i] = yi;
-        mx = fmax(mx, fabs(yi));
-    }
-    // block maximum: shuffle tree per warp, then the 8 warp values (two barriers)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) rm[warp] = mx;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double v = rm[0];
-        for (int w = 1; w < kPrepThreads / 32; ++w) v = fmax(v, rm[w]);
-        rm[0] = v;
-    }
-    __syncthreads();
-    int e = 0;
-    if (rm[0] > 0.0) frexp(rm[0], &e);
-    ++e;  // |y| < 2^{e-1}
-    const double inv = pow2i(-e), scale = pow2i(e);
-    uint8_t* out = yslices + (size_t)f * fbytes;
-    double s1 = 0.0, s2 = 0.0;
-    for (int64_t w4 = threadIdx.x; w4 < nk / 4; w4 += blockDim.x) {  // 4 consecutive elements per word
-        const int64_t i0 = w4 * 4, kc = i0 / kKc;
-        const int kb = (int)(i0 % kKc);
-        uint32_t word[kBSl] = {};
+    // y of four columns i0 .. i0 + 3 (the solve left z reversed), with their scales
+    auto load = [&](int64_t i0, double (&y)[4], double (&di)[4]) {
+        float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+        double2 d0 = make_double2(0.0, 0.0), d1 = d0;
+        if (live && i0 < n) {  // n_pad is a multiple of 4
+            z = *reinterpret_cast<const float4*>(row + na - 4 - i0);
+            d0 = *reinterpret_cast<const double2*>(d + i0);
+            d1 = *reinterpret_cast<const double2*>(d + i0 + 2);
+        }
+        const double di_[4] = {d0.x, d0.y, d1.x, d1.y};
+        const float z_[4] = {z.w, z.z, z.y, z.x};
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const int64_t i = i0 + q;
-            double v = i < n_pad ? yrow[i] * inv : 0.0;  // |v| < 1/2, exact
-            double rec = 0.0;          // the rounded value, in units of the last digit
+            di[q] = di_[q];
+            y[q] = i0 + q < n ? di_[q] * (double)z_[q] : 0.0;
+        }
+    };
+    double mx = 0.0;
+#pragma unroll 4
+    for (int64_t i0 = 4 * lane; i0 < n_pad; i0 += 128) {
+        double y[4], di[4];
+        load(i0, y, di);
 #pragma unroll
-            for (int t = 0; t < kBSl; ++t) {
-                const int dg = next_digit(v);
-                rec = fma(rec, 128.0, (double)dg);  // exact: |rec| < 2^{7 kBSl}
-                word[t] |= ((uint32_t)dg & 0xFFu) << (8 * q);
-            }
-            if (live && i < n) {
-                const double yh = rec * pow2i(-7 * kBSl) * scale;  // exact
-                const double zh = yh / d[i];
-                s1 = fma(xt[j * n + i], yh, s1);
+        for (int q = 0; q < 4; ++q) mx = fmax(mx, fabs(y[q]));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    int e = 0;
+    if (mx > 0.0) frexp(mx, &e);
+    ++e;  // |y| < 2^{e-1}
+    // y / 2^e rounded to 28 bits: an integer whose four balanced 7-bit digits are those of itself plus 64
+    // in every place, minus 64
+    static_assert(kBSl == 4, "28 bits");
+    const double inv = pow2i(7 * kBSl - e), scale = pow2i(e - 7 * kBSl);
+    uint8_t* out = yslices + (size_t)f * fbytes;
+    double s1 = 0.0, s2 = 0.0;
+#pragma unroll 2
+    for (int64_t i0 = 4 * lane; i0 < nk; i0 += 128) {  // 4 consecutive elements per word
+        const int64_t kc = i0 / kKc;
+        uint32_t word[kBSl] = {};
+        double y[4], di[4];
+        load(i0, y, di);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int rec = __double2int_rn(y[q] * inv);  // |rec| <= 2^27
+            const uint32_t u = (uint32_t)(rec + 0x08102040);
+            word[0] |= ((u >> 21) - 64u & 0xFFu) << (8 * q);
+            word[1] |= ((u >> 14 & 127u) - 64u & 0xFFu) << (8 * q);
+            word[2] |= ((u >> 7 & 127u) - 64u & 0xFFu) << (8 * q);
+            word[3] |= ((u & 127u) - 64u & 0xFFu) << (8 * q);
+            if (live && i0 + q < n) {
+                const double yh = (double)rec * scale;  // exact
+                const double zh = yh / di[q];
+                s1 = fma(x[i0 + q], yh, s1);
                 s2 = fma(zh, zh, s2);
             }
         }
 #pragma unroll
         for (int t = 0; t < kBSl; ++t)
-            *reinterpret_cast<uint32_t*>(out + ((size_t)(kc * kBSl + t) * m_pad) * kKc + swz(j, kb)) = word[t];
+            *reinterpret_cast<uint32_t*>(out + ((size_t)(kc * kBSl + t) * m_pad) * kKc + swz(j, 4 * lane)) = word[t];
     }
-    // block sums in a fixed order: shuffle tree per warp, then the 8 warp sums in warp order
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         s1 += __shfl_xor_sync(0xffffffffu, s1, o);
         s2 += __shfl_xor_sync(0xffffffffu, s2, o);
     }
     if (lane == 0) {
-        r1[warp] = s1;
-        r2[warp] = s2;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double u1 = r1[0], u2 = r2[0];
-        for (int w = 1; w < kPrepThreads / 32; ++w) {
-            u1 += r1[w];
-            u2 += r2[w];
-        }
-        t12[((size_t)f * m_pad + j) * 2] = u1;
-        t12[((size_t)f * m_pad + j) * 2 + 1] = u2;
+        t12[((size_t)f * m_pad + j) * 2] = s1;
+        t12[((size_t)f * m_pad + j) * 2 + 1] = s2;
         yexp[(size_t)f * m_pad + j] = e;
     }
 }
@@ -440,11 +441,9 @@ int launch_refine_terms_oz(const TallGeometry& ga, int64_t nf, const float* a, c
     int32_t* yexp = reinterpret_cast<int32_t*>(ysl + fbytes * (size_t)nf);
     double* t12 = reinterpret_cast<double*>(yexp + ((size_t)nf * m_pad + 1) / 2 * 2);
     double* part = t12 + (size_t)nf * 2 * m_pad;
-    const size_t prep_smem = sizeof(double) * (size_t)n_pad;
-    GWB_CUDA(cudaFuncSetAttribute(k_refine_prep_oz, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep_smem));
     if (m_pad > 65535) fail(GWB200_BAD_SHAPE, "refined form: more than 65535 right-hand sides per frequency");
-    k_refine_prep_oz<<<dim3((unsigned)nf, (unsigned)m_pad), kPrepThreads, prep_smem, s>>>(
-        a, ga.ld, ga.stride, ga.n_pad, gm.n_pad, gm.n, n_pad, nk, gm.m, m_pad, xt, dvec, ysl, fbytes, yexp, t12);
+    k_refine_prep_oz<<<dim3((unsigned)((nf + kPrepWarps - 1) / kPrepWarps), (unsigned)m_pad), 32 * kPrepWarps, 0, s>>>(
+        a, ga.ld, ga.stride, ga.n_pad, gm.n_pad, gm.n, n_pad, nk, gm.m, m_pad, (int)nf, xt, dvec, ysl, fbytes, yexp, t12);
     GWB_LAUNCH("k_refine_prep_oz");
     const uint8_t* asl = static_cast<const uint8_t*>(ct_slices);
     const int32_t* aex = reinterpret_cast<const int32_t*>(asl + (size_t)kASl * r128 * nk);
