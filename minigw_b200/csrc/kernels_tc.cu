@@ -475,7 +475,7 @@ int64_t tc_panel_rows(const TallGeometry& g, int64_t c_begin) { return round_up(
 
 int launch_update32_tc(const TallGeometry& g, int64_t nf, float* a, int64_t c_begin, const float* panel,
                        unsigned long long* sched, unsigned long long* err, cudaStream_t s, int max_ctas,
-                       int64_t row_min) {
+                       int64_t row_min, TileRows which) {
     const int64_t T = (g.n_pad - c_begin + kTcN - 1) / kTcN;  // the last column tile may be 64 wide
     if (T <= 0 || nf <= 0) return 0;
     const int64_t H = g.rows - c_begin;
@@ -510,6 +510,13 @@ int launch_update32_tc(const TallGeometry& g, int64_t nf, float* a, int64_t c_be
     // row_min > c_begin (the solve-only pass): only the row tiles that reach row_min have work
     const int64_t i0 = std::max<int64_t>(0, (row_min - c_begin) / kTcM);
     us.per_f = (NI - i0) * us.NS;
+    if (which == TileRows::kFirst) {  // row tile 0 has one column tile
+        us.NI = 1;
+        us.NS = us.per_f = 1;
+    } else if (which == TileRows::kRest) {
+        us.per_f -= us.NS;
+        if (us.per_f == 0) return 0;
+    }
     us.total = nf * us.per_f;
     const unsigned grid = (unsigned)std::min<int64_t>(us.total, max_ctas > 0 ? std::min(max_ctas, sm_count()) : sm_count());
     // GWB200_TEST_EXPIRE_WAIT=1 (tests only): one CTA withholds its first operand stage, so a
