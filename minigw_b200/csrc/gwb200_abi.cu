@@ -427,7 +427,7 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
     UpdateProfiler prof(prof_env && prof_env[0] == '1', s);
     int64_t chunks = 0;
     const SideStream* side = nullptr;  // a capped handle's share of the GPU is taken by its own kernels
-    if (!small && !mixed && g.n_pad > kNb && h->persistent_ctas == 0) {
+    if (!small && g.n_pad > kNb && h->persistent_ctas == 0) {
         h->side.ensure();
         side = &h->side;
     }
@@ -464,7 +464,7 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
                                               h->err(), s, prof.enabled ? &prof : nullptr,
                                               mixed_tc ? h->panel32.as<float>() : nullptr,
                                               h->tc_sched.as<unsigned long long>(), h->persistent_ctas,
-                                              /*keep_rows=*/refine);
+                                              /*keep_rows=*/refine, /*solve_only=*/false, side);
             if (refine)  // qacc <- 2 x^T y - z^T z - y^T V y (FP64 energy functional at the FP32 solve)
                 launches += launch_refine_chunk(g, nf, h->a.as<float>(), h->xt.as<double>(),
                                                 h->dvec.as<double>(), fac, h->refine.p,

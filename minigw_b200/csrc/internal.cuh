@@ -241,9 +241,10 @@ int launch_build_tall32(const TallGeometry& g, const double* v, const double* xt
 // right-hand sides against a factor that is already there.
 int launch_factor_chunk32(const TallGeometry& g, int64_t nf, float* a, double* qacc, unsigned long long* err_pivot,
                           cudaStream_t s, UpdateProfiler* prof, float* panel, unsigned long long* sched, int max_ctas,
-                          bool keep_rows, bool solve_only = false);
+                          bool keep_rows, bool solve_only = false, const SideStream* side = nullptr);
 // Work counters of the persistent updates of one factorisation, one per outer block.
-inline size_t sched_bytes(const TallGeometry& g) { return sizeof(unsigned long long) * (size_t)(g.n_pad / (2 * kNb) + 1); }
+inline size_t sched_slots(const TallGeometry& g) { return (size_t)(g.n_pad / (2 * kNb) + 1); }
+inline size_t sched_bytes(const TallGeometry& g) { return sizeof(unsigned long long) * 2 * sched_slots(g); }
 int launch_clear_sched(const TallGeometry& g, unsigned long long* sched, cudaStream_t s);
 // kernels_refine.cu: FP64 energy-functional correction of the mixed form.  launch_pchol factors
 // V = C C^T (pivoted, FP64; `work` of pchol_bytes(n)), returns the rank r and C^T (r_pad x n_pad,
@@ -297,9 +298,11 @@ int launch_refine_terms(const TallGeometry& ga, int64_t nf, const float* a, cons
 // kernel's work counter.  A device wait that expires records pivot 0 in err_pivot.
 size_t tc_panel_bytes_per_freq(const TallGeometry& g);
 int64_t tc_panel_rows(const TallGeometry& g, int64_t c_begin);
+// kFirst: the first 128 rows alone (the next diagonal block), kRest: the others.
+enum class TileRows { kAll, kFirst, kRest };
 int launch_update32_tc(const TallGeometry& g, int64_t nf, float* a, int64_t c_begin, const float* panel,
                        unsigned long long* sched, unsigned long long* err_pivot, cudaStream_t s, int max_ctas = 0,
-                       int64_t row_min = 0);
+                       int64_t row_min = 0, TileRows which = TileRows::kAll);
 // kernels_c64.cu: eta != 0 (complex symmetric M = I - S V S, S = diag(Pi0)^1/2).  Planes a_re/a_im
 // of geometry g; svec 2*n_pad, qacc 2*m_pad doubles per frequency.
 int launch_factor_chunk_c(const TallGeometry& g, int64_t nf, const double* delta, const double* omega, double eta,

@@ -12,6 +12,7 @@
 // There is no FP64 refinement: the result carries FP32-level error (stated, not hidden, by
 // bench.py and the tests).
 #include "panel_common.cuh"
+#include "tc_common.cuh"
 
 #include <cmath>
 
@@ -436,50 +437,69 @@ int launch_build_tall32(const TallGeometry& g, const double* v, const double* xt
 namespace {
 
 template <int NB>
-int launch_block32(const TallGeometry& g, int64_t nf, float* a, int64_t k, double* qacc, unsigned long long* err_pivot,
-                   cudaStream_t s, float* panel, bool solve_only, bool keep) {
-    int launches = 0;
-    if (!solve_only) {
-        GWB_CUDA(cudaFuncSetAttribute(k_diag32<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiag32Smem));
-        k_diag32<NB><<<(unsigned)nf, 256, kDiag32Smem, s>>>(a, g.ld, g.stride, k, err_pivot);
-        GWB_LAUNCH("k_diag32");
-        ++launches;
-    }
-    // the rows below: all of them for the update's operands, else while factoring; the solve-only
-    // pass works on the right-hand sides alone
+void launch_diag32(const TallGeometry& g, int64_t nf, float* a, int64_t k, unsigned long long* err_pivot, cudaStream_t s) {
+    GWB_CUDA(cudaFuncSetAttribute(k_diag32<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiag32Smem));
+    k_diag32<NB><<<(unsigned)nf, 256, kDiag32Smem, s>>>(a, g.ld, g.stride, k, err_pivot);
+    GWB_LAUNCH("k_diag32");
+}
+
+// the rows below a diagonal block: all of them for the update's operands, else while factoring; the
+// solve-only pass works on the right-hand sides alone
+template <int NB>
+int launch_rows32(const TallGeometry& g, int64_t nf, float* a, int64_t k, double* qacc, cudaStream_t s, float* panel,
+                  bool solve_only, bool keep) {
     const int64_t row0 = solve_only && !panel ? g.n_pad : k + NB;
     const int64_t rows_end = panel ? row0 + tc_panel_rows(g, row0) : g.rows;
     const int64_t tiles = (rows_end - row0) / 16;
-    if (tiles <= 0) return launches;
+    if (tiles <= 0) return 0;
     GWB_CUDA(cudaFuncSetAttribute(k_panel32<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanel32Smem<NB>));
     const int64_t gx = panel_grid((tiles + kPanelWarps - 1) / kPanelWarps, nf, 1);
     k_panel32<NB><<<dim3((unsigned)gx, (unsigned)nf), 32 * kPanelWarps, kPanel32Smem<NB>, s>>>(
         a, g.ld, g.stride, k, row0, g.rows, rows_end, solve_only ? g.n_pad : row0, g.n_pad, panel, keep ? 1 : 0, qacc,
         g.m_pad);
     GWB_LAUNCH("k_panel32");
-    return launches + 1;
+    return 1;
 }
 
 }  // namespace
 
 int launch_factor_chunk32(const TallGeometry& g, int64_t nf, float* a, double* qacc, unsigned long long* err_pivot,
                           cudaStream_t s, UpdateProfiler* prof, float* panel, unsigned long long* sched, int max_ctas,
-                          bool keep_rows, bool solve_only) {
+                          bool keep_rows, bool solve_only, const SideStream* side) {
     const size_t smem_update = 4 * 64 * kLdkf * sizeof(float);
     GWB_CUDA(cudaFuncSetAttribute(k_update32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_update));
     const int64_t nsq = g.n_pad / kNb, nrt = g.rows / kNb;
     constexpr int64_t kOuter = 2;
     int launches = 0;
     if (panel && nsq > kOuter) launches += launch_clear_sched(g, sched, s);
+    // As in the plain form the next diagonal block is factored beside the trailing update; its own update
+    // comes first, from the same kernel (its rounding is the form's): 2000 pairs x 64 frequencies 5029 -> 4912
+    // us.  (Not in batches, whose lanes already overlap, nor in the refinement's solve.)
+    if (prof || max_ctas > 0 || solve_only || !panel || nf >= tc::sm_count()) side = nullptr;
+    auto diag = [&](int64_t ob) {
+        if (solve_only) return;
+        nsq - ob >= kOuter ? launch_diag32<128>(g, nf, a, ob * kNb, err_pivot, s)
+                           : launch_diag32<64>(g, nf, a, ob * kNb, err_pivot, s);
+        ++launches;
+    };
+    diag(0);
     for (int64_t ob = 0; ob < nsq; ob += kOuter) {
         const int64_t q = std::min(kOuter, nsq - ob), tc0 = ob + q;
         float* pan = tc0 < nsq ? panel : nullptr;  // operands of the trailing update, when there is one
         const bool keep = keep_rows || !panel;     // the mma.sync update reads the rows themselves
-        launches += q == kOuter ? launch_block32<128>(g, nf, a, ob * kNb, qacc, err_pivot, s, pan, solve_only, keep)
-                                : launch_block32<64>(g, nf, a, ob * kNb, qacc, err_pivot, s, pan, solve_only, keep);
+        launches += q == kOuter ? launch_rows32<128>(g, nf, a, ob * kNb, qacc, s, pan, solve_only, keep)
+                                : launch_rows32<64>(g, nf, a, ob * kNb, qacc, s, pan, solve_only, keep);
         if (tc0 >= nsq) break;
         if (prof) prof->begin();
-        if (pan) {  // trailing update on tcgen05
+        if (side) {
+            unsigned long long* counter = sched + ob / kOuter;
+            launches += launch_update32_tc(g, nf, a, tc0 * kNb, pan, counter + sched_slots(g), err_pivot, s, 0, 0,
+                                           TileRows::kFirst);
+            SideScope beside(side, s);
+            diag(tc0);
+            launches += launch_update32_tc(g, nf, a, tc0 * kNb, pan, counter, err_pivot, beside.stream(), 0, 0,
+                                           TileRows::kRest);
+        } else if (pan) {  // trailing update on tcgen05
             launches += launch_update32_tc(g, nf, a, tc0 * kNb, pan, sched + ob / kOuter, err_pivot, s, max_ctas,
                                            solve_only ? g.n_pad : 0);
         } else {
@@ -493,6 +513,7 @@ int launch_factor_chunk32(const TallGeometry& g, int64_t nf, float* a, double* q
             }
         }
         if (prof) prof->end((double)nf * update_flops32(g, ob * kNb, (int)q, tc0 * kNb, nsq * kNb));
+        if (!side) diag(tc0);
     }
     return launches;
 }
