@@ -214,15 +214,6 @@ def workload_config(args, wl, world: int) -> dict:
             "inputs smaller than L2 (a parity-size workload, not flushed between steps)"}
 
 
-def traffic_oz(workload: str):
-    """DRAM bytes per k_update64_oz launch from the committed ncu capture, if one exists."""
-    try:
-        return json.loads((ROOT / "profiles" / "k_update64_oz_traffic.json").read_text())["workloads"][workload][
-            "bytes_per_launch"]
-    except (OSError, ValueError, KeyError):
-        return None
-
-
 def hbm_peak_gbs() -> float:
     """Measured HBM copy bandwidth of this pool's B200s (MEASURED_PEAKS.json), else the fallback."""
     try:
@@ -618,26 +609,25 @@ def run_b200(args, wl):
     kernel_used = be.update_kernel()
     if args.precision == "fp64" and kernel_used == 6 and achieved:
         # the autotuner chose the int8 tensor-core emulation of the FP64 update (k_slice_panel64 +
-        # k_update64_oz, timed together): bound by the FP64 C read+write, 16 bytes per updated
-        # element per K = 128 pass, i.e. flops_update / 16 bytes; the int8 work is 26 products of
+        # k_update64_oz, timed together).  Against HBM: the FP64 C read+write, 16 bytes per updated
+        # element per K = 256 pass, i.e. flops_update / 32 bytes; the int8 work is 21 products of
         # 6-digit slices per FP64 product
-        gbs = upd_flops / 16.0 / (upd_ms * 1e-3) / 1e9
+        gbs = upd_flops / 32.0 / (upd_ms * 1e-3) / 1e9
         result["roofline"] = {
             "bound": "hbm", "kernel": "k_update64_oz (FP64 trailing update emulated on int8 tcgen05, with "
                                       "k_slice_panel64)",
             "achieved": gbs, "peak": hbm_peak_gbs(), "unit": "GB/s", "frac": gbs / hbm_peak_gbs(),
             "peak_source": hbm_peak_source(),
-            "tflops_fp64_equivalent": achieved, "int8_tops": achieved * 26.0,
-            "vs_fp64_dmma_peak": achieved / peak_fp64, "launches": upd_n, "traffic": traffic_oz(wl.name),
-            "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per k_update64_oz launch "
-                              "(profiles/k_update64_oz_traffic.json)" if traffic_oz(wl.name) else None}
+            "tflops_fp64_equivalent": achieved, "int8_tops": achieved * 21.0,
+            "vs_fp64_dmma_peak": achieved / peak_fp64, "launches": upd_n, "traffic": None,
+            "traffic_source": None}
     if args.precision in ("mixed", "mixed-refined") and achieved:
-        # the tcgen05 3xTF32 trailing update (k_split_panel32 + k_update32_tc, timed together) is
+        # the tcgen05 3xTF32 trailing update (k_update32_tc; the panel solve writes its operands) is
         # bound by the FP32 C read+write, 8 bytes per updated element per K = 128 pass, i.e.
         # flops_update / 32 bytes (flops = 2 K per element)
         gbs = upd_flops / 32.0 / (upd_ms * 1e-3) / 1e9
         result["roofline"] = {
-            "bound": "hbm", "kernel": "k_update32_tc (tcgen05 kind::tf32 3xTF32 trailing update, with k_split_panel32)",
+            "bound": "hbm", "kernel": "k_update32_tc (tcgen05 kind::tf32 3xTF32 trailing update)",
             "achieved": gbs, "peak": hbm_peak_gbs(), "unit": "GB/s", "frac": gbs / hbm_peak_gbs(),
             "peak_source": hbm_peak_source(),
             "tflops_fp32_equivalent": achieved, "launches": upd_n, "traffic": None,

@@ -5,8 +5,8 @@
 //   * the tall matrices stored in FP32 (eps has eigenvalues >= 1, entries O(1..100)), halving HBM
 //     footprint and traffic;
 //   * each 64x64 diagonal block factored and inverted in FP64 in shared memory, stored as FP32;
-//   * the panel solve and the trailing updates on the tensor cores through mma.sync m16n8k8 TF32
-//     with the 3xTF32 split (a = a_hi + a_lo, each a TF32 value; a*b ~ a_hi b_hi + a_hi b_lo +
+//   * the panel solve and the trailing updates on the tensor cores (mma.sync m16n8k8 TF32; the updates
+//     on tcgen05 where kernels_tc.cu takes them) with the 3xTF32 split (a = a_hi + a_lo, each a TF32 value; a*b ~ a_hi b_hi + a_hi b_lo +
 //     a_lo b_hi, accumulated in FP32), about 21 significant bits per product;
 //   * the squared norms, the G0 frequency contraction, Pade and QP in FP64.
 // There is no FP64 refinement: the result carries FP32-level error (stated, not hidden, by
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(32 * kPanelWarps, 1)
     }
 }
 
-// Trailing / look-left update on FP32 tiles (3xTF32), same tile enumeration and K chunking as the
+// Trailing update on FP32 tiles (3xTF32), same tile enumeration and K chunking as the
 // FP64 k_update: output column tiles [tc0, tc0+T), lower square tiles then all RHS tiles
 // (rhs_only: the RHS tiles alone, for the solve-only pass against a finished factor).
 __global__ void __launch_bounds__(256, 3) k_update32(float* __restrict__ a, int64_t ld, int64_t stride, int64_t kb0,
