@@ -147,7 +147,7 @@ template <int NB>
 struct PanelShape {
     static constexpr int kLd = NB + 4;  // = 4 mod 16 (fragment loads on distinct banks)
     static constexpr int kTiles = NB / 32;  // column tiles of 8 per warp
-    static constexpr size_t kSmem = sizeof(double) * ((size_t)NB * kLd + 2 * kRowTile * kLd + 4 * kRowTile);
+    static constexpr size_t kSmem = sizeof(double) * ((size_t)NB * kLd + 2 * kRowTile * kLd + 8 * kRowTile);
 };
 
 template <int NB>
@@ -179,15 +179,21 @@ __global__ void __launch_bounds__(kPanelThreads, 1)
         if (c < (r < kNb ? kNb : NB)) cp_async16(Y + r * LD + c, A + (size_t)(k + r) * ld + k + c);
     }
     load_rows(blockIdx.x, 0);
-    int buf = 0;
-    for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x, buf ^= 1) {
-        if (tile + (int)gridDim.x < ntile) {
-            load_rows(tile + gridDim.x, buf ^ 1);
-            asm volatile("cp.async.wait_group 1;\n" ::);
-        } else {
-            asm volatile("cp.async.wait_group 0;\n" ::);
-        }
+    // squared norms of a right-hand-side tile, from the warps' sums in red[its buffer], after a barrier
+    auto add_norms = [&](int tile, int b) {
+        const int64_t r = row0 + (int64_t)tile * kRowTile - n_pad + threadIdx.x;
+        const double* v = red + b * 4 * kRowTile + threadIdx.x;
+        if (r >= (int64_t)threadIdx.x && threadIdx.x < kRowTile)  // n_pad is a multiple of the tile
+            qacc[(size_t)blockIdx.y * ldq + r] += (v[0] + v[kRowTile]) + (v[2 * kRowTile] + v[3 * kRowTile]);
+    };
+    // one barrier per tile: a warp stores its rows while others still multiply (4480 rows x 128 frequencies
+    // 468 us with a second barrier, 458 without; multiplying alone takes 357)
+    int buf = 0, tile = blockIdx.x;
+    for (; tile < ntile; tile += gridDim.x, buf ^= 1) {
+        asm volatile("cp.async.wait_group 0;\n" ::);
         __syncthreads();
+        if (tile != (int)blockIdx.x) add_norms(tile - gridDim.x, buf ^ 1);
+        if (tile + (int)gridDim.x < ntile) load_rows(tile + gridDim.x, buf ^ 1);
         const double* X = Xs + buf * kRowTile * LD + (r0 + g) * LD + t;
         // column tiles of this warp, ascending: cg, 7 - cg(, 8 + cg, 15 - cg)
         auto col = [&](int i) { return (i >> 1) * 8 + ((i & 1) ? 7 - cg : cg); };
@@ -213,8 +219,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1)
             for (int i = 0; i < NT; ++i)
                 *reinterpret_cast<double2*>(A + (size_t)(row + 8 * h) * ld + k + 8 * col(i) + 2 * t) =
                     make_double2(acc[h][i][0], acc[h][i][1]);
-        const bool rhs = row0 + (int64_t)tile * kRowTile >= n_pad;  // n_pad is a multiple of the tile
-        if (rhs) {  // squared row norms, summed in a fixed order
+        if (row0 + (int64_t)tile * kRowTile >= n_pad) {  // squared row norms, summed in a fixed order
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 double s = 0.0;
@@ -222,16 +227,12 @@ __global__ void __launch_bounds__(kPanelThreads, 1)
                 for (int i = 0; i < NT; ++i) s = fma(acc[h][i][1], acc[h][i][1], fma(acc[h][i][0], acc[h][i][0], s));
                 s += __shfl_xor_sync(0xffffffffu, s, 1);
                 s += __shfl_xor_sync(0xffffffffu, s, 2);
-                if (t == 0) red[cg * kRowTile + r0 + 8 * h + g] = s;
+                if (t == 0) red[(buf * 4 + cg) * kRowTile + r0 + 8 * h + g] = s;
             }
         }
-        __syncthreads();
-        if (rhs && threadIdx.x < kRowTile) {
-            const int r = threadIdx.x;
-            qacc[(size_t)blockIdx.y * ldq + (row0 + (int64_t)tile * kRowTile - n_pad) + r] +=
-                (red[r] + red[kRowTile + r]) + (red[2 * kRowTile + r] + red[3 * kRowTile + r]);
-        }
     }
+    __syncthreads();
+    add_norms(tile - gridDim.x, buf ^ 1);
 }
 
 // Whole frequencies of a small system (n <= NB <= 128), one CTA each: the scale vector, eps, its factor
