@@ -183,8 +183,9 @@ int launch_panel64(const TallGeometry& g, int64_t nf, double* a, int64_t k, int6
 bool small_system(const TallGeometry& g);
 int launch_small64(const TallGeometry& g, int64_t nf, const double* delta, const double* omega, const double* v,
                    const double* xt, double* q, int64_t ldq, unsigned long long* err_pivot, cudaStream_t s);
-// CTAs per frequency of a panel kernel over `tiles` row tiles of nf frequencies, per_sm CTAs per SM
-int64_t panel_grid(int64_t tiles, int64_t nf, int64_t per_sm);
+// CTAs per frequency of a kernel over `tiles` row tiles of nf frequencies, per_sm CTAs per SM; head: what a
+// CTA spends before its first tile, in tile times (a panel kernel's load of the block's tiles: two)
+int64_t panel_grid(int64_t tiles, int64_t nf, int64_t per_sm, double head = 2.0);
 // kernels_oz.cu: FP64 trailing update C -= P P^T (columns [kb0, c_begin) of the panel, 128 or 256, into
 // columns [c_begin, c_end), rows [c_begin, rows)) from exact int8 products of 6-digit row slices
 // (tcgen05 kind::i8).  Two launches.

@@ -235,13 +235,15 @@ __global__ void __launch_bounds__(kPanelThreads, 1)
     add_norms(tile - gridDim.x, buf ^ 1);
 }
 
-// Whole frequencies of a small system (n <= NB <= 128), one CTA each: the scale vector, eps, its factor
+// Whole frequencies of a small system (n <= NB <= 128), a CTA or more each: the scale vector, eps, its factor
 // and inverse in shared memory, then the right-hand sides in 32-row tiles, of which only the forms
 // leave the SM.  The arithmetic and its order are those of k_scale_vectors, k_build_tall, k_diag64,
 // k_panel64 and k_negate_copy, whose five launches and tall matrices it replaces: at this size they
 // spent their time in launches and the matrices' way through memory (24 orbitals, 200 frequencies:
 // 113 us of kernels; this one 39).  NB is the next of 64, 96 and 128, so that up to n = 96 two CTAs
-// share an SM.
+// share an SM.  The row tiles are dealt out over the grid's y; each of a frequency's CTAs factors its
+// block again, on SMs that would be idle (116 pairs, 3600 rows: one CTA per frequency took 472 to 479 us
+// at 1 to 64 frequencies, where the panel kernels take 57 to 312 and these 39 to 260).
 template <int NB>
 struct SmallShape {
     static constexpr int kXLd = NB + 4;
@@ -278,7 +280,7 @@ __global__ void __launch_bounds__(DiagShape<NB>::kThreads) k_small64(int n, int 
     const int g = lane >> 2, t = lane & 3;
     const int r0 = 16 * (warp & 1), cg = warp >> 1;
     auto col = [&](int i) { return (i >> 1) * 8 + ((i & 1) ? 7 - cg : cg); };  // as in k_panel64
-    for (int row = 0; row < m; row += kRowTile) {
+    for (int row = kRowTile * blockIdx.y; row < m; row += kRowTile * gridDim.y) {
         for (int idx = threadIdx.x; idx < kRowTile * NB; idx += Sh::kThreads) {
             const int r = idx / NB, c = idx % NB;
             X[r * XL + c] = (row + r < m && c < n) ? d[c] * xt[(size_t)(row + r) * n + c] : 0.0;
@@ -327,8 +329,12 @@ int launch_small(const TallGeometry& g, int64_t nf, const double* delta, const d
                  const double* xt, double* q, int64_t ldq, unsigned long long* err_pivot, cudaStream_t s) {
     const size_t smem = SmallShape<NB>::kSmem;
     GWB_CUDA(cudaFuncSetAttribute(k_small64<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_small64<NB><<<(unsigned)nf, DiagShape<NB>::kThreads, smem, s>>>((int)g.n, (int)g.m, delta, omega, v, xt, q, ldq,
-                                                                     err_pivot);
+    // the factorisation costs as much as 8 row tiles at every NB; at NB = 64 two CTAs on an SM are as
+    // fast as one (35 pairs, 288 rows, 148 frequencies: 33 us as 148 CTAs, 31 as 296), from 96 on they
+    // take turns (80 pairs, 336 rows: 53 and 70)
+    const int64_t gy = panel_grid((g.m + kRowTile - 1) / kRowTile, nf, NB == 64 ? 2 : 1, 8.0);
+    k_small64<NB><<<dim3((unsigned)nf, (unsigned)gy), DiagShape<NB>::kThreads, smem, s>>>(
+        (int)g.n, (int)g.m, delta, omega, v, xt, q, ldq, err_pivot);
     GWB_LAUNCH("k_small64");
     return 1;
 }
@@ -356,14 +362,14 @@ int launch_rows(const TallGeometry& g, int64_t nf, double* a, int64_t k, double*
 
 }  // namespace
 
-// The fewest tile times over the waves, counting two for a CTA's load of the block's tiles.
-int64_t panel_grid(int64_t tiles, int64_t nf, int64_t per_sm) {
+// The fewest tile times over the waves.
+int64_t panel_grid(int64_t tiles, int64_t nf, int64_t per_sm, double head) {
     const int64_t slots = 148 * per_sm;
     int64_t best = 1;
     double best_cost = 0.0;
     for (int64_t gx = 1; gx <= std::min<int64_t>(tiles, 64); ++gx) {
         const double waves = (double)((nf * gx + slots - 1) / slots);
-        const double cost = waves * ((double)((tiles + gx - 1) / gx) + 2.0);
+        const double cost = waves * ((double)((tiles + gx - 1) / gx) + head);
         if (gx == 1 || cost < best_cost) {
             best = gx;
             best_cost = cost;

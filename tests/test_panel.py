@@ -142,3 +142,36 @@ def test_complex_reported_pivot(pivot):
         with pytest.raises(GwB200Error) as e:
             be.screened_forms_complex(np.array([0.3]), sl.states, eta=0.02)
         assert e.value.status == "GWB200_NOT_SPD" and f"pivot {pivot + 1} " in str(e.value)
+
+
+@pytest.mark.parametrize("n,nstates", [(35, 8), (64, 5), (65, 5), (96, 6), (97, 6), (128, 4)])
+def test_small_system_with_many_rows(n, nstates):
+    """Systems of one kernel (n <= 128) whose row tiles are dealt out over the idle SMs: one frequency, a
+    few, and more than there are SMs, the same forms bit for bit."""
+    from minigw_b200 import B200Backend
+
+    sl = _system(n, n // 2, nstates, 1500 + n)
+    omegas = np.array([1e-3, 0.4, 7.0])
+    with B200Backend(0) as be:
+        be.load_slices(sl)
+        q, _ = be.screened_forms(omegas, sl.states)
+        one, _ = be.screened_forms(omegas[1:2], sl.states)
+        many, _ = be.screened_forms(np.tile(omegas, 100), sl.states)
+    ref = _forms(sl, omegas)
+    assert np.abs(q - ref).max() <= 1e-11 * np.abs(ref).max()  # as above
+    np.testing.assert_array_equal(one[0], q[1])
+    np.testing.assert_array_equal(many.reshape(100, 3, -1), np.broadcast_to(q.reshape(3, -1), (100, 3, q[0].size)))
+
+
+def test_few_frequencies_of_many_rows_use_the_idle_sms():
+    """Two frequencies leave 146 SMs idle: 3510 rows (110 row tiles) may not take three times as long as 117
+    rows (4 tiles).  Walked by one CTA per frequency they take ten times as long."""
+    from minigw_b200 import B200Backend
+
+    def best(nstates):
+        sl = _system(116, 50, nstates, 1700)
+        with B200Backend(0) as be:
+            be.load_slices(sl)
+            return min(be.screened_forms(np.array([0.1, 1.0]), sl.states)[1]["device_ms_screening"] for _ in range(10))
+
+    assert best(30) < 3 * best(1)
