@@ -89,8 +89,9 @@ struct SideStream {
     }
 };
 
-// Work on the side stream, behind what `s` holds at the scope's start and before what `s` is given after the
-// scope (also where the scope is left by an exception).
+// Work on the side stream, behind what `s` holds at the scope's start and before what `s` is given after
+// join().  A scope that is left without it, by an exception, joins as well, and waits for the side stream on
+// the host where that fails: what reads the results, or frees their buffers, waits for `s` alone.
 class SideScope {
     const SideStream* side_;
     cudaStream_t s_;
@@ -108,8 +109,16 @@ class SideScope {
         begun_ = true;
         return side_->stream;
     }
+    void join() {
+        if (!begun_) return;
+        cuda_check(cudaEventRecord(side_->join, side_->stream), "cudaEventRecord", __FILE__, __LINE__);
+        cuda_check(cudaStreamWaitEvent(s_, side_->join, 0), "cudaStreamWaitEvent", __FILE__, __LINE__);
+        begun_ = false;
+    }
     ~SideScope() {
-        if (begun_ && cudaEventRecord(side_->join, side_->stream) == cudaSuccess) cudaStreamWaitEvent(s_, side_->join, 0);
+        if (begun_ && (cudaEventRecord(side_->join, side_->stream) != cudaSuccess ||
+                       cudaStreamWaitEvent(s_, side_->join, 0) != cudaSuccess))
+            cudaStreamSynchronize(side_->stream);
     }
 };
 

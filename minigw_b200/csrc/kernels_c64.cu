@@ -753,6 +753,7 @@ int launch_factor_chunk_c(const TallGeometry& g, int64_t nf, const double* delta
         k_update_c<<<dim3((unsigned)(T * L - T * (T - 1) / 2 + T * (nrt - nsq) - 1), (unsigned)nf), 256, kUpdateSmemC,
                      beside.stream()>>>(a_re, a_im, g.ld, g.stride, (tc0 - nk) * kNb, nk, tc0, T, nsq);
         GWB_LAUNCH("k_update_c");
+        beside.join();
         ++launches;
     }
     return launches;

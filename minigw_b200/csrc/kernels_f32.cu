@@ -499,6 +499,7 @@ int launch_factor_chunk32(const TallGeometry& g, int64_t nf, float* a, double* q
             diag(tc0);
             launches += launch_update32_tc(g, nf, a, tc0 * kNb, pan, counter, err_pivot, beside.stream(), 0, 0,
                                            TileRows::kRest);
+            beside.join();
         } else if (pan) {  // trailing update on tcgen05
             launches += launch_update32_tc(g, nf, a, tc0 * kNb, pan, sched + ob / kOuter, err_pivot, s, max_ctas,
                                            solve_only ? g.n_pad : 0);

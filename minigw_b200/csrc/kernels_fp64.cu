@@ -509,6 +509,7 @@ int launch_factor_chunk(const TallGeometry& g, int64_t nf, double* a, double* qa
             launch_variant(variant, g, nf, a, kb, (int)q, tc0, nsq - tc0, beside.stream(), next);
             ++launches;
         }
+        beside.join();
         const int nk = (int)(tc0 - kb / kNb);
         if (prof)
             prof->end((double)nf * (update_flops(g, kb, nk, tc0 * kNb, c_end * kNb) -
