@@ -426,11 +426,8 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
     const char* prof_env = std::getenv("GWB200_PROFILE");
     UpdateProfiler prof(prof_env && prof_env[0] == '1', s);
     int64_t chunks = 0;
-    const SideStream* side = nullptr;  // a capped handle's share of the GPU is taken by its own kernels
-    if (!small && g.n_pad > kNb && h->persistent_ctas == 0) {
-        h->side.ensure();
-        side = &h->side;
-    }
+    // a capped handle's share of the GPU is taken by its own kernels
+    SideStream* side = h->persistent_ctas == 0 ? &h->side : nullptr;
     int upd_variant = -1;  // FP64 update kernel, tuned on the first chunk (full size) of this geometry
     for (int64_t f0 = 0; f0 < nfreq; f0 += fc) {
         const int64_t nf = std::min(fc, nfreq - f0);

@@ -73,7 +73,8 @@ inline TallGeometry make_geometry(int64_t n, int64_t m) {
     return g;
 }
 
-// A second stream of one handle for work beside its own, with the events that order the two.
+// A second stream of one handle for work beside its own, with the events that order the two; made by the first
+// scope that is given it.
 struct SideStream {
     cudaStream_t stream = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
@@ -93,13 +94,15 @@ struct SideStream {
 // join().  A scope that is left without it, by an exception, joins as well, and waits for the side stream on
 // the host where that fails: what reads the results, or frees their buffers, waits for `s` alone.
 class SideScope {
-    const SideStream* side_;
+    SideStream* side_;
     cudaStream_t s_;
     bool begun_ = false;
 
   public:
-    SideScope(const SideStream* side, cudaStream_t s) : side_(side), s_(s) {
-        if (side_) cuda_check(cudaEventRecord(side_->fork, s_), "cudaEventRecord", __FILE__, __LINE__);
+    SideScope(SideStream* side, cudaStream_t s) : side_(side), s_(s) {
+        if (!side_) return;
+        side_->ensure();
+        cuda_check(cudaEventRecord(side_->fork, s_), "cudaEventRecord", __FILE__, __LINE__);
     }
     SideScope(const SideScope&) = delete;
     SideScope& operator=(const SideScope&) = delete;
@@ -178,7 +181,7 @@ int launch_build_tall(const TallGeometry& g, const double* v, const double* xt, 
 int launch_factor_chunk(const TallGeometry& g, int64_t nf, double* a, double* qacc,
                         unsigned long long* err_pivot, cudaStream_t s, UpdateProfiler* prof, int variant,
                         void* oz = nullptr, unsigned long long* sched = nullptr, int max_ctas = 0,
-                        const SideStream* side = nullptr);
+                        SideStream* side = nullptr);
 // kernels_panel.cu, the panel step of columns [k, k + width), width 64 or 128.  launch_diag64: the
 // diagonal block, replaced by its inverse factor, after its update by the `depth` columns before it (0,
 // 128 or 256).  launch_panel64: every row below; the squared norms of the right-hand-side rows are added to
@@ -251,7 +254,7 @@ int launch_build_tall32(const TallGeometry& g, const double* v, const double* xt
 // right-hand sides against a factor that is already there.
 int launch_factor_chunk32(const TallGeometry& g, int64_t nf, float* a, double* qacc, unsigned long long* err_pivot,
                           cudaStream_t s, UpdateProfiler* prof, float* panel, unsigned long long* sched, int max_ctas,
-                          bool keep_rows, bool solve_only = false, const SideStream* side = nullptr);
+                          bool keep_rows, bool solve_only = false, SideStream* side = nullptr);
 // Work counters of the persistent updates of one factorisation, one per outer block.
 inline size_t sched_slots(const TallGeometry& g) { return (size_t)(g.n_pad / (2 * kNb) + 1); }
 inline size_t sched_bytes(const TallGeometry& g) { return sizeof(unsigned long long) * 2 * sched_slots(g); }
@@ -317,7 +320,7 @@ int launch_update32_tc(const TallGeometry& g, int64_t nf, float* a, int64_t c_be
 // of geometry g; svec 2*n_pad, qacc 2*m_pad doubles per frequency.
 int launch_factor_chunk_c(const TallGeometry& g, int64_t nf, const double* delta, const double* omega, double eta,
                           const double* v, const double* xt, double* a_re, double* a_im, double* svec, double* qacc,
-                          unsigned long long* err_pivot, cudaStream_t s, const SideStream* side = nullptr);
+                          unsigned long long* err_pivot, cudaStream_t s, SideStream* side = nullptr);
 int launch_forms_out_c(const double* qacc, int64_t nf, int64_t m, int64_t ldq, double* q_out, int64_t ldq_out,
                        cudaStream_t s);
 int launch_sigma_contract_c(const double* qall, int64_t nf_int, int64_t nstates, int64_t nmo, int64_t ldq,

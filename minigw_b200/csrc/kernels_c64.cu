@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(256) k_sigma_contract_c(const double* __restri
 
 int launch_factor_chunk_c(const TallGeometry& g, int64_t nf, const double* delta, const double* omega, double eta,
                           const double* v, const double* xt, double* a_re, double* a_im, double* svec, double* qacc,
-                          unsigned long long* err_pivot, cudaStream_t s, const SideStream* side) {
+                          unsigned long long* err_pivot, cudaStream_t s, SideStream* side) {
     const size_t smem_diag = sizeof(double) * (2 * kPlane + kCWork);
     GWB_CUDA(cudaFuncSetAttribute(k_diag_c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_diag));
     GWB_CUDA(cudaFuncSetAttribute(k_panel_c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmemC));

@@ -465,7 +465,7 @@ int launch_rows32(const TallGeometry& g, int64_t nf, float* a, int64_t k, double
 
 int launch_factor_chunk32(const TallGeometry& g, int64_t nf, float* a, double* qacc, unsigned long long* err_pivot,
                           cudaStream_t s, UpdateProfiler* prof, float* panel, unsigned long long* sched, int max_ctas,
-                          bool keep_rows, bool solve_only, const SideStream* side) {
+                          bool keep_rows, bool solve_only, SideStream* side) {
     const size_t smem_update = 4 * 64 * kLdkf * sizeof(float);
     GWB_CUDA(cudaFuncSetAttribute(k_update32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_update));
     const int64_t nsq = g.n_pad / kNb, nrt = g.rows / kNb;

@@ -471,7 +471,7 @@ const char* update_variant_name(int v) {
 
 int launch_factor_chunk(const TallGeometry& g, int64_t nf, double* a, double* qacc, unsigned long long* err_pivot,
                         cudaStream_t s, UpdateProfiler* prof, int variant, void* oz, unsigned long long* sched,
-                        int max_ctas, const SideStream* side) {
+                        int max_ctas, SideStream* side) {
     const bool use_oz = oz && variant == kUpdateOzaki;
     if (variant < 0 || variant >= kNumVariants)  // untuned caller: GWB200_UPDATE_VARIANT, else the default
         variant = env_update_variant() >= 0 ? env_update_variant() : kDefaultUpdateVariant;

@@ -52,9 +52,18 @@ int main(int, char** argv) {
     cudaStream_t own = (cudaStream_t)(size_t)0x1000;
     try {
         if (mode == "unused") return 0;
-        side.ensure();
+        if (mode == "none") {
+            SideScope beside(nullptr, own);
+            std::printf("on %s\n", name(beside.stream()));
+            beside.join();
+            return 0;
+        }
+        if (mode == "twice") {
+            SideScope first(&side, own);
+            first.stream();
+            first.join();
+        }
         SideScope beside(&side, own);
-        if (mode == "untouched") return 0;
         beside.stream();
         std::puts("work");
         if (mode == "throws") fail(GWB200_CUDA_ERROR, "launch");
@@ -76,12 +85,13 @@ def run(tmp_path_factory):
 
     def go(mode, fails=""):
         out = subprocess.run([str(d / "side"), mode, fails], check=True, capture_output=True, text=True).stdout
-        return [line for line in out.splitlines() if line not in ("stream", "event")]
+        return out.splitlines()
 
     return go
 
 
-BEGIN = ["record 2 on own", "1 waits for 2", "work"]  # stream 1, events 2 (fork) and 3 (join)
+MADE = ["stream", "event", "event"]  # stream 1, events 2 (fork) and 3 (join)
+BEGIN = MADE + ["record 2 on own", "1 waits for 2", "work"]
 
 
 def test_joined_once(run):
@@ -98,3 +108,10 @@ def test_a_join_that_fails_is_reported(run, fails):
 def test_left_by_an_exception(run):
     assert run("throws") == BEGIN + ["record 3 on 1", "own waits for 3", "error 6"]
     assert run("throws", "own waits for 3")[-2:] == ["synchronise 1", "error 6"]
+
+
+def test_made_by_the_first_scope_alone(run):
+    assert run("unused") == []
+    assert run("none") == ["on own"]
+    twice = run("twice")
+    assert twice[:3] == MADE and not {"stream", "event"} & set(twice[3:])
