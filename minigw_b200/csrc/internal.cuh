@@ -208,9 +208,9 @@ int launch_update64_oz(const TallGeometry& g, int64_t nf, double* a, int64_t kb0
                        void* slices, unsigned long long* sched, unsigned long long* err_pivot, cudaStream_t s,
                        int max_ctas = 0, int64_t row_min = 0);
 // Autotuner of the FP64 trailing-update kernel: GWB200_UPDATE_VARIANT if set, else the fastest
-// candidate on this geometry's largest trailing update, timed once per (device, n_pad, rows, nf)
-// per process in the workspace `a` (nf tall matrices) BEFORE the matrices are built there (the
-// timing overwrites it).  The default is kept unless another candidate is more than 3% faster.
+// candidate on the updates by this geometry's first pair of outer blocks, timed once per (device,
+// n_pad, rows, nf) per process in the workspace `a` (nf tall matrices) BEFORE the matrices are built
+// there (the timing overwrites it).  The default is kept unless another candidate is more than 3% faster.
 // oz != NULL adds the int8 emulation of the outer updates (kernels_oz.cu) as a candidate
 // (kUpdateOzaki), timed with the slicing; GWB200_FP64_UPDATE=dmma / =ozaki force either side.
 // Timed candidates: the default DMMA kernel and the int8 emulation (all six DMMA variants with

@@ -406,9 +406,12 @@ int tune_update_variant(const TallGeometry& g, int64_t nf, double* a, cudaStream
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tuned.find(key);
     if (it != g_tuned.end()) return it->second;
-    // Time the candidates on the largest trailing update of this geometry (K = 128 from column 0
-    // onto columns [128, n_pad) and all RHS rows), in the workspace before the tall matrix is built
-    // there: the values are irrelevant to the timing and are overwritten afterwards.
+    // Time the candidates on the first steps of this geometry's factorisation, in the workspace before the
+    // tall matrix is built there: the values are irrelevant to the timing and are overwritten afterwards.  The
+    // steps are those of launch_factor_chunk, without the diagonal blocks: the first block's trailing update
+    // and, where the int8 update takes blocks in pairs, the second's too, so that its K = 256 kernel, which
+    // does most of its work, is in the comparison (timed at K = 128 over all columns it was taken for 317
+    // pairs x 64 frequencies, 261 us a call, where DMMA takes 236).
     cudaEvent_t e0, e1;
     GWB_CUDA(cudaEventCreate(&e0));
     GWB_CUDA(cudaEventCreate(&e1));
@@ -425,10 +428,15 @@ int tune_update_variant(const TallGeometry& g, int64_t nf, double* a, cudaStream
     };
     float best_ms = 0.f, def_ms = 0.f;
     int best = -1;
+    const bool pair = nsq > 4;
+    const int64_t first = std::min<int64_t>(2, nsq - 2), second = std::min<int64_t>(2, nsq - 4);  // tiles of the next blocks
     for (int v = 0; v < kNumVariants; ++v) {
         if (!all && v != kDefaultUpdateVariant) continue;
         GWB_CUDA(cudaFuncSetAttribute(kVariants[v].fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVariants[v].smem));
-        const float ms = time_it([&] { launch_variant(v, g, nf, a, 0, 2, 2, nsq - 2, s); });
+        const float ms = time_it([&] {
+            launch_variant(v, g, nf, a, 0, 2, 2, nsq - 2, s, first);
+            if (pair) launch_variant(v, g, nf, a, 2 * kNb, 2, 4, nsq - 4, s, second);
+        });
         times[v] = ms;
         if (v == kDefaultUpdateVariant) def_ms = ms;
         if (best < 0 || ms < best_ms) {
@@ -439,7 +447,8 @@ int tune_update_variant(const TallGeometry& g, int64_t nf, double* a, cudaStream
     if (oz) {  // the int8 emulation of the outer update (kernels_oz.cu), slicing included
         const float ms = time_it([&] {
             launch_clear_sched(g, sched, s);
-            launch_update64_oz(g, nf, a, 0, 2 * kNb, g.n_pad, oz, sched, err_pivot, s);
+            launch_update64_oz(g, nf, a, 0, 2 * kNb, pair ? 4 * kNb : g.n_pad, oz, sched, err_pivot, s, 0, first * kNb);
+            if (pair) launch_update64_oz(g, nf, a, 0, 4 * kNb, g.n_pad, oz, sched + 1, err_pivot, s, 0, second * kNb);
         });
         times[kUpdateOzaki] = ms;
         if (ms < best_ms) {
