@@ -382,7 +382,7 @@ void compute_forms(gwb200_handle* h, const double* omega, int64_t nfreq, const i
         size_t budget = (size_t)((double)avail * 0.85);
         if (h->mem_limit > 0) {  // the handle's cap minus what the system and panels already hold
             const size_t resident = h->pqo.bytes + h->xdiag.bytes + h->v.bytes + h->xt.bytes + h->qall.bytes +
-                                    h->out.bytes + h->pchol.bytes + h->pchol_sl.bytes +
+                                    h->in.bytes + h->out.bytes + h->pchol.bytes + h->pchol_sl.bytes +
                                     h->qx.bytes + h->sigmx.bytes + ((size_t)1 << 20);
             const size_t lim = (size_t)h->mem_limit;
             const size_t room = lim > resident ? lim - resident : 0;
@@ -1198,6 +1198,7 @@ int gwb200_qp(gwb200_handle* h, const double* omega, int64_t nfreq, const double
         if (nfreq <= 0) fail(GWB200_BAD_SHAPE, "nfreq must be positive");
         if (npade <= 0) fail(GWB200_BAD_SHAPE, "Pade: npar must be positive");
         check_states(h, states, nstates);
+        check_npade(npade);
         cudaStream_t s = h->stream;
         // grid, the states' rows and the state list: one pinned upload; one read back
         const size_t nb_om = sizeof(double) * nfreq, nb_st = sizeof(int64_t) * nstates;
@@ -1230,17 +1231,25 @@ int gwb200_pade_sweep(gwb200_handle* h, const double* omega, int64_t nfreq, cons
         if (!omega || !sigma_row || !out) fail(GWB200_BAD_ARGUMENT, "null input or output array");
         if (nfreq <= 0 || npts <= 0) fail(GWB200_BAD_SHAPE, "nfreq and npts must be positive");
         if (npade <= 0) fail(GWB200_BAD_SHAPE, "Pade: npar must be positive");
+        check_npade(npade);  // no copy of the caller's arrays is in flight when a call is refused
         cudaStream_t s = h->stream;
-        // kept by the handle: allocating and freeing them per call synchronised the device each time
+        // kept by the handle: allocating and freeing them per call synchronised the device each time.  A
+        // capped handle gives them back, its cap is for the solves.
         h->sweep.ensure(sizeof(double) * ((size_t)nfreq * 3 + 3 * (size_t)npts));
         double* dom = h->sweep.as<double>();
         double* drow = dom + nfreq;
         double* dout = drow + 2 * nfreq;
-        GWB_CUDA(cudaMemcpyAsync(dom, omega, sizeof(double) * nfreq, cudaMemcpyHostToDevice, s));
-        GWB_CUDA(cudaMemcpyAsync(drow, sigma_row, sizeof(double) * 2 * nfreq, cudaMemcpyHostToDevice, s));
-        launch_pade_sweep(drow, dom, nfreq, npade, npts, fermi, x_start, interval, dout, s);
-        GWB_CUDA(cudaMemcpyAsync(out, dout, sizeof(double) * 3 * (size_t)npts, cudaMemcpyDeviceToHost, s));
+        try {
+            GWB_CUDA(cudaMemcpyAsync(dom, omega, sizeof(double) * nfreq, cudaMemcpyHostToDevice, s));
+            GWB_CUDA(cudaMemcpyAsync(drow, sigma_row, sizeof(double) * 2 * nfreq, cudaMemcpyHostToDevice, s));
+            launch_pade_sweep(drow, dom, nfreq, npade, npts, fermi, x_start, interval, dout, s);
+            GWB_CUDA(cudaMemcpyAsync(out, dout, sizeof(double) * 3 * (size_t)npts, cudaMemcpyDeviceToHost, s));
+        } catch (...) {
+            cudaStreamSynchronize(s);
+            throw;
+        }
         GWB_CUDA(cudaStreamSynchronize(s));
+        if (h->mem_limit > 0) h->sweep.release();
     });
 }
 
@@ -1328,7 +1337,7 @@ size_t batch_avail(const gwb200_handle* w) {
     size_t avail = free_b + held;
     if (w->mem_limit > 0) {
         size_t resident = (size_t)1 << 20;
-        for (const DevBuf* b : {&w->pqo, &w->xdiag, &w->v, &w->xt, &w->dvec, &w->qall, &w->out, &w->a,
+        for (const DevBuf* b : {&w->pqo, &w->xdiag, &w->v, &w->xt, &w->dvec, &w->qall, &w->in, &w->out, &w->a,
                                 &w->qacc, &w->panel32})
             resident += b->bytes;
         const size_t lim = (size_t)w->mem_limit;

@@ -238,6 +238,7 @@ int launch_sigma_contract(const double* qall, int64_t nf_int, int64_t nstates, i
 int launch_qp(const double* sigma, const double* omega, int64_t nfreq, const int64_t* states, int64_t nstates,
               int64_t npade, const double* mo, double fermi, const double* sigx, const double* vxc_diag, double* qp,
               cudaStream_t s);
+void check_npade(int64_t npade);  // GWB200_BAD_SHAPE beyond the kernels' limit
 int launch_pade_sweep(const double* sigma_row, const double* omega, int64_t nfreq, int64_t npade, int64_t npts,
                       double fermi, double x_start, double interval, double* out, cudaStream_t s);
 int launch_negate_copy(const double* qacc, int64_t nf, int64_t m, int64_t ldq_in, double* q_out, int64_t ldq_out,

@@ -287,10 +287,14 @@ int launch_sigma_contract(const double* qall, int64_t nf_int, int64_t nstates, i
     return 1;
 }
 
+void check_npade(int64_t npade) {
+    if (npade > kMaxPade) fail(GWB200_BAD_SHAPE, "npade exceeds the device Pade limit of 128");
+}
+
 int launch_qp(const double* sigma, const double* omega, int64_t nfreq, const int64_t* states, int64_t nstates,
               int64_t npade, const double* mo, double fermi, const double* sigx, const double* vxc_diag, double* qp,
               cudaStream_t s) {
-    if (npade > kMaxPade) fail(GWB200_BAD_SHAPE, "npade exceeds the device Pade limit of 128");
+    check_npade(npade);
     k_qp<<<(unsigned)nstates, 32, 0, s>>>(sigma, omega, (int)nfreq, states, (int)npade, mo, fermi, sigx, vxc_diag, qp);
     GWB_LAUNCH("k_qp");
     return 1;
@@ -298,7 +302,7 @@ int launch_qp(const double* sigma, const double* omega, int64_t nfreq, const int
 
 int launch_pade_sweep(const double* sigma_row, const double* omega, int64_t nfreq, int64_t npade, int64_t npts,
                       double fermi, double x_start, double interval, double* out, cudaStream_t s) {
-    if (npade > kMaxPade) fail(GWB200_BAD_SHAPE, "npade exceeds the device Pade limit of 128");
+    check_npade(npade);
     k_pade_sweep<<<(unsigned)std::min<int64_t>((npts + 127) / 128, 8 * 148), 128, 0, s>>>(
         sigma_row, omega, (int)nfreq, (int)npade, (int)npts, fermi, x_start, interval, out);
     GWB_LAUNCH("k_pade_sweep");

@@ -40,3 +40,32 @@ def test_sweep_and_qp_bit_exact(oracle_lib, cfg1_input, nfreq, npade):
             sx = be.sigma_x_diag()
             qp = be.qp(om, sigma, npade, states)
             np.testing.assert_array_equal(qp[states], oracle_lib.qp(cfg1_input, sx, om, sigma, states, npade)[states])
+
+
+def test_sweep_refuses_too_many_parameters_before_any_device_work():
+    """A sweep of more points than any device holds and more parameters than the kernels take is refused for the
+    parameters: nothing was allocated, and no copy of the caller's arrays begun, when the call returns."""
+    from minigw_b200 import B200Backend
+    from minigw_b200._lib import STATUS, dptr, lib
+
+    om, row, out = np.linspace(0.1, 1.0, 200), np.zeros(200, complex), np.zeros(3)
+    with B200Backend(0) as be:
+        rc = lib.gwb200_pade_sweep(be._h, dptr(om), 200, dptr(row), 129, 10**12, 0.0, -6.5, 0.1, dptr(out))
+    assert STATUS[rc] == "GWB200_BAD_SHAPE" and b"Pade limit" in lib.gwb200_last_error()
+
+
+def test_sweep_of_a_capped_handle_keeps_no_memory():
+    import torch
+
+    from minigw_b200 import B200Backend
+
+    om = np.linspace(0.1, 1.0, 40)
+    row = 0.1 / (1j * om + 0.5)
+    npts = 4_000_000  # 96 MB of points
+    torch.cuda.mem_get_info(0)
+    with B200Backend(0) as be:
+        be.set_memory_limit(1 << 27)
+        be.pade_sweep(om, row, 8, npts=1000)
+        before = torch.cuda.mem_get_info(0)[0]
+        be.pade_sweep(om, row, 8, npts=npts)
+        assert before - torch.cuda.mem_get_info(0)[0] < 16 << 20
