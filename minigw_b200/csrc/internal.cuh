@@ -31,6 +31,7 @@ struct Failure : std::runtime_error {
 
 inline void cuda_check(cudaError_t e, const char* what, const char* file, int line) {
     if (e != cudaSuccess) {
+        cudaGetLastError();  // reported here, not by the next launch's check
         const int code = (e == cudaErrorMemoryAllocation) ? GWB200_OOM : GWB200_CUDA_ERROR;
         fail(code, std::string(what) + ": " + cudaGetErrorString(e) + " (" + file + ":" + std::to_string(line) + ")");
     }

@@ -69,3 +69,15 @@ def test_sweep_of_a_capped_handle_keeps_no_memory():
         before = torch.cuda.mem_get_info(0)[0]
         be.pade_sweep(om, row, 8, npts=npts)
         assert before - torch.cuda.mem_get_info(0)[0] < 16 << 20
+
+
+def test_a_failed_allocation_does_not_fail_the_next_call():
+    from minigw_b200 import B200Backend
+    from minigw_b200._lib import STATUS, dptr, lib
+
+    om, out = np.linspace(0.1, 1.0, 40), np.zeros(3)
+    row = 0.1 / (1j * om + 0.5)
+    with B200Backend(0) as be:
+        rc = lib.gwb200_pade_sweep(be._h, dptr(om), 40, dptr(row), 8, 10**12, 0.0, -6.5, 0.1, dptr(out))
+        assert STATUS[rc] == "GWB200_OOM"
+        assert np.isfinite(be.pade_sweep(om, row, 8, npts=100)).all()

@@ -29,6 +29,7 @@ static cudaError_t call(const std::string& what) {
 }
 extern "C" {
 const char* cudaGetErrorString(cudaError_t) { return "fake error"; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
     *s = (cudaStream_t)(size_t)++g_made;
     return call("stream");
