@@ -177,8 +177,9 @@ __global__ void __launch_bounds__(256) k_slice_panel64(const double* __restrict_
     for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
     // the row scale 2^e k / 64, k = 33 .. 65, with |x| <= 0.498 of it, so that six digits of -128 .. 127
     // reach it (a power of two alone leaves half a bit of each row unused on average)
+    // (a row below the normal range, whose scale and its inverse a double does not hold, counts as zero)
     double scale = 1.0, inv = 1.0;
-    if (m > 0.0) {
+    if (m >= 0x1p-1022) {
         int e;
         const double k = ceil(frexp(m, &e) * (64.0 / 0.996));
         scale = pow2(e) * (k * 0x1p-5);

@@ -175,3 +175,23 @@ def test_few_frequencies_of_many_rows_use_the_idle_sms():
             return min(be.screened_forms(np.array([0.1, 1.0]), sl.states)[1]["device_ms_screening"] for _ in range(10))
 
     assert best(30) < 3 * best(1)
+
+
+def test_int8_update_with_rows_near_the_end_of_the_exponent_range(monkeypatch):
+    """Rows that couple to the columns before them by 1e-295 .. 1e-323 alone, subnormal ones among them: nothing
+    of theirs reaches the forms, and their scales may not either."""
+    from minigw_b200 import B200Backend
+
+    monkeypatch.setenv("GWB200_FP64_UPDATE", "ozaki")
+    n, first = 449, 390
+    sl = _system(n, n // 2, 1, 2100)
+    weak = 10.0 ** -np.linspace(295.0, 323.0, n - first)
+    sl.vph[first:, :] = weak[:, None]
+    sl.vph[:, first:] = weak[None, :]
+    sl.vph[np.arange(first, n), np.arange(first, n)] = 0.5
+    omegas = np.array([1e-2, 0.9])
+    with B200Backend(0) as be:
+        be.load_slices(sl)
+        q, _ = be.screened_forms(omegas, sl.states)
+    ref = _forms(sl, omegas)
+    assert np.abs(q - ref).max() <= 1e-11 * np.abs(ref).max()  # as above
