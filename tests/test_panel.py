@@ -195,3 +195,20 @@ def test_int8_update_with_rows_near_the_end_of_the_exponent_range(monkeypatch):
         q, _ = be.screened_forms(omegas, sl.states)
     ref = _forms(sl, omegas)
     assert np.abs(q - ref).max() <= 1e-11 * np.abs(ref).max()  # as above
+
+
+@pytest.mark.parametrize("n", [65, 129, 193, 257])
+def test_complex_next_block_beside_the_update(n):
+    """eta != 0: the next diagonal block factored beside the trailing update (few frequencies) or before it (more
+    than there are SMs), the same forms bit for bit."""
+    from minigw_b200 import B200Backend
+
+    sl = _system(n, n // 2, 1, 2300 + n)
+    few = np.array([1e-3, 0.4, 7.0])
+    with B200Backend(0) as be:
+        be.load_slices(sl)
+        q, _ = be.screened_forms_complex(few, sl.states, eta=0.02)
+        many, _ = be.screened_forms_complex(np.tile(few, 67), sl.states, eta=0.02)
+    ref = _forms_complex(sl, few, 0.02)
+    assert np.abs(q - ref).max() <= 1e-11 * np.abs(ref).max()
+    np.testing.assert_array_equal(many.reshape(67, 3, -1), np.broadcast_to(q.reshape(3, -1), (67, 3, q[0].size)))
