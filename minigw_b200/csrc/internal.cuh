@@ -42,9 +42,6 @@ inline void cuda_check(cudaError_t e, const char* what, const char* file, int li
 // Block size of the right-looking Cholesky (rows/cols of one diagonal block) and
 // the square tile edge of every DMMA tile kernel.
 constexpr int kNb = 64;
-// Padded shared-memory row stride (doubles) of a 64-wide tile: 68*8 B rows put the
-// 8 rows touched by one m8n8k4 fragment load on distinct banks.
-constexpr int kLds = 68;
 // Default variant of the trailing-update kernel (index into the table in kernels_fp64.cu).
 constexpr int kDefaultUpdateVariant = 0;
 
@@ -286,7 +283,7 @@ int launch_refine_chunk(const TallGeometry& g, int64_t nf, float* a, const doubl
 bool refine_gram_on_int8(int64_t n_pad);
 // kernels_gram_oz.cu: y^T V y = ||C^T y||^2 from int8 digit slices (tcgen05 kind::i8).
 int64_t gram_oz_rows(int64_t r);
-// the int8 path (exact int32 sums, y of a right-hand side in shared memory) takes n_pad up to 25600; beyond, DMMA
+// the int8 path takes n_pad up to 25600 (its int32 sums are exact to 65536, but it was not run beyond); above, DMMA
 bool gram_oz_fits(int64_t n_pad);
 size_t refine_oz_bytes_per_freq(const TallGeometry& g, int64_t r);
 size_t gram_oz_system_bytes(int64_t n_pad, int64_t r);

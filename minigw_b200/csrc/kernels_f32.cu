@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(256) k_diag32(float* __restrict__ a, int64_t l
         }
     };
     __syncthreads();
-    panel::factor_diag<kNb, false>(S, work, k, err_pivot);
+    panel::factor_diag<kNb>(S, work, k, err_pivot);
     inverse_out(A);
     if (NB == 128) {
         const int lane = tid & 31, w = tid >> 5;
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(256) k_diag32(float* __restrict__ a, int64_t l
             }
         if (tid < kNb) S[tid * LD + kNb] = 0.0;  // the last identity column
         __syncthreads();
-        panel::factor_diag<kNb, false>(S, work, k + kNb, err_pivot);
+        panel::factor_diag<kNb>(S, work, k + kNb, err_pivot);
         inverse_out(A22);
     }
 }

@@ -64,7 +64,7 @@ __global__ void k_gather_panel(const double* __restrict__ pqo, int nmo, int nocc
 }
 
 // Sigma_x[p,p] = -sum_{i<nocc} eri[p,i,p,i] in the reference's order (src/gw/sigma.cpp:29-36);
-// xdiag[p*nocc + i] = eri[p,i,p,i] (uploaded element by element).
+// xdiag[p*nocc + i] = eri[p,i,p,i] (gathered on the host).
 __global__ void k_sigma_x_diag(const double* __restrict__ xdiag, int nmo, int nocc, double* __restrict__ out) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= nmo) return;
@@ -124,9 +124,7 @@ __global__ void k_build_tall(int64_t n, int64_t m, int64_t n_pad, int64_t ld, in
 }
 
 // ---------------------------------------------------------------------------
-// DMMA 64x64x64 tile product:  acc += sgn * As(64x64) * Bs(64x64)^T, both in shared memory,
-// row-major with stride kLds.  8 warps; warp w owns rows 16*(w/2)..+15, cols 32*(w%2)..+31,
-// i.e. 2 x 4 fragments of the m8n8k4 f64 MMA.  Fragment layout (PTX ISA, mma.m8n8k4 .f64):
+// Fragments of the m8n8k4 f64 MMA (PTX ISA, mma.m8n8k4 .f64):
 // A: a = A[lane/4][lane%4]; B: b = B[lane%4][lane/4]; C: {C[lane/4][2*(lane%4)], +1}.
 __device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -134,19 +132,16 @@ __device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
                  : "d"(a), "d"(b));
 }
 
+__device__ __forceinline__ void cp_async_16(double* smem_dst, const double* gsrc) {
+    const unsigned saddr = (unsigned)__cvta_generic_to_shared(smem_dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(saddr), "l"(gsrc));
+}
 // Trailing update C -= sum_chunks P_i P_j^T of the output column tiles [tc0, tc0+T) (64-wide,
 // absolute tile indices): every tile on or below the diagonal in the square block but the first
 // `skip` row tiles, then every tile of the right-hand-side rows.  The contraction runs over nk
 // 64-wide column chunks of the factored panels starting at column kb0 in K slices, so K = 64*nk
 // costs one read and one write of C: nk = 2 (16 flop per byte of C traffic).
-__device__ __forceinline__ void cp_async_16(double* smem_dst, const double* gsrc) {
-    const unsigned saddr = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(saddr), "l"(gsrc));
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.commit_group;\n" ::);
-    asm volatile("cp.async.wait_group 0;\n" ::);
-}
+//
 // Update kernel family: 64x64 output tile per CTA, warp tile (8*WM) x (8*WN) of m8n8k4 DMMA
 // fragments, K streamed in KC-wide slices through a STAGES-deep cp.async pipeline.
 template <int KC>

@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(256) k_slice_ct(const double* __restrict__ ct,
 // its row of xt.  Bound by the bytes of z and the digits and by their FP64 arithmetic; a warp reads its
 // row twice (the second time from L1) instead of staging y in shared memory: 389 us at 720 rows of 2000
 // x 64 frequencies, where a block per row with its barriers and one conversion per digit took 611.
-constexpr int64_t kPrepMaxNpad = 25600;  // larger systems take the FP64 Gram kernel
+constexpr int64_t kPrepMaxNpad = 25600;  // larger systems, on which this path was not run, take the FP64 Gram kernel
 constexpr int kPrepWarps = 8;
 
 __global__ void __launch_bounds__(32 * kPrepWarps)

@@ -237,8 +237,8 @@ __global__ void __launch_bounds__(kOzThreads, 1)
     extern __shared__ __align__(1024) uint8_t osm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t base = smem_u32(osm);
-    const uint32_t abuf = (base + kHeader + 1023u) & ~1023u;  // A slices 3-6, 1024-aligned
-    const uint32_t ring = abuf + (kOzSlices - kOzTmemSlices) * kSliceA;  // B stages (A slices 3-6 before)
+    const uint32_t abuf = (base + kHeader + 1023u) & ~1023u;  // A slices 5-6, 1024-aligned
+    const uint32_t ring = abuf + (kOzSlices - kOzTmemSlices) * kSliceA;  // B stages, and with KH = 2 A slices
     const uint32_t stg0 = ring + kOzStages * kStageB;          // epilogue staging rows
     volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(osm + kOffAbort);
     volatile int64_t* uslot = reinterpret_cast<volatile int64_t*>(osm + kOffUnit);
@@ -500,7 +500,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
                 }
             } else {
                 for (int64_t c = c0; ok && c < c1; ++c) {
-                    // group X (levels 4-8, sa + t >= 2) once the epilogue has read the previous tile's
+                    // group X (levels 4-7, sa + t >= 2) once the epilogue has read the previous tile's
                     if (!mbar_wait_fast(tempty(0), acc_ph ^ 1u, abort_flag, err)) {
                         ok = false;
                         break;
@@ -607,7 +607,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
                 // Levels combined exactly: adjacent pairs S2 2^8 + S3 (|S2| <= 128^2 256, below 2^31), S4 2^8
                 // + S5 and S6 2^8 + S7 (below 2^33), the latter two as one integer m of at most 49 bits (an
                 // exact double between the groups); value = p23 2^-24 + m 2^-56 with one rounding, scaled
-                // by 2^{e_r + e_c}.
+                // by c_r c_c.
                 const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * 32);
                 auto wait_group = [&](int g) {
                     uint32_t got = 1;
@@ -664,7 +664,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
                             const int j = 4 * j4 + k;
                             const int32_t p23 = (int32_t)v[0][j] * 256 + (int32_t)v[1][j];
                             // (p23 2^32 + m) rounded once is 2^56 times the value rounded once: the
-                            // 2^-56 joins the exact power-of-two scale
+                            // 2^-56 is in row_scale
                             val[k] = fma((double)p23, 0x1p32, m_d[16 * h16 + j]) *
                                      (row_scale * sj[k]);  // an exact product
                         }

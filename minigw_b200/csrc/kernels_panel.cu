@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(DiagShape<NB>::kThreads) k_diag64(double* __re
         }
     }
     __syncthreads();
-    factor_diag<NB, false>(S, S + DiagShape<NB>::kBlockDoubles, k, err_pivot);
+    factor_diag<NB>(S, S + DiagShape<NB>::kBlockDoubles, k, err_pivot);
     // the inverse in place of the block; above the diagonal zeros (not the upper right 64 x 64, which
     // nothing reads).  A warp takes 4 rows x 8 columns: the transposed reads are 2-way bank conflicts.
     const int rr = (threadIdx.x >> 3) & 3, cc = threadIdx.x & 7;
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(DiagShape<NB>::kThreads) k_small64(int n, int 
         S[idx] = x;
     }
     __syncthreads();
-    factor_diag<NB, false>(S, work, 0, err_pivot);
+    factor_diag<NB>(S, work, 0, err_pivot);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int r0 = 16 * (warp & 1), cg = warp >> 1;

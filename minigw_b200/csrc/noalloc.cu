@@ -59,10 +59,12 @@ void screened_forms_noalloc(int64_t n, int64_t m, const double* d_v, const doubl
                             const double* d_omega, int64_t nfreq, double* d_q_out, cudaStream_t s) {
     if (n <= 0 || m <= 0 || nfreq <= 0) fail(GWB200_BAD_SHAPE, "n, m and nfreq must be positive");
     const TallGeometry g = make_geometry(n, m);
-    const size_t per_freq = (size_t)g.stride + (size_t)g.n_pad + (size_t)kNb * kNb + (size_t)g.m_pad;
-    if (per_freq > kStaticScratchDoubles - kHeaderDoubles)
+    const size_t per_freq = (size_t)g.stride + (size_t)g.n_pad + (size_t)g.m_pad;
+    // the size rule of the interface, which counts 4096 doubles more than a frequency takes
+    const size_t rule = per_freq + 4096;
+    if (rule > kStaticScratchDoubles - kHeaderDoubles)
         fail(GWB200_BAD_SHAPE, "system too large for the 4 MiB static scratch: one frequency needs " +
-                                   std::to_string(per_freq * sizeof(double)) + " bytes ((n64+m64)*n64 + n64 + 4096 + "
+                                   std::to_string(rule * sizeof(double)) + " bytes ((n64+m64)*n64 + n64 + 4096 + "
                                    "m64 doubles with n64, m64 = n, m rounded up to 64)");
     require_device_pointer(d_v, "V_ph");
     require_device_pointer(d_xt, "panel");
@@ -75,8 +77,7 @@ void screened_forms_noalloc(int64_t n, int64_t m, const double* d_v, const doubl
     const int64_t fc = (int64_t)std::min<size_t>((size_t)nfreq, (kStaticScratchDoubles - kHeaderDoubles) / per_freq);
     double* a = base + kHeaderDoubles;
     double* dvec = a + (size_t)fc * g.stride;
-    double* linv = dvec + (size_t)fc * g.n_pad;
-    double* qacc = linv + (size_t)fc * kNb * kNb;
+    double* qacc = dvec + (size_t)fc * g.n_pad;
 
     // The scratch keeps the previous call's contents: reset the pivot flag; qacc is cleared per chunk.
     GWB_CUDA(cudaMemsetAsync(err, 0xFF, sizeof(unsigned long long), s));

@@ -174,10 +174,10 @@ __device__ __forceinline__ unsigned factor_rows16(const double* __restrict__ S, 
     return bad;
 }
 
-// Warp 0: factors the panel's diagonal block; the transposed inverse to Wt[c][r] and, with kKeepL,
-// the factor back to S.  Returns the failed pivots as a bit mask.
-template <int LD, bool kKeepL>
-__device__ __forceinline__ unsigned factor_panel16(double* __restrict__ S, double* __restrict__ Wt,
+// Warp 0: factors the panel's diagonal block; the transposed inverse to Wt[c][r].  Returns the failed
+// pivots as a bit mask.
+template <int LD>
+__device__ __forceinline__ unsigned factor_panel16(const double* __restrict__ S, double* __restrict__ Wt,
                                                    double* __restrict__ rows2, double* __restrict__ piv, int c0) {
     const int lane = threadIdx.x & 31, r = lane & 15;
     double x[16];
@@ -189,20 +189,16 @@ __device__ __forceinline__ unsigned factor_panel16(double* __restrict__ S, doubl
     if (lane >= 16) {
 #pragma unroll
         for (int c = 0; c < 16; ++c) Wt[c * kWtLd + r] = x[c];
-    } else if (kKeepL) {
-#pragma unroll
-        for (int c = 0; c < 16; ++c)
-            if (c <= r) S[(c0 + r) * LD + c0 + c] = x[c];
     }
     return bad;
 }
 
 // Factors the block in S (lower triangle given, everything above the diagonal zero) and leaves the
-// transposed inverse: L^{-1}[c][r] = S[r][c + 1], c >= r.  With kKeepL the lower triangle of S is
-// L.  A pivot that is not > 0 records the 1-based global row k0 + j + 1 in *err (the minimum) and
-// counts as 1.  work: DiagShape::kWorkDoubles, 16-byte aligned.  All DiagShape::kThreads threads call
-// it after a barrier; ends with a barrier.
-template <int NB, bool kKeepL>
+// transposed inverse: L^{-1}[c][r] = S[r][c + 1], c >= r (the lower triangle does not end as L).  A
+// pivot that is not > 0 records the 1-based global row k0 + j + 1 in *err (the minimum) and counts as 1.
+// work: DiagShape::kWorkDoubles, 16-byte aligned.  All DiagShape::kThreads threads call it after a
+// barrier; ends with a barrier.
+template <int NB>
 __device__ __forceinline__ void factor_diag(double* __restrict__ S, double* __restrict__ work, int64_t k0,
                                             unsigned long long* err) {
     constexpr int LD = DiagShape<NB>::kLd, kWarps = DiagShape<NB>::kThreads / 32;
@@ -214,7 +210,7 @@ __device__ __forceinline__ void factor_diag(double* __restrict__ S, double* __re
         // a panel's update reads its own inverse while warp 0 writes the next panel's
         double* Wt = piv + 16 + (c0 & 16) * kWtLd;
         if (warp == 0) {
-            const unsigned bad = factor_panel16<LD, kKeepL>(S, Wt, rows2, piv, c0);
+            const unsigned bad = factor_panel16<LD>(S, Wt, rows2, piv, c0);
             if (bad && lane == 0) atomicMin(err, (unsigned long long)(k0 + c0 + __ffs(bad)));
         }
         __syncthreads();

@@ -209,3 +209,17 @@ def test_reference_executable_with_b200_fails_loudly_without_gpu(tmp_path):
     r = subprocess.run([str(exe), "--linalg-backend", "b200", "--input-dir", str(GOLDEN / "h2o"), "--output-dir",
                         str(tmp_path)], capture_output=True, text=True, timeout=120)
     assert r.returncode != 0 and "CUDA" in r.stderr
+
+
+@pytest.mark.parametrize("n,m,fits", [(320, 320, True), (64, 7936, True), (1, 7937, False), (64, 8000, False), (128, 3904, True),
+                                      (128, 3905, False), (448, 704, True), (448, 705, False)])
+def test_noalloc_size_rule(n, m, fits):
+    """(n64 + m64) n64 + n64 + 4096 + m64 <= 524256 doubles: what does not fit is refused for its shape, what fits
+    gets as far as the check of its pointers (host memory here)."""
+    import ctypes as C
+
+    from minigw_b200._lib import STATUS, lib
+
+    p = C.c_void_p(np.zeros(1).ctypes.data)
+    rc = lib.gwb200_screened_forms_noalloc(n, m, p, p, p, p, 2, p, None)
+    assert STATUS[rc] == ("GWB200_BAD_ARGUMENT" if fits else "GWB200_BAD_SHAPE")
