@@ -359,16 +359,13 @@ __device__ void factor_diag_c(double* __restrict__ Sr, double* __restrict__ Si, 
     __syncthreads();
 }
 
-__device__ __forceinline__ void cp_async16c(double* dst, const double* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
-}
 // 32 or 64 rows of `w` doubles of both planes into shared memory (row stride ldm), one plane `plane` apart
 __device__ __forceinline__ void load_rows_c(double* dst, int plane, int ldm, const double* re, const double* im, int64_t ld,
                                             int rows, int w) {
     for (int idx = threadIdx.x; idx < rows * (w / 2); idx += blockDim.x) {
         const int r = idx / (w / 2), c = 2 * (idx % (w / 2));
-        cp_async16c(dst + r * ldm + c, re + (size_t)r * ld + c);
-        cp_async16c(dst + plane + r * ldm + c, im + (size_t)r * ld + c);
+        panel::cp_async16(dst + r * ldm + c, re + (size_t)r * ld + c);
+        panel::cp_async16(dst + plane + r * ldm + c, im + (size_t)r * ld + c);
     }
 }
 

@@ -82,17 +82,12 @@ __device__ __forceinline__ void store_fragments(float* __restrict__ s, const flo
                 make_float2(acc[j][2 * h], acc[j][2 * h + 1]);
 }
 
-__device__ __forceinline__ void cp_async_16f(float* smem_dst, const float* gsrc) {
-    const unsigned saddr = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(saddr), "l"(gsrc));
-}
-
 // 64 x W floats of global (row stride ld) into shared memory (row stride LD), 16-byte pieces.
 template <int W, int LD>
 __device__ __forceinline__ void load_f32_async(float* __restrict__ s, const float* __restrict__ gsrc, int64_t ld) {
     for (int idx = threadIdx.x; idx < 64 * (W / 4); idx += blockDim.x) {
         const int r = idx / (W / 4), c4 = idx % (W / 4);
-        cp_async_16f(s + r * LD + 4 * c4, gsrc + (size_t)r * ld + 4 * c4);
+        panel::cp_async16(s + r * LD + 4 * c4, gsrc + (size_t)r * ld + 4 * c4);
     }
 }
 
@@ -276,8 +271,8 @@ __global__ void __launch_bounds__(32 * kPanelWarps, 1)
         if (inside) {
             const float* src = A + (size_t)r0 * ld + k;
             for (int idx = lane; idx < 16 * (NB / 4); idx += 32)
-                cp_async_16f(X + idx / (NB / 4) * LD + 4 * (idx % (NB / 4)),
-                             src + (size_t)(idx / (NB / 4)) * ld + 4 * (idx % (NB / 4)));
+                panel::cp_async16(X + idx / (NB / 4) * LD + 4 * (idx % (NB / 4)),
+                                  src + (size_t)(idx / (NB / 4)) * ld + 4 * (idx % (NB / 4)));
         }
         asm volatile("cp.async.commit_group;\n" ::);
         asm volatile("cp.async.wait_group 0;\n" ::);

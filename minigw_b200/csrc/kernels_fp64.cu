@@ -124,18 +124,6 @@ __global__ void k_build_tall(int64_t n, int64_t m, int64_t n_pad, int64_t ld, in
 }
 
 // ---------------------------------------------------------------------------
-// Fragments of the m8n8k4 f64 MMA (PTX ISA, mma.m8n8k4 .f64):
-// A: a = A[lane/4][lane%4]; B: b = B[lane%4][lane/4]; C: {C[lane/4][2*(lane%4)], +1}.
-__device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                 : "+d"(c[0]), "+d"(c[1])
-                 : "d"(a), "d"(b));
-}
-
-__device__ __forceinline__ void cp_async_16(double* smem_dst, const double* gsrc) {
-    const unsigned saddr = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(saddr), "l"(gsrc));
-}
 // Trailing update C -= sum_chunks P_i P_j^T of the output column tiles [tc0, tc0+T) (64-wide,
 // absolute tile indices): every tile on or below the diagonal in the square block but the first
 // `skip` row tiles, then every tile of the right-hand-side rows.  The contraction runs over nk
@@ -150,7 +138,7 @@ __device__ __forceinline__ void load_slice_async(double* __restrict__ s, const d
     constexpr int LD = KC + 4;  // (KC+4)*8 bytes per row: the 8 rows of one fragment load hit distinct banks
     for (int idx = threadIdx.x; idx < 64 * (KC / 2); idx += nthreads) {
         const int r = idx / (KC / 2), c2 = idx % (KC / 2);
-        cp_async_16(s + r * LD + 2 * c2, gsrc + (size_t)r * ld + 2 * c2);
+        panel::cp_async16(s + r * LD + 2 * c2, gsrc + (size_t)r * ld + 2 * c2);
     }
 }
 
@@ -169,7 +157,7 @@ __device__ __forceinline__ void warp_mma(const double* __restrict__ As, const do
 #pragma unroll
         for (int i = 0; i < WM; ++i)
 #pragma unroll
-            for (int j = 0; j < WN; ++j) dmma_8x8x4(acc[i][j], af[i], bf[j]);
+            for (int j = 0; j < WN; ++j) panel::dmma(acc[i][j], af[i], bf[j]);
     }
 }
 

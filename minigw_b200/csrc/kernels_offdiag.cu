@@ -14,7 +14,7 @@
 //                          warp, the warps' parts added in a fixed order;
 //   k_sigma_contract_pairs one CTA per (output frequency, pair s <= t): the contraction, a fixed
 //                          reduction tree; both triangles written.
-#include "internal.cuh"
+#include "panel_common.cuh"
 
 #include <type_traits>
 
@@ -63,9 +63,7 @@ __global__ void __launch_bounds__(32 * kXWarps) k_cross_forms(const double* __re
         for (int i = 0; i < NT; ++i)
 #pragma unroll
             for (int j = i; j < NT; ++j, ++p)
-                asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                             : "+d"(acc[p][0]), "+d"(acc[p][1])
-                             : "d"(x[i]), "d"(x[j]));
+                panel::dmma(acc[p], x[i], x[j]);
     }
     double* out = qx + ((size_t)f * nmo + k) * ns * ns;
     int p = 0;

@@ -30,10 +30,6 @@ using namespace panel;
 constexpr int kPanelThreads = 256;
 constexpr int kRowTile = 32;
 
-__device__ __forceinline__ void cp_async16(double* dst, const double* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
-}
-
 // With kUpdate the block first takes the update by the `depth` (128 or 256) columns before it, which the trailing
 // update then leaves out: the block depends on the previous panel alone and is factored while the
 // rest of the trailing update runs.

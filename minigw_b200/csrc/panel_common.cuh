@@ -38,10 +38,18 @@ __device__ __forceinline__ double scale_value(double delta, double w) {
     return sqrt(__dmul_rn(4.0, delta) / __fma_rn(w, w, __dmul_rn(delta, delta)));
 }
 
+// One m8n8k4 product.  Fragments (PTX ISA, mma.m8n8k4 .f64): a = A[lane/4][lane%4], b = B[lane%4][lane/4],
+// c = C[lane/4][2*(lane%4)] and the next.
 __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
                  : "+d"(c[0]), "+d"(c[1])
                  : "d"(a), "d"(b));
+}
+
+// 16 bytes of global to shared memory, asynchronously
+template <class T>
+__device__ __forceinline__ void cp_async16(T* dst, const T* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
 }
 
 // d > 0 (infinity included, NaN not), on the integer pipe
