@@ -214,6 +214,26 @@ def workload_config(args, wl, world: int) -> dict:
             "inputs smaller than L2 (a parity-size workload, not flushed between steps)"}
 
 
+def int8_tops_n64(sm_mhz: float) -> float:
+    """int8 TOP/s of 148 SMs that issue a tcgen05.mma kind::i8 of M=128, N=64, K=32 every 48 cycles."""
+    return 148 * 2 * 128 * 64 * 32 / 48 * sm_mhz * 1e6 / 1e12
+
+
+def int8_update_bytes(n: int, m: int, nfreq: int) -> float:
+    """FP64 C bytes (read and write) of one solve's int8 trailing updates: outer blocks of 128 columns in pairs
+    while columns remain behind the pair, the first of a pair onto the second's columns, both onto the rest;
+    the next diagonal block is left out (launch_factor_chunk)."""
+    elements = 0
+    for tc0 in range(128, n, 128):
+        pair_end = (tc0 - 128) // 256 * 256 + 256
+        c_end = tc0 + 128 if pair_end < n and tc0 < pair_end else n
+        c_end, nxt = min(c_end, n), min(128, n - tc0)
+        cols = c_end - tc0
+        lower = cols * n - (tc0 + c_end - 1) * cols // 2  # sum of n - c over the columns
+        elements += lower + m * cols - nxt * (nxt + 1) // 2
+    return 16.0 * nfreq * elements
+
+
 def hbm_peak_gbs() -> float:
     """Measured HBM copy bandwidth of this pool's B200s (MEASURED_PEAKS.json), else the fallback."""
     try:
@@ -505,8 +525,8 @@ def run_b200(args, wl):
     # weights and states (run_g0w0); Sigma_c, Sigma_x diagonal, QP energies and the pivot flag back
     nmo, nocc, nf, ns = wl.nmo, wl.nocc, wl.nfreq, len(states)
     nph = nocc * (nmo - nocc)
-    h2d = 8 * (nph * nph + ns * nmo * nph + nmo * nocc + 2 * nmo) + (16 * nf + 8 * ns)
-    d2h = 16 * nmo * nf + 8 * nmo + 8 * nmo + 8
+    h2d = 8 * (nph * nph + ns * nmo * nph + nmo * nocc + 2 * nmo) + (8 + 16 * nf + 8 * ns)
+    d2h = 8 + 16 * ns * nf + 8 * ns + 8 * nmo  # pivot word, Sigma_c rows and QP energies of the states, Sigma_x
     ee0, ee1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     barrier()
     torch.cuda.synchronize()
@@ -609,18 +629,23 @@ def run_b200(args, wl):
     kernel_used = be.update_kernel()
     if args.precision == "fp64" and kernel_used == 6 and achieved:
         # the autotuner chose the int8 tensor-core emulation of the FP64 update (k_slice_panel64 +
-        # k_update64_oz, timed together).  Against HBM: the FP64 C read+write, 16 bytes per updated
-        # element per K = 256 pass, i.e. flops_update / 32 bytes; the int8 work is 21 products of
-        # 6-digit slices per FP64 product
-        gbs = upd_flops / 32.0 / (upd_ms * 1e-3) / 1e9
+        # k_update64_oz, timed together): 21 int8 products of 6-digit slices per FP64 product, against the rate
+        # of its instruction; and the FP64 C read and write of its passes against HBM
+        sm_mhz = clock_info.get("sm_mhz") or clock_info.get("sm_max_mhz") or 1965.0
+        tops, peak_tops = achieved * 21.0, int8_tops_n64(sm_mhz)
+        m = ns * nmo
+        nf_solved = round(stats[0]["flops_screening"] / (nph**3 / 3 + nph**2 * m + 3 * nph * m))  # a shard's, if split
+        gbs = len(stats) * int8_update_bytes(nph, m, nf_solved) / (upd_ms * 1e-3) / 1e9
         result["roofline"] = {
-            "bound": "hbm", "kernel": "k_update64_oz (FP64 trailing update emulated on int8 tcgen05, with "
-                                      "k_slice_panel64)",
-            "achieved": gbs, "peak": hbm_peak_gbs(), "unit": "GB/s", "frac": gbs / hbm_peak_gbs(),
-            "peak_source": hbm_peak_source(),
-            "tflops_fp64_equivalent": achieved, "int8_tops": achieved * 21.0,
-            "vs_fp64_dmma_peak": achieved / peak_fp64, "launches": upd_n, "traffic": None,
-            "traffic_source": None}
+            "bound": "tensor", "kernel": "k_update64_oz (FP64 trailing update emulated on int8 tcgen05, with "
+                                         "k_slice_panel64)",
+            "achieved": tops, "peak": peak_tops, "unit": "int8 TOP/s", "frac": tops / peak_tops,
+            "peak_source": "148 SMs x one tcgen05.mma kind::i8 M=128 N=64 K=32 per 48 cycles (microbenchmark) at "
+                           f"{sm_mhz:.0f} MHz",
+            "tflops_fp64_equivalent": achieved, "vs_fp64_dmma_peak": achieved / peak_fp64, "launches": upd_n,
+            "hbm": {"achieved": gbs, "peak": hbm_peak_gbs(), "unit": "GB/s", "frac": gbs / hbm_peak_gbs(),
+                    "peak_source": hbm_peak_source(), "bytes": "FP64 C read and write of every pass"},
+            "traffic": None, "traffic_source": None}
     if args.precision in ("mixed", "mixed-refined") and achieved:
         # the tcgen05 3xTF32 trailing update (k_update32_tc; the panel solve writes its operands) is
         # bound by the FP32 C read+write, 8 bytes per updated element per K = 128 pass, i.e.
@@ -832,7 +857,7 @@ def run_batch(args):
     launches_batch = last["stats"]["kernel_launches"]
     launches_each = sum(r["stats"]["kernel_launches"] for r in outs_each[-1])
     h2d = 16 * nfreq + 8 * sum(len(s) for s in states)
-    d2h = sum(16 * nmo * nfreq + 8 * nmo for nmo in nmos) + 8
+    d2h = 8 + sum(16 * len(s) * nfreq + 8 * len(s) for s in states)  # rows and QP energies of the states
     result = {
         "metric": "gw_solves_per_s", "value": args.molecules * 1e3 / ms_batch, "unit": "GW solves/s", "n_gpus": 1,
         "steps": args.steps, "warmup": max(3, args.warmup), "ms_per_step": ms_batch, "higher_is_better": True,

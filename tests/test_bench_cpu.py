@@ -66,3 +66,22 @@ def test_batch_cpu_baseline_samples_and_interpolates(monkeypatch):
     assert cb["kind"] == "reference" and cb["unit"] == "GW solves/s"
     assert cb["value"] >= 6 / (6 * 16 ** 2 * per_pair_max) * (1 - 1e-9)
     assert np.isfinite(cb["value"]) and cb["cores"] >= 1
+
+
+@pytest.mark.parametrize("n", [128, 130, 200, 256, 257, 320, 321, 384, 500, 513, 1125])
+def test_int8_update_bytes_follow_the_factorisation(n):
+    """Block by block as launch_factor_chunk takes them, column by column."""
+    import bench
+
+    m, nsq, elements = 37, -(-n // 64), 0
+    for ob in range(0, nsq, 2):
+        tc0 = ob + min(2, nsq - ob)
+        if tc0 >= nsq:
+            break
+        nxt = min(2, nsq - tc0)
+        pairs = nsq - ob // 4 * 4 > 4
+        c_end = tc0 + nxt if pairs and ob % 4 == 0 else nsq
+        elements += sum(n - c + m for c in range(tc0 * 64, min(c_end * 64, n)))
+        d = min(nxt * 64, n - tc0 * 64)
+        elements -= d * (d + 1) // 2
+    assert bench.int8_update_bytes(n, m, 3) == 16.0 * 3 * elements
