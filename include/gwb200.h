@@ -355,7 +355,9 @@ int gwb200_server_counters(gwb200_server* s, int64_t* merged_batches, int64_t* m
  * stream with systems[0]'s workspaces.  Outputs (either array, or any entry, may be NULL):
  * sigma_out[i] nmo_i x nfreq[i] complex row-major, qp_out[i] nmo_i (NaN where not requested).
  * *nbuckets_out: the buckets used.  stats: totals of the call (flops at the true sizes, device
- * times, launches).  Each result is bit-identical to the molecule's own gwb200_run_g0w0. */
+ * times, launches).  Each result is bit-identical to the molecule's own gwb200_run_g0w0; in the plain
+ * form where both take the same trailing-update kernel, which is picked by timing per geometry
+ * unless GWB200_FP64_UPDATE names it or the handle's memory is capped (to rounding otherwise). */
 int gwb200_run_g0w0_batch(gwb200_handle* const* systems, int64_t nsys, const int64_t* nfreq,
                           const int64_t* npade, const int64_t* const* states, const int64_t* nstates,
                           int precision, double* const* sigma_out, double* const* qp_out,

@@ -752,7 +752,8 @@ std::vector<std::vector<size_t>> batch_assign(const std::vector<BatchChunk>& chu
 // the padded work, the cost model's defaults (GWB200_BATCH_STEP_US / GWB200_BATCH_TFLOPS override).
 // Measured on 16 molecules of 20 to 120 orbitals x 64 frequencies on 4 lanes, refined mixed form: 22.6
 // ms at 8-15 us, 23.9 at 30, 25.4 at 60, 30.7 at 240 (one bucket per molecule 22.2); plain form, 16 to
-// 96 orbitals: 9.7 ms at 8-15 us, 11.1 at 30, 12.2 at 80.
+// 96 orbitals: 9.7 ms at 8-15 us, 11.1 at 30, 12.2 at 80.  64 molecules of 20 to 160 orbitals, at 12 / 30 /
+// 60 / 80 us: mixed 163 / 166 / 168 / 171 ms, plain 296 / 300 / 305 / 304, refined 260 / 265 / 265 / 271.
 double batch_step_us() {
     if (const char* e = std::getenv("GWB200_BATCH_STEP_US")) return std::max(0.0, std::atof(e));
     return 12.0;

@@ -6,8 +6,9 @@
 //               (panel_common.cuh); the inverse replaces the block in the tall matrix (the factor
 //               itself is not read again: the screened forms need the solved rows alone).  A chain of
 //               pivots on one SM, so the next block's runs beside the trailing update on the other
-//               SMs: it takes its own update by the panel first (31 us without, 40 with it, at any
-//               number of frequencies up to the SMs), which the trailing update leaves out.
+//               SMs: it takes its own update by the panel first, which the trailing update leaves out
+//               (31 us without, 41 with 128 columns, 52 with 256, at any number of frequencies up to the
+//               SMs).
 //   k_panel64   rows below: P = A L^{-T} with the whole block's inverse, so the second 64 columns
 //               need no separate update by the first.  The inverse is triangular, so column tile c
 //               (8 wide) takes k < 8 (c + 1) only: 0.53 of the square product, less work than two
